@@ -809,8 +809,12 @@ class CudaKernels:
             return self._linear_tc(a, w, out, mode, defer=defer and mode in ("store", "add"))
         if a.dtype == torch.float32 and out.dtype != torch.float32:
             _fail("a float32 product is stored as float32")
+        fn = self._f("gemm_simt", "gfb_gemm_simt_scratch_floats")
+        fn.restype = c_long
+        need = fn(c_int(M), c_int(N), c_int(K))
+        partial = torch.empty(need, dtype=torch.float32, device=a.device) if need > 0 else None
         self._call("gemm_simt", "gfb_gemm_simt", _ptr(a), _ptr(w), _ptr(out), c_int(_dt(a)), c_int(_dt(out)),
-                   c_int(M), c_int(N), c_int(K), c_int(_EPI[mode]), _stream())
+                   c_int(M), c_int(N), c_int(K), c_int(_EPI[mode]), _ptr(partial), _stream())
 
     def _tc_fits(self, M, N, K, mode) -> bool:
         """The tensor-core kernel takes rows of whole 16-byte units (TMA) and stores in 16-byte vectors."""
