@@ -38,6 +38,7 @@ LIBRARIES = {
     "embedding": (["embedding.cu"], [], []),
     "latent": (["latent.cu"], [], []),
     "recurrent": (["recurrent.cu"], [], []),
+    "delta_chunk": (["delta_chunk.cu"], [], []),
     "moe": (["moe.cu"], [], []),
     "gla": (["gla.cu"], [], []),
     "streams": (["streams.cu"], [], []),
