@@ -39,6 +39,7 @@ LIBRARIES = {
     "latent": (["latent.cu"], [], []),
     "recurrent": (["recurrent.cu"], [], []),
     "delta_chunk": (["delta_chunk.cu"], [], []),
+    "ssd_chunk": (["ssd_chunk.cu"], [], []),
     "moe": (["moe.cu"], [], []),
     "gla": (["gla.cu"], [], []),
     "streams": (["streams.cu"], [], []),
