@@ -128,10 +128,10 @@ __device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr) {
 }
 // MN-major operand tile with 128-byte swizzle: rows are K (keys), 64 MN elements (dims) per 128-byte
 // row; 8-row groups 1024 bytes apart (stride offset), the next 64 dims one half tile further (leading offset)
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t saddr) {
+__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t saddr, uint32_t half_bytes = HALF_BYTES) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)(HALF_BYTES >> 4) << 16;
+    d |= (uint64_t)(half_bytes >> 4) << 16;
     d |= (uint64_t)(1024 >> 4) << 32;
     d |= (uint64_t)1 << 46;
     d |= (uint64_t)2 << 61;
@@ -1058,6 +1058,302 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     }
 }
 
+// ---- prompts against a shared latent ---------------------------------------------------------------
+// All heads read the same cached rows (gfb_latent_attention states the arithmetic): keys are whole rows of R + 64 numbers (R = 128, 256,
+// 384 or 512), values their first R.  A tile is 128 (token, head) pairs of one sequence.  A 32-bit accumulator of 128 x 512 would take
+// all of an SM's tensor memory, so an item is a tile AND one half of the value columns: two blocks score the same keys, each
+// adds its own half of P V.  That is 1.5 times the products of one pass, on a pipe that the scores alone (36 MMAs of 128 x 64 per page) keep
+// busy while four softmax warps, a row per thread, work on the page before.
+//
+// A page's rows lie in shared memory as swizzled pieces of [64 keys][64 dims]: the block's own value half (also the B operand of P V,
+// MN-major) and the rest (the other half and the rotated part), each with two stages of its own, so that a page's rest is free again when
+// its scores are done and its own half when its P V is.  What makes room for both (144 KB) is Q: the 256 numbers of the own half stand in
+// tensor memory as the A operand (128 columns), only the rest (80 KB) in shared memory.
+//   tensor memory: O 0..255, two score buffers of 64 columns (P overwrites the first 32 of its own) 256..383, Q's half 384..511
+//
+// Measured (16 heads, R = 512, one prompt): 4,096 tokens 449 us, 650 TFLOP/s of scores and weighted sums, where the
+// mma.sync kernel (gfb_latent_attention, which decode steps and other sizes keep) took 1,723 us, 169 TFLOP/s.
+constexpr int LK = 64;                          // keys per iteration: one page
+constexpr int PIECE_BYTES = LK * 128;           // [64 keys][64 dims]
+constexpr int QPIECE_BYTES = ROWS * 128;        // [128 rows][64 dims]
+constexpr uint32_t LCOL_S = 256, LCOL_Q = 384;
+constexpr int LAT_THREADS = 192;
+
+struct LatBars {
+    unsigned long long q_full, qt_full;           // Q's rest in shared memory (TMA), Q's own half in tensor memory (four softmax warps)
+    unsigned long long rest_full[2], own_full[2];
+    unsigned long long rest_done[2];              // the scores' first part has read the rest of page j (a commit)
+    unsigned long long s_full[2], pv_done[2];     // scores of page j are there; P V of page j is done (which also frees the own half's stage)
+    unsigned long long p_ready, o_full;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+__global__ void __launch_bounds__(LAT_THREADS, 1)
+latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __nv_bfloat16* __restrict__ q,
+                         __nv_bfloat16* __restrict__ out, const int* __restrict__ page_table, int max_pages, int n_pages_pool, GfbBatch b, int H,
+                         int R, float scale_log2e, int window, const float* __restrict__ sink, int n_x, int* status) {
+    extern __shared__ uint8_t smem_raw[];
+    if (threadIdx.x == 0) { prefetch_map(&map_q); prefetch_map(&map_k); }
+    const int hc = R / 128, rc = hc + 1;          // pieces of the own half and of the rest
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t qs = base, rs = qs + rc * QPIECE_BYTES, os = rs + 2 * rc * PIECE_BYTES;
+    LatBars* bars = reinterpret_cast<LatBars*>(aligned + rc * QPIECE_BYTES + 2 * (rc + hc) * PIECE_BYTES);
+    volatile int* abort_flag = &bars->abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int Dk = R + 64;
+
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&bars->q_full), 1);
+        mbar_init(smem_u32(&bars->qt_full), 4);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(smem_u32(&bars->rest_full[s]), 1);
+            mbar_init(smem_u32(&bars->own_full[s]), 1);
+            mbar_init(smem_u32(&bars->rest_done[s]), 1);
+            mbar_init(smem_u32(&bars->s_full[s]), 1);
+            mbar_init(smem_u32(&bars->pv_done[s]), 1);
+        }
+        mbar_init(smem_u32(&bars->p_ready), 4);
+        mbar_init(smem_u32(&bars->o_full), 1);
+        bars->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+
+    // the item: a tile of rows (the latest rows of the last sequence first: they see the most keys) and a half of the value columns
+    const int half = blockIdx.x & 1;
+    int seq = -1, m0 = 0;
+    {
+        int left = n_x - 1 - (int)(blockIdx.x >> 1);
+        for (int i = 0; i < b.n_seqs; i++) {
+            const int nt = ((b.cu_seqlens[i + 1] - b.cu_seqlens[i]) * H + ROWS - 1) / ROWS;
+            if (left < nt) { seq = i; m0 = left * ROWS; break; }
+            left -= nt;
+        }
+    }
+    if (seq >= 0) {
+        const int t0 = b.cu_seqlens[seq], rows_here = min(ROWS, (b.cu_seqlens[seq + 1] - t0) * H - m0);
+        const int slot = b.slots[seq], start = b.lengths[slot];
+        const int first_pos = start + m0 / H, last_pos = start + (m0 + rows_here - 1) / H;
+        const int blk0 = window > 0 ? max(0, first_pos - window + 1) / LK : 0, n_iter = last_pos / LK + 1 - blk0;
+        const int own0 = half * hc * 64;              // the own half's first number in a row
+        const size_t row0 = (size_t)t0 * H + m0;      // the tile's first row of q and out
+
+        if (warp == 0) {
+            if (lane == 0) {
+                // the rest of a row: the other half's pieces, then the rotated part
+                mbar_expect_tx(smem_u32(&bars->q_full), (uint32_t)rc * QPIECE_BYTES);
+                for (int c = 0; c < rc; c++)
+                    tma_load_2d(qs + c * QPIECE_BYTES, &map_q, c < hc ? (1 - half) * hc * 64 + c * 64 : R, (int)row0, smem_u32(&bars->q_full));
+                const int* pt = page_table + (size_t)slot * max_pages;
+                for (int j = 0; j < n_iter; j++) {
+                    const int s = j & 1;
+                    const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+                    const int pi = blk0 + j;
+                    int page = pi < max_pages ? pt[pi] : -1;
+                    if (page < 0 || page >= n_pages_pool) { gfb_report(status, GFB_ERR_PAGE_TABLE, slot, pi); page = 0; }
+                    if (!mbar_wait(smem_u32(&bars->rest_done[s]), ph ^ 1u, abort_flag, status, 21)) break;
+                    mbar_expect_tx(smem_u32(&bars->rest_full[s]), (uint32_t)rc * PIECE_BYTES);
+                    for (int c = 0; c < rc; c++)
+                        tma_load_2d(rs + (s * rc + c) * PIECE_BYTES, &map_k, c < hc ? (1 - half) * hc * 64 + c * 64 : R, page * LK, smem_u32(&bars->rest_full[s]));
+                    if (!mbar_wait(smem_u32(&bars->pv_done[s]), ph ^ 1u, abort_flag, status, 22)) break;
+                    mbar_expect_tx(smem_u32(&bars->own_full[s]), (uint32_t)hc * PIECE_BYTES);
+                    for (int c = 0; c < hc; c++)
+                        tma_load_2d(os + (s * hc + c) * PIECE_BYTES, &map_k, own0 + c * 64, page * LK, smem_u32(&bars->own_full[s]));
+                }
+            }
+        } else if (warp == 1) {
+            if (lane == 0) {
+                const uint32_t idesc_s = idesc_bf16(ROWS, LK, 0), idesc_o = idesc_bf16(ROWS, hc * 64, 1);
+                auto issue_s = [&](int j) -> bool {
+                    const int s = j & 1;
+                    const uint32_t ph = (uint32_t)(j >> 1) & 1u, d = tmem + LCOL_S + s * LK;
+                    if (!mbar_wait(smem_u32(&bars->rest_full[s]), ph, abort_flag, status, 23)) return false;
+                    tc_fence_after();
+                    for (int c = 0; c < rc; c++) {
+                        const uint64_t da = desc_kmajor(qs + c * QPIECE_BYTES), db = desc_kmajor(rs + (s * rc + c) * PIECE_BYTES);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) umma_ss(d, da + 2 * k, db + 2 * k, idesc_s, (c | k) != 0);
+                    }
+                    umma_commit(smem_u32(&bars->rest_done[s]));
+                    if (!mbar_wait(smem_u32(&bars->own_full[s]), ph, abort_flag, status, 24)) return false;
+                    tc_fence_after();
+                    for (int c = 0; c < hc; c++) {
+                        const uint64_t db = desc_kmajor(os + (s * hc + c) * PIECE_BYTES);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) umma_ts(d, tmem + LCOL_Q + c * 32 + k * 8, db + 2 * k, idesc_s, 1);
+                    }
+                    umma_commit(smem_u32(&bars->s_full[s]));
+                    return true;
+                };
+                bool ok = mbar_wait(smem_u32(&bars->q_full), 0, abort_flag, status, 25);
+                ok = ok && mbar_wait(smem_u32(&bars->qt_full), 0, abort_flag, status, 26);
+                tc_fence_after();
+                ok = ok && issue_s(0);
+                for (int j = 0; j < n_iter && ok; j++) {
+                    // the next page's scores go ahead of this page's P V (their buffer's last P was read by the P V before, in order)
+                    if (j + 1 < n_iter) ok = issue_s(j + 1);
+                    ok = ok && mbar_wait(smem_u32(&bars->p_ready), (uint32_t)j & 1u, abort_flag, status, 27);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const int s = j & 1;
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)                       // 16 keys per MMA: 8 columns of P, 2 KB of every piece
+                        umma_ts(tmem, tmem + LCOL_S + s * LK + kk * 8, desc_mnmajor(os + s * hc * PIECE_BYTES + kk * 2048, PIECE_BYTES), idesc_o, (j | kk) != 0);
+                    umma_commit(smem_u32(&bars->pv_done[s]));
+                    if (j + 1 == n_iter) umma_commit(smem_u32(&bars->o_full));
+                }
+            }
+        } else {
+            const int quarter = warp & 3;
+            const int r = quarter * 32 + lane;
+            const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+            const bool row_ok = r < rows_here;
+            const int row_pos = start + (m0 + r) / H;
+            const int row_lo = window > 0 ? max(0, row_pos - window + 1) : 0;
+            const int last_lo = window > 0 ? max(0, last_pos - window + 1) : 0;
+            // Q's own half into tensor memory: a row per thread, two numbers per column (rows beyond the tile: zeros)
+            {
+                const uint4* src = reinterpret_cast<const uint4*>(q + (row0 + (row_ok ? r : 0)) * Dk + own0);
+                for (int c = 0; c < 2 * hc; c++) {
+                    uint32_t v[16];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const uint4 x = row_ok ? src[c * 4 + i] : make_uint4(0u, 0u, 0u, 0u);
+                        v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+                    }
+                    tmem_st16(lane_base + LCOL_Q + c * 16, v);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&bars->qt_full));
+            }
+            float m_run = -INFINITY, l_run = 0.f;
+            bool ok = true;
+            for (int j = 0; j < n_iter; j++) {
+                const int s = j & 1, key0 = (blk0 + j) * LK;
+                ok = mbar_wait(smem_u32(&bars->s_full[s]), (uint32_t)(j >> 1) & 1u, abort_flag, status, 28);
+                if (!ok) break;
+                tc_fence_after();
+                uint32_t raw[2][32];
+                tmem_ld32_issue(lane_base + LCOL_S + s * LK, raw[0]);
+                tmem_ld32_issue(lane_base + LCOL_S + s * LK + 32, raw[1]);
+                tmem_ld_wait32(raw[0]);
+                tmem_ld_wait32(raw[1]);
+                float v[2][32];
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[c][i] = __uint_as_float(raw[c][i]);
+                // only pages on the diagonal, at the window's edge or of a tile with empty rows
+                if (key0 + LK - 1 > first_pos || key0 < last_lo || rows_here < ROWS) {
+#pragma unroll
+                    for (int c = 0; c < 2; c++)
+#pragma unroll
+                        for (int i = 0; i < 32; i++) {
+                            const int kj = key0 + c * 32 + i;
+                            if (!(row_ok && kj <= row_pos && kj >= row_lo)) v[c][i] = -INFINITY;
+                        }
+                }
+                float mx4[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const float* x = &v[c >> 1][(c & 1) * 16];
+                    mx4[c] = fmaxf(x[0], x[1]);
+#pragma unroll
+                    for (int i = 2; i < 16; i += 2) mx4[c] = max3(mx4[c], x[i], x[i + 1]);
+                }
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                // the reference maximum follows lazily, in steps of 2^8 (as in the kernels above)
+                float m_new = m_run;
+                if (mx > m_run && (m_run == -INFINITY || (mx - m_run) * scale_log2e > 8.f)) m_new = mx;
+                const float corr = (m_run == -INFINITY || m_new == m_run) ? 1.f : fast_exp2((m_run - m_new) * scale_log2e);
+                const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * scale_log2e;
+                float rsum[2] = {0.f, 0.f};
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    uint32_t pk[16];
+                    float odd = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float a0, a1;
+                        fma2(v[c][i], v[c][i + 1], scale_log2e, mneg, a0, a1);
+                        const float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
+                        add2(rsum[c], odd, p0, p1);
+                        pk[i >> 1] = pack2(p0, p1);
+                    }
+                    rsum[c] += odd;
+                    tmem_st16(lane_base + LCOL_S + s * LK + c * 16, pk);
+                }
+                // O follows a new reference, behind the previous P V: the scores of this page were issued behind the P V of page j - 2,
+                // and that of page j + 1 waits for this warp, so the barrier's phase is the awaited one or the one before it
+                if (j > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
+                    ok = mbar_wait(smem_u32(&bars->pv_done[(j - 1) & 1]), (uint32_t)((j - 1) >> 1) & 1u, abort_flag, status, 29);
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < 2 * hc; c++) {
+                        float o[32];
+                        tmem_ld32(lane_base + c * 32, o);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) o[i] *= corr;
+                        tmem_st32(lane_base + c * 32, o);
+                    }
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&bars->p_ready));
+                l_run = l_run * corr + (rsum[0] + rsum[1]);
+                m_run = m_new;
+            }
+            if (ok) ok = mbar_wait(smem_u32(&bars->o_full), 0, abort_flag, status, 30);
+            if (ok) {
+                tc_fence_after();
+                if (sink != nullptr && m_run != -INFINITY) l_run += fast_exp2(sink[(m0 + r) % H] * 1.4426950408889634f - m_run * scale_log2e);
+                const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+                __nv_bfloat16* dst = out + (row0 + r) * R + own0;
+#pragma unroll 1
+                for (int c = 0; c < 2 * hc; c++) {
+                    float o[32];
+                    tmem_ld32(lane_base + c * 32, o);                      // warp-collective: also for idle rows
+                    if (row_ok) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 8) {
+                            uint4 pk;
+                            pk.x = pack2(o[i] * inv, o[i + 1] * inv); pk.y = pack2(o[i + 2] * inv, o[i + 3] * inv);
+                            pk.z = pack2(o[i + 4] * inv, o[i + 5] * inv); pk.w = pack2(o[i + 6] * inv, o[i + 7] * inv);
+                            *reinterpret_cast<uint4*>(dst + c * 32 + i) = pk;
+                        }
+                    }
+                }
+            }
+        }
+    }
+    if (*abort_flag) {
+        unsigned long long w0 = global_ns();
+        while (global_ns() - w0 < 50000ull) __nanosleep(1000);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1314,4 +1610,40 @@ GFB_API int gfb_attn_prefill_tc_capped(const void* q, void* out, void* k_pool, v
         return gfb_check(e, "gfb_attn_prefill_tc (kept first positions)");
     }
     return 0;
+}
+
+// Prompts against a shared latent (the arguments are gfb_latent_attention's): q bfloat16 [T, H, R + 64], out bfloat16 [T, H * R], cached rows of
+// R + 64 numbers in pages of 64, R = 128, 256, 384 or 512, scale > 0; everything 16-byte aligned.
+GFB_API int gfb_latent_prefill_tc(const void* q, void* out, void* k_pool, const int* page_table, int max_pages, int page_size, int n_pages,
+                                  const int* cu_seqlens, const int* tok_seq, const int* slots, const int* lengths, int n_seqs, int n_tokens, int H,
+                                  int Dk, int R, float scale, int window, const float* sink, int* status, cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (page_size != PAGE || R < 128 || R > 512 || R % 128 || Dk != R + 64 || !(scale > 0.f) || H < 1)
+        return gfb_fail("gfb_latent_prefill_tc: rows of %d with %d value columns in pages of %d, scale %f", Dk, R, page_size, scale);
+    if ((((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool) & 15) != 0) return gfb_fail("gfb_latent_prefill_tc: operands must be 16-byte aligned");
+    if ((long long)n_pages * PAGE > 2147483647LL || (long long)n_tokens * H + ROWS > 2147483647LL)
+        return gfb_fail("gfb_latent_prefill_tc: %d pages or %d x %d rows do not fit the 32-bit row coordinate of a tensor map", n_pages, n_tokens, H);
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return gfb_fail("gfb_latent_prefill_tc: the driver does not export cuTensorMapEncodeTiled");
+    CUtensorMap mq, mk;
+    for (int i = 0; i < 2; i++) {
+        cuuint64_t dims[2] = {(cuuint64_t)Dk, i ? (cuuint64_t)n_pages * PAGE : (cuuint64_t)n_tokens * H};
+        cuuint64_t strides[1] = {(cuuint64_t)Dk * 2};
+        cuuint32_t box[2] = {64, (cuuint32_t)(i ? LK : ROWS)};
+        cuuint32_t es[2] = {1, 1};
+        CUresult r = enc(i ? &mk : &mq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, i ? k_pool : const_cast<void*>(q), dims, strides, box, es,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return gfb_fail("gfb_latent_prefill_tc: tensor map refused (%d)", (int)r);
+    }
+    GfbBatch b{cu_seqlens, tok_seq, slots, lengths, n_seqs, n_tokens};
+    const int hc = R / 128;
+    const size_t smem = 1024 + (size_t)(hc + 1) * QPIECE_BYTES + 2 * (size_t)(2 * hc + 1) * PIECE_BYTES + sizeof(LatBars);
+    cudaError_t e = cudaFuncSetAttribute(latent_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return gfb_fail("gfb_latent_prefill_tc: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
+    const long n_x = ((long)n_tokens * H + ROWS - 1) / ROWS + n_seqs;          // an upper bound of the tiles; surplus blocks find no work
+    if (2 * n_x > 2147483647L) return gfb_fail("gfb_latent_prefill_tc: %ld tiles", n_x);
+    e = gfb_launch(latent_prefill_tc_kernel, dim3((unsigned)(2 * n_x)), dim3(LAT_THREADS), smem, stream, mq, mk, (const __nv_bfloat16*)q,
+                   (__nv_bfloat16*)out, page_table, max_pages, n_pages, b, H, R, scale * 1.4426950408889634f, window, sink, (int)n_x, status);
+    return gfb_check(e, "gfb_latent_prefill_tc");
 }

@@ -947,6 +947,14 @@ class CudaKernels:
         if (values_in_keys and not biased and not special and q.dtype == torch.bfloat16 and n_kv == 1 and chunk is None
                 and head_dim % 16 == 0 and dv % 16 == 0 and dv <= 512 and dv < head_dim and kv.page_size % 32 == 0
                 and (64 + 2 * 32) * (head_dim + 8) * 2 <= 220 * 1024):
+            if (batch.max_q_len > 1 and kv.page_size == 64 and head_dim == dv + 64 and dv % 128 == 0 and scale > 0
+                    and (q.data_ptr() | out.data_ptr() | kv.k_pool.data_ptr()) % 16 == 0):
+                # prompts at the sizes the tcgen05 kernel is built for (it takes the maximum of unscaled scores, so scale > 0)
+                self._label = "gfb_latent_attention"
+                return self._call("attention_tc", "gfb_latent_prefill_tc", _ptr(q), _ptr(out), _ptr(kv.k_pool), _ptr(kv.page_table),
+                                  c_int(kv.page_table.shape[1]), c_int(kv.page_size), c_int(kv.k_pool.shape[0]), *self._batch_args(batch),
+                                  c_int(n_head), c_int(head_dim), c_int(dv), c_float(scale), c_int(window or 0), _ptr(sink), _ptr(batch.status),
+                                  _stream())
             # a latent that all heads share: the tensor-core kernel that fetches every cached row once per 64 (token, head)
             # pairs of a sequence (a decode step's heads are the rows of one MMA)
             splits, scratch = 1, None

@@ -1,0 +1,40 @@
+"""Prompts against a shared latent on tcgen05: every rank the kernel takes, heads that fill a tile of 128 (token, head) rows or straddle it,
+one to many pages, windows and sinks, sequences that go on behind cached tokens, against 64-bit softmax attention."""
+import dataclasses
+
+import pytest
+import torch
+
+from gpt_fast_b200 import ops
+from gpt_fast_b200.ops.types import PagedKV
+from test_kernels_gpu import DEV, REF, make_batch, rnd
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("R", [128, 256, 384, 512])
+@pytest.mark.parametrize("H,q_lens,starts,window,sinks", [
+    (1, [2], [0], None, False),                          # two rows
+    (16, [8, 9], [0, 56], None, False),                  # one whole tile, one and a bit, up to a page's edge
+    (7, [130, 3, 65], [0, 63, 640], None, True),         # tiles that end inside a token
+    (48, [20, 40], [1, 700], 64, True),                  # windows that begin inside a page
+    (16, [300], [0], 1, False),
+    (16, [200, 1, 64], [0, 5, 64], 500, False),
+])
+def test_latent_prompts(R, H, q_lens, starts, window, sinks):
+    dtype = torch.bfloat16
+    batch, table, n_pages = make_batch(q_lens, starts, 6, 64, 16, seed=3)
+    kv = PagedKV(rnd(n_pages, 1, 64, R + 64, dtype=dtype, scale=0.5, seed=1), torch.zeros(n_pages, 1, 64, 0, dtype=dtype, device=DEV), table, 64)
+    q, sink = rnd(batch.n_tokens, H, R + 64, dtype=dtype, scale=0.5, seed=2), rnd(H, seed=4, scale=2.0) if sinks else None
+    guard = torch.full((batch.n_tokens + 1, H * R), 7.0, dtype=dtype, device=DEV)
+    out = guard[:-1]
+    ops.attention(q, kv, batch, out, H, 1, R + 64, 0.25, window, sink=sink, v_head_dim=R, values_in_keys=True)
+    ops.check_status(batch.status)
+    assert bool((guard[-1] == 7.0).all())
+    cpu = dataclasses.replace(batch, **{f: getattr(batch, f).cpu() for f in ("cu_seqlens", "tok_seq", "slots", "lengths", "status")})
+    want = torch.empty(batch.n_tokens, H * R, dtype=torch.float64)
+    REF.attention(q.cpu(), PagedKV(kv.k_pool.cpu(), kv.v_pool.cpu(), table.cpu(), 64), cpu, want, H, 1, R + 64, 0.25, window,
+                  sink=sink.cpu() if sinks else None, v_head_dim=R, values_in_keys=True)
+    # P and the output are rounded to bfloat16 once each (2^-9), values are of size 0.5 to 2
+    torch.testing.assert_close(out.double().cpu(), want, rtol=2e-2, atol=1e-2)
+    assert float((out.double().cpu() - want).norm() / want.norm()) < 5e-3
