@@ -1354,6 +1354,124 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
 }
 
+// ---- a product with a weight per head -----------------------------------------------------------------
+// out[t, h, n] = sum_k in[t, h, k] W_h[k, n], optionally times a sigmoid gate (gfb_headwise_linear states the arguments): latent attention's
+// move of the queries into the latent space and of the attended latent out of it.  A block takes 128 tokens of one head and 128 columns:
+// A is the tokens' rows through a map over the whole input (the head is a column offset), B the weight as it lies, [k][n], an MN-major operand
+// in two pieces of 64 columns.  Three stages of 64 k (32 KB each), so that two blocks share an SM and one's epilogue runs under the other's
+// loads.  The epilogue passes 32-bit rows through shared memory, so that gates and results move as whole lines.
+//
+// What bounds it is memory (K = 128 or 512: 4,096 tokens of 16 heads read and write 90 MB).  The mma.sync form (64 x 64 tiles without a
+// pipeline), us for 4,096 tokens, 16 heads, 128 -> 512 and back: 234 -> 105 (34 us alone for
+// 128 -> 512, without the events' cost).
+constexpr int HW_STAGES = 3, HW_STAGE_BYTES = 2 * HALF_BYTES, HW_PITCH = 132;
+constexpr uint32_t HW_SMEM = 1024 + HW_STAGES * HW_STAGE_BYTES + 128;
+static_assert(4 * 32 * HW_PITCH * 4 <= HW_STAGES * HW_STAGE_BYTES, "the epilogue's rows take the ring's place");
+
+struct HwBars {
+    unsigned long long full[HW_STAGES], empty[HW_STAGES], done;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+__global__ void __launch_bounds__(192)
+headwise_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, int in_off, int in_stride,
+                   __nv_bfloat16* __restrict__ out, int ld_out, int out_off, int out_stride, const __nv_bfloat16* __restrict__ gate, int ld_gate,
+                   int gate_off, int gate_cols, int n_tokens, int K, int N, int* status) {
+    extern __shared__ uint8_t smem_raw[];
+    if (threadIdx.x == 0) { prefetch_map(&map_a); prefetch_map(&map_w); }
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
+    HwBars* bars = reinterpret_cast<HwBars*>(aligned + HW_STAGES * HW_STAGE_BYTES);
+    volatile int* abort_flag = &bars->abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = blockIdx.x * ROWS, h = blockIdx.y, n0 = blockIdx.z * 128, nkb = K / 64;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < HW_STAGES; s++) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
+        mbar_init(smem_u32(&bars->done), 1);
+        bars->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(128u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int kb = 0; kb < nkb; kb++) {
+                const int s = kb % HW_STAGES;
+                if (!mbar_wait(smem_u32(&bars->empty[s]), ((uint32_t)(kb / HW_STAGES) & 1u) ^ 1u, abort_flag, status, 31)) break;
+                const uint32_t full = smem_u32(&bars->full[s]), at = base + s * HW_STAGE_BYTES;
+                mbar_expect_tx(full, HW_STAGE_BYTES);
+                tma_load_2d(at, &map_a, in_off + h * in_stride + kb * 64, t0, full);
+                tma_load_2d(at + HALF_BYTES, &map_w, n0, h * K + kb * 64, full);
+                tma_load_2d(at + HALF_BYTES + PIECE_BYTES, &map_w, n0 + 64, h * K + kb * 64, full);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = idesc_bf16(ROWS, 128, 1);
+            bool ok = true;
+            for (int kb = 0; kb < nkb && ok; kb++) {
+                const int s = kb % HW_STAGES;
+                ok = mbar_wait(smem_u32(&bars->full[s]), (uint32_t)(kb / HW_STAGES) & 1u, abort_flag, status, 32);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t at = base + s * HW_STAGE_BYTES;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    umma_ss(tmem, desc_kmajor(at) + 2 * k, desc_mnmajor(at + HALF_BYTES + k * 2048, PIECE_BYTES), idesc, (kb | k) != 0);
+                umma_commit(smem_u32(&bars->empty[s]));
+            }
+            if (ok) umma_commit(smem_u32(&bars->done));
+        }
+    } else {
+        const int q = warp & 3;
+        float* mine = reinterpret_cast<float*>(aligned) + q * 32 * HW_PITCH;
+        if (mbar_wait(smem_u32(&bars->done), 0, abort_flag, status, 33)) {      // every copy has landed and been read
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < 128; c += 32) {
+                float v[32];
+                tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c, v);
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(mine + lane * HW_PITCH + c + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            }
+            __syncwarp();
+            const int rows = min(32, n_tokens - (t0 + q * 32));
+#pragma unroll 4
+            for (int r = 0; r < rows; r++) {
+                const size_t t = (size_t)(t0 + q * 32 + r);
+                float4 v = *reinterpret_cast<const float4*>(mine + r * HW_PITCH + lane * 4);
+                if (gate != nullptr) {
+                    const __nv_bfloat16* g = gate + t * ld_gate + gate_off + (gate_cols == 1 ? h : h * N + n0 + lane * 4);
+                    float z[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) z[i] = 1.0f / (1.0f + expf(-__bfloat162float(g[gate_cols == 1 ? 0 : i])));
+                    v.x *= z[0]; v.y *= z[1]; v.z *= z[2]; v.w *= z[3];
+                }
+                *reinterpret_cast<uint2*>(out + t * ld_out + out_off + (size_t)h * out_stride + n0 + lane * 4) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+            }
+        }
+    }
+    if (*abort_flag) {
+        unsigned long long w0 = global_ns();
+        while (global_ns() - w0 < 50000ull) __nanosleep(1000);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128u) : "memory");
+    }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1646,4 +1764,34 @@ GFB_API int gfb_latent_prefill_tc(const void* q, void* out, void* k_pool, const 
     e = gfb_launch(latent_prefill_tc_kernel, dim3((unsigned)(2 * n_x)), dim3(LAT_THREADS), smem, stream, mq, mk, (const __nv_bfloat16*)q,
                    (__nv_bfloat16*)out, page_table, max_pages, n_pages, b, H, R, scale * 1.4426950408889634f, window, sink, (int)n_x, status);
     return gfb_check(e, "gfb_latent_prefill_tc");
+}
+
+// gfb_headwise_linear (whose arguments these are) on tcgen05: bfloat16, K a multiple of 64, N of 128, input and weight 16-byte aligned with
+// ld_in, in_off and in_stride multiples of 8, output 8-byte aligned with ld_out, out_off and out_stride multiples of 4.
+GFB_API int gfb_headwise_linear_tc(const void* in, int ld_in, int in_off, int in_stride, const void* w, void* out, int ld_out, int out_off,
+                                   int out_stride, const void* gate, int ld_gate, int gate_off, int gate_cols, int n_tokens, int H, int K, int N,
+                                   int* status, cudaStream_t stream) {
+    if (n_tokens <= 0 || H <= 0 || N <= 0) return 0;
+    if (K < 64 || K % 64 || N % 128 || ld_in % 8 || in_off % 8 || in_stride % 8 || ld_out % 4 || out_off % 4 || out_stride % 4 ||
+        (((uintptr_t)in | (uintptr_t)w) & 15) || ((uintptr_t)out & 7))
+        return gfb_fail("gfb_headwise_linear_tc: %d -> %d per head, rows of %d and %d, or pointers that are not aligned", K, N, ld_in, ld_out);
+    if (H > 65535 || N / 128 > 65535 || (long long)H * K > 2147483647LL) return gfb_fail("gfb_headwise_linear_tc: %d heads of %d x %d exceed the grid limit", H, K, N);
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return gfb_fail("gfb_headwise_linear_tc: the driver does not export cuTensorMapEncodeTiled");
+    CUtensorMap ma, mw;
+    for (int i = 0; i < 2; i++) {
+        cuuint64_t dims[2] = {i ? (cuuint64_t)N : (cuuint64_t)ld_in, i ? (cuuint64_t)H * K : (cuuint64_t)n_tokens};
+        cuuint64_t strides[1] = {dims[0] * 2};
+        cuuint32_t box[2] = {64, (cuuint32_t)(i ? 64 : ROWS)};
+        cuuint32_t es[2] = {1, 1};
+        CUresult r = enc(i ? &mw : &ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(i ? w : in), dims, strides, box, es,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return gfb_fail("gfb_headwise_linear_tc: tensor map refused (%d)", (int)r);
+    }
+    cudaError_t e = cudaFuncSetAttribute(headwise_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HW_SMEM);
+    if (e != cudaSuccess) return gfb_fail("gfb_headwise_linear_tc: %u bytes of shared memory refused: %s", HW_SMEM, cudaGetErrorString(e));
+    e = gfb_launch(headwise_tc_kernel, dim3((n_tokens + ROWS - 1) / ROWS, H, N / 128), dim3(192), HW_SMEM, stream, ma, mw, in_off, in_stride,
+                   (__nv_bfloat16*)out, ld_out, out_off, out_stride, (const __nv_bfloat16*)gate, ld_gate, gate_off, gate_cols, n_tokens, K, N, status);
+    return gfb_check(e, "gfb_headwise_linear_tc");
 }

@@ -384,6 +384,8 @@ class CudaKernels:
                    c_float(eps), c_int(n_head), c_int(head_dim), c_int(rot_dim), c_int(rank), c_int(_PAIRING[pairing]),
                    c_int(1 if append else 0), _ptr(batch.status), _stream())
 
+    HEADWISE_FEW_TOKENS = 64           # up to this many tokens a tile of 128 is mostly empty: the smaller tiles of the mma.sync form
+
     def headwise_linear(self, a, w, out, n_head, k, n, a_off=0, a_stride=None, out_off=0, out_stride=None, gate=None, gate_off=0,
                         gate_per_head=False):
         T = a.shape[0]
@@ -400,6 +402,13 @@ class CudaKernels:
             _need(gate, a.dtype, name="gate")
             if gate.shape[0] != T or gate_off + n_head * (1 if gate_per_head else n) > gate.shape[1]:
                 _fail("head-wise product: the gate does not fit")
+        if (a.dtype == torch.bfloat16 and T > self.HEADWISE_FEW_TOKENS and k % 64 == 0 and n % 128 == 0
+                and (a.shape[1] | a_off | a_stride) % 8 == 0 and (out.shape[1] | out_off | out_stride) % 4 == 0
+                and (a.data_ptr() | w.data_ptr()) % 16 == 0 and out.data_ptr() % 8 == 0):
+            self._call("attention_tc", "gfb_headwise_linear_tc", _ptr(a), c_int(a.shape[1]), c_int(a_off), c_int(a_stride), _ptr(w), _ptr(out),
+                       c_int(out.shape[1]), c_int(out_off), c_int(out_stride), _ptr(gate), c_int(gate.shape[1] if gate is not None else 0),
+                       c_int(gate_off), c_int(1 if gate_per_head else n), c_int(T), c_int(n_head), c_int(k), c_int(n), _ptr(self.status), _stream())
+            return
         self._call("latent", "gfb_headwise_linear", _ptr(a), c_int(_dt(a)), c_int(a.shape[1]), c_int(a_off), c_int(a_stride), _ptr(w), _ptr(out), c_int(out.shape[1]), c_int(out_off), c_int(out_stride), _ptr(gate),
                    c_int(gate.shape[1] if gate is not None else 0), c_int(gate_off), c_int(1 if gate_per_head else n), c_int(T), c_int(n_head),
                    c_int(k), c_int(n),
