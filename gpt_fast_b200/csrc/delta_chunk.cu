@@ -23,9 +23,9 @@
 // do, which keeps their rounding where it was.  T is made from the inverses of its four 16 x 16 diagonal blocks.
 //
 // What bounds it: the token-by-token kernel took 0.48 us per token whatever the hardware's width (a chain of dependent instructions;
-// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 323 us, of which
-// delta_chunk_kernel 168, delta_scan_kernel 120, delta_out_kernel 42.  Against 64-bit sums (700 tokens of 4 heads, outputs): 2.1e-7 where the
-// decays are close to one (token by token 3.4e-7), 1.6e-7 where they are fast (1.5e-7).
+// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 312 us, of which delta_chunk_kernel 158 (shared
+// memory and issue slots: with single FMAs instead of pairs 168), delta_scan_kernel 120, delta_out_kernel 42.  Against 64-bit sums (700 tokens
+// of 4 heads, outputs): 2.3e-7 where the decays are close to one (token by token 3.6e-7), 1.6e-7 to 1.9e-7 where they are fast (1.5e-7).
 #include "common.cuh"
 
 GFB_DEFINE_LAST_ERROR()
@@ -45,6 +45,19 @@ __device__ __forceinline__ float ldw(const void* p, int dt, size_t i) {
 }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+// two 32-bit numbers per instruction (sm_100), each rounded as by the single form
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 r; const f32x2 m = pack2(-1.f, -1.f); asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(m), "l"(a)); return r; }
+__device__ __forceinline__ float half_sum(f32x2 v) { float a, b; unpack2(v, a, b); return a + b; }
+// 2^x for x <= 0 (results below 2^-126 become zero)
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ f32x2 ex22(f32x2 v) { float a, b; unpack2(v, a, b); return pack2(ex2(a), ex2(b)); }
+__device__ __forceinline__ ulonglong2 ldp(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }      // four numbers as two pairs
 __device__ __forceinline__ void copy16(float* smem, const float* gmem) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem) : "memory");
@@ -131,8 +144,9 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
     __syncthreads();
     const float rate = expf(ldw(a_log, w_dt, h)) * LOG2E;
     // Thread (ty, tx) owns tokens ty + 16 r (one per sub-chunk) against tokens tx + 16 c: B in [0], A in [1]
-    // (far: sub-chunks (1,0), (2,1), (2,0), (3,2), (3,1), (3,0))
-    float far[2][6] = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}}, near[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    // (far: sub-chunks (1,0), (2,1), (2,0), (3,2), (3,1), (3,0)),
+    // and every sum as that of its even and that of its odd channels
+    f32x2 far[2][6] = {{0ull, 0ull, 0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull, 0ull, 0ull}}, near[2][4] = {{0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull}};
     const int dd = tid & 31, oct = tid >> 5;        // staging: a channel, eight tokens
 #pragma unroll 1
     for (int d0 = 0; d0 < d; d0 += DT) {
@@ -167,16 +181,16 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
                 if (m < sub) ahead += w;
                 if (m > sub) behind += w;
             }
-            if (!(oct & 1)) sm.M[sub][dd] = exp2f((float)whole);
-            const float pa = exp2f((float)ahead), pb = exp2f((float)behind);
+            if (!(oct & 1)) sm.M[sub][dd] = ex2((float)whole);
+            const float pa = ex2((float)ahead), pb = ex2((float)behind);
             double run = before;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int j = oct * 8 + i;
                 run += (double)gi[i];
-                const float L = (float)run, e = exp2f(L);
+                const float L = (float)run, e = ex2(L);
                 // the decays behind the token within its sub-chunk: never above zero, also where rounding made the two sums cross
-                const float kh = ki[i] * exp2f(fminf((float)(whole - run), 0.f));
+                const float kh = ki[i] * ex2(fminf((float)(whole - run), 0.f));
                 sm.q[j][dd] = qi[i];
                 sm.k[j][dd] = ki[i];
                 sm.L[j][dd] = L;
@@ -188,56 +202,48 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
                 W[(size_t)j * d + ch] = sm.beta[j] * (ki[i] * e * pa);       // the right-hand side that becomes W
                 gi[i] = qi[i] * e * pa;
             }
-            if (oct == 0) dec[ch] = exp2f((float)(whole + behind));
+            if (oct == 0) dec[ch] = ex2((float)(whole + behind));
             float4* out = reinterpret_cast<float4*>(QB + (size_t)ch * PC + oct * 8);
             out[0] = make_float4(gi[0], gi[1], gi[2], gi[3]);
             out[1] = make_float4(gi[4], gi[5], gi[6], gi[7]);
         }
         __syncthreads();
-#define DOT4(acc, p, s) acc = fmaf(p.x, s.x, fmaf(p.y, s.y, fmaf(p.z, s.z, fmaf(p.w, s.w, acc))))
-#define MUL4(p, s) make_float4(p.x * s.x, p.y * s.y, p.z * s.z, p.w * s.w)
-        float pf[2][6] = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}}, pn[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll 1
         for (int x = 0; x < DT; x += 4) {
             {
-                const float4 M1 = ld4(&sm.M[1][x]), M2 = ld4(&sm.M[2][x]);
-                const float4 h0 = ld4(&sm.kh[tx][x]), h1 = ld4(&sm.kh[tx + 16][x]), h2 = ld4(&sm.kh[tx + 32][x]);
+                const ulonglong2 M1 = ldp(&sm.M[1][x]), M2 = ldp(&sm.M[2][x]);
+                const ulonglong2 h0 = ldp(&sm.kh[tx][x]), h1 = ldp(&sm.kh[tx + 16][x]), h2 = ldp(&sm.kh[tx + 32][x]);
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
                     const float(*rows)[DTP] = m == 0 ? sm.qt : sm.kt;
-                    const float4 r1 = ld4(&rows[ty + 16][x]), r2 = ld4(&rows[ty + 32][x]), r3 = ld4(&rows[ty + 48][x]);
-                    const float4 a2 = MUL4(r2, M1), a3 = MUL4(r3, M2), b3 = MUL4(a3, M1);
-                    DOT4(pf[m][0], r1, h0);
-                    DOT4(pf[m][1], r2, h1);
-                    DOT4(pf[m][2], a2, h0);
-                    DOT4(pf[m][3], r3, h2);
-                    DOT4(pf[m][4], a3, h1);
-                    DOT4(pf[m][5], b3, h0);
+                    const ulonglong2 r1 = ldp(&rows[ty + 16][x]), r2 = ldp(&rows[ty + 32][x]), r3 = ldp(&rows[ty + 48][x]);
+                    const f32x2 a2x = mul2(r2.x, M1.x), a2y = mul2(r2.y, M1.y), a3x = mul2(r3.x, M2.x), a3y = mul2(r3.y, M2.y);
+                    const f32x2 b3x = mul2(a3x, M1.x), b3y = mul2(a3y, M1.y);
+                    fma2(far[m][0], r1.x, h0.x); fma2(far[m][0], r1.y, h0.y);
+                    fma2(far[m][1], r2.x, h1.x); fma2(far[m][1], r2.y, h1.y);
+                    fma2(far[m][2], a2x, h0.x); fma2(far[m][2], a2y, h0.y);
+                    fma2(far[m][3], r3.x, h2.x); fma2(far[m][3], r3.y, h2.y);
+                    fma2(far[m][4], a3x, h1.x); fma2(far[m][4], a3y, h1.y);
+                    fma2(far[m][5], b3x, h0.x); fma2(far[m][5], b3y, h0.y);
                 }
             }
             if (tx <= ty) {
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
-                    const float4 q4 = ld4(&sm.q[ty + 16 * r][x]), c4 = ld4(&sm.k[ty + 16 * r][x]), k4 = ld4(&sm.k[tx + 16 * r][x]);
-                    const float4 li = ld4(&sm.L[ty + 16 * r][x]), lj = ld4(&sm.L[tx + 16 * r][x]);
-                    const float4 ri = ld4(&sm.Lo[ty + 16 * r][x]), rj = ld4(&sm.Lo[tx + 16 * r][x]);
-                    const float4 e = make_float4(k4.x * exp2f((li.x - lj.x) + (ri.x - rj.x)), k4.y * exp2f((li.y - lj.y) + (ri.y - rj.y)),
-                                                 k4.z * exp2f((li.z - lj.z) + (ri.z - rj.z)), k4.w * exp2f((li.w - lj.w) + (ri.w - rj.w)));
-                    DOT4(pn[0][r], q4, e);
-                    DOT4(pn[1][r], c4, e);
+                    const ulonglong2 li = ldp(&sm.L[ty + 16 * r][x]), lj = ldp(&sm.L[tx + 16 * r][x]);
+                    const ulonglong2 ri = ldp(&sm.Lo[ty + 16 * r][x]), rj = ldp(&sm.Lo[tx + 16 * r][x]);
+                    const ulonglong2 k2 = ldp(&sm.k[tx + 16 * r][x]);
+                    const f32x2 ex = mul2(k2.x, ex22(add2(sub2(li.x, lj.x), sub2(ri.x, rj.x))));
+                    const f32x2 ey = mul2(k2.y, ex22(add2(sub2(li.y, lj.y), sub2(ri.y, rj.y))));
+                    const ulonglong2 q2 = ldp(&sm.q[ty + 16 * r][x]), c2 = ldp(&sm.k[ty + 16 * r][x]);
+                    fma2(near[0][r], q2.x, ex); fma2(near[0][r], q2.y, ey);
+                    fma2(near[1][r], c2.x, ex); fma2(near[1][r], c2.y, ey);
                 }
             }
         }
-#pragma unroll
-        for (int m = 0; m < 2; m++) {
-#pragma unroll
-            for (int i = 0; i < 6; i++) far[m][i] += pf[m][i];
-#pragma unroll
-            for (int r = 0; r < 4; r++) near[m][r] += pn[m][r];
-        }
     }
     __syncthreads();                                 // the matrices take the place of q, k, L
-    // B to memory (transposed, zeros above the diagonal), diag(beta) A to shared memory
+    // B transposed (zeros above the diagonal) and diag(beta) A; T is kept transposed too, so that four rows of it are one load
 #pragma unroll
     for (int r = 0; r < 4; r++) {
         const int i = ty + 16 * r;
@@ -246,14 +252,18 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
         for (int cc = 0; cc < 4; cc++) {
             const int j = tx + 16 * cc;
             const int f = cc < r ? (r == 1 ? 0 : r == 2 ? 2 - cc : 5 - cc) : 0;
-            const float bv = cc < r ? far[0][f] : (cc == r && tx <= ty) ? near[0][r] : 0.f;
-            const float av = cc < r ? far[1][f] : (cc == r && tx < ty) ? near[1][r] : 0.f;
-            QB[(size_t)(d + j) * PC + i] = bv;
+            const float bv = cc < r ? half_sum(far[0][f]) : (cc == r && tx <= ty) ? half_sum(near[0][r]) : 0.f;
+            const float av = cc < r ? half_sum(far[1][f]) : (cc == r && tx < ty) ? half_sum(near[1][r]) : 0.f;
+            sm.R[j][i] = bv;
             sm.N[i][j] = be * av;
-            sm.T[i][j] = 0.f;
+            sm.T[j][i] = 0.f;
         }
     }
     __syncthreads();
+    for (int e = tid; e < PC * 16; e += THREADS) {
+        const int j = e >> 4, i = (e & 15) * 4;
+        *reinterpret_cast<float4*>(QB + (size_t)(d + j) * PC + i) = ld4(&sm.R[j][i]);
+    }
     // the inverses of the diagonal blocks of I + N: a thread per column, forward substitution
     if (tid < PC) {
         const int o = (tid >> 4) * SUB, col = tid & 15;
@@ -264,7 +274,7 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
 #pragma unroll
             for (int j = 0; j < i; j++) v = fmaf(-sm.N[o + i][o + j], x[j], v);
             x[i] = v;                                // zero above the diagonal by itself
-            sm.T[o + i][o + col] = v;
+            sm.T[o + col][o + i] = v;
         }
     }
     // blocks below the diagonal, one diagonal of blocks after the other: T_rc = -T_rr sum_(c <= m < r) N_rm T_mc
@@ -273,7 +283,7 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
         for (int k = 0; k < 4 - off; k++) {          // thread (ty, tx): one number of each block
             const int r = k + off;
             float v = 0.f;
-            for (int m = k * SUB; m < r * SUB; m++) v = fmaf(sm.N[r * SUB + ty][m], sm.T[m][k * SUB + tx], v);
+            for (int m = k * SUB; m < r * SUB; m++) v = fmaf(sm.N[r * SUB + ty][m], sm.T[k * SUB + tx][m], v);
             sm.P[k][ty][tx] = v;
         }
         __syncthreads();
@@ -281,11 +291,11 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             const int r = k + off;
             float v = 0.f;
 #pragma unroll
-            for (int m = 0; m < SUB; m++) v = fmaf(sm.T[r * SUB + ty][r * SUB + m], sm.P[k][m][tx], v);
-            sm.T[r * SUB + ty][k * SUB + tx] = -v;
+            for (int m = 0; m < SUB; m++) v = fmaf(sm.T[r * SUB + m][r * SUB + ty], sm.P[k][m][tx], v);
+            sm.T[k * SUB + tx][r * SUB + ty] = -v;
         }
     }
-    // W = T (diag(beta) Kt) in place, Y = T (diag(beta) V): 64 columns at a time, a thread has rows ty + 16 r and four columns
+    // W = T (diag(beta) Kt) in place, Y = T (diag(beta) V): 64 columns at a time
     const int tiles = (d + dv) / 64;
     for (int tile = 0; tile < tiles; tile++) {
         const bool of_w = tile * 64 < d;
@@ -307,42 +317,39 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             *reinterpret_cast<float4*>(&sm.R[j][cc]) = v;
         }
         __syncthreads();
+        // rows 4 ty .. + 3 (their sub-chunk and those before it), columns 4 tx .. + 3
         float acc[4][4];
 #pragma unroll
         for (int r = 0; r < 4; r++)
 #pragma unroll
             for (int cc = 0; cc < 4; cc++) acc[r][cc] = 0.f;
+        for (int J = 0; J <= ty >> 2; J++) {
+            f32x2 part[4][2] = {{0ull, 0ull}, {0ull, 0ull}, {0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll
-        for (int J = 0; J < 4; J++) {
-            float part[4][4];
-#pragma unroll
-            for (int r = J; r < 4; r++)
-#pragma unroll
-                for (int cc = 0; cc < 4; cc++) part[r][cc] = 0.f;
-#pragma unroll 4
             for (int jj = 0; jj < SUB; jj++) {
-                const float4 v = ld4(&sm.R[16 * J + jj][4 * tx]);
-#pragma unroll
-                for (int r = J; r < 4; r++) {
-                    const float a = sm.T[ty + 16 * r][16 * J + jj];
-                    part[r][0] = fmaf(a, v.x, part[r][0]); part[r][1] = fmaf(a, v.y, part[r][1]);
-                    part[r][2] = fmaf(a, v.z, part[r][2]); part[r][3] = fmaf(a, v.w, part[r][3]);
-                }
+                const ulonglong2 v = ldp(&sm.R[16 * J + jj][4 * tx]);
+                const float4 t4 = ld4(&sm.T[16 * J + jj][4 * ty]);
+                const f32x2 t0 = pack2(t4.x, t4.x), t1 = pack2(t4.y, t4.y), t2 = pack2(t4.z, t4.z), t3 = pack2(t4.w, t4.w);
+                fma2(part[0][0], t0, v.x); fma2(part[0][1], t0, v.y);
+                fma2(part[1][0], t1, v.x); fma2(part[1][1], t1, v.y);
+                fma2(part[2][0], t2, v.x); fma2(part[2][1], t2, v.y);
+                fma2(part[3][0], t3, v.x); fma2(part[3][1], t3, v.y);
             }
 #pragma unroll
-            for (int r = J; r < 4; r++)
-#pragma unroll
-                for (int cc = 0; cc < 4; cc++) acc[r][cc] += part[r][cc];
+            for (int r = 0; r < 4; r++) {
+                float a, e, i, o;
+                unpack2(part[r][0], a, e);
+                unpack2(part[r][1], i, o);
+                acc[r][0] += a; acc[r][1] += e; acc[r][2] += i; acc[r][3] += o;
+            }
         }
 #pragma unroll
         for (int r = 0; r < 4; r++) {
-            const int i = ty + 16 * r;
+            const int i = 4 * ty + r;
             float* dst = of_w ? W + (size_t)i * d + c0 + 4 * tx : SU + (size_t)(d + i) * dv + c0 + 4 * tx;
             *reinterpret_cast<float4*>(dst) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
         }
     }
-#undef DOT4
-#undef MUL4
 }
 
 // A block has S [d][16] of one (sequence, head) in shared memory, transposed, and two stages of W, Kh, Y and the decays: the next
