@@ -237,9 +237,21 @@ __device__ __forceinline__ bool epilogue_warps_all(bool flag) {
 
 __device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.f + __expf(-g)) * u; }
 
+// 1 / d for d >= 1, infinite or not a number: the hardware's estimate and two steps of Newton's method, each with its residual from one
+// FMA (Markstein 1990).  The division it stands for ends in a branch for rare operands, and an epilogue whose every number branches runs
+// them one behind the other: 8,192 rows by 3,584 x 2,048 took 139 us with it and 97 so, as the same product with SiLU.  From 1 to infinity
+// five numbers differ from 1.0f / d, each in its last bit.
+__device__ __forceinline__ float reciprocal(float d) {
+    float y;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(d));
+    y = fmaf(y, fmaf(-d, y, 1.0f), y);
+    y = fmaf(y, fmaf(-d, y, 1.0f), y);
+    return d == INFINITY ? 0.f : y;
+}
+
 __device__ __forceinline__ float glu_clamp(float g, float u, const Groups& gp) {
     if (gp.limit > 0.f) { g = fminf(g, gp.limit); u = fminf(fmaxf(u, -gp.limit), gp.limit); }
-    return g * (1.0f / (1.0f + expf(-gp.alpha * g))) * (u + gp.shift);
+    return g * reciprocal(1.0f + expf(-gp.alpha * g)) * (u + gp.shift);
 }
 
 // the gated activation of an epilogue: SiLU(g) u, or the clamped form with the product's constants
