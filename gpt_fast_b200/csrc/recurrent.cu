@@ -657,6 +657,185 @@ GFB_API int gfb_delta_rule(float* qkv, int ldq, int q_off, int k_off, int v_off,
     return gfb_check(e, "gfb_delta_rule");
 }
 
+// One token per sequence (a decode step) in one launch: what delta_prepare_kernel does, the token's step and its output.  Four warps take a
+// slice of a (sequence, head)'s columns, a lane RPT rows of four of them: the state comes and goes once in 16-byte accesses, all of a lane's
+// in flight at once while the block makes its unit vectors and decays.  Sums run in the order of delta_rule_kernel (RPT terms per lane, a
+// butterfly over a column's lanes for S^T k, the lanes' parts in ascending order for the output), so a token's result is the same bits.
+// What bounds it is latency: 8 sequences of 16 heads of 128 x 128 (8.4 MB each way) take 11.0 us alone; in a captured decode step of the mixer, whose
+// conv, products and norm surround it, delta_prepare_kernel and delta_rule_kernel in its place cost 32 us more (75.6 -> 43.2).
+template <typename TD, int RPT>
+__global__ void __launch_bounds__(32 * SCAN_WARPS)
+delta_decode_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off, int v_off, const TD* __restrict__ beta_raw, int ld_b, int beta_off,
+                    const float* __restrict__ a_raw, int ld_a, int a_off, const void* __restrict__ dt_bias, const void* __restrict__ a_log, int w_dt,
+                    float* __restrict__ state, size_t state_ld, float* __restrict__ out, GfbBatch b, int H, int KH, int d, int dv, float q_scale,
+                    float unit_eps, int RG, int head_decay) {
+    extern __shared__ __align__(16) float sm[];
+    float* sQ = sm;                       // [d] each
+    float* sK = sQ + d;
+    float* sG = sK + d;
+    float* sO = sG + d;                   // [columns of the block][RG]: the lanes' parts of the outputs
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    const int s = blockIdx.x, h = blockIdx.y, kh = h / (H / KH);
+    const int CQ = 32 / RG, cols = SCAN_WARPS * CQ * 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rg = lane % RG, c0 = (warp * CQ + lane / RG) * 4, p = blockIdx.z * cols + c0;
+    const int t = b.cu_seqlens[s];
+    const bool active = p < dv;           // (dv is a multiple of four)
+    float* S = state + (size_t)b.slots[s] * state_ld + (size_t)h * d * dv;
+    float4 st[RPT];
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        const int i = rg * RPT + r;
+        st[r] = active && i < d ? *reinterpret_cast<const float4*>(S + (size_t)i * dv + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float* row = qkv + (size_t)t * ldq;
+    if (warp < 2) {                       // warp 0: q, warp 1: k
+        const float* vec = row + (warp ? k_off : q_off) + (size_t)kh * d;
+        float ss = 0.f;
+        for (int c = lane; c < d; c += 32) ss = fmaf(vec[c], vec[c], ss);
+        ss = gfb_warp_sum(ss);
+        const float f = (1.0f / sqrtf(ss + unit_eps)) * (warp ? 1.0f : q_scale);
+        for (int c = lane; c < d; c += 32) (warp ? sK : sQ)[c] = vec[c] * f;
+    } else {                              // warps 2 and 3: the decays
+        const float* ar = a_raw + (size_t)t * ld_a + a_off;
+        const float rate = expf(ldw(a_log, w_dt, h));
+        for (int c = tid - 64; c < d; c += 64) {
+            const size_t at = head_decay ? (size_t)h : (size_t)h * d + c;
+            sG[c] = expf(-rate * softplus_f(ar[at] + ldw(dt_bias, w_dt, at)));
+        }
+    }
+    const float beta = sigmoid_f(gfb_to_f32(beta_raw[(size_t)t * ld_b + beta_off + h]));
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (active) { const float* vp = row + v_off + (size_t)h * dv + p; v = make_float4(vp[0], vp[1], vp[2], vp[3]); }
+    __syncthreads();
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        const int i = rg * RPT + r;
+        const float g = i < d ? sG[i] : 0.f, k = i < d ? sK[i] : 0.f;
+        st[r].x *= g; st[r].y *= g; st[r].z *= g; st[r].w *= g;
+        acc.x = fmaf(st[r].x, k, acc.x); acc.y = fmaf(st[r].y, k, acc.y); acc.z = fmaf(st[r].z, k, acc.z); acc.w = fmaf(st[r].w, k, acc.w);
+    }
+    acc.x = group_sum(acc.x, RG); acc.y = group_sum(acc.y, RG); acc.z = group_sum(acc.z, RG); acc.w = group_sum(acc.w, RG);
+    const float4 u = make_float4(beta * (v.x - acc.x), beta * (v.y - acc.y), beta * (v.z - acc.z), beta * (v.w - acc.w));
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        const int i = rg * RPT + r;
+        const float k = i < d ? sK[i] : 0.f, q = i < d ? sQ[i] : 0.f;
+        st[r].x = fmaf(k, u.x, st[r].x); st[r].y = fmaf(k, u.y, st[r].y); st[r].z = fmaf(k, u.z, st[r].z); st[r].w = fmaf(k, u.w, st[r].w);
+        o.x = fmaf(st[r].x, q, o.x); o.y = fmaf(st[r].y, q, o.y); o.z = fmaf(st[r].z, q, o.z); o.w = fmaf(st[r].w, q, o.w);
+        if (active && i < d) *reinterpret_cast<float4*>(S + (size_t)i * dv + p) = st[r];
+    }
+    sO[c0 * RG + rg] = o.x; sO[(c0 + 1) * RG + rg] = o.y; sO[(c0 + 2) * RG + rg] = o.z; sO[(c0 + 3) * RG + rg] = o.w;
+    __syncthreads();
+    for (int c = tid; c < cols; c += 32 * SCAN_WARPS) {
+        const int col = blockIdx.z * cols + c;
+        if (col < dv) out[((size_t)t * H + h) * dv + col] = sum_parts(sO + c * RG, RG);
+    }
+}
+
+// The same for the state space: dt, decay, the token's step and its output in one launch, in the order of ssd_scan_kernel.
+template <typename TD, int RPT>
+__global__ void __launch_bounds__(32 * SCAN_WARPS)
+ssd_decode_kernel(const float* __restrict__ x, int ldx, int b_off, int c_off, const TD* __restrict__ dt_raw, int ld_dt, int dt_off,
+                  const void* __restrict__ dt_bias, const void* __restrict__ a_log, const void* __restrict__ skip, int w_dt, float* __restrict__ state,
+                  size_t state_ld, float* __restrict__ out, GfbBatch b, int H, int P, int N, int G, int RG) {
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    const int s = blockIdx.x, h = blockIdx.y, g = h / (H / G);
+    const int CQ = 32 / RG, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rg = lane % RG, p = ((blockIdx.z * SCAN_WARPS + warp) * CQ + lane / RG) * 4;
+    const int t = b.cu_seqlens[s];
+    const bool active = p < P;            // (P is a multiple of four)
+    float* S = state + (size_t)b.slots[s] * state_ld + (size_t)h * N * P;
+    const float* row = x + (size_t)t * ldx;
+    float4 st[RPT];
+    float bb[RPT], cc[RPT];
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        const int n = rg * RPT + r;
+        st[r] = active && n < N ? *reinterpret_cast<const float4*>(S + (size_t)n * P + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        bb[r] = n < N ? row[b_off + g * N + n] : 0.f;
+        cc[r] = n < N ? row[c_off + g * N + n] : 0.f;
+    }
+    float4 xp = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (active) { const float* q = row + (size_t)h * P + p; xp = make_float4(q[0], q[1], q[2], q[3]); }
+    const float dx = softplus_f(gfb_to_f32(dt_raw[(size_t)t * ld_dt + dt_off + h]) + ldw(dt_bias, w_dt, h));
+    const float a = expf(-expf(ldw(a_log, w_dt, h)) * dx), dskip = skip != nullptr ? ldw(skip, w_dt, h) : 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        const int n = rg * RPT + r;
+        const float db = dx * bb[r];
+        st[r].x = fmaf(a, st[r].x, db * xp.x); st[r].y = fmaf(a, st[r].y, db * xp.y);
+        st[r].z = fmaf(a, st[r].z, db * xp.z); st[r].w = fmaf(a, st[r].w, db * xp.w);
+        acc.x = fmaf(st[r].x, cc[r], acc.x); acc.y = fmaf(st[r].y, cc[r], acc.y); acc.z = fmaf(st[r].z, cc[r], acc.z); acc.w = fmaf(st[r].w, cc[r], acc.w);
+        if (active && n < N) *reinterpret_cast<float4*>(S + (size_t)n * P + p) = st[r];
+    }
+    acc.x = group_sum(acc.x, RG); acc.y = group_sum(acc.y, RG); acc.z = group_sum(acc.z, RG); acc.w = group_sum(acc.w, RG);
+    if (rg == 0 && active) {
+        float* o = out + ((size_t)t * H + h) * P + p;
+        o[0] = acc.x + dskip * xp.x; o[1] = acc.y + dskip * xp.y; o[2] = acc.z + dskip * xp.z; o[3] = acc.w + dskip * xp.w;
+    }
+}
+
+// As gfb_delta_rule where every sequence of the step has exactly one token: value heads of a multiple of four, a 16-byte aligned state with
+// state_ld % 4 == 0, at most 256 rows (what gfb_delta_rule's shared memory takes); qkv and a_raw are only read.
+GFB_API int gfb_delta_decode(const float* qkv, int ldq, int q_off, int k_off, int v_off, const void* beta_raw, int b_dt, int ld_b, int beta_off,
+                             const float* a_raw, int ld_a, int a_off, const void* dt_bias, const void* a_log, int w_dt, float* state, long state_ld,
+                             float* out, const int* cu_seqlens, const int* tok_seq, const int* slots, const int* lengths, int n_seqs, int n_tokens,
+                             int H, int KH, int d, int dv, float q_scale, float unit_eps, int head_decay, cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (KH <= 0 || H % KH) return gfb_fail("gfb_delta_decode: %d heads do not divide into %d query/key heads", H, KH);
+    if (n_tokens != n_seqs || dv % 4 || state_ld % 4 || ((uintptr_t)state & 15)) return gfb_fail("gfb_delta_decode: %d tokens of %d sequences, value heads of %d, a state stride of %ld", n_tokens, n_seqs, dv, state_ld);
+    int RG = 0;
+    const int rpt = pick_rpt(d, &RG, (long)n_seqs * H >= 512);
+    if (!rpt || d > 256) return gfb_fail("gfb_delta_decode: a state of %d rows per head does not fit a lane's registers", d);
+    const int cols = SCAN_WARPS * (32 / RG) * 4;
+    const unsigned slices = (unsigned)((dv + cols - 1) / cols);
+    if (H > 65535 || slices > 65535) return gfb_fail("gfb_delta_decode: %d heads of %d columns exceed the grid limit", H, dv);
+    const size_t smem = (3 * (size_t)d + (size_t)cols * RG) * sizeof(float);
+    GfbBatch b{cu_seqlens, tok_seq, slots, lengths, n_seqs, n_tokens};
+    cudaError_t e;
+#define GO(TD, R)                                                                                                                              \
+    e = gfb_launch(delta_decode_kernel<TD, R>, dim3(n_seqs, H, slices), dim3(32 * SCAN_WARPS), smem, stream, qkv, ldq, q_off, k_off, v_off, (const TD*)beta_raw, \
+                   ld_b, beta_off, a_raw, ld_a, a_off, dt_bias, a_log, w_dt, state, (size_t)state_ld, out, b, H, KH, d, dv, q_scale, unit_eps, RG, head_decay)
+    if (b_dt == GFB_BF16) { if (rpt == 8) GO(__nv_bfloat16, 8); else GO(__nv_bfloat16, 16); }
+    else if (b_dt == GFB_F32) { if (rpt == 8) GO(float, 8); else GO(float, 16); }
+    else return gfb_fail("gfb_delta_decode: unknown type %d", b_dt);
+#undef GO
+    return gfb_check(e, "gfb_delta_decode");
+}
+
+// As gfb_ssd_scan where every sequence of the step has exactly one token: columns a multiple of four, a 16-byte aligned state with
+// state_ld % 4 == 0.
+GFB_API int gfb_ssd_decode(const float* x, int ldx, int b_off, int c_off, const void* dt_raw, int dt_dt, int ld_dt, int dt_off, const void* dt_bias,
+                           const void* a_log, const void* skip, int w_dt, float* state, long state_ld, float* out, const int* cu_seqlens,
+                           const int* tok_seq, const int* slots, const int* lengths, int n_seqs, int n_tokens, int H, int P, int N, int G,
+                           cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (G <= 0 || H % G) return gfb_fail("gfb_ssd_decode: %d heads do not divide into %d groups", H, G);
+    if (n_tokens != n_seqs || P % 4 || state_ld % 4 || ((uintptr_t)state & 15)) return gfb_fail("gfb_ssd_decode: %d tokens of %d sequences, %d columns, a state stride of %ld", n_tokens, n_seqs, P, state_ld);
+    int RG = 0;
+    const int rpt = pick_rpt(N, &RG, (long)n_seqs * H >= 512);
+    if (!rpt || rpt > 16) return gfb_fail("gfb_ssd_decode: a state of %d rows per head does not fit a lane's registers", N);
+    const int cols = SCAN_WARPS * (32 / RG) * 4;
+    const unsigned slices = (unsigned)((P + cols - 1) / cols);
+    if (H > 65535 || slices > 65535) return gfb_fail("gfb_ssd_decode: %d heads of %d columns exceed the grid limit", H, P);
+    GfbBatch b{cu_seqlens, tok_seq, slots, lengths, n_seqs, n_tokens};
+    cudaError_t e;
+#define GO(TD, R)                                                                                                                              \
+    e = gfb_launch(ssd_decode_kernel<TD, R>, dim3(n_seqs, H, slices), dim3(32 * SCAN_WARPS), 0, stream, x, ldx, b_off, c_off, (const TD*)dt_raw, ld_dt, dt_off, \
+                   dt_bias, a_log, skip, w_dt, state, (size_t)state_ld, out, b, H, P, N, G, RG)
+    if (dt_dt == GFB_BF16) { if (rpt == 8) GO(__nv_bfloat16, 8); else GO(__nv_bfloat16, 16); }
+    else if (dt_dt == GFB_F32) { if (rpt == 8) GO(float, 8); else GO(float, 16); }
+    else return gfb_fail("gfb_ssd_decode: unknown type %d", dt_dt);
+#undef GO
+    return gfb_check(e, "gfb_ssd_decode");
+}
+
 // ------------------------------------------------------------------------------ gated group norm ----
 // One warp per (token, group of `gs` columns), or one block for a large group (BLOCK): v = y, times act(gate) first if
 // gate_first; n = v / sqrt(mean(v^2) + eps) * weight[col % w_len]; times act(gate) behind the norm otherwise.

@@ -545,6 +545,10 @@ class CudaKernels:
                               c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
                               _ptr(out), _ptr(scratch), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state),
                               c_int(n_groups), _stream())
+        if batch.max_q_len == 1 and T == batch.n_seqs and n_state <= 512 and head_dim % 4 == 0 and state.shape[1] % 4 == 0 and sp.value % 16 == 0:
+            return self._call("recurrent", "gfb_ssd_decode", _ptr(x), c_int(x.shape[1]), c_int(b_off), c_int(c_off), _ptr(dt_src), c_int(_dt(dt_src)),
+                              c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
+                              _ptr(out), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups), _stream())
         self._call("recurrent", "gfb_ssd_scan", _ptr(x), c_int(x.shape[1]), c_int(b_off), c_int(c_off), _ptr(dt_src), c_int(_dt(dt_src)),
                    c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
                    _ptr(out), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups), _stream())
@@ -579,6 +583,12 @@ class CudaKernels:
                               c_int(a_src.shape[1]), c_int(a_off), _ptr(dt_bias), _ptr(a_log), c_int(_dt(dt_bias)), sp, sld, _ptr(out),
                               _ptr(scratch), *self._batch_args(batch), c_int(n_head), c_int(n_qk), c_int(head_dim), c_int(v_head_dim),
                               c_float(q_scale), c_float(unit_eps), c_int(1 if head_decay else 0), _stream())
+        if batch.max_q_len == 1 and T == batch.n_seqs and head_dim <= 256 and v_head_dim % 4 == 0 and state.shape[1] % 4 == 0 and sp.value % 16 == 0:
+            return self._call("recurrent", "gfb_delta_decode", _ptr(qkv), c_int(qkv.shape[1]), c_int(q_off), c_int(k_off), c_int(v_off),
+                              _ptr(beta_src), c_int(_dt(beta_src)), c_int(beta_src.shape[1]), c_int(beta_off), _ptr(a_src),
+                              c_int(a_src.shape[1]), c_int(a_off), _ptr(dt_bias), _ptr(a_log), c_int(_dt(dt_bias)), sp, sld, _ptr(out),
+                              *self._batch_args(batch), c_int(n_head), c_int(n_qk), c_int(head_dim), c_int(v_head_dim), c_float(q_scale),
+                              c_float(unit_eps), c_int(1 if head_decay else 0), _stream())
         self._call("recurrent", "gfb_delta_rule", _ptr(qkv), c_int(qkv.shape[1]), c_int(q_off), c_int(k_off), c_int(v_off),
                    _ptr(beta_src), c_int(_dt(beta_src)), c_int(beta_src.shape[1]), c_int(beta_off), _ptr(a_src), c_int(a_src.shape[1]),
                    c_int(a_off), _ptr(dt_bias), _ptr(a_log), c_int(_dt(dt_bias)), sp, sld, _ptr(out), *self._batch_args(batch),
