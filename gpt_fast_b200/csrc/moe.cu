@@ -47,12 +47,14 @@ struct RouteArgs {
     int mode, groups, keep, group_terms, shared;
 };
 
-// one token's choice by one warp: `logits` are the token's E router logits
+// one token's choice by one warp: `logits` are the token's E router logits.  EPL experts per lane (E <= 32 EPL): every step of the choice
+// walks over a lane's experts, so the usual 8 to 32 of them are not walked over as 512.
+template <int EPL>
 __device__ __forceinline__ void route_token(const float* __restrict__ logits, const void* __restrict__ correction, int c_dt,
                                             const RouteArgs& ra, int* __restrict__ idx, float* __restrict__ weights, int lane) {
     const int E = ra.E, top = ra.top, mode = ra.mode;
     const float scale = ra.scale;
-    float s[MAX_EPL], c[MAX_EPL];
+    float s[EPL], c[EPL];
     float z_max = -INFINITY, z_inv = 0.f;
     if (mode == ROUTE_SOFTMAX) {
         for (int e = lane; e < E; e += 32) z_max = fmaxf(z_max, logits[e]);
@@ -62,7 +64,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
         z_inv = 1.0f / gfb_warp_sum(sum);
     }
 #pragma unroll
-    for (int i = 0; i < MAX_EPL; i++) {
+    for (int i = 0; i < EPL; i++) {
         const int e = lane + 32 * i;
         if (e < E) {
             s[i] = mode == ROUTE_SOFTMAX_TOP ? logits[e] : mode == ROUTE_SOFTMAX ? expf(logits[e] - z_max) * z_inv : sigmoid_f(logits[e]);
@@ -80,7 +82,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
         for (int g = 0; g < ra.groups; g++) {
             float m = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < MAX_EPL; i++)
+            for (int i = 0; i < EPL; i++)
                 if ((lane + 32 * i) / per == g) m = fmaxf(m, c[i]);            // (experts beyond E are -inf)
             const float top1 = gfb_warp_max(m);
             if (ra.group_terms > 1 && per > 1) {
@@ -89,7 +91,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
                 float second = -INFINITY;
                 bool skip = lane == holder;
 #pragma unroll
-                for (int i = 0; i < MAX_EPL; i++)
+                for (int i = 0; i < EPL; i++)
                     if ((lane + 32 * i) / per == g) {
                         if (skip && c[i] == top1) skip = false;
                         else second = fmaxf(second, c[i]);
@@ -113,7 +115,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
             if (best_g < 32) kept |= 1u << best_g;
         }
 #pragma unroll
-        for (int i = 0; i < MAX_EPL; i++) {
+        for (int i = 0; i < EPL; i++) {
             const int e = lane + 32 * i;
             if (e < E && !(kept >> (e / per) & 1u)) c[i] = -INFINITY;
         }
@@ -125,7 +127,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
         float best = -INFINITY, best_s = 0.f;
         int best_e = 0x7fffffff;
 #pragma unroll
-        for (int i = 0; i < MAX_EPL; i++)
+        for (int i = 0; i < EPL; i++)
             if (c[i] > best) { best = c[i]; best_e = lane + 32 * i; best_s = s[i]; }     // ascending e per lane: the lowest index wins a tie
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -134,7 +136,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
             if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; best_s = os; }
         }
 #pragma unroll
-        for (int i = 0; i < MAX_EPL; i++)
+        for (int i = 0; i < EPL; i++)
             if (lane + 32 * i == best_e) c[i] = -INFINITY;
         if (mode == ROUTE_SOFTMAX_TOP) {
             if (r == 0) first = best_s;
@@ -162,6 +164,7 @@ static int check_route(const RouteArgs& ra, const char* what) {
     return 0;
 }
 
+template <int EPL>
 __global__ void __launch_bounds__(32 * ROUTE_WARPS)
 moe_route_kernel(const float* __restrict__ logits, int ld, const void* __restrict__ correction, int c_dt, RouteArgs ra,
                  int* __restrict__ idx, float* __restrict__ weights, int T) {
@@ -171,7 +174,7 @@ moe_route_kernel(const float* __restrict__ logits, int ld, const void* __restric
     const int t = blockIdx.x * ROUTE_WARPS + (threadIdx.x >> 5);
     if (t >= T) return;
     const size_t at = (size_t)t * (ra.top + ra.shared);
-    route_token(logits + (size_t)t * ld, correction, c_dt, ra, idx + at, weights + at, lane);
+    route_token<EPL>(logits + (size_t)t * ld, correction, c_dt, ra, idx + at, weights + at, lane);
 }
 
 // idx int32 and weights float32 [T, top + shared]
@@ -180,8 +183,13 @@ GFB_API int gfb_moe_route(const float* logits, int ld, const void* correction, i
     if (T <= 0) return 0;
     const RouteArgs ra{E, top, scale, mode, groups, keep, group_terms, shared ? 1 : 0};
     if (check_route(ra, "gfb_moe_route")) return 1;
-    cudaError_t e = gfb_launch(moe_route_kernel, dim3((T + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(32 * ROUTE_WARPS), 0, stream, logits, ld,
-                               correction, c_dt, ra, idx, weights, T);
+    cudaError_t e;
+#define GO(EPL) e = gfb_launch(moe_route_kernel<EPL>, dim3((T + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(32 * ROUTE_WARPS), 0, stream, logits, ld, \
+                               correction, c_dt, ra, idx, weights, T)
+    if (E <= 32) GO(1);
+    else if (E <= 128) GO(4);
+    else GO(MAX_EPL);
+#undef GO
     return gfb_check(e, "gfb_moe_route");
 }
 
@@ -217,7 +225,7 @@ __device__ __forceinline__ bool rows_wide(const T* base, int n) {
 // staged in shared memory in 32-bit) and its first warp chooses.
 constexpr int ROUTER_WARPS = 8;
 
-template <typename T>
+template <typename T, int EPL>
 __global__ void __launch_bounds__(32 * ROUTER_WARPS)
 moe_router_kernel(const T* __restrict__ h, const T* __restrict__ router, const void* __restrict__ correction, int c_dt, RouteArgs ra,
                   int* __restrict__ idx, float* __restrict__ weights, int D, int n_extra, float* __restrict__ extra) {
@@ -240,10 +248,78 @@ moe_router_kernel(const T* __restrict__ h, const T* __restrict__ router, const v
     }
     __syncthreads();
     const size_t at = (size_t)t * (ra.top + ra.shared);
-    if (warp == 0) route_token(z, correction, c_dt, ra, idx + at, weights + at, lane);
+    if (warp == 0) route_token<EPL>(z, correction, c_dt, ra, idx + at, weights + at, lane);
 }
 
-// h [T, D] and router [>= E + n_extra, D] of type dt (further rows are padding); few tokens only: a block per token.
+// Prompts: a block takes ROUTER_TOKENS tokens, whose inputs sit in shared memory as they are, and a warp takes two of the router's rows at a
+// time against all of them (sums in row_dot's order, so a token's logits are the same bits as alone); then a warp chooses for each token.
+// What bounds it is the conversions and FMAs of a warp's row pair: 2,048 tokens of 2,048 for 16 experts 16.9 us
+// (the product on the tensor cores, zero-padded to 128 columns, and the choice behind it took 19 + 11.1 us and a launch between them).
+constexpr int ROUTER_TOKENS = 8;
+
+template <typename T, int EPL>
+__global__ void __launch_bounds__(32 * ROUTER_WARPS)
+moe_router_tokens_kernel(const T* __restrict__ h, const T* __restrict__ router, const void* __restrict__ correction, int c_dt, RouteArgs ra,
+                         int* __restrict__ idx, float* __restrict__ weights, int n_tokens, int D, int n_extra, float* __restrict__ extra) {
+    constexpr int N = Vec<T>::N;
+    const int E = ra.E, rows = E + n_extra;
+    extern __shared__ __align__(16) unsigned char rt_raw[];      // the inputs [ROUTER_TOKENS][D], then the logits [ROUTER_TOKENS][rows]
+    T* hs = reinterpret_cast<T*>(rt_raw);
+    float* z = reinterpret_cast<float*>(rt_raw + (size_t)ROUTER_TOKENS * D * sizeof(T));
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t0 = blockIdx.x * ROUTER_TOKENS, nt = min(ROUTER_TOKENS, n_tokens - t0);
+#pragma unroll 4
+    for (int i = threadIdx.x * N; i < ROUTER_TOKENS * D; i += blockDim.x * N)         // (rows are side by side and whole 16-byte pieces)
+        *reinterpret_cast<uint4*>(hs + i) = i < nt * D ? *reinterpret_cast<const uint4*>(h + (size_t)t0 * D + i) : make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (int e = warp; e < rows; e += 2 * ROUTER_WARPS) {
+        const bool two = e + ROUTER_WARPS < rows;
+        const T* row[2] = {router + (size_t)e * D, router + (size_t)(two ? e + ROUTER_WARPS : e) * D};
+        float acc[2][ROUTER_TOKENS];
+#pragma unroll
+        for (int t = 0; t < ROUTER_TOKENS; t++) acc[0][t] = acc[1][t] = 0.f;
+#pragma unroll 2
+        for (int c = lane * N; c < D; c += 32 * N) {
+            const uint4 r0 = *reinterpret_cast<const uint4*>(row[0] + c), r1 = *reinterpret_cast<const uint4*>(row[1] + c);
+            float w[2][N];
+#pragma unroll
+            for (int k = 0; k < N; k++) { w[0][k] = gfb_to_f32(reinterpret_cast<const T*>(&r0)[k]); w[1][k] = gfb_to_f32(reinterpret_cast<const T*>(&r1)[k]); }
+#pragma unroll
+            for (int t = 0; t < ROUTER_TOKENS; t++) {
+                const uint4 hv = *reinterpret_cast<const uint4*>(hs + (size_t)t * D + c);
+#pragma unroll
+                for (int k = 0; k < N; k++) {
+                    const float v = gfb_to_f32(reinterpret_cast<const T*>(&hv)[k]);
+                    acc[0][t] = fmaf(w[0][k], v, acc[0][t]);
+                    acc[1][t] = fmaf(w[1][k], v, acc[1][t]);
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (k == 1 && !two) break;
+            const int ee = e + k * ROUTER_WARPS;
+#pragma unroll
+            for (int t = 0; t < ROUTER_TOKENS; t++) {
+                const float d = gfb_warp_sum(acc[k][t]);
+                if (lane == 0) {
+                    z[t * rows + ee] = d;
+                    if (ee >= E && t < nt) extra[(size_t)(t0 + t) * n_extra + (ee - E)] = d;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int t = warp; t < nt; t += ROUTER_WARPS) {
+        const size_t at = (size_t)(t0 + t) * (ra.top + ra.shared);
+        route_token<EPL>(z + t * rows, correction, c_dt, ra, idx + at, weights + at, lane);
+    }
+}
+
+// h [T, D] and router [>= E + n_extra, D] of type dt (further rows are padding).  Up to 64 tokens: a block per token; beyond, rows of whole
+// 16-byte pieces whose eight inputs fit shared memory: a block per eight tokens; other rows are refused.
 // The logits of the n_extra rows behind the experts' go to extra float32 [T, n_extra].
 GFB_API int gfb_moe_router(const void* h, const void* router, int dt, const void* correction, int c_dt, int E, int top, float scale,
                            int* idx, float* weights, int T, int D, int mode, int groups, int keep, int group_terms, int shared, int n_extra, float* extra,
@@ -252,16 +328,31 @@ GFB_API int gfb_moe_router(const void* h, const void* router, int dt, const void
     const RouteArgs ra{E, top, scale, mode, groups, keep, group_terms, shared ? 1 : 0};
     if (check_route(ra, "gfb_moe_router")) return 1;
     if (n_extra < 0 || (n_extra > 0 && extra == nullptr)) return gfb_fail("gfb_moe_router: %d further rows without a place for their logits", n_extra);
-    const size_t smem = (size_t)(D + E + n_extra) * sizeof(float);
-    if (smem > 48 * 1024) return gfb_fail("gfb_moe_router: %zu bytes of shared memory", smem);
-    cudaError_t e;
-    if (dt == GFB_BF16)
-        e = gfb_launch(moe_router_kernel<__nv_bfloat16>, dim3((unsigned)T), dim3(32 * ROUTER_WARPS), smem, stream, (const __nv_bfloat16*)h,
-                       (const __nv_bfloat16*)router, correction, c_dt, ra, idx, weights, D, n_extra, extra);
-    else if (dt == GFB_F32)
-        e = gfb_launch(moe_router_kernel<float>, dim3((unsigned)T), dim3(32 * ROUTER_WARPS), smem, stream, (const float*)h, (const float*)router,
-                       correction, c_dt, ra, idx, weights, D, n_extra, extra);
+    const bool few = T <= 64;
+    const size_t smem = few ? (size_t)(D + E + n_extra) * sizeof(float)
+                            : ROUTER_TOKENS * ((size_t)D * (dt == GFB_BF16 ? 2 : 4) + (size_t)(E + n_extra) * sizeof(float));
+    if (smem > (few ? 48 : 200) * 1024) return gfb_fail("gfb_moe_router: %zu bytes of shared memory", smem);
+    const int per = dt == GFB_BF16 ? 8 : 4;
+    if (!few && (D % per || (((uintptr_t)h | (uintptr_t)router) & 15))) return gfb_fail("gfb_moe_router: rows of %d numbers are not whole 16-byte pieces", D);
+    cudaError_t e = cudaSuccess;
+#define GO(T_, EPL)                                                                                                                          \
+    do {                                                                                                                                     \
+        if (few) {                                                                                                                           \
+            e = gfb_launch(moe_router_kernel<T_, EPL>, dim3((unsigned)T), dim3(32 * ROUTER_WARPS), smem, stream, (const T_*)h, (const T_*)router, \
+                           correction, c_dt, ra, idx, weights, D, n_extra, extra);                                                           \
+        } else {                                                                                                                             \
+            if (smem > 48 * 1024) e = cudaFuncSetAttribute(moe_router_tokens_kernel<T_, EPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            if (e == cudaSuccess)                                                                                                            \
+                e = gfb_launch(moe_router_tokens_kernel<T_, EPL>, dim3((unsigned)((T + ROUTER_TOKENS - 1) / ROUTER_TOKENS)), dim3(32 * ROUTER_WARPS), \
+                               smem, stream, (const T_*)h, (const T_*)router, correction, c_dt, ra, idx, weights, T, D, n_extra, extra);      \
+        }                                                                                                                                    \
+    } while (0)
+#define PICK(T_) do { if (E <= 32) GO(T_, 1); else if (E <= 128) GO(T_, 4); else GO(T_, MAX_EPL); } while (0)
+    if (dt == GFB_BF16) PICK(__nv_bfloat16);
+    else if (dt == GFB_F32) PICK(float);
     else return gfb_fail("gfb_moe_router: unknown type %d", dt);
+#undef PICK
+#undef GO
     return gfb_check(e, "gfb_moe_router");
 }
 

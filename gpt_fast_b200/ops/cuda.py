@@ -733,7 +733,7 @@ class CudaKernels:
         self._call("moe", "gfb_moe_route", _ptr(logits), c_int(logits.shape[1]), _ptr(correction), c_int(_dt(correction)), c_int(E),
                    c_int(top), c_float(scale), _ptr(idx), _ptr(weights), c_int(T), *self._route_args(score, groups, shared), _stream())
 
-    MOE_ROUTER_FEW_TOKENS = 64         # up to this many tokens the router's product and its choice are one launch
+    MOE_ROUTER_FEW_TOKENS = 64         # up to this many tokens a block per token, beyond it one per eight tokens (rows of whole 16-byte pieces)
 
     def moe_router(self, h, router, correction, top, scale, idx, weights, score="sigmoid", extra=None, groups=(1, 1),
                    shared=False) -> bool:
@@ -741,8 +741,12 @@ class CudaKernels:
         slots = top + (1 if shared else 0)
         E = correction.shape[0]
         n_extra = 0 if extra is None else extra.shape[1]
-        if T > self.MOE_ROUTER_FEW_TOKENS or (D + E + n_extra) * 4 > 48 * 1024:
-            return False
+        if T <= self.MOE_ROUTER_FEW_TOKENS:
+            if (D + E + n_extra) * 4 > 48 * 1024:
+                return False
+        elif (8 * (D * h.element_size() + 4 * (E + n_extra)) > 200 * 1024 or E + n_extra > 128 or D * h.element_size() % 16
+              or (h.data_ptr() | router.data_ptr()) % 16):
+            return False                               # the product on the tensor cores and the choice behind it
         if score not in self._ROUTE_SCORES:
             _fail(f"unknown router score '{score}'")
         if extra is not None:
