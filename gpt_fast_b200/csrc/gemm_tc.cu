@@ -436,8 +436,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         group = gp.tile_group[SWAP ? blockIdx.y : blockIdx.x];     // the tile of tokens
     }
     const bool idle = GROUPED && group < 0;
-    const int xrow0 = GROUPED && SWAP ? group * gp.group_rows + row0 : row0;      // where the weights' rows start
-    const int ycol0 = GROUPED && !SWAP ? group * gp.group_rows + col0 : col0;
+    static_assert(!GROUPED || SWAP, "row tiles with weights of their own are the columns of the MMA here");
+    const int xrow0 = GROUPED ? group * gp.group_rows + row0 : row0;              // where the weights' rows start
 
     if (idle) {
     } else if (warp == 0) {
@@ -451,7 +451,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                     mbar_expect_tx(full, X_TILE_BYTES + Y_TILE_BYTES);
                     if (SWAP) tma_load_2d_hint(xs + i * X_TILE_BYTES, &map_x, (kb0 + i) * BK, xrow0, full, pol);
                     else tma_load_2d(xs + i * X_TILE_BYTES, &map_x, (kb0 + i) * BK, xrow0, full);
-                    tma_load_2d(ys + i * Y_TILE_BYTES, &map_y, (kb0 + i) * BK, ycol0, full);
+                    tma_load_2d(ys + i * Y_TILE_BYTES, &map_y, (kb0 + i) * BK, col0, full);
                 } else if (SWAP) tma_load_2d(ys + i * Y_TILE_BYTES, &map_y, (kb0 + i) * BK, col0, full);
                 else tma_load_2d(xs + i * X_TILE_BYTES, &map_x, (kb0 + i) * BK, row0, full);
             }
@@ -463,7 +463,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                 mbar_expect_tx(full, X_TILE_BYTES + Y_TILE_BYTES);
                 if (SWAP) tma_load_2d_hint(xs + s * X_TILE_BYTES, &map_x, (kb0 + i) * BK, xrow0, full, pol);
                 else tma_load_2d(xs + s * X_TILE_BYTES, &map_x, (kb0 + i) * BK, xrow0, full);
-                tma_load_2d(ys + s * Y_TILE_BYTES, &map_y, (kb0 + i) * BK, ycol0, full);
+                tma_load_2d(ys + s * Y_TILE_BYTES, &map_y, (kb0 + i) * BK, col0, full);
             }
         }
     } else if (warp == 1) {
@@ -1167,10 +1167,10 @@ int launch(const CUtensorMap& mx, const CUtensorMap& my, void* out, float* parti
     return gfb_check(e, "gfb_gemm_tc");
 }
 
-template <int BN, int EPI, typename TO, bool SWAP = false>
+template <int BN, int EPI, typename TO>
 int launch_grouped(const CUtensorMap& mx, const CUtensorMap& my, void* out, int R, int Cc, int K, int ldo, int stages, int* status,
                    const Groups& gp, cudaStream_t stream) {
-    auto kern = gemm_tc_kernel<BN, SWAP, EPI, TO, true>;
+    auto kern = gemm_tc_kernel<BN, true, EPI, TO, true>;
     size_t smem = smem_bytes(BN, stages);
     static size_t configured = 0;
     if (smem > configured) {
@@ -1382,16 +1382,15 @@ GFB_API int gfb_gemm_tc(const void* A, const void* W, void* out, int out_dt, int
 
 // Row tiles that each use one of `groups` weight matrices: out[r] = A[r] * W[tile_group[r / tile_rows]]^T for A [rows, K]
 // (rows a multiple of tile_rows), W [groups, N, K].  tile_rows 16, 32, 64: the swapped orientation of a decode step (128 weight
-// rows x a tile of tokens per block); 128: 128 tokens x 128 or 64 weight rows per block; in both a tile whose entry is negative is
-// skipped.  tile_rows 256: pairs of SMs walk over the first *tiles_used row tiles (the entries with rows come first).
+// rows x a tile of tokens per block); a tile whose entry is negative is skipped.  tile_rows 256: pairs of SMs walk over the first *tiles_used row tiles (the entries with rows come first).
 // epi: EPI_STORE with out float32 [rows, N], EPI_GLU_CLAMP with out bfloat16 [rows, N / 2] from alternating gate/up
 // rows of W, or EPI_RELU2 with out bfloat16 [rows, N].
 GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out_dt, int rows, int tile_rows, int groups, int N, int K,
                                 int epi, const int* tile_group, const int* tiles_used, float limit, float alpha, float shift,
                                 int* status, cudaStream_t stream) {
     if (rows <= 0 || N <= 0 || groups <= 0) return 0;
-    if ((tile_rows != 16 && tile_rows != 32 && tile_rows != 64 && tile_rows != 128 && tile_rows != 256) || rows % tile_rows)
-        return gfb_fail("gfb_gemm_tc_grouped: %d rows in tiles of %d (16 to 256 rows, whole tiles)", rows, tile_rows);
+    if ((tile_rows != 16 && tile_rows != 32 && tile_rows != 64 && tile_rows != 256) || rows % tile_rows)
+        return gfb_fail("gfb_gemm_tc_grouped: %d rows in tiles of %d (16, 32, 64 or 256 rows, whole tiles)", rows, tile_rows);
     if (tile_rows == 256 && tiles_used == nullptr) return gfb_fail("gfb_gemm_tc_grouped: tiles of 256 rows need the count of tiles with rows");
     if (K <= 0 || K % 8) return gfb_fail("gfb_gemm_tc_grouped: K = %d must be a positive multiple of 8 (16-byte rows for TMA)", K);
     if (N % 8) return gfb_fail("gfb_gemm_tc_grouped: N = %d must be a multiple of 8", N);
@@ -1400,7 +1399,7 @@ GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out
     if ((long)groups * N > 0x7fffffffL) return gfb_fail("gfb_gemm_tc_grouped: %d matrices of %d rows exceed a tensor map's coordinates", groups, N);
     const Groups gp{tile_group, N, limit, alpha, shift, tiles_used};
     CUtensorMap mx, my;
-    if (tile_rows < 128) {
+    if (tile_rows < 256) {
         // few tokens per group: the weights' rows are the rows of the MMA, a tile of tokens its columns
         // rings short enough for two blocks per SM: one block's set-up and epilogue hide behind the other's stream of weights
         int STAGES = (100 * 1024) / (X_TILE_BYTES + tile_rows * BK * 2);
@@ -1410,9 +1409,9 @@ GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out
         const bool glu = epi == EPI_GLU_CLAMP && out_dt == GFB_BF16, store = epi == EPI_STORE && out_dt == GFB_F32;
         const bool relu2 = epi == EPI_RELU2 && out_dt == GFB_BF16;
         const int ldo = glu ? N / 2 : N;
-#define GS(B) return relu2 ? launch_grouped<B, EPI_RELU2, __nv_bfloat16, true>(mx, my, out, N, rows, K, ldo, STAGES, status, gp, stream) \
-                         : glu ? launch_grouped<B, EPI_GLU_CLAMP, __nv_bfloat16, true>(mx, my, out, N, rows, K, ldo, STAGES, status, gp, stream) \
-                         : launch_grouped<B, EPI_STORE, float, true>(mx, my, out, N, rows, K, ldo, STAGES, status, gp, stream)
+#define GS(B) return relu2 ? launch_grouped<B, EPI_RELU2, __nv_bfloat16>(mx, my, out, N, rows, K, ldo, STAGES, status, gp, stream) \
+                         : glu ? launch_grouped<B, EPI_GLU_CLAMP, __nv_bfloat16>(mx, my, out, N, rows, K, ldo, STAGES, status, gp, stream) \
+                         : launch_grouped<B, EPI_STORE, float>(mx, my, out, N, rows, K, ldo, STAGES, status, gp, stream)
         if (glu || store || relu2) {
             if (tile_rows == 16) GS(16);
             if (tile_rows == 32) GS(32);
@@ -1422,29 +1421,12 @@ GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out
         return gfb_fail("gfb_gemm_tc_grouped: unsupported epilogue %d / output type %d", epi, out_dt);
     }
     if (make_map(&mx, A, rows, K, BM)) return 1;
-    if (tile_rows == 256) {
-        if (make_map(&my, W, groups * N, K, 128)) return 1;
-        if (epi == EPI_GLU_CLAMP && out_dt == GFB_BF16)
-            return launch_pair_grouped<EPI_GLU_CLAMP, __nv_bfloat16>(mx, my, out, rows, N, K, N / 2, status, gp, stream);
-        if (epi == EPI_RELU2 && out_dt == GFB_BF16)
-            return launch_pair_grouped<EPI_RELU2, __nv_bfloat16>(mx, my, out, rows, N, K, N, status, gp, stream);
-        if (epi == EPI_STORE && out_dt == GFB_F32)
-            return launch_pair_grouped<EPI_STORE, float>(mx, my, out, rows, N, K, N, status, gp, stream);
-        return gfb_fail("gfb_gemm_tc_grouped: unsupported epilogue %d / output type %d", epi, out_dt);
-    }
-    // Few row tiles (a decode step) are bound by the stream of weights: tiles of 64 columns then give twice the blocks,
-    // each with its own ring of copies in flight.
-    constexpr int STAGES = 6;
-    const bool narrow = (long)(rows / BM) * ((N + 127) / 128) < 2 * 148;
-    if (make_map(&my, W, groups * N, K, narrow ? 64 : 128)) return 1;
+    if (make_map(&my, W, groups * N, K, 128)) return 1;
     if (epi == EPI_GLU_CLAMP && out_dt == GFB_BF16)
-        return narrow ? launch_grouped<64, EPI_GLU_CLAMP, __nv_bfloat16>(mx, my, out, rows, N, K, N / 2, STAGES, status, gp, stream)
-                      : launch_grouped<128, EPI_GLU_CLAMP, __nv_bfloat16>(mx, my, out, rows, N, K, N / 2, STAGES, status, gp, stream);
+        return launch_pair_grouped<EPI_GLU_CLAMP, __nv_bfloat16>(mx, my, out, rows, N, K, N / 2, status, gp, stream);
     if (epi == EPI_RELU2 && out_dt == GFB_BF16)
-        return narrow ? launch_grouped<64, EPI_RELU2, __nv_bfloat16>(mx, my, out, rows, N, K, N, STAGES, status, gp, stream)
-                      : launch_grouped<128, EPI_RELU2, __nv_bfloat16>(mx, my, out, rows, N, K, N, STAGES, status, gp, stream);
+        return launch_pair_grouped<EPI_RELU2, __nv_bfloat16>(mx, my, out, rows, N, K, N, status, gp, stream);
     if (epi == EPI_STORE && out_dt == GFB_F32)
-        return narrow ? launch_grouped<64, EPI_STORE, float>(mx, my, out, rows, N, K, N, STAGES, status, gp, stream)
-                      : launch_grouped<128, EPI_STORE, float>(mx, my, out, rows, N, K, N, STAGES, status, gp, stream);
+        return launch_pair_grouped<EPI_STORE, float>(mx, my, out, rows, N, K, N, status, gp, stream);
     return gfb_fail("gfb_gemm_tc_grouped: unsupported epilogue %d / output type %d", epi, out_dt);
 }

@@ -704,10 +704,11 @@ class CudaKernels:
 
     # -- mixture of experts ------------------------------------------------------------------
     MOE_TILE_ROWS = 64                 # rows of a tile of the sorted form on CUDA cores
-    MOE_TC_TILE_ROWS = 128             # ... and on the tensor cores (the rows of one MMA)
     MOE_FEW_TOKENS = 32                # up to this many tokens a warp per output number streams the weight rows (CUDA-core forms)
     MOE_TC_FEW_TOKENS = 0              # ... where the tensor-core tiles run: they stream a chosen expert's weights once per step by TMA
-    MOE_PAIR_ROWS_PER_EXPERT = 384     # (token, expert) pairs per expert from which the row tiles have 256 rows
+    # (token, expert) pairs per expert from which a prompt's row tiles have 256 rows, for pairs of SMs, and not 64.  16 experts of 1,792 x 2,048,
+    # us with 64 | 256: 64 pairs each 142 | 149, 128 158 | 144, 256 226 | 165; 32 of 768 x 2,048: 64 119 | 140, 128 160 | 150, 256 237 | 200
+    MOE_PAIR_ROWS_PER_EXPERT = 128
     _EPI_GLU_CLAMP = 8
 
     _ROUTE_SCORES = {"sigmoid": 0, "softmax_top": 1, "softmax": 2, "sigmoid_plain": 3}
@@ -780,14 +781,13 @@ class CudaKernels:
         dt = c_int(_dt(h))
         sizes = (c_int(T), c_int(top), c_int(E), c_int(F), c_int(D))
         if h.dtype == torch.bfloat16 and T > self.MOE_TC_FEW_TOKENS and D % 8 == 0 and F % 8 == 0 and E * max(N1, D) < 2 ** 31:
-            # sorted by expert in tiles of 128 rows, both products on the tensor cores: gather the rows, gate/up with the
+            # sorted by expert in tiles, both products on the tensor cores: gather the rows, gate/up with the
             # activation in the epilogue, down into 32-bit rows, then the weighted sum into the stream in pair order
             pairs = T * top
-            # from about two full tiles per expert on: tiles of 256 rows for pairs of SMs (tcgen05 cta_group::2)
             # a decode step: an expert has at most T rows, so tiles of at least T rows (the columns of the swapped MMA) read
-            # every chosen expert's weights exactly once
-            rows = (16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else
-                    self.MOE_TC_TILE_ROWS * (2 if pairs >= self.MOE_PAIR_ROWS_PER_EXPERT * E else 1))
+            # every chosen expert's weights exactly once; prompts of many rows per expert: tiles of 256 rows for pairs of SMs
+            # (tcgen05 cta_group::2)
+            rows = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 or pairs < self.MOE_PAIR_ROWS_PER_EXPERT * E else 256
             tiles = (pairs + min(E, pairs) * (rows - 1)) // rows
             plan = torch.empty(tiles * rows + pairs + tiles + 1, dtype=torch.int32, device=h.device)
             row_pair, pair_row = plan[:tiles * rows], plan[tiles * rows:tiles * rows + pairs]
