@@ -22,7 +22,7 @@
 // 16 bytes per lane and load, the token's input staged in shared memory.  Many tokens (a prompt): the pairs are sorted by
 // expert (gfb_moe_plan: each expert's rows padded to whole tiles) and the products run tile by tile, each tile with its
 // expert's weights, the rows' results brought back to pair order.  The tiles run on the tensor cores (bfloat16: the
-// grouped product of the tcgen05 library between gfb_moe_gather_rows and gfb_moe_combine_rows, tiles of 128 rows) or on
+// grouped product of the tcgen05 library between gfb_moe_gather_rows and gfb_moe_combine_rows, tiles of 16 to 256 rows) or on
 // CUDA cores (32-bit, and shapes the tensor-core tiles do not take: moe_tiles_simt_kernel, tiles of 64 rows).  In every
 // form a number is one sum over k in 32-bit in an order that does not depend on the other rows, so a token's result does
 // not depend on what else is in the batch.
@@ -216,13 +216,34 @@ __device__ __forceinline__ float row_dot(const T* __restrict__ row, const float*
     return gfb_warp_sum(acc);
 }
 
+// row_dot (its sums in the same order) of two rows of whole aligned 16-byte pieces
+template <typename T>
+__device__ __forceinline__ void two_rows_dot(const T* __restrict__ row0, const T* __restrict__ row1, const float* __restrict__ v, int n, int lane,
+                                             float (&out)[2]) {
+    constexpr int N = Vec<T>::N;
+    float a0 = 0.f, a1 = 0.f;
+#pragma unroll 4
+    for (int c = lane * N; c < n; c += 32 * N) {
+        const uint4 r0 = *reinterpret_cast<const uint4*>(row0 + c), r1 = *reinterpret_cast<const uint4*>(row1 + c);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            a0 = fmaf(gfb_to_f32(reinterpret_cast<const T*>(&r0)[i]), v[c + i], a0);
+            a1 = fmaf(gfb_to_f32(reinterpret_cast<const T*>(&r1)[i]), v[c + i], a1);
+        }
+    }
+    out[0] = gfb_warp_sum(a0);
+    out[1] = gfb_warp_sum(a1);
+}
+
 template <typename T>
 __device__ __forceinline__ bool rows_wide(const T* base, int n) {
     return n % Vec<T>::N == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
 }
 
-// A decode step's router in one launch: a block per token computes the E logits (a warp per expert row, the token's input
-// staged in shared memory in 32-bit) and its first warp chooses.
+// A decode step's router in one launch: a block per token computes the E logits (a warp per two expert rows, the token's input staged in
+// shared memory in 32-bit) and its first warp chooses.  What bounds it is latency: the rows are weights, so they are asked into L2 before the
+// wait for the kernel ahead, and eight 16-byte loads of a lane are in flight at once.  8 tokens of 2,048 for 16 experts, alone and
+// with cold caches: one load at a time 11.7 us, 11.3 so.
 constexpr int ROUTER_WARPS = 8;
 
 template <typename T, int EPL>
@@ -234,17 +255,29 @@ moe_router_kernel(const T* __restrict__ h, const T* __restrict__ router, const v
     float* z = rs + D;
     gfb_pdl_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = blockIdx.x;
+    const int t = blockIdx.x, rows = E + n_extra;
+    for (int e = warp; e < rows; e += ROUTER_WARPS)
+        for (int c = lane * (128 / (int)sizeof(T)); c < D; c += 32 * (128 / (int)sizeof(T)))
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(router + (size_t)e * D + c));
     gfb_pdl_wait();
     for (int i = threadIdx.x; i < D; i += blockDim.x) rs[i] = gfb_to_f32(h[(size_t)t * D + i]);
     __syncthreads();
     const bool wide = rows_wide(router, D);
-    for (int e = warp; e < E + n_extra; e += ROUTER_WARPS) {
-        const float d = row_dot(router + (size_t)e * D, rs, D, lane, wide);
-        if (lane == 0) {
-            z[e] = d;
-            if (e >= E) extra[(size_t)t * n_extra + (e - E)] = d;      // rows behind the experts': their logits are handed out as they are
+    for (int e = warp; e < rows; e += 2 * ROUTER_WARPS) {
+        const int n = e + ROUTER_WARPS < rows ? 2 : 1;
+        float d[2];
+        if (wide) {
+            two_rows_dot(router + (size_t)e * D, router + (size_t)(e + (n - 1) * ROUTER_WARPS) * D, rs, D, lane, d);
+        } else {
+            d[0] = row_dot(router + (size_t)e * D, rs, D, lane, false);
+            if (n == 2) d[1] = row_dot(router + (size_t)(e + ROUTER_WARPS) * D, rs, D, lane, false);
         }
+        if (lane == 0)
+            for (int k = 0; k < n; k++) {
+                const int ee = e + k * ROUTER_WARPS;
+                z[ee] = d[k];
+                if (ee >= E) extra[(size_t)t * n_extra + (ee - E)] = d[k];     // rows behind the experts': their logits are handed out as they are
+            }
     }
     __syncthreads();
     const size_t at = (size_t)t * (ra.top + ra.shared);
@@ -614,6 +647,98 @@ GFB_API int gfb_moe_gather_rows(const void* h, const int* row_pair, void* hs, in
     cudaError_t e = gfb_launch(moe_gather_rows_kernel, dim3((unsigned)rows), dim3(128), 0, stream, (const uint4*)h, row_pair, (uint4*)hs, top,
                                D / 8);
     return gfb_check(e, "gfb_moe_gather_rows");
+}
+
+// The plan and the gathered rows of a step of few pairs in one launch: a block per tile (and quarter of its columns) counts the pairs by
+// expert for itself, finds its tile's expert in the scan of the counts, lists that expert's pairs in their order and copies their rows.  What
+// bounds a decode step here is the chain of launches: 24 pairs of 17 experts, rows of 2,048, took 5.5 + 3.5 us as two, 4.9 us so.
+constexpr int PLAN_FEW_PAIRS = 1024, PLAN_FEW_EXPERTS = 1024, PLAN_FEW_ROWS = 64;
+
+__global__ void __launch_bounds__(256)
+moe_plan_gather_kernel(const int* __restrict__ idx, int n_pairs, int E, int tile_rows, const uint4* __restrict__ h, uint4* __restrict__ hs, int top,
+                       int vec_per_row, int* __restrict__ row_pair, int* __restrict__ pair_row, int* __restrict__ tile_expert,
+                       int* __restrict__ tiles_used) {
+    __shared__ int experts[PLAN_FEW_PAIRS], count[PLAN_FEW_EXPERTS], mine[PLAN_FEW_ROWS], my_expert, my_first, total;
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    const int tid = threadIdx.x, lane = tid & 31, tile = blockIdx.x;
+    const bool writer = blockIdx.y == 0;             // one of a tile's blocks writes the plan
+    for (int e = tid; e < E; e += blockDim.x) count[e] = 0;
+    if (tid < tile_rows) mine[tid] = -1;
+    if (tid == 0) my_expert = -1;
+    __syncthreads();
+    for (int p = tid; p < n_pairs; p += blockDim.x) {
+        const int e = idx[p];
+        const bool valid = e >= 0 && e < E;
+        experts[p] = valid ? e : -1;
+        if (valid) atomicAdd(&count[e], 1);
+        else if (writer && tile == 0) pair_row[p] = -1;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int at = 0;                                  // tiles of the experts so far
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane, tiles = e < E ? (count[e] + tile_rows - 1) / tile_rows : 0;
+            int sum = tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += v;
+            }
+            const int first = at + sum - tiles;
+            if (tile >= first && tile < first + tiles) { my_expert = e; my_first = (tile - first) * tile_rows; }
+            at += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) total = at;
+        __syncwarp();
+        const int e = my_expert;
+        if (e >= 0) {
+            int rank = -my_first;
+            for (int p0 = 0; p0 < n_pairs; p0 += 32) {
+                const int p = p0 + lane;
+                const bool in = p < n_pairs && experts[p] == e;
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                const int r = rank + __popc(m & ((1u << lane) - 1u));
+                if (in && r >= 0 && r < tile_rows) {
+                    mine[r] = p;
+                    if (writer) pair_row[p] = tile * tile_rows + r;
+                }
+                rank += __popc(m);
+            }
+        }
+    }
+    __syncthreads();
+    if (writer) {
+        if (tid == 0) {
+            tile_expert[tile] = my_expert;
+            if (tile == 0) *tiles_used = total;
+        }
+        if (tid < tile_rows) row_pair[tile * tile_rows + tid] = mine[tid];
+    }
+    if (my_expert < 0) return;
+    const int per = (vec_per_row + gridDim.y - 1) / gridDim.y, v0 = blockIdx.y * per, n = min(per, vec_per_row - v0);
+    for (int i = tid; i < tile_rows * n; i += blockDim.x) {
+        const int r = i / n, c = v0 + i - r * n, p = mine[r];
+        hs[(size_t)(tile * tile_rows + r) * vec_per_row + c] = p < 0 ? make_uint4(0u, 0u, 0u, 0u) : h[(size_t)(p / top) * vec_per_row + c];
+    }
+}
+
+// gfb_moe_plan and gfb_moe_gather_rows in one launch: at most 1,024 pairs and experts, tiles of at most 64 rows; tiles without rows are not
+// written in hs
+GFB_API int gfb_moe_plan_gather(const int* idx, int n_pairs, int E, int tile_rows, const void* h, void* hs, int top, int D, int* row_pair,
+                                int* pair_row, int* tile_expert, int max_tiles, int* tiles_used, cudaStream_t stream) {
+    if (n_pairs <= 0) return 0;
+    const long busy = n_pairs < E ? n_pairs : E;
+    if (tile_rows < 1 || tile_rows > PLAN_FEW_ROWS || n_pairs > PLAN_FEW_PAIRS || E > PLAN_FEW_EXPERTS)
+        return gfb_fail("gfb_moe_plan_gather: %d pairs of %d experts in tiles of %d rows", n_pairs, E, tile_rows);
+    if ((long)max_tiles < ((long)n_pairs + busy * (tile_rows - 1)) / tile_rows)
+        return gfb_fail("gfb_moe_plan_gather: %d tiles of %d rows cannot hold %d pairs of %d experts", max_tiles, tile_rows, n_pairs, E);
+    if (D < 8 || D % 8 || ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(hs)) & 15))
+        return gfb_fail("gfb_moe_plan_gather: rows of %d bfloat16 numbers are not whole 16-byte pieces", D);
+    const int vec = D / 8, cuts = vec >= 256 ? 4 : 1;
+    cudaError_t e = gfb_launch(moe_plan_gather_kernel, dim3(max_tiles, cuts), dim3(256), 0, stream, idx, n_pairs, E, tile_rows, (const uint4*)h,
+                               (uint4*)hs, top, vec, row_pair, pair_row, tile_expert, tiles_used);
+    return gfb_check(e, "gfb_moe_plan_gather");
 }
 
 // x[t] += sum_r weights[t, r] * y[pair_row[t * top + r]] in ascending r (store: x[t] = that sum); y in the plan's sorted order, D % 4 == 0

@@ -706,6 +706,7 @@ class CudaKernels:
     MOE_TILE_ROWS = 64                 # rows of a tile of the sorted form on CUDA cores
     MOE_FEW_TOKENS = 32                # up to this many tokens a warp per output number streams the weight rows (CUDA-core forms)
     MOE_TC_FEW_TOKENS = 0              # ... where the tensor-core tiles run: they stream a chosen expert's weights once per step by TMA
+    MOE_PLAN_GATHER = 1024             # up to this many pairs and experts a decode step's plan and its gathered rows are one launch
     # (token, expert) pairs per expert from which a prompt's row tiles have 256 rows, for pairs of SMs, and not 64.  16 experts of 1,792 x 2,048,
     # us with 64 | 256: 64 pairs each 142 | 149, 128 158 | 144, 256 226 | 165; 32 of 768 x 2,048: 64 119 | 140, 128 160 | 150, 256 237 | 200
     MOE_PAIR_ROWS_PER_EXPERT = 128
@@ -792,10 +793,14 @@ class CudaKernels:
             plan = torch.empty(tiles * rows + pairs + tiles + 1, dtype=torch.int32, device=h.device)
             row_pair, pair_row = plan[:tiles * rows], plan[tiles * rows:tiles * rows + pairs]
             tile_expert, tiles_used = plan[tiles * rows + pairs:-1], plan[-1:]
-            self._call("moe", "gfb_moe_plan", _ptr(idx), c_int(pairs), c_int(E), c_int(rows), _ptr(row_pair), _ptr(pair_row),
-                       _ptr(tile_expert), c_int(tiles), _ptr(tiles_used), _stream())
             hs = torch.empty(tiles * rows, D, dtype=h.dtype, device=h.device)
-            self._call("moe", "gfb_moe_gather_rows", _ptr(h), _ptr(row_pair), _ptr(hs), c_int(tiles * rows), c_int(top), c_int(D), _stream())
+            if rows <= 64 and pairs <= self.MOE_PLAN_GATHER and E <= self.MOE_PLAN_GATHER:
+                self._call("moe", "gfb_moe_plan_gather", _ptr(idx), c_int(pairs), c_int(E), c_int(rows), _ptr(h), _ptr(hs), c_int(top), c_int(D),
+                           _ptr(row_pair), _ptr(pair_row), _ptr(tile_expert), c_int(tiles), _ptr(tiles_used), _stream())
+            else:
+                self._call("moe", "gfb_moe_plan", _ptr(idx), c_int(pairs), c_int(E), c_int(rows), _ptr(row_pair), _ptr(pair_row),
+                           _ptr(tile_expert), c_int(tiles), _ptr(tiles_used), _stream())
+                self._call("moe", "gfb_moe_gather_rows", _ptr(h), _ptr(row_pair), _ptr(hs), c_int(tiles * rows), c_int(top), c_int(D), _stream())
             mid = torch.empty(tiles * rows, F, dtype=h.dtype, device=h.device)
             self._label = f"moe_{act}_tc {N1}x{D}"
             self._call("gemm_tc", "gfb_gemm_tc_grouped", _ptr(hs), _ptr(w13), _ptr(mid), c_int(_dt(mid)), c_int(tiles * rows), c_int(rows), c_int(E),
