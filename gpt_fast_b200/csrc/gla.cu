@@ -259,11 +259,16 @@ gla_out_kernel(const T* __restrict__ src, int ld, int q_off, int k_off, int v_of
     }
     const float* Ug = U + ((size_t)w * H + h) * d * dv;
     float far[4][4];                                // scores of tokens in different sub-chunks: [r][c], c < r
-    float near[4];                                  // scores within a sub-chunk: token ty against tx
+    // Scores within a sub-chunk: row u has u earlier tokens and row 15 - u has 15 - u, so that the two together fill 15 of 16 lanes, and the
+    // last lane takes the later row's own pair.  128 threads are a sub-chunk, which leaves two sub-chunks to a thread where a square has
+    // four; the first eight tokens' own pairs, whose decay is one, are taken by eight threads each.  2,048 tokens of 16 heads of 128 x 128:
+    // 129 us with the square, 112 so.
+    const int u = ty & 7, fi = (tid >> 7) * SUB + (tx < u ? u : 15 - u), fj = (tid >> 7) * SUB + (tx < u ? tx : tx - u);
+    const int di = (tid >> 6) * SUB + ((tid >> 3) & 7);
+    float near[2] = {0.f, 0.f}, diag = 0.f;
     float o[NG][4][4];
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-        near[r] = 0.f;
 #pragma unroll
         for (int cc = 0; cc < 4; cc++) {
             far[r][cc] = 0.f;
@@ -328,16 +333,14 @@ gla_out_kernel(const T* __restrict__ src, int ld, int q_off, int k_off, int v_of
                 DOT4(far[3][0], b3, h0);
 #undef DOT4
             }
-            if (tx <= ty) {
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const float4 q4 = ld4(&sm.q[ty + 16 * r][x]), k4 = ld4(&sm.k[tx + 16 * r][x]);
-                    const float4 li = ld4(&sm.L[ty + 16 * r][x]), lj = ld4(&sm.L[tx + 16 * r][x]);
-                    near[r] = fmaf(q4.x * k4.x, exp2f(li.x - lj.x), near[r]);
-                    near[r] = fmaf(q4.y * k4.y, exp2f(li.y - lj.y), near[r]);
-                    near[r] = fmaf(q4.z * k4.z, exp2f(li.z - lj.z), near[r]);
-                    near[r] = fmaf(q4.w * k4.w, exp2f(li.w - lj.w), near[r]);
-                }
+            for (int r = 0; r < 2; r++) {
+                const int i = fi + 32 * r, j = fj + 32 * r;
+                const float4 q4 = ld4(&sm.q[i][x]), k4 = ld4(&sm.k[j][x]), li = ld4(&sm.L[i][x]), lj = ld4(&sm.L[j][x]);
+                near[r] = fmaf(q4.x * k4.x, exp2f(li.x - lj.x), near[r]);
+                near[r] = fmaf(q4.y * k4.y, exp2f(li.y - lj.y), near[r]);
+                near[r] = fmaf(q4.z * k4.z, exp2f(li.z - lj.z), near[r]);
+                near[r] = fmaf(q4.w * k4.w, exp2f(li.w - lj.w), near[r]);
             }
             // the carried state: q 2^(L + the sub-chunks before)
             const float p1[4] = {M0.x, M0.y, M0.z, M0.w}, m1[4] = {M1.x, M1.y, M1.z, M1.w}, m2[4] = {M2.x, M2.y, M2.z, M2.w};
@@ -359,6 +362,10 @@ gla_out_kernel(const T* __restrict__ src, int ld, int q_off, int k_off, int v_of
                 }
             }
         }
+        {
+            const float4 q4 = ld4(&sm.q[di][(tid & 7) * 4]), k4 = ld4(&sm.k[di][(tid & 7) * 4]);
+            diag = fmaf(q4.x, k4.x, fmaf(q4.y, k4.y, fmaf(q4.z, k4.z, fmaf(q4.w, k4.w, diag))));
+        }
     }
     __syncthreads();                                 // the scores take the place of q, k, L
     // scores to shared memory: row ty + 16 r, column tx + 16 c (columns of later sub-chunks are never read)
@@ -366,8 +373,13 @@ gla_out_kernel(const T* __restrict__ src, int ld, int q_off, int k_off, int v_of
     for (int r = 0; r < 4; r++) {
 #pragma unroll
         for (int cc = 0; cc < r; cc++) sm.A[ty + 16 * r][tx + 16 * cc] = far[r][cc];
-        sm.A[ty + 16 * r][tx + 16 * r] = tx <= ty ? near[r] : 0.f;
+        if (tx > ty) sm.A[ty + 16 * r][tx + 16 * r] = 0.f;
     }
+#pragma unroll
+    for (int r = 0; r < 2; r++) sm.A[fi + 32 * r][fj + 32 * r] = near[r];
+#pragma unroll
+    for (int o8 = 1; o8 < 8; o8 <<= 1) diag += __shfl_xor_sync(0xffffffffu, diag, o8);
+    if ((tid & 7) == 0) sm.A[di][di] = diag;
     __syncthreads();
 #pragma unroll
     for (int J = 0; J < 4; J++) {
