@@ -23,9 +23,10 @@
 // do, which keeps their rounding where it was.  T is made from the inverses of its four 16 x 16 diagonal blocks.
 //
 // What bounds it: the token-by-token kernel took 0.48 us per token whatever the hardware's width (a chain of dependent instructions;
-// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 312 us, of which delta_chunk_kernel 158 (shared
-// memory and issue slots: with single FMAs instead of pairs 168), delta_scan_kernel 120, delta_out_kernel 42.  Against 64-bit sums (700 tokens
-// of 4 heads, outputs): 2.3e-7 where the decays are close to one (token by token 3.6e-7), 1.6e-7 to 1.9e-7 where they are fast (1.5e-7).
+// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 302 us, of which delta_chunk_kernel 145 (issue
+// slots: single FMAs instead of pairs 168, pairs of a sub-chunk as a square 158), delta_scan_kernel 120, delta_out_kernel 42.  Against 64-bit
+// sums (700 tokens of 4 heads, outputs): 2.3e-7 where the decays are close to one (token by token 3.6e-7), 1.6e-7 to 1.8e-7 where they are
+// fast (1.5e-7).
 #include "common.cuh"
 
 GFB_DEFINE_LAST_ERROR()
@@ -146,7 +147,12 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
     // Thread (ty, tx) owns tokens ty + 16 r (one per sub-chunk) against tokens tx + 16 c: B in [0], A in [1]
     // (far: sub-chunks (1,0), (2,1), (2,0), (3,2), (3,1), (3,0)),
     // and every sum as that of its even and that of its odd channels
-    f32x2 far[2][6] = {{0ull, 0ull, 0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull, 0ull, 0ull}}, near[2][4] = {{0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull}};
+    f32x2 far[2][6] = {{0ull, 0ull, 0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull, 0ull, 0ull}}, near[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, diag = 0ull;
+    // Pairs within a sub-chunk: row u has u earlier tokens and row 15 - u has 15 - u, so that the two together fill 15 of 16 lanes, and the last
+    // lane takes the later row's own pair.  128 threads are a sub-chunk, which leaves two sub-chunks to a thread where a square has four; the
+    // first eight tokens' own pairs, whose decay is one, are taken by eight threads each.
+    const int u = ty & 7, fi = (tid >> 7) * SUB + (tx < u ? u : 15 - u), fj = (tid >> 7) * SUB + (tx < u ? tx : tx - u);
+    const int di = (tid >> 6) * SUB + ((tid >> 3) & 7);
     const int dd = tid & 31, oct = tid >> 5;        // staging: a channel, eight tokens
 #pragma unroll 1
     for (int d0 = 0; d0 < d; d0 += DT) {
@@ -227,19 +233,22 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
                     fma2(far[m][5], b3x, h0.x); fma2(far[m][5], b3y, h0.y);
                 }
             }
-            if (tx <= ty) {
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const ulonglong2 li = ldp(&sm.L[ty + 16 * r][x]), lj = ldp(&sm.L[tx + 16 * r][x]);
-                    const ulonglong2 ri = ldp(&sm.Lo[ty + 16 * r][x]), rj = ldp(&sm.Lo[tx + 16 * r][x]);
-                    const ulonglong2 k2 = ldp(&sm.k[tx + 16 * r][x]);
-                    const f32x2 ex = mul2(k2.x, ex22(add2(sub2(li.x, lj.x), sub2(ri.x, rj.x))));
-                    const f32x2 ey = mul2(k2.y, ex22(add2(sub2(li.y, lj.y), sub2(ri.y, rj.y))));
-                    const ulonglong2 q2 = ldp(&sm.q[ty + 16 * r][x]), c2 = ldp(&sm.k[ty + 16 * r][x]);
-                    fma2(near[0][r], q2.x, ex); fma2(near[0][r], q2.y, ey);
-                    fma2(near[1][r], c2.x, ex); fma2(near[1][r], c2.y, ey);
-                }
+            for (int r = 0; r < 2; r++) {
+                const int i = fi + 32 * r, j = fj + 32 * r;
+                const ulonglong2 li = ldp(&sm.L[i][x]), lj = ldp(&sm.L[j][x]);
+                const ulonglong2 ri = ldp(&sm.Lo[i][x]), rj = ldp(&sm.Lo[j][x]);
+                const ulonglong2 k2 = ldp(&sm.k[j][x]);
+                const f32x2 ex = mul2(k2.x, ex22(add2(sub2(li.x, lj.x), sub2(ri.x, rj.x))));
+                const f32x2 ey = mul2(k2.y, ex22(add2(sub2(li.y, lj.y), sub2(ri.y, rj.y))));
+                const ulonglong2 q2 = ldp(&sm.q[i][x]), c2 = ldp(&sm.k[i][x]);
+                fma2(near[0][r], q2.x, ex); fma2(near[0][r], q2.y, ey);
+                fma2(near[1][r], c2.x, ex); fma2(near[1][r], c2.y, ey);
             }
+        }
+        {
+            const ulonglong2 q2 = ldp(&sm.q[di][(tid & 7) * 4]), k2 = ldp(&sm.k[di][(tid & 7) * 4]);
+            fma2(diag, q2.x, k2.x); fma2(diag, q2.y, k2.y);
         }
     }
     __syncthreads();                                 // the matrices take the place of q, k, L
@@ -252,13 +261,22 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
         for (int cc = 0; cc < 4; cc++) {
             const int j = tx + 16 * cc;
             const int f = cc < r ? (r == 1 ? 0 : r == 2 ? 2 - cc : 5 - cc) : 0;
-            const float bv = cc < r ? half_sum(far[0][f]) : (cc == r && tx <= ty) ? half_sum(near[0][r]) : 0.f;
-            const float av = cc < r ? half_sum(far[1][f]) : (cc == r && tx < ty) ? half_sum(near[1][r]) : 0.f;
-            sm.R[j][i] = bv;
-            sm.N[i][j] = be * av;
             sm.T[j][i] = 0.f;
+            if (cc == r && tx <= ty) continue;       // below
+            sm.R[j][i] = cc < r ? half_sum(far[0][f]) : 0.f;
+            if (cc < r) sm.N[i][j] = be * half_sum(far[1][f]);
         }
     }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const int i = fi + 32 * r, j = fj + 32 * r;
+        sm.R[j][i] = half_sum(near[0][r]);
+        if (j < i) sm.N[i][j] = sm.beta[i] * half_sum(near[1][r]);
+    }
+    float own = half_sum(diag);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) own += __shfl_xor_sync(0xffffffffu, own, o);
+    if ((tid & 7) == 0) sm.R[di][di] = own;
     __syncthreads();
     for (int e = tid; e < PC * 16; e += THREADS) {
         const int j = e >> 4, i = (e & 15) * 4;
