@@ -6,9 +6,10 @@
 //
 //     y_i = 2^(L_i) S_0^T C_i + sum_(j<=i) (C_i . B_j) 2^(L_i - L_j) dt_j x_j + D_h x_i,     S_0' = 2^(L_end) S_0 + sum_j 2^(L_end - L_j) dt_j B_j x_j^T
 //
-// Three launches:
-//   ssd_scores_kernel   a block per (chunk, group, 16 tokens): C_i . B_j, which all heads of a group share, and C transposed
-//   ssd_state_kernel    a block per (sequence, head, 32 columns) walks over the chunks with its part of S in registers and leaves the S_0s
+// Four launches:
+//   ssd_scores_kernel   a block per (chunk, group, 16 tokens): C_i . B_j, which all heads of a group share, C transposed, and the heads' factors
+//   ssd_add_kernel      a block per (chunk, head, 64 rows, 64 columns): what the chunk adds to the state
+//   ssd_state_kernel    four numbers of a (sequence, head)'s state per thread walk over the chunks and leave the S_0s
 //   ssd_out_kernel      a block per (chunk, head, 64 columns): one product with K = state rows + 64
 //
 // Everything is 32-bit FMAs; the sums L and their differences are 64-bit (64 numbers per chunk and head), so that a decay between two tokens
@@ -16,9 +17,10 @@
 // token-by-token kernel's lanes do, which keeps their rounding where it was.
 //
 // What bounds it: the token-by-token kernel is a chain of dependent instructions per token (sequences of 77, 788 and 1,500 tokens,
-// 64 heads of 128 x 64: 1,135 us).  Here 2.4 GFMA and the S_0s' way through L2: 274 us,
-// of which ssd_state_kernel 156, ssd_out_kernel 121, ssd_scores_kernel 8.  Against 64-bit sums (700 tokens of 4 heads, outputs): 2.0e-7 where
-// the decays are close to one (token by token 6.2e-7), 1.3e-7 where they are fast (0.9e-7 to 1.1e-7).
+// 64 heads of 128 x 64: 1,135 us).  Here 2.4 GFMA and the S_0s' way through L2: about 220 us (alone and with cold caches ssd_scores_kernel 10,
+// ssd_add_kernel 77, ssd_state_kernel 78, ssd_out_kernel 121).  With the state in a block's registers, walking over a sequence's chunks as it
+// added them up, the longest sequence's 24 chunks took 6.5 us each on less than a block per SM: 274 us.  Against 64-bit sums (700 tokens of
+// 4 heads, outputs): 1.8e-7 where the decays are close to one (token by token 6.2e-7), 1.3e-7 where they are fast (0.9e-7 to 1.1e-7).
 #include "common.cuh"
 
 GFB_DEFINE_LAST_ERROR()
@@ -27,7 +29,6 @@ namespace {
 
 constexpr int PC = 64;
 constexpr int THREADS = 256;
-constexpr int VC = 32;                    // columns per block of ssd_state_kernel
 constexpr double LOG2E = 1.4426950408889634;
 
 __device__ __forceinline__ float ldw(const void* p, int dt, size_t i) {
@@ -62,12 +63,15 @@ __device__ __forceinline__ bool chunk_work(const GfbBatch& b, int w, ChunkWork& 
     return false;
 }
 
-// A chunk's scratch, in floats: per group the scores, transposed ([j][i]), and C transposed ([N][PC]); per head S_0 [N][P]
+// A chunk's scratch, in floats: per group the scores, transposed ([j][i]), and C transposed ([N][PC]); per head the tokens' factors
+// 2^(L_end - L_j) dt_j, the chunk's decay behind them, and S_0 [N][P]
+constexpr int WD = PC + 4;
 struct Sizes {
     int H, P, N, G;
     __host__ __device__ size_t scores(int g) const { return (size_t)g * (PC * PC + N * PC); }
     __host__ __device__ size_t c_t(int g) const { return scores(g) + PC * PC; }
-    __host__ __device__ size_t s0(int h) const { return scores(G) + (size_t)h * N * P; }
+    __host__ __device__ size_t w(int h) const { return scores(G) + (size_t)h * WD; }
+    __host__ __device__ size_t s0(int h) const { return w(H) + (size_t)h * N * P; }
     __host__ __device__ size_t all() const { return s0(H); }
 };
 
@@ -94,10 +98,14 @@ __device__ __forceinline__ void chunk_decays(const TD* __restrict__ dt_raw, int 
     L[2 * lane + 1] = run;
 }
 
-template <int N>
+template <typename TD, int N>
 __global__ void __launch_bounds__(THREADS)
-ssd_scores_kernel(const float* __restrict__ x, int ldx, int b_off, int c_off, float* __restrict__ scratch, GfbBatch b, int first_chunk, Sizes z) {
+ssd_scores_kernel(const float* __restrict__ x, int ldx, int b_off, int c_off, const TD* __restrict__ dt_raw, int ld_dt, int dt_off,
+                  const void* __restrict__ dt_bias, const void* __restrict__ a_log, int w_dt, float* __restrict__ scratch, GfbBatch b, int first_chunk,
+                  Sizes z) {
     extern __shared__ __align__(16) float sm[];
+    __shared__ double sL[THREADS / 32][PC];
+    __shared__ float sDt[THREADS / 32][PC];
     float(*Bs)[N + 4] = reinterpret_cast<float(*)[N + 4]>(sm);                  // [PC]
     float(*Cs)[N + 4] = reinterpret_cast<float(*)[N + 4]>(sm + PC * (N + 4));   // [16]
     gfb_pdl_launch();
@@ -115,6 +123,19 @@ ssd_scores_kernel(const float* __restrict__ x, int ldx, int b_off, int c_off, fl
         else copy16(&Cs[r - PC][p], row + c_off + g * N + p, live);
     }
     copy_commit();
+    // meanwhile the factors of the group's heads, a warp per head, dealt to the chunk's four blocks
+    const int lane = tid & 31, warp = tid >> 5, per_group = z.H / z.G;
+    for (int k = blockIdx.z * (THREADS / 32) + warp; k < per_group; k += PC / 16 * (THREADS / 32)) {
+        const int h = g * per_group + k;
+        chunk_decays(dt_raw, ld_dt, dt_off + h, c.t0, c.n, ldw(dt_bias, w_dt, h), (double)expf(ldw(a_log, w_dt, h)) * LOG2E, lane, sDt[warp], sL[warp]);
+        __syncwarp();
+        const double end = sL[warp][PC - 1];
+        float* w = mine + z.w(h);
+#pragma unroll
+        for (int q = 0; q < 2; q++) w[lane + 32 * q] = sDt[warp][lane + 32 * q] * exp2f((float)(end - sL[warp][lane + 32 * q]));
+        if (lane == 0) w[PC] = exp2f((float)end);
+        __syncwarp();
+    }
     copy_wait<0>();
     __syncthreads();
     const int i = tid & 15, jg = tid >> 4;
@@ -136,98 +157,95 @@ ssd_scores_kernel(const float* __restrict__ x, int ldx, int b_off, int c_off, fl
     for (int k = jg; k < N; k += 16) mine[z.c_t(g) + (size_t)k * PC + i0 + i] = Cs[i][k];
 }
 
-// A thread has 4 state rows x 4 columns of S in registers, a warp 32 x 16; two stages of B and x, so that the next chunk's copies run under
-// the current one's products.
-template <int N>
-struct StateSmem {
-    float B[2][PC][N];
-    float X[2][PC][VC];
-    float w[2][PC];
-    float dt[PC];
-    double L[PC];
-    float decay[2];
-};
+// What a chunk adds to the state, all chunks side by side: dS = sum_j B_j (w_j x_j)^T into S_0's place, 64 rows x 64 columns per block, four warps of
+// 32 x 32, a lane 8 x 4 sums in two groups of four rows; 32 tokens per stage, two stages.
+constexpr int ADD_THREADS = 128, HC = PC / 2;
 
-template <typename TD, int N>
-__global__ void __launch_bounds__(N * VC / 16)
-ssd_state_kernel(const float* __restrict__ x, int ldx, int b_off, const TD* __restrict__ dt_raw, int ld_dt, int dt_off, const void* __restrict__ dt_bias,
-                 const void* __restrict__ a_log, int w_dt, float* __restrict__ scratch, float* __restrict__ state, size_t state_ld, GfbBatch b,
-                 int first_chunk, int n_chunks, Sizes z) {
-    constexpr int NT = N * VC / 16;                  // threads
-    extern __shared__ __align__(16) unsigned char raw[];
-    StateSmem<N>& sm = *reinterpret_cast<StateSmem<N>*>(raw);
+__global__ void __launch_bounds__(ADD_THREADS)
+ssd_add_kernel(const float* __restrict__ x, int ldx, int b_off, float* __restrict__ scratch, GfbBatch b, int first_chunk, Sizes z) {
+    __shared__ __align__(16) float B[2][HC][64], X[2][HC][64], w[PC];
     gfb_pdl_launch();
     gfb_pdl_wait();
-    const int s = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * VC, g = h / (z.H / z.G);
-    int seq0 = 0;
-    for (int i = 0; i < s; i++) seq0 += (b.cu_seqlens[i + 1] - b.cu_seqlens[i] + PC - 1) / PC;
-    const int q0 = b.cu_seqlens[s], qlen = b.cu_seqlens[s + 1] - q0;
-    const int lo = max(seq0, first_chunk), hi = min(seq0 + (qlen + PC - 1) / PC, first_chunk + n_chunks);
-    if (lo >= hi) return;
+    ChunkWork c;
+    if (!chunk_work(b, first_chunk + blockIdx.x, c)) return;
+    const int h = blockIdx.y, g = h / (z.H / z.G), n0 = (int)blockIdx.z % (z.N / 64) * 64, p0 = (int)blockIdx.z / (z.N / 64) * 64;
+    float* mine = scratch + (size_t)blockIdx.x * z.all();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // a warp: 8 groups of four rows x 4 groups of four columns
-    const int n0 = (warp >> 1) * 32 + (lane >> 2) * 4, c0 = (warp & 1) * 16 + (lane & 3) * 4;
-    const float bias = ldw(dt_bias, w_dt, h);
-    const double rate = (double)expf(ldw(a_log, w_dt, h)) * LOG2E;
-    float* Sg = state + (size_t)b.slots[s] * state_ld + (size_t)h * N * z.P + p0;
-    float S[4][4];
+    const int r0 = (warp & 1) * 32 + (lane >> 3) * 4, c0 = (warp >> 1) * 32 + (lane & 7) * 4;
+    const float *bx = x + b_off + g * z.N + n0, *xx = x + (size_t)h * z.P + p0;
+    auto fetch = [&](int st, int j0) {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) S[i][j] = Sg[(size_t)(n0 + i) * z.P + c0 + j];
-    auto fetch = [&](int st, int w) {
-        const int t0 = q0 + (w - seq0) * PC, n = min(PC, qlen - (w - seq0) * PC);
-        for (int e = tid; e < PC * (N / 4); e += NT) {
-            const int j = e / (N / 4), p = (e - j * (N / 4)) * 4;
-            copy16(&sm.B[st][j][p], x + (size_t)(t0 + min(j, n - 1)) * ldx + b_off + g * N + p, j < n);
-        }
-        for (int e = tid; e < PC * (VC / 4); e += NT) {
-            const int j = e / (VC / 4), p = (e - j * (VC / 4)) * 4;
-            copy16(&sm.X[st][j][p], x + (size_t)(t0 + min(j, n - 1)) * ldx + (size_t)h * z.P + p0 + p, j < n);
+        for (int i = 0; i < HC * 16 / ADD_THREADS; i++) {
+            const int e = tid + ADD_THREADS * i, k = e >> 4, p = (e & 15) * 4, j = j0 + k;
+            const size_t row = (size_t)(c.t0 + (j < c.n ? j : 0)) * ldx;
+            copy16(&B[st][k][p], bx + row + p, j < c.n);
+            copy16(&X[st][k][p], xx + row + p, j < c.n);
         }
         copy_commit();
-        if (warp == 0) {
-            chunk_decays(dt_raw, ld_dt, dt_off + h, t0, n, bias, rate, lane, sm.dt, sm.L);
-            __syncwarp();
-            const double end = sm.L[PC - 1];
-#pragma unroll
-            for (int k = 0; k < 2; k++) sm.w[st][2 * lane + k] = sm.dt[2 * lane + k] * exp2f((float)(end - sm.L[2 * lane + k]));
-            if (lane == 0) sm.decay[st] = exp2f((float)end);
-            __syncwarp();
-        }
     };
-    fetch(0, lo);
-    int st = 0;
-    for (int w = lo; w < hi; w++, st ^= 1) {
-        float* S0 = scratch + (size_t)(w - first_chunk) * z.all() + z.s0(h) + p0;
+    fetch(0, 0);
+    if (tid < PC) w[tid] = mine[z.w(h) + tid];
+    float acc[8][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(S0 + (size_t)(n0 + i) * z.P + c0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-        copy_wait<0>();
-        __syncthreads();                             // this chunk's inputs have landed; everybody is done with the other stage
-        if (w + 1 < hi) fetch(st ^ 1, w + 1);
-        const float d = sm.decay[st];
+    for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; j++) S[i][j] *= d;
+    for (int st = 0; st < 2; st++) {
+        if (st == 0) { fetch(1, HC); copy_wait<1>(); } else copy_wait<0>();
+        __syncthreads();
 #pragma unroll 8
-        for (int t = 0; t < PC; t++) {
-            const float4 bv = ld4(&sm.B[st][t][n0]);
-            float4 xv = ld4(&sm.X[st][t][c0]);
-            const float wt = sm.w[st][t];
-            xv.x *= wt; xv.y *= wt; xv.z *= wt; xv.w *= wt;
-            const float br[4] = {bv.x, bv.y, bv.z, bv.w};
+        for (int k = 0; k < HC; k++) {
+            const float4 a = ld4(&B[st][k][r0]), a2 = ld4(&B[st][k][r0 + 16]);
+            float4 v = ld4(&X[st][k][c0]);
+            const float wk = w[st * HC + k];
+            v.x *= wk; v.y *= wk; v.z *= wk; v.w *= wk;
+            const float av[8] = {a.x, a.y, a.z, a.w, a2.x, a2.y, a2.z, a2.w};
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                S[i][0] = fmaf(br[i], xv.x, S[i][0]); S[i][1] = fmaf(br[i], xv.y, S[i][1]);
-                S[i][2] = fmaf(br[i], xv.z, S[i][2]); S[i][3] = fmaf(br[i], xv.w, S[i][3]);
+            for (int i = 0; i < 8; i++) {
+                acc[i][0] = fmaf(av[i], v.x, acc[i][0]); acc[i][1] = fmaf(av[i], v.y, acc[i][1]);
+                acc[i][2] = fmaf(av[i], v.z, acc[i][2]); acc[i][3] = fmaf(av[i], v.w, acc[i][3]);
             }
         }
     }
+    float* S0 = mine + z.s0(h) + p0 + c0;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < 8; i++)
+        *reinterpret_cast<float4*>(S0 + (size_t)(n0 + r0 + (i & 3) + 16 * (i >> 2)) * z.P) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+}
+
+// The walk over a sequence's chunks, four numbers of the state per thread: S_0 of a chunk takes the place of what the chunk adds, S <- decay S + dS.
+// Bound by that traffic; AHEAD chunks' loads are in flight together.
+constexpr int AHEAD = 4;
+
+__global__ void __launch_bounds__(THREADS)
+ssd_state_kernel(float* scratch, float* __restrict__ state, size_t state_ld, GfbBatch b, int first_chunk, int n_chunks, Sizes z) {
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    const int s = blockIdx.x, h = blockIdx.y, at = (blockIdx.z * THREADS + threadIdx.x) * 4;
+    int seq0 = 0;
+    for (int i = 0; i < s; i++) seq0 += (b.cu_seqlens[i + 1] - b.cu_seqlens[i] + PC - 1) / PC;
+    const int lo = max(seq0, first_chunk), hi = min(seq0 + (b.cu_seqlens[s + 1] - b.cu_seqlens[s] + PC - 1) / PC, first_chunk + n_chunks);
+    if (lo >= hi || at >= z.N * z.P) return;
+    float* Sg = state + (size_t)b.slots[s] * state_ld + (size_t)h * z.N * z.P + at;      // (of any alignment)
+    float4 S = make_float4(Sg[0], Sg[1], Sg[2], Sg[3]);
+    for (int w0 = lo; w0 < hi; w0 += AHEAD) {
+        float4 add[AHEAD];
+        float d[AHEAD];
 #pragma unroll
-        for (int j = 0; j < 4; j++) Sg[(size_t)(n0 + i) * z.P + c0 + j] = S[i][j];
+        for (int i = 0; i < AHEAD; i++) {
+            const float* m = scratch + (size_t)(min(w0 + i, hi - 1) - first_chunk) * z.all();
+            add[i] = ld4(m + z.s0(h) + at);
+            d[i] = m[z.w(h) + PC];
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) {
+            if (w0 + i >= hi) break;
+            *reinterpret_cast<float4*>(scratch + (size_t)(w0 + i - first_chunk) * z.all() + z.s0(h) + at) = S;
+            S = make_float4(fmaf(S.x, d[i], add[i].x), fmaf(S.y, d[i], add[i].y), fmaf(S.z, d[i], add[i].z), fmaf(S.w, d[i], add[i].w));
+        }
+    }
+    Sg[0] = S.x; Sg[1] = S.y; Sg[2] = S.z; Sg[3] = S.w;
 }
 
 // Tokens x columns, 64 x 64 per block: four warps of 32 x 32, a lane has 8 x 4 sums in two groups of four rows.  First C S_0 (both k-major, 32
@@ -355,7 +373,7 @@ GFB_API int gfb_ssd_chunks(const float* x, int ldx, int b_off, int c_off, const 
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
     if (G <= 0 || H % G) return gfb_fail("gfb_ssd_chunks: %d heads do not divide into %d groups", H, G);
     if ((N != 64 && N != 128) || P < 64 || P % 64) return gfb_fail("gfb_ssd_chunks: states of %d x %d", N, P);
-    if (H > 65535 || G > 65535 || P / VC > 65535) return gfb_fail("gfb_ssd_chunks: %d heads of %d columns exceed the grid limit", H, P);
+    if (H > 65535 || G > 65535 || P / 8 > 65535) return gfb_fail("gfb_ssd_chunks: %d heads of %d columns exceed the grid limit", H, P);
     if (ldx % 4 || b_off % 4 || c_off % 4 || (((uintptr_t)x | (uintptr_t)out | (uintptr_t)scratch) & 15))
         return gfb_fail("gfb_ssd_chunks: rows, B and C, output and scratch must be 16-byte aligned");
     const Sizes z{H, P, N, G};
@@ -365,12 +383,8 @@ GFB_API int gfb_ssd_chunks(const float* x, int ldx, int b_off, int c_off, const 
     cudaError_t e = cudaSuccess;
 #define ALLOW(K, bytes) if (e == cudaSuccess) e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))
     if (N == 128) {
-        ALLOW(ssd_scores_kernel<128>, score_smem);
-        if (dt_dt == GFB_BF16) { ALLOW((ssd_state_kernel<bf16, 128>), sizeof(StateSmem<128>)); }
-        else { ALLOW((ssd_state_kernel<float, 128>), sizeof(StateSmem<128>)); }
-    } else {
-        if (dt_dt == GFB_BF16) { ALLOW((ssd_state_kernel<bf16, 64>), sizeof(StateSmem<64>)); }
-        else { ALLOW((ssd_state_kernel<float, 64>), sizeof(StateSmem<64>)); }
+        if (dt_dt == GFB_BF16) { ALLOW((ssd_scores_kernel<bf16, 128>), score_smem); }
+        else { ALLOW((ssd_scores_kernel<float, 128>), score_smem); }
     }
 #undef ALLOW
     if (e != cudaSuccess) return gfb_fail("gfb_ssd_chunks: %s", cudaGetErrorString(e));
@@ -378,25 +392,22 @@ GFB_API int gfb_ssd_chunks(const float* x, int ldx, int b_off, int c_off, const 
     const long all = (long)n_tokens / PC + n_seqs, step = chunks_at_once(n_tokens, n_seqs, z);
     for (long first = 0; first < all; first += step) {
         const int n = (int)(all - first < step ? all - first : step);
-        const dim3 sgrid(n_seqs, H, P / VC), ogrid(n, H, P / 64);
-        e = N == 128 ? gfb_launch(ssd_scores_kernel<128>, dim3(n, G, PC / 16), dim3(THREADS), score_smem, stream, x, ldx, b_off, c_off, scratch, b, (int)first, z)
-                     : gfb_launch(ssd_scores_kernel<64>, dim3(n, G, PC / 16), dim3(THREADS), score_smem, stream, x, ldx, b_off, c_off, scratch, b, (int)first, z);
-#define STATE(TD, N_)                                                                                                                                    \
-    if (e == cudaSuccess)                                                                                                                                \
-        e = gfb_launch(ssd_state_kernel<TD, N_>, sgrid, dim3(N_ * VC / 16), sizeof(StateSmem<N_>), stream, x, ldx, b_off, (const TD*)dt_raw, ld_dt, dt_off,    \
-                       dt_bias, a_log, w_dt, scratch, state, (size_t)state_ld, b, (int)first, n, z)
+        const dim3 ogrid(n, H, P / 64);
+#define SCORES(TD, N_)                                                                                                                                   \
+    e = gfb_launch(ssd_scores_kernel<TD, N_>, dim3(n, G, PC / 16), dim3(THREADS), score_smem, stream, x, ldx, b_off, c_off, (const TD*)dt_raw, ld_dt, dt_off, \
+                   dt_bias, a_log, w_dt, scratch, b, (int)first, z)
 #define OUT(TD)                                                                                                                                          \
     if (e == cudaSuccess)                                                                                                                                \
         e = gfb_launch(ssd_out_kernel<TD>, ogrid, dim3(OUT_THREADS), 0, stream, x, ldx, (const TD*)dt_raw, ld_dt, dt_off, dt_bias, a_log, skip, w_dt,     \
                        (const float*)scratch, out, b, (int)first, z)
-        if (dt_dt == GFB_BF16) {
-            if (N == 128) { STATE(bf16, 128); } else { STATE(bf16, 64); }
-            OUT(bf16);
-        } else {
-            if (N == 128) { STATE(float, 128); } else { STATE(float, 64); }
-            OUT(float);
-        }
-#undef STATE
+        if (N == 128) { if (dt_dt == GFB_BF16) SCORES(bf16, 128); else SCORES(float, 128); }
+        else { if (dt_dt == GFB_BF16) SCORES(bf16, 64); else SCORES(float, 64); }
+        if (e == cudaSuccess) e = gfb_launch(ssd_add_kernel, dim3(n, H, N / 64 * (P / 64)), dim3(ADD_THREADS), 0, stream, x, ldx, b_off, scratch, b, (int)first, z);
+        if (e == cudaSuccess)
+            e = gfb_launch(ssd_state_kernel, dim3(n_seqs, H, (N * P / 4 + THREADS - 1) / THREADS), dim3(THREADS), 0, stream, scratch, state, (size_t)state_ld, b,
+                           (int)first, n, z);
+        if (dt_dt == GFB_BF16) { OUT(bf16); } else { OUT(float); }
+#undef SCORES
 #undef OUT
         if (gfb_check(e, "gfb_ssd_chunks")) return 1;
     }
