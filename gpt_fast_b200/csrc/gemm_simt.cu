@@ -45,6 +45,12 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
     return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
 }
 
+// two 32-bit numbers per instruction (sm_100), each rounded as by the single form
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+
 // numbers k .. k + 3 of row r of an operand with `rows` rows; zeros beyond its ends.  WIDE: rows of whole 4-number units, aligned
 template <typename T, bool WIDE>
 __device__ __forceinline__ float4 fetch4(const T* __restrict__ p, int r, int rows, int k, int k_end, int K) {
@@ -90,11 +96,11 @@ gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restr
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int k_begin = SPLIT ? (int)blockIdx.z * SLICE : 0, k_last = SPLIT ? min(K, k_begin + SLICE) : K;
     const int lr = tid >> 2, lk = (tid & 3) * 4;                    // the row (of every 32) and the four k this thread loads
-    float acc[TM][TN];
+    f32x2 sum[TM][TN / 2];                        // neighbouring columns share an FMA instruction
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
+        for (int j = 0; j < TN / 2; j++) sum[i][j] = 0ull;
 
     float4 ra[LA], rw[LW];
     auto fetch = [&](int k0) {
@@ -122,9 +128,10 @@ gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restr
     for (int k0 = k_begin; k0 < k_last; k0 += BK, s ^= 1) {
         const bool more = k0 + BK < k_last;
         if (more) fetch(k0 + BK);
-#pragma unroll
+#pragma unroll 8
         for (int k = 0; k < BK; k++) {
-            float a[TM], w[TN];
+            float a[TM];
+            f32x2 w[TN / 2];
             if (TM == 8) {
                 const float4 a0 = *reinterpret_cast<const float4*>(&As[s][k][am]), a1 = *reinterpret_cast<const float4*>(&As[s][k][am + 16]);
                 a[0] = a0.x; a[1] = a0.y; a[2 % TM] = a0.z; a[3 % TM] = a0.w; a[4 % TM] = a1.x; a[5 % TM] = a1.y; a[6 % TM] = a1.z; a[7 % TM] = a1.w;
@@ -134,13 +141,15 @@ gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restr
             }
 #pragma unroll
             for (int j = 0; j < TN; j += 4) {
-                const float4 v = *reinterpret_cast<const float4*>(&Ws[s][k][wn + 8 * j]);
-                w[j] = v.x; w[j + 1] = v.y; w[j + 2] = v.z; w[j + 3] = v.w;
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&Ws[s][k][wn + 8 * j]);
+                w[j / 2] = v.x; w[j / 2 + 1] = v.y;
             }
 #pragma unroll
-            for (int i = 0; i < TM; i++)
+            for (int i = 0; i < TM; i++) {
+                const f32x2 both = pack2(a[i], a[i]);
 #pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+                for (int j = 0; j < TN / 2; j++) fma2(sum[i][j], both, w[j]);
+            }
         }
         if (!SPLIT && (k0 + BK) % SLICE == 0 && more) {             // a slice ends: into the running total (the first one as it is)
             const bool first = k0 < SLICE;
@@ -150,12 +159,15 @@ gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restr
 #pragma unroll
                 for (int j = 0; j < TN; j++) {
                     const int n = n0 + wn + (j & 3) + 32 * (j >> 2);
+                    float v[2];
+                    unpack2(sum[i][j / 2], v[0], v[1]);
                     if (m < M && n < N) {
                         float* t = partial + (size_t)m * N + n;
-                        *t = first ? acc[i][j] : *t + acc[i][j];
+                        *t = first ? v[j & 1] : *t + v[j & 1];
                     }
-                    acc[i][j] = 0.f;
                 }
+#pragma unroll
+                for (int j = 0; j < TN / 2; j++) sum[i][j] = 0ull;
             }
         }
         if (more) stage(s ^ 1);
@@ -166,18 +178,21 @@ gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restr
     for (int i = 0; i < TM; i++) {
         const int m = m0 + am + (i & 3) + 16 * (i >> 2);
         if (m >= M) continue;
+        float acc[TN];
+#pragma unroll
+        for (int j = 0; j < TN; j += 2) unpack2(sum[i][j / 2], acc[j], acc[j + 1]);
 #pragma unroll
         for (int j = 0; j < TN; j++) {
             const int n = n0 + wn + (j & 3) + 32 * (j >> 2);
             if (n >= N) continue;
             if (SPLIT) {
-                partial[((size_t)blockIdx.z * M + m) * N + n] = acc[i][j];
+                partial[((size_t)blockIdx.z * M + m) * N + n] = acc[j];
             } else if (K > SLICE) {
                 const float* t = partial + (size_t)m * N;
                 const int other = EPI == EPI_SWIGLU ? (n ^ 1) : n;
-                finish<TC, EPI>(C, m, n, N, t[n] + acc[i][j], t[other] + acc[i][j ^ 1]);
+                finish<TC, EPI>(C, m, n, N, t[n] + acc[j], t[other] + acc[j ^ 1]);
             } else {
-                finish<TC, EPI>(C, m, n, N, acc[i][j], acc[i][j ^ 1]);
+                finish<TC, EPI>(C, m, n, N, acc[j], acc[j ^ 1]);
             }
         }
     }
