@@ -384,7 +384,9 @@ class CudaKernels:
                    c_float(eps), c_int(n_head), c_int(head_dim), c_int(rot_dim), c_int(rank), c_int(_PAIRING[pairing]),
                    c_int(1 if append else 0), _ptr(batch.status), _stream())
 
-    HEADWISE_FEW_TOKENS = 64           # up to this many tokens a tile of 128 is mostly empty: the smaller tiles of the mma.sync form
+    # up to this many tokens the smaller tiles of the mma.sync form (16 heads, 128 -> 512, us with it | on tcgen05: 16 tokens 22.1 | 22.9,
+    # 48 23.4 | 23.4, 64 26.8 | 22.8, 256 29.2 | 18.9)
+    HEADWISE_FEW_TOKENS = 48
 
     def headwise_linear(self, a, w, out, n_head, k, n, a_off=0, a_stride=None, out_off=0, out_stride=None, gate=None, gate_off=0,
                         gate_per_head=False):
@@ -518,9 +520,9 @@ class CudaKernels:
                    _ptr(out), c_int(_dt(out)), _ptr(scratch), *self._batch_args(batch), c_int(int(batch.max_q_len)), c_int(C), c_int(blocks),
                    _stream())
 
-    # A step whose longest sequence has this many tokens takes the state space in chunks of 64 (token by
-    # token costs about 0.4 us per token of the longest sequence, the chunks' three launches about 20 us)
-    SSD_CHUNK_TOKENS = 128
+    # A step whose longest sequence has this many tokens takes the state space in chunks of 64.  64 heads of 128 x 64, us token by token |
+    # in chunks: one sequence of 48 57 | 58, of 64 63 | 62, of 128 87 | 61; eight of 32 103 | 105, of 48 134 | 109, of 128 279 | 149
+    SSD_CHUNK_TOKENS = 64
 
     def ssd_scan(self, x, b_off, c_off, dt_src, dt_off, dt_bias, a_log, skip, state, state_off, out, batch, n_head, head_dim,
                  n_state, n_groups):
@@ -553,9 +555,10 @@ class CudaKernels:
                    c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
                    _ptr(out), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups), _stream())
 
-    # A step whose longest sequence has this many tokens takes the delta rule in chunks of 64 (token by token costs about
-    # 0.5 us per token of the longest sequence, the chunks' three launches about 25 us)
-    DELTA_CHUNK_TOKENS = 128
+    # A step whose longest sequence has this many tokens takes the delta rule in chunks of 64, and a step of three times as many tokens
+    # does so from three tenths on: the chunks of several sequences are side by side, their tokens one by one are not.  16 heads of 128 x 128,
+    # us token by token | in chunks: one sequence of 128 100 | 112, of 192 132 | 115; eight of 32 166 | 172, of 48 216 | 174, of 128 470 | 204
+    DELTA_CHUNK_TOKENS = 160
 
     def delta_rule(self, qkv, offsets, beta_src, beta_off, a_src, a_off, dt_bias, a_log, state, state_off, out, batch, n_head,
                    n_qk, head_dim, v_head_dim, q_scale, unit_eps=1e-6, head_decay=False):
@@ -573,7 +576,8 @@ class CudaKernels:
         _need(a_log, dt_bias.dtype, (n_head,), "A_log")
         _need(out, torch.float32, (T, n_head, v_head_dim), "delta-rule output")
         sp, sld = self._state_args(state, state_off, n_head * head_dim * v_head_dim)
-        if (batch.max_q_len >= self.DELTA_CHUNK_TOKENS and head_dim in (64, 128) and v_head_dim % 64 == 0 and out.data_ptr() % 16 == 0):
+        line = self.DELTA_CHUNK_TOKENS
+        if (batch.max_q_len >= (line if T < 3 * line else 3 * line // 10) and head_dim in (64, 128) and v_head_dim % 64 == 0 and out.data_ptr() % 16 == 0):
             fn = self._f("delta_chunk", "gfb_delta_chunks_scratch_floats")
             fn.restype = c_long
             need = fn(c_int(T), c_int(batch.n_seqs), c_int(n_head), c_int(head_dim), c_int(v_head_dim))
