@@ -1401,8 +1401,14 @@ GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out
     CUtensorMap mx, my;
     if (tile_rows < 256) {
         // few tokens per group: the weights' rows are the rows of the MMA, a tile of tokens its columns
-        // rings short enough for two blocks per SM: one block's set-up and epilogue hide behind the other's stream of weights
-        int STAGES = (100 * 1024) / (X_TILE_BYTES + tile_rows * BK * 2);
+        // Rings short enough for two blocks per SM: one block's set-up and epilogue hide behind the other's stream of weights.  For three with
+        // tiles of 16 rows, where the blocks are more than two per SM and, once those of tiles without rows are taken off (a tenth or more), no
+        // more than three: 24 pairs of 17 experts, 3,584 x 2,048, are some 360 blocks, and the second round of them left most SMs idle (a decode
+        // step of 8 tokens through the layer 76.6 -> 72.2 us; 476 blocks with rows took 123 us with two, 125 with three).  Tiles of 32 and 64 rows
+        // leave room for three stages only then, and lose more than that (32 experts of 1,792 x 2,048, 24 tokens: 129 us with two, 143 with three).
+        const long blocks = (long)(rows / tile_rows) * ((N + BM - 1) / BM);
+        const bool three = tile_rows == 16 && blocks > 2 * 148 && blocks <= 500;
+        int STAGES = ((three ? 73 : 100) * 1024) / (X_TILE_BYTES + tile_rows * BK * 2);
         STAGES = STAGES < 2 ? 2 : STAGES > 8 ? 8 : STAGES;
         if (make_map(&mx, W, groups * N, K, BM)) return 1;
         if (make_map(&my, A, rows, K, tile_rows)) return 1;
