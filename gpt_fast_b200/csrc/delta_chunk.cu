@@ -23,8 +23,9 @@
 // do, which keeps their rounding where it was.  T is made from the inverses of its four 16 x 16 diagonal blocks.
 //
 // What bounds it: the token-by-token kernel took 0.48 us per token whatever the hardware's width (a chain of dependent instructions;
-// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 302 us, of which delta_chunk_kernel 145 (issue
-// slots: single FMAs instead of pairs 168, pairs of a sub-chunk as a square 158), delta_scan_kernel 120, delta_out_kernel 42.  Against 64-bit
+// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 302 us, of which delta_chunk_kernel 145 (shared
+// memory and the latency of its staging loads, issue slots 31 %; single FMAs instead of pairs 168, pairs of a sub-chunk as a square 158),
+// delta_scan_kernel 120 (shared memory, 76 %), delta_out_kernel 42.  Against 64-bit
 // sums (700 tokens of 4 heads, outputs): 2.3e-7 where the decays are close to one (token by token 3.6e-7), 1.6e-7 to 1.8e-7 where they are
 // fast (1.5e-7).
 #include "common.cuh"
