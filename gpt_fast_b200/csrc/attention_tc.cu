@@ -1084,7 +1084,10 @@ struct LatBars {
     unsigned long long rest_full[2], own_full[2];
     unsigned long long rest_done[2];              // the scores' first part has read the rest of page j (a commit)
     unsigned long long s_full[2], pv_done[2];     // scores of page j are there; P V of page j is done (which also frees the own half's stage)
-    unsigned long long p_ready, o_full;
+    // all four warps' P of page j, a barrier per score buffer: the scores of page j + 1 are issued ahead of the wait for P of page j, so a
+    // warp may arrive for page j + 1 while another has not arrived for page j, and one barrier would count the two together.  An arrival for
+    // page j + 2 needs that page's scores, which are issued behind the wait for page j.
+    unsigned long long p_ready[2], o_full;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -1113,8 +1116,8 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             mbar_init(smem_u32(&bars->rest_done[s]), 1);
             mbar_init(smem_u32(&bars->s_full[s]), 1);
             mbar_init(smem_u32(&bars->pv_done[s]), 1);
+            mbar_init(smem_u32(&bars->p_ready[s]), 4);
         }
-        mbar_init(smem_u32(&bars->p_ready), 4);
         mbar_init(smem_u32(&bars->o_full), 1);
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1204,10 +1207,10 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 for (int j = 0; j < n_iter && ok; j++) {
                     // the next page's scores go ahead of this page's P V (their buffer's last P was read by the P V before, in order)
                     if (j + 1 < n_iter) ok = issue_s(j + 1);
-                    ok = ok && mbar_wait(smem_u32(&bars->p_ready), (uint32_t)j & 1u, abort_flag, status, 27);
+                    const int s = j & 1;
+                    ok = ok && mbar_wait(smem_u32(&bars->p_ready[s]), (uint32_t)(j >> 1) & 1u, abort_flag, status, 27);
                     if (!ok) break;
                     tc_fence_after();
-                    const int s = j & 1;
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++)                       // 16 keys per MMA: 8 columns of P, 2 KB of every piece
                         umma_ts(tmem, tmem + LCOL_S + s * LK + kk * 8, desc_mnmajor(os + s * hc * PIECE_BYTES + kk * 2048, PIECE_BYTES), idesc_o, (j | kk) != 0);
@@ -1315,7 +1318,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->p_ready));
+                if (lane == 0) mbar_arrive(smem_u32(&bars->p_ready[s]));
                 l_run = l_run * corr + (rsum[0] + rsum[1]);
                 m_run = m_new;
             }

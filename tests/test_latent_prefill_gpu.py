@@ -38,3 +38,29 @@ def test_latent_prompts(R, H, q_lens, starts, window, sinks):
     # P and the output are rounded to bfloat16 once each (2^-9), values are of size 0.5 to 2
     torch.testing.assert_close(out.double().cpu(), want, rtol=2e-2, atol=1e-2)
     assert float((out.double().cpu() - want).norm() / want.norm()) < 5e-3
+
+
+def test_one_warp_that_rescales_every_page():
+    """Rows whose maxima rise by more than 2^8 from page to page, in one of the four softmax warps: that warp is late for every page, and
+    the others' weights of the next page are not counted for it.  The same bits in every run."""
+    dtype, H, R, n = torch.bfloat16, 16, 256, 640
+    batch, table, n_pages = make_batch([n], [0], 1, 64, 16, seed=5)
+    pool = rnd(n_pages, 1, 64, R + 64, dtype=dtype, scale=0.5, seed=1)
+    for i in range(n // 64):
+        pool[table[0, i].item(), 0, :, R] = float(i)
+    q = rnd(n, H, R + 64, dtype=dtype, scale=0.5, seed=2)
+    q[:, :, R] = 0.0
+    late = torch.arange(n, device=DEV) % 8 // 2 == 1                  # tokens 2 and 3 of eight: rows 32 to 63 of every tile
+    q[late, :, R] = 32.0
+    kv = PagedKV(pool, torch.zeros(n_pages, 1, 64, 0, dtype=dtype, device=DEV), table, 64)
+    runs = []
+    for _ in range(20):
+        out = torch.empty(n, H * R, dtype=dtype, device=DEV)
+        ops.attention(q, kv, batch, out, H, 1, R + 64, 0.25, v_head_dim=R, values_in_keys=True)
+        runs.append(out)
+    ops.check_status(batch.status)
+    assert all(torch.equal(r.view(torch.int16), runs[0].view(torch.int16)) for r in runs)
+    cpu = dataclasses.replace(batch, **{f: getattr(batch, f).cpu() for f in ("cu_seqlens", "tok_seq", "slots", "lengths", "status")})
+    want = torch.empty(n, H * R, dtype=torch.float64)
+    REF.attention(q.cpu(), PagedKV(kv.k_pool.cpu(), kv.v_pool.cpu(), table.cpu(), 64), cpu, want, H, 1, R + 64, 0.25, v_head_dim=R, values_in_keys=True)
+    assert float((runs[0].double().cpu() - want).norm() / want.norm()) < 5e-3
