@@ -50,7 +50,9 @@ struct Bars {
     unsigned long long k_full[KV_STAGES];     // (a K stage is free again when the scores of its block are done: s_full,
     unsigned long long v_full[KV_STAGES];     //  a V stage when its P V is: pv_done; a commit per barrier costs MMA issue time)
     unsigned long long s_full[2], s_empty[2];
-    unsigned long long p_ready;
+    // P of the even / odd key blocks is written: one barrier would count two blocks together, since the scores of the next block are
+    // issued ahead of the wait for P of this one and the quarters of the rows do not wait for one another
+    unsigned long long p_ready[2];
     unsigned long long pv_done[2];            // P V of the even / odd key blocks has landed
     unsigned long long o_full;                // the item's last P V has landed (one phase per item)
     unsigned long long xch[4];                // per quarter of the rows: both warps of a row have written their half's maximum
@@ -399,8 +401,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         for (int s = 0; s < 2; s++) {
             mbar_init(smem_u32(&bars->s_full[s]), 1);
             mbar_init(smem_u32(&bars->s_empty[s]), 8);
+            mbar_init(smem_u32(&bars->p_ready[s]), 8);
         }
-        mbar_init(smem_u32(&bars->p_ready), 8);
         for (int s = 0; s < 4; s++) {
             mbar_init(smem_u32(&bars->xch[s]), 2);
             mbar_init(smem_u32(&bars->fin[s]), 2);
@@ -501,7 +503,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     if (!ok) break;
                     const int s = jj % KV_STAGES;
                     ok = mbar_wait(smem_u32(&bars->v_full[s]), (jj / KV_STAGES) & 1u, abort_flag, status, 6);
-                    ok = ok && mbar_wait(smem_u32(&bars->p_ready), jj & 1u, abort_flag, status, 7);
+                    ok = ok && mbar_wait(smem_u32(&bars->p_ready[jj & 1u]), (jj >> 1) & 1u, abort_flag, status, 7);
                     // the first P V of an item overwrites O: the previous item's output must have been read
                     if (ok && j == 0 && it > 0) ok = mbar_wait(smem_u32(&bars->o_free), (it - 1u) & 1u, abort_flag, status, 12);
                     if (!ok) break;
@@ -671,7 +673,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->p_ready));
+                if (lane == 0) mbar_arrive(smem_u32(&bars->p_ready[sb]));
                 l_run = l_run * corr + rs;
                 m_run = m_new;
             }

@@ -65,7 +65,7 @@ def walk(blocks, warps, n_bars, reads_counted):
     return wrong
 
 
-@pytest.mark.parametrize("struct,warps,reads_counted", [("LatBars", 4, False)])
+@pytest.mark.parametrize("struct,warps,reads_counted", [("Bars", 4, True), ("LatBars", 4, False)])
 def test_no_product_runs_ahead_of_its_weights(struct, warps, reads_counted):
     assert walk(6, warps, p_barriers(struct), reads_counted) == set()
 
