@@ -239,23 +239,40 @@ static bool split(int M, int N, int K) {
     return slices_of(K) > 1 && slices_of(K) <= 65535 && tiles < 6 * 148;
 }
 
+// The rows of A that one launch takes.  Partial sums stay below 256 MB (or are one row tile's), as the chunked recurrences' scratch does:
+// a product that needs more is done in portions of rows behind one another, in the same scratch.  28 slices of 1,728 x 4,096 would be
+// 793 MB beside a result of 28.
+constexpr long SCRATCH_BYTES = 256L << 20;
+struct Portion { int rows; bool apart; };         // apart: slices in blocks of their own
+static Portion portion(int M, int N, int K) {
+    const int bm = tile_rows(M), slices = slices_of(K);
+    if (slices == 1) return {M, false};
+    bool apart = split(M, N, K);
+    long most = SCRATCH_BYTES / 4 / N / (apart ? slices : 1) / bm * bm;
+    if (apart && most < bm) {
+        apart = false;
+        most = SCRATCH_BYTES / 4 / N / bm * bm;
+    }
+    if (most < bm) most = bm;
+    return {M < most ? M : (int)most, apart};
+}
+
 // Floats of scratch of a product (0: none).
 GFB_API long gfb_gemm_simt_scratch_floats(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= SLICE) return 0;
-    return (long)(split(M, N, K) ? slices_of(K) : 1) * M * N;
+    const Portion p = portion(M, N, K);
+    return (long)(p.apart ? slices_of(K) : 1) * p.rows * N;
 }
 
 template <typename TA, typename TW, typename TC, int EPI>
-static int run(const void* A, const void* W, void* C, int M, int N, int K, float* partial, cudaStream_t stream) {
+static int run(const TA* A, const TW* W, TC* C, int M, int N, int K, bool apart, float* partial, cudaStream_t stream) {
     const int bm = tile_rows(M), bn = tile_cols(bm);
-    const bool apart = split(M, N, K);
     const dim3 grid((N + bn - 1) / bn, (M + bm - 1) / bm, apart ? slices_of(K) : 1);
-    if (grid.y > 65535) return gfb_fail("gfb_gemm_simt: M = %d is too large", M);
     const bool wide = K % 4 == 0 && ((uintptr_t)A & (4 * sizeof(TA) - 1)) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
     cudaError_t e;
 #define GO(WM_, WN_, TM_, WIDE_) \
-    e = apart ? gfb_launch(gemm_simt_kernel<TA, TW, float, EPI_STORE, WM_, WN_, TM_, WIDE_, true>, grid, dim3(THREADS), 0, stream, (const TA*)A, (const TW*)W, (float*)nullptr, M, N, K, partial) \
-              : gfb_launch(gemm_simt_kernel<TA, TW, TC, EPI, WM_, WN_, TM_, WIDE_, false>, grid, dim3(THREADS), 0, stream, (const TA*)A, (const TW*)W, (TC*)C, M, N, K, partial)
+    e = apart ? gfb_launch(gemm_simt_kernel<TA, TW, float, EPI_STORE, WM_, WN_, TM_, WIDE_, true>, grid, dim3(THREADS), 0, stream, A, W, (float*)nullptr, M, N, K, partial) \
+              : gfb_launch(gemm_simt_kernel<TA, TW, TC, EPI, WM_, WN_, TM_, WIDE_, false>, grid, dim3(THREADS), 0, stream, A, W, C, M, N, K, partial)
     if (bm == 16) { if (wide) GO(2, 2, 2, true); else GO(2, 2, 2, false); }
     else if (bm == 32) { if (wide) GO(1, 4, 8, true); else GO(1, 4, 8, false); }
     else { if (wide) GO(2, 2, 8, true); else GO(2, 2, 8, false); }
@@ -263,19 +280,30 @@ static int run(const void* A, const void* W, void* C, int M, int N, int K, float
     if (gfb_check(e, "gfb_gemm_simt")) return 1;
     if (!apart) return 0;
     const size_t pairs = (size_t)M * ((N + 1) / 2);
-    e = gfb_launch(gemm_simt_sum_kernel<TC, EPI>, dim3((unsigned)((pairs + 255) / 256)), dim3(256), 0, stream, (const float*)partial, (TC*)C, M, N, slices_of(K));
+    e = gfb_launch(gemm_simt_sum_kernel<TC, EPI>, dim3((unsigned)((pairs + 255) / 256)), dim3(256), 0, stream, (const float*)partial, C, M, N, slices_of(K));
     return gfb_check(e, "gfb_gemm_simt (sum)");
+}
+
+template <typename TA, typename TW, typename TC, int EPI>
+static int portions(const void* A, const void* W, void* C, int M, int N, int K, float* partial, cudaStream_t stream) {
+    if ((M + tile_rows(M) - 1) / tile_rows(M) > 65535) return gfb_fail("gfb_gemm_simt: M = %d is too large", M);
+    const Portion p = portion(M, N, K);
+    const size_t out_cols = EPI == EPI_SWIGLU ? N / 2 : N;
+    for (int m = 0; m < M; m += p.rows)
+        if (run<TA, TW, TC, EPI>((const TA*)A + (size_t)m * K, (const TW*)W, (TC*)C + m * out_cols, M - m < p.rows ? M - m : p.rows, N, K, p.apart, partial, stream))
+            return 1;
+    return 0;
 }
 
 template <typename TA, typename TW, typename TC>
 static int launch(const void* A, const void* W, void* C, int M, int N, int K, int epi, float* partial, cudaStream_t stream) {
-    if (epi == EPI_STORE) return run<TA, TW, TC, EPI_STORE>(A, W, C, M, N, K, partial, stream);
-    if (epi == EPI_ADD) return run<TA, TW, TC, EPI_ADD>(A, W, C, M, N, K, partial, stream);
-    if (epi == EPI_SWIGLU) return run<TA, TW, TC, EPI_SWIGLU>(A, W, C, M, N, K, partial, stream);
-    if (epi == EPI_GELU) return run<TA, TW, TC, EPI_GELU>(A, W, C, M, N, K, partial, stream);
-    if (epi == EPI_GELU_TANH) return run<TA, TW, TC, EPI_GELU_TANH>(A, W, C, M, N, K, partial, stream);
-    if (epi == EPI_SILU) return run<TA, TW, TC, EPI_SILU>(A, W, C, M, N, K, partial, stream);
-    if (epi == EPI_RELU2) return run<TA, TW, TC, EPI_RELU2>(A, W, C, M, N, K, partial, stream);
+    if (epi == EPI_STORE) return portions<TA, TW, TC, EPI_STORE>(A, W, C, M, N, K, partial, stream);
+    if (epi == EPI_ADD) return portions<TA, TW, TC, EPI_ADD>(A, W, C, M, N, K, partial, stream);
+    if (epi == EPI_SWIGLU) return portions<TA, TW, TC, EPI_SWIGLU>(A, W, C, M, N, K, partial, stream);
+    if (epi == EPI_GELU) return portions<TA, TW, TC, EPI_GELU>(A, W, C, M, N, K, partial, stream);
+    if (epi == EPI_GELU_TANH) return portions<TA, TW, TC, EPI_GELU_TANH>(A, W, C, M, N, K, partial, stream);
+    if (epi == EPI_SILU) return portions<TA, TW, TC, EPI_SILU>(A, W, C, M, N, K, partial, stream);
+    if (epi == EPI_RELU2) return portions<TA, TW, TC, EPI_RELU2>(A, W, C, M, N, K, partial, stream);
     return gfb_fail("gfb_gemm_simt: unknown epilogue %d", epi);
 }
 

@@ -39,3 +39,18 @@ def test_a_row_has_the_same_bits_in_every_batch(N, K):
         part = torch.empty(rows, N, device=DEV)
         ops.linear(a[:rows].contiguous(), w, part)
         assert torch.equal(part, whole[:rows]), rows
+
+
+@pytest.mark.parametrize("mode", ["store", "add", "swiglu"])
+@pytest.mark.parametrize("M,N,K", [(600, 4096, 14336), (1100, 70000, 520)])      # 28 slices in blocks of their own; totals of slices in one block
+def test_portions_of_rows_have_the_same_bits(M, N, K, mode):
+    a, w = rnd(M, K, seed=6), rnd(N, K, seed=7)
+    cols = N // 2 if mode == "swiglu" else N
+    start = rnd(M, cols, seed=8)
+    whole = torch.cat([start, torch.full((1, cols), 7.0, device=DEV)])
+    ops.linear(a, w, whole[:M], mode)
+    assert bool((whole[M] == 7.0).all())
+    for lo, hi in ((0, 33), (M // 2 - 20, M // 2 + 60), (M - 17, M)):
+        part = start[lo:hi].clone()
+        ops.linear(a[lo:hi].contiguous(), w, part, mode)
+        assert torch.equal(part, whole[lo:hi]), lo
