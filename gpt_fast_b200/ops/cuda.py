@@ -492,7 +492,7 @@ class CudaKernels:
         sp, sld = self._state_args(state, state_off, (taps - 1) * channels)
         self._call("recurrent", "gfb_short_conv", _ptr(src), c_int(_dt(src)), c_int(src.shape[1]), c_int(col_off), c_int(channels),
                    _ptr(weight), _ptr(bias), _ptr(in_bias), c_int(_dt(weight)), c_int(taps), sp, sld, _ptr(out), *self._batch_args(batch),
-                   c_int(1 if act else 0), _stream())
+                   c_int(int(batch.max_q_len)), c_int(1 if act else 0), _stream())
 
     def rglru(self, u, w_a, w_i, b_a, b_i, lam, decay_scale, y_src, y_off, y_bias, state, state_off, out, batch):
         T = batch.n_tokens

@@ -31,6 +31,11 @@ def test_convolution_by_four_channels(dtype, taps, lens):
     torch.testing.assert_close(state.double(), want_state, rtol=1e-6, atol=1e-6)
 
 
+@pytest.mark.parametrize("lens", [[1] * 40 + [30], [2] * 30 + [1] * 9, [1] * 255 + [257], [300] + [1] * 20])
+def test_convolution_of_a_long_sequence_among_single_tokens(lens):
+    test_convolution_by_four_channels(torch.bfloat16, 4, lens)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("first", [True, False])
 @pytest.mark.parametrize("groups,gs", [(3, 4), (2, 128), (5, 132), (1, 512), (2, 516), (1, 4096), (1, 4100), (1, 8192)])
