@@ -69,6 +69,38 @@ def decode_slices(max_kv_len: int, page_size: int, blocks: int, sm_count: int) -
     return best
 
 
+def fewest_chunks(n_tokens: int, n_seqs: int, longest: int) -> int:
+    """Chunks of 64 tokens that `n_seqs` sequences of `n_tokens` altogether, the longest of `longest`, make at least (at most n_seqs - 1
+    more): the step's lengths are on the device, but every sequence has a chunk of its own, however short it is."""
+    return -(-longest // 64) + max(n_seqs - 1, -(-(n_tokens - longest) // 64))
+
+
+def delta_in_chunks(n_tokens: int, n_seqs: int, longest: int, n_head: int, head_dim: int, v_head_dim: int, line: float) -> bool:
+    """Whether a step of the delta rule takes the kernels that work in chunks.  A cost model fitted to measurements on a B200 (one to 433
+    sequences of 1 to 2,048 tokens, 16 heads of 128 x 128 and 4 of 64 x 64), in tokens of a lone sequence (0.45 us at 128 rows).  Token by
+    token the longest sequence is the chain of the step; 16 heads of 128 x 128 fill the chip, and then the tokens count; a sequence's state
+    comes and goes.  In chunks every chunk costs the same whether it has 64 tokens or one, three quarters more where the chunks' scratch
+    and the states outgrow L2.  us token by token | in chunks, 16 heads of 128 x 128: one sequence of 128 102 | 115, of 256 162 | 125; eight
+    of 32 164 | 173, of 64 264 | 176; one of 512 beside 7 of one token 303 | 217, beside 63 382 | 911; 255 of one and one of 64 357 | 5,341."""
+    w = n_head * head_dim * v_head_dim / 2 ** 18
+    chunks = fewest_chunks(n_tokens, n_seqs, longest)
+    room = 4 * n_head * (chunks * (128 * head_dim + (head_dim + 64) * (64 + v_head_dim)) + n_seqs * head_dim * v_head_dim)
+    each = max(0.129 * w, 0.025) * (1.75 if room > 100e6 else 1.0)
+    return max(longest, w * n_tokens) + 1.5 * w * n_seqs >= line * (0.75 + head_dim / 512) * (1 + each * chunks)
+
+
+def ssd_in_chunks(n_tokens: int, n_seqs: int, longest: int, n_head: int, head_dim: int, n_state: int, line: float) -> bool:
+    """The same for the state space (64 and 16 heads of 128 x 64; a token of a lone sequence is 0.32 us).  From 512 (sequence, head) pairs on
+    the token-by-token kernel keeps 16 rows per lane and takes two thirds of the time.  us token by token | in chunks, 64 heads: one
+    sequence of 48 58 | 59, of 128 87 | 64; eight of 32 103 | 102, of 48 134 | 104; one of 512 beside 7 of one token 301 | 134, beside 63
+    373 | 946; 255 of one and one of 64 495 | 5,614."""
+    w = n_head * head_dim * n_state / 2 ** 19
+    chunks = fewest_chunks(n_tokens, n_seqs, longest)
+    room = 4 * n_head * n_state * head_dim * (chunks + n_seqs)
+    each = max(0.23 * w, 0.02) * (1.9 if room > 100e6 else 1.0)
+    return max(longest, 41 + (0.81 if n_seqs * n_head >= 512 else 1.32) * w * n_tokens) + 5 * w * n_seqs >= line * (1 + each * chunks)
+
+
 class CudaKernels:
     """The operations of `ops`, bound to the sm_100a libraries.  A library is
     compiled and loaded when its first function is needed."""
@@ -520,9 +552,8 @@ class CudaKernels:
                    _ptr(out), c_int(_dt(out)), _ptr(scratch), *self._batch_args(batch), c_int(int(batch.max_q_len)), c_int(C), c_int(blocks),
                    _stream())
 
-    # A step whose longest sequence has this many tokens takes the state space in chunks of 64.  64 heads of 128 x 64, us token by token |
-    # in chunks: one sequence of 48 57 | 58, of 64 63 | 62, of 128 87 | 61; eight of 32 103 | 105, of 48 134 | 109, of 128 279 | 149
-    SSD_CHUNK_TOKENS = 64
+    # what a step in chunks costs at least, in tokens of a lone sequence token by token (`ssd_in_chunks`)
+    SSD_CHUNK_TOKENS = 95
 
     def ssd_scan(self, x, b_off, c_off, dt_src, dt_off, dt_bias, a_log, skip, state, state_off, out, batch, n_head, head_dim,
                  n_state, n_groups):
@@ -537,8 +568,9 @@ class CudaKernels:
             _need(v, dt_bias.dtype, (n_head,), name)
         _need(out, torch.float32, (T, n_head, head_dim), "scan output")
         sp, sld = self._state_args(state, state_off, n_head * n_state * head_dim)
-        if (batch.max_q_len >= self.SSD_CHUNK_TOKENS and n_state in (64, 128) and head_dim % 64 == 0 and x.shape[1] % 4 == 0 and b_off % 4 == 0
-                and c_off % 4 == 0 and x.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0):
+        if (n_state in (64, 128) and head_dim % 64 == 0 and x.shape[1] % 4 == 0 and b_off % 4 == 0 and c_off % 4 == 0 and x.data_ptr() % 16 == 0
+                and out.data_ptr() % 16 == 0
+                and ssd_in_chunks(T, batch.n_seqs, int(batch.max_q_len), n_head, head_dim, n_state, self.SSD_CHUNK_TOKENS)):
             fn = self._f("ssd_chunk", "gfb_ssd_chunks_scratch_floats")
             fn.restype = c_long
             need = fn(c_int(T), c_int(batch.n_seqs), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups))
@@ -555,10 +587,8 @@ class CudaKernels:
                    c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
                    _ptr(out), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups), _stream())
 
-    # A step whose longest sequence has this many tokens takes the delta rule in chunks of 64, and a step of three times as many tokens
-    # does so from three tenths on: the chunks of several sequences are side by side, their tokens one by one are not.  16 heads of 128 x 128,
-    # us token by token | in chunks: one sequence of 128 100 | 112, of 192 132 | 115; eight of 32 166 | 172, of 48 216 | 174, of 128 470 | 204
-    DELTA_CHUNK_TOKENS = 160
+    # the same for the delta rule (`delta_in_chunks`)
+    DELTA_CHUNK_TOKENS = 132
 
     def delta_rule(self, qkv, offsets, beta_src, beta_off, a_src, a_off, dt_bias, a_log, state, state_off, out, batch, n_head,
                    n_qk, head_dim, v_head_dim, q_scale, unit_eps=1e-6, head_decay=False):
@@ -576,8 +606,8 @@ class CudaKernels:
         _need(a_log, dt_bias.dtype, (n_head,), "A_log")
         _need(out, torch.float32, (T, n_head, v_head_dim), "delta-rule output")
         sp, sld = self._state_args(state, state_off, n_head * head_dim * v_head_dim)
-        line = self.DELTA_CHUNK_TOKENS
-        if (batch.max_q_len >= (line if T < 3 * line else 3 * line // 10) and head_dim in (64, 128) and v_head_dim % 64 == 0 and out.data_ptr() % 16 == 0):
+        if (head_dim in (64, 128) and v_head_dim % 64 == 0 and out.data_ptr() % 16 == 0
+                and delta_in_chunks(T, batch.n_seqs, int(batch.max_q_len), n_head, head_dim, v_head_dim, self.DELTA_CHUNK_TOKENS)):
             fn = self._f("delta_chunk", "gfb_delta_chunks_scratch_floats")
             fn.restype = c_long
             need = fn(c_int(T), c_int(batch.n_seqs), c_int(n_head), c_int(head_dim), c_int(v_head_dim))
