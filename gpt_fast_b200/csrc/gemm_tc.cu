@@ -1384,10 +1384,10 @@ GFB_API int gfb_gemm_tc(const void* A, const void* W, void* out, int out_dt, int
 // (rows a multiple of tile_rows), W [groups, N, K].  tile_rows 16, 32, 64: the swapped orientation of a decode step (128 weight
 // rows x a tile of tokens per block); a tile whose entry is negative is skipped.  tile_rows 256: pairs of SMs walk over the first *tiles_used row tiles (the entries with rows come first).
 // epi: EPI_STORE with out float32 [rows, N], EPI_GLU_CLAMP with out bfloat16 [rows, N / 2] from alternating gate/up
-// rows of W, or EPI_RELU2 with out bfloat16 [rows, N].
+// rows of W, or EPI_RELU2 with out bfloat16 [rows, N].  blocks_per_sm: how many blocks of tiles of 16 rows are to share an SM (2 or 3).
 GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out_dt, int rows, int tile_rows, int groups, int N, int K,
                                 int epi, const int* tile_group, const int* tiles_used, float limit, float alpha, float shift,
-                                int* status, cudaStream_t stream) {
+                                int blocks_per_sm, int* status, cudaStream_t stream) {
     if (rows <= 0 || N <= 0 || groups <= 0) return 0;
     if ((tile_rows != 16 && tile_rows != 32 && tile_rows != 64 && tile_rows != 256) || rows % tile_rows)
         return gfb_fail("gfb_gemm_tc_grouped: %d rows in tiles of %d (16, 32, 64 or 256 rows, whole tiles)", rows, tile_rows);
@@ -1402,13 +1402,11 @@ GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out
     if (tile_rows < 256) {
         // few tokens per group: the weights' rows are the rows of the MMA, a tile of tokens its columns
         // Rings short enough for two blocks per SM: one block's set-up and epilogue hide behind the other's stream of weights.  For three with
-        // tiles of 16 rows, where the blocks are more than two per SM and, once those of tiles without rows are taken off (a tenth or more), no
-        // more than three: 24 pairs of 17 experts, 3,584 x 2,048, are some 360 blocks, and the second round of them left most SMs idle (a decode
-        // step of 8 tokens through the layer 76.6 -> 72.2 us; 476 blocks with rows took 123 us with two, 125 with three).  Tiles of 32 and 64 rows
-        // leave room for three stages only then, and lose more than that (32 experts of 1,792 x 2,048, 24 tokens: 129 us with two, 143 with three).
-        const long blocks = (long)(rows / tile_rows) * ((N + BM - 1) / BM);
-        const bool three = tile_rows == 16 && blocks > 2 * 148 && blocks <= 500;
-        int STAGES = ((three ? 73 : 100) * 1024) / (X_TILE_BYTES + tile_rows * BK * 2);
+        // tiles of 16 rows, where the caller expects more blocks with rows than two per SM and no more than three: the second round of two
+        // left most SMs idle (8 tokens, 4 of 17 experts, 3,584 x 2,048: some 400 blocks, the layer 76.6 -> 72.2 us; 16 tokens, some 470, took
+        // 123 us with two and 125 with three).  Tiles of 32 and 64 rows leave room for three stages only then, and lose more than that
+        // (32 experts of 1,792 x 2,048, 24 tokens: 129 us with two, 143 with three).
+        int STAGES = ((blocks_per_sm == 3 && tile_rows == 16 ? 73 : 100) * 1024) / (X_TILE_BYTES + tile_rows * BK * 2);
         STAGES = STAGES < 2 ? 2 : STAGES > 8 ? 8 : STAGES;
         if (make_map(&mx, W, groups * N, K, BM)) return 1;
         if (make_map(&my, A, rows, K, tile_rows)) return 1;

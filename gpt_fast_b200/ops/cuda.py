@@ -69,6 +69,16 @@ def decode_slices(max_kv_len: int, page_size: int, blocks: int, sm_count: int) -
     return best
 
 
+def expert_blocks_per_sm(n_tokens: int, top: int, n_experts: int, n_rows: int, sm_count: int) -> int:
+    """How many blocks of the experts' products in a decode step are to share an SM.  With tiles of 16 rows (at most 16 tokens) a chosen
+    expert is one tile, of one block per 128 of its n_rows weight rows; evenly routed tokens choose E (1 - (1 - top / E)^T) experts.  Three
+    where two per SM would need a second round and three do not."""
+    if n_tokens > 16:
+        return 2
+    chosen = n_experts * (1.0 - (1.0 - min(1.0, top / n_experts)) ** n_tokens)
+    return 3 if 2 * sm_count < chosen * -(-n_rows // 128) <= 3 * sm_count else 2
+
+
 def fewest_chunks(n_tokens: int, n_seqs: int, longest: int) -> int:
     """Chunks of 64 tokens that `n_seqs` sequences of `n_tokens` altogether, the longest of `longest`, make at least (at most n_seqs - 1
     more): the step's lengths are on the device, but every sequence has a chunk of its own, however short it is."""
@@ -839,12 +849,12 @@ class CudaKernels:
             self._label = f"moe_{act}_tc {N1}x{D}"
             self._call("gemm_tc", "gfb_gemm_tc_grouped", _ptr(hs), _ptr(w13), _ptr(mid), c_int(_dt(mid)), c_int(tiles * rows), c_int(rows), c_int(E),
                        c_int(N1), c_int(D), c_int(_EPI["relu2"] if relu2 else self._EPI_GLU_CLAMP), _ptr(tile_expert), _ptr(tiles_used), c_float(limit), c_float(alpha),
-                       c_float(shift), _ptr(self.status), _stream())
+                       c_float(shift), c_int(expert_blocks_per_sm(T, top, E, N1, self.sm_count)), _ptr(self.status), _stream())
             y = torch.empty(tiles * rows, D, dtype=torch.float32, device=h.device)
             self._label = f"moe_down_tc {D}x{F}"
             self._call("gemm_tc", "gfb_gemm_tc_grouped", _ptr(mid), _ptr(w2), _ptr(y), c_int(_dt(y)), c_int(tiles * rows), c_int(rows), c_int(E),
                        c_int(D), c_int(F), c_int(_EPI["store"]), _ptr(tile_expert), _ptr(tiles_used), c_float(0.0), c_float(0.0), c_float(0.0),
-                       _ptr(self.status), _stream())
+                       c_int(expert_blocks_per_sm(T, top, E, D, self.sm_count)), _ptr(self.status), _stream())
             self._call("moe", "gfb_moe_combine_rows", _ptr(y), _ptr(pair_row), _ptr(weights), _ptr(x), c_int(T), c_int(top), c_int(D), keep,
                        _stream())
             return
