@@ -1434,3 +1434,14 @@ GFB_API int gfb_gemm_tc_grouped(const void* A, const void* W, void* out, int out
         return launch_pair_grouped<EPI_STORE, float>(mx, my, out, rows, N, K, N, status, gp, stream);
     return gfb_fail("gfb_gemm_tc_grouped: unsupported epilogue %d / output type %d", epi, out_dt);
 }
+
+// out[i] = reciprocal(in[i]): the epilogue's own, for a comparison with the division it stands for
+__global__ void reciprocal_kernel(const float* __restrict__ in, float* __restrict__ out, long n) {
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) out[i] = reciprocal(in[i]);
+}
+
+GFB_API int gfb_reciprocal(const float* in, float* out, long n, cudaStream_t stream) {
+    if (n <= 0) return 0;
+    reciprocal_kernel<<<1184, 256, 0, stream>>>(in, out, n);
+    return gfb_check(cudaGetLastError(), "gfb_reciprocal");
+}
