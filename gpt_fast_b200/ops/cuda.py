@@ -86,29 +86,32 @@ def fewest_chunks(n_tokens: int, n_seqs: int, longest: int) -> int:
 
 
 def delta_in_chunks(n_tokens: int, n_seqs: int, longest: int, n_head: int, head_dim: int, v_head_dim: int, line: float) -> bool:
-    """Whether a step of the delta rule takes the kernels that work in chunks.  A cost model fitted to measurements on a B200 (one to 433
-    sequences of 1 to 2,048 tokens, 16 heads of 128 x 128 and 4 of 64 x 64), in tokens of a lone sequence (0.45 us at 128 rows).  Token by
-    token the longest sequence is the chain of the step; 16 heads of 128 x 128 fill the chip, and then the tokens count; a sequence's state
-    comes and goes.  In chunks every chunk costs the same whether it has 64 tokens or one, three quarters more where the chunks' scratch
-    and the states outgrow L2.  us token by token | in chunks, 16 heads of 128 x 128: one sequence of 128 102 | 115, of 256 162 | 125; eight
-    of 32 164 | 173, of 64 264 | 176; one of 512 beside 7 of one token 303 | 217, beside 63 382 | 911; 255 of one and one of 64 357 | 5,341."""
+    """Whether a step of the delta rule takes the kernels that work in chunks.  A cost model fitted to measurements on a B200 (39 mixes of 1
+    to 433 sequences of 1 to 2,048 tokens, 4 to 32 heads of 64 x 64 to 128 x 256; it takes a form that is more than 5 % slower,
+    by up to 21 %, in 8 of 234 steps), in tokens of a lone sequence (0.45 us at 128 rows).  Token by token the longest sequence is the chain of the step; 16
+    heads of 128 x 128 fill the chip, and then the tokens count (a quarter as much from 512 (sequence, head) pairs on, where a lane has
+    16 rows); a sequence's state comes and goes.  In chunks every chunk costs the same whether it has 64 tokens or one, more where the
+    chunks' scratch and the states outgrow L2.  us token by token | in chunks, 16 heads of 128 x 128: one sequence of 128 102 | 115, of 256
+    162 | 125; eight of 32 164 | 173, of 64 264 | 176; 64 of 32 460 | 945; one of 512 beside 7 of one token 303 | 217, beside 63 382 | 911;
+    255 of one and one of 64 357 | 5,341."""
     w = n_head * head_dim * v_head_dim / 2 ** 18
     chunks = fewest_chunks(n_tokens, n_seqs, longest)
     room = 4 * n_head * (chunks * (128 * head_dim + (head_dim + 64) * (64 + v_head_dim)) + n_seqs * head_dim * v_head_dim)
-    each = max(0.129 * w, 0.025) * (1.75 if room > 100e6 else 1.0)
-    return max(longest, w * n_tokens) + 1.5 * w * n_seqs >= line * (0.75 + head_dim / 512) * (1 + each * chunks)
+    each = (0.023 + 0.113 * w) * (1.26 if room > 100e6 else 1.0)
+    busy = (23 if head_dim < 128 else 0) + (0.222 if n_seqs * n_head >= 512 else 0.916) * w * n_tokens
+    return max(longest, busy) + 0.88 * w * n_seqs >= line * (0.79 + head_dim / 1290) * (1 + each * chunks)
 
 
 def ssd_in_chunks(n_tokens: int, n_seqs: int, longest: int, n_head: int, head_dim: int, n_state: int, line: float) -> bool:
-    """The same for the state space (64 and 16 heads of 128 x 64; a token of a lone sequence is 0.32 us).  From 512 (sequence, head) pairs on
-    the token-by-token kernel keeps 16 rows per lane and takes two thirds of the time.  us token by token | in chunks, 64 heads: one
-    sequence of 48 58 | 59, of 128 87 | 64; eight of 32 103 | 102, of 48 134 | 104; one of 512 beside 7 of one token 301 | 134, beside 63
-    373 | 946; 255 of one and one of 64 495 | 5,614."""
+    """The same for the state space (8 to 128 heads of 64 x 64 to 128 x 128; a token of a lone sequence is 0.32 us; a form that is more than 5 %
+    slower, by up to 9 %, in 5 of 234 steps).  us token by token | in chunks, 64 heads of 128 x 64: one sequence of 48 58 | 59, of 128 87 | 64; eight of 32
+    103 | 102, of 48 134 | 104; one of 512 beside 7 of one token 301 | 134, beside 63 373 | 946; 255 of one and one of 64 495 | 5,614."""
     w = n_head * head_dim * n_state / 2 ** 19
     chunks = fewest_chunks(n_tokens, n_seqs, longest)
     room = 4 * n_head * n_state * head_dim * (chunks + n_seqs)
-    each = max(0.23 * w, 0.02) * (1.9 if room > 100e6 else 1.0)
-    return max(longest, 41 + (0.81 if n_seqs * n_head >= 512 else 1.32) * w * n_tokens) + 5 * w * n_seqs >= line * (1 + each * chunks)
+    each = (0.009 + 0.129 * w) * (2.2 if room > 100e6 else 1.0)
+    busy = 13 + (0.49 if n_seqs * n_head >= 512 else 1.15) * w * n_tokens
+    return max(longest, busy) + 2.3 * w * n_seqs >= line * (1 + each * chunks)
 
 
 class CudaKernels:
@@ -563,7 +566,7 @@ class CudaKernels:
                    _stream())
 
     # what a step in chunks costs at least, in tokens of a lone sequence token by token (`ssd_in_chunks`)
-    SSD_CHUNK_TOKENS = 95
+    SSD_CHUNK_TOKENS = 90
 
     def ssd_scan(self, x, b_off, c_off, dt_src, dt_off, dt_bias, a_log, skip, state, state_off, out, batch, n_head, head_dim,
                  n_state, n_groups):

@@ -17,7 +17,7 @@ def test_fewest_chunks(lens):
                                             ([48] * 8, True, True), ([64] * 8, True, True), ([16] * 32, False, False), ([8] * 64, False, False),
                                             ([512] + [1] * 7, True, True), ([64] + [1] * 15, False, False), ([64] + [1] * 255, False, False),
                                             ([160] + [1] * 63, False, False), ([512] + [1] * 63, False, False), ([512] + [1] * 255, False, False),
-                                            ([48] + [1] * 432, False, False), ([256] * 2 + [1] * 30, False, False), ([1, 3, 9, 27, 81, 200], True, True)])
+                                            ([48] + [1] * 432, False, False), ([32] * 64, False, None), ([64] * 64, False, None), ([1000] * 4 + [1] * 12, None, True), ([256] * 2 + [1] * 30, False, False), ([1, 3, 9, 27, 81, 200], True, True)])
 def test_the_faster_form_is_taken(lens, delta, ssd):
     step = sum(lens), len(lens), max(lens)
     assert delta in (None, delta_in_chunks(*step, 16, 128, 128, DELTA_LINE))
