@@ -360,15 +360,16 @@ def _route_options(score, groups, shared) -> dict:
 def moe_router(h, router, correction, top: int, scale: float, idx, weights, score: str = "sigmoid", n_extra: int = 0, groups=None,
                shared: bool = False):
     """Router logits z = h router^T (32-bit) and `moe_route` on them.  h [T, D]; router [>= E + n_extra, D] (rows beyond
-    those are padding).  A set of kernels may do both in one launch (`moe_router` returning True); otherwise the
-    product and the choice run one after the other.  n_extra: that many rows behind the experts' are further 32-bit
+    those are padding).  A set of kernels may do both in one launch (`moe_router` returning True) and may say where that
+    is slower (`moe_router_pays`); otherwise the product and the choice run one after the other.  n_extra: that many rows behind the experts' are further 32-bit
     products of the same input (a gate, say); returns (tensor float32 [T, >= n_extra], first column) where their logits
     are, or None."""
     k = kernels()
     fused = getattr(k, "moe_router", None)
     E = correction.shape[0]
     kw = _route_options(score, groups, shared)
-    if fused is not None:
+    pays = getattr(k, "moe_router_pays", None)
+    if fused is not None and (pays is None or pays(h, E + n_extra)):
         extra = None
         if n_extra:
             extra = torch.empty(h.shape[0], n_extra, dtype=torch.float32, device=h.device)

@@ -79,6 +79,20 @@ def expert_blocks_per_sm(n_tokens: int, top: int, n_experts: int, n_rows: int, s
     return 3 if 2 * sm_count < chosen * -(-n_rows // 128) <= 3 * sm_count else 2
 
 
+def router_in_one_launch(n_tokens: int, n_rows: int, dim: int, wide: bool) -> bool:
+    """Whether a router of `n_rows` rows of `dim` numbers (wide: 32-bit ones) and its choice run in one launch.  Beyond 64 tokens that launch
+    works on CUDA cores, 16 rows per pass of a block, where the product of two launches is on the tensor cores for bfloat16.  us in one |
+    in two, captured: bfloat16, rows of 1,024: 16 of them 65 tokens 12.2 | 14.0, 3,072 16.9 | 18.5, 4,096 22.9 | 19.9; 17 of them 65 tokens
+    16.6 | 14.2; rows of 2,048: 16 of them 512 tokens 18.0 | 15.5, 1,024 (from 513 on the product has other tiles) 19.2 | 22.1, 2,048
+    19.9 | 23.4, 4,096 32.4 | 26.0; 64 of them 256 tokens 40 | 16.  32-bit: 16 rows of 2,048 24 | 41, 64 of 1,024 37 | 41, 64 of 2,048 52 | 42, 16
+    of 4,096 256 tokens 41 | 42, 4,096 tokens 129 | 120."""
+    if n_tokens <= 64:
+        return True
+    if wide:
+        return -(-n_rows // 16) * dim <= 4096 and (dim < 4096 or n_tokens <= 1024)
+    return n_rows <= 16 and (n_tokens <= 3072 if dim <= 1024 else 512 < n_tokens <= 2048)
+
+
 def fewest_chunks(n_tokens: int, n_seqs: int, longest: int) -> int:
     """Chunks of 64 tokens that `n_seqs` sequences of `n_tokens` altogether, the longest of `longest`, make at least (at most n_seqs - 1
     more): the step's lengths are on the device, but every sequence has a chunk of its own, however short it is."""
@@ -783,6 +797,10 @@ class CudaKernels:
                    c_int(top), c_float(scale), _ptr(idx), _ptr(weights), c_int(T), *self._route_args(score, groups, shared), _stream())
 
     MOE_ROUTER_FEW_TOKENS = 64         # up to this many tokens a block per token, beyond it one per eight tokens (rows of whole 16-byte pieces)
+
+    def moe_router_pays(self, h, n_rows) -> bool:
+        """Whether `moe_router` is faster than the product and the choice behind it."""
+        return router_in_one_launch(h.shape[0], n_rows, h.shape[1], h.dtype == torch.float32)
 
     def moe_router(self, h, router, correction, top, scale, idx, weights, score="sigmoid", extra=None, groups=(1, 1),
                    shared=False) -> bool:

@@ -1,7 +1,7 @@
-"""How many blocks of the experts' products share an SM in a decode step (host rule, no GPU)."""
+"""The rules of the experts' kernels: blocks per SM of a decode step's products, launches of the router and of the plan (host only, no GPU)."""
 import pytest
 
-from gpt_fast_b200.ops.cuda import expert_blocks_per_sm
+from gpt_fast_b200.ops.cuda import expert_blocks_per_sm, router_in_one_launch
 
 
 @pytest.mark.parametrize("T,top,E,N,want", [(8, 4, 17, 3584, 3), (16, 4, 17, 3584, 2), (1, 4, 17, 3584, 2), (1, 16, 64, 3584, 2), (17, 4, 17, 3584, 2),
@@ -10,3 +10,11 @@ def test_three_where_two_would_need_a_second_round(T, top, E, N, want):
     assert expert_blocks_per_sm(T, top, E, N, 148) == want
     live = E * (1 - (1 - min(1, top / E)) ** T) * -(-N // 128)
     assert want == 2 or 2 * 148 < live <= 3 * 148
+
+
+@pytest.mark.parametrize("T,rows,D,wide,want", [(64, 128, 4096, False, True), (65, 16, 1024, False, True), (65, 17, 1024, False, False), (3072, 16, 1024, False, True),
+                                                (4096, 16, 1024, False, False), (256, 16, 2048, False, False), (1024, 16, 2048, False, True),
+                                                (2048, 8, 4096, False, True), (4096, 8, 4096, False, False), (256, 64, 2048, False, False),
+                                                (256, 32, 2048, True, True), (256, 64, 1024, True, True), (256, 64, 2048, True, False), (2048, 16, 4096, True, False)])
+def test_the_router_in_one_launch_where_that_is_faster(T, rows, D, wide, want):
+    assert router_in_one_launch(T, rows, D, wide) is want
