@@ -93,6 +93,16 @@ def router_in_one_launch(n_tokens: int, n_rows: int, dim: int, wide: bool) -> bo
     return n_rows <= 16 and (n_tokens <= 3072 if dim <= 1024 else 512 < n_tokens <= 2048)
 
 
+def plan_with_rows(pairs: int, n_experts: int, dim: int) -> bool:
+    """Whether the plan of the experts' tiles and the gathered rows are one launch.  Every block of it counts all pairs for itself, which
+    grows with them, and copies the rows of one tile, in four parts from 2,048 numbers on; the plan of two launches grows with the
+    experts.  us in one | in two, captured: 8 tokens, 3 of 17 experts 8.4 | 12.0; 64 tokens of 2,048: 4 of 16 experts 10.2 | 12.0, 8 of 16
+    12.5 | 12.3, 8 of 64 11.7 | 24.0; 64 tokens of 1,024: 4 of 8 16.0 | 9.3, 4 of 16 14.1 | 11.4, 4 of 32 12.5 | 14.7; 256 tokens, 4 of 32: of
+    1,024 19.6 | 16.4, of 2,048 15.8 | 16.8."""
+    most = n_experts * n_experts // (1 if dim >= 2048 else 2)
+    return pairs <= min(most, 1024) and n_experts <= 1024          # (1,024 of either fill the kernel's shared memory)
+
+
 def fewest_chunks(n_tokens: int, n_seqs: int, longest: int) -> int:
     """Chunks of 64 tokens that `n_seqs` sequences of `n_tokens` altogether, the longest of `longest`, make at least (at most n_seqs - 1
     more): the step's lengths are on the device, but every sequence has a chunk of its own, however short it is."""
@@ -767,7 +777,6 @@ class CudaKernels:
     MOE_TILE_ROWS = 64                 # rows of a tile of the sorted form on CUDA cores
     MOE_FEW_TOKENS = 32                # up to this many tokens a warp per output number streams the weight rows (CUDA-core forms)
     MOE_TC_FEW_TOKENS = 0              # ... where the tensor-core tiles run: they stream a chosen expert's weights once per step by TMA
-    MOE_PLAN_GATHER = 1024             # up to this many pairs and experts a decode step's plan and its gathered rows are one launch
     # (token, expert) pairs per expert from which a prompt's row tiles have 256 rows, for pairs of SMs, and not 64.  16 experts of 1,792 x 2,048,
     # us with 64 | 256: 64 pairs each 142 | 149, 128 158 | 144, 256 226 | 165; 32 of 768 x 2,048: 64 119 | 140, 128 160 | 150, 256 237 | 200
     MOE_PAIR_ROWS_PER_EXPERT = 128
@@ -859,7 +868,7 @@ class CudaKernels:
             row_pair, pair_row = plan[:tiles * rows], plan[tiles * rows:tiles * rows + pairs]
             tile_expert, tiles_used = plan[tiles * rows + pairs:-1], plan[-1:]
             hs = torch.empty(tiles * rows, D, dtype=h.dtype, device=h.device)
-            if rows <= 64 and pairs <= self.MOE_PLAN_GATHER and E <= self.MOE_PLAN_GATHER:
+            if rows <= 64 and plan_with_rows(pairs, E, D):
                 self._call("moe", "gfb_moe_plan_gather", _ptr(idx), c_int(pairs), c_int(E), c_int(rows), _ptr(h), _ptr(hs), c_int(top), c_int(D),
                            _ptr(row_pair), _ptr(pair_row), _ptr(tile_expert), c_int(tiles), _ptr(tiles_used), _stream())
             else:
