@@ -172,7 +172,10 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
         double sum = 0.0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            gi[i] = oct * 8 + i < c.n ? -rate * softplus_f(gi[i] + bias) : 0.f;
+            // 2^-4096 is zero against any 32-bit number, so a decay that forgets everything is that: an infinite one (A_log above 88, an
+            // infinite input) would leave the sums, and the differences of them, without a value.  (Not a number stays that.)
+            const float g = oct * 8 + i < c.n ? -rate * softplus_f(gi[i] + bias) : 0.f;
+            gi[i] = g < -4096.f ? -4096.f : g;
             sum += (double)gi[i];
         }
         __syncthreads();                            // the previous pass is done with everything below
@@ -197,7 +200,8 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
                 run += (double)gi[i];
                 const float L = (float)run, e = ex2(L);
                 // the decays behind the token within its sub-chunk: never above zero, also where rounding made the two sums cross
-                const float kh = ki[i] * ex2(fminf((float)(whole - run), 0.f));
+                const float rest = (float)(whole - run);
+                const float kh = ki[i] * ex2(rest > 0.f ? 0.f : rest);
                 sm.q[j][dd] = qi[i];
                 sm.k[j][dd] = ki[i];
                 sm.L[j][dd] = L;

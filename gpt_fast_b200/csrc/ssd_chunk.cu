@@ -75,7 +75,14 @@ struct Sizes {
     __host__ __device__ size_t all() const { return s0(H); }
 };
 
-// dt [PC] and L [PC] of a chunk by one warp (every lane two neighbouring tokens; tokens beyond the chunk have dt = 0)
+// The exponent of a token's decay.  2^-4096 is zero against any 32-bit number, so a decay that forgets everything is that: an infinite one
+// (A_log above 88) would leave its sums, and the differences of them, without a value.  (Not a number stays that.)
+__device__ __forceinline__ double decay_exponent(double rate, float dt) {
+    const double a = -rate * (double)dt;
+    return a < -4096.0 ? -4096.0 : a;
+}
+
+// dt [PC] and L [PC] of a chunk by one warp (every lane two neighbouring tokens; tokens beyond the chunk have dt = 0 and decay by nothing)
 template <typename TD>
 __device__ __forceinline__ void chunk_decays(const TD* __restrict__ dt_raw, int ld_dt, int col, int t0, int n, float bias, double rate, int lane,
                                              float* dt, double* L) {
@@ -86,15 +93,15 @@ __device__ __forceinline__ void chunk_decays(const TD* __restrict__ dt_raw, int 
         d[k] = j < n ? softplus_f(gfb_to_f32(dt_raw[(size_t)(t0 + j) * ld_dt + col]) + bias) : 0.f;
         dt[j] = d[k];
     }
-    const double a0 = -rate * (double)d[0], a1 = a0 - rate * (double)d[1];
-    double run = a1;                                 // sum up to and with this lane
+    const double a0 = 2 * lane < n ? decay_exponent(rate, d[0]) : 0.0;
+    double run = a0 + (2 * lane + 1 < n ? decay_exponent(rate, d[1]) : 0.0);        // sum up to and with this lane
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double v = __shfl_up_sync(0xffffffffu, run, o);
         if (lane >= o) run += v;
     }
-    const double before = run - a1;
-    L[2 * lane] = before + a0;
+    const double before = __shfl_up_sync(0xffffffffu, run, 1);      // (not run minus this lane's: the second token is not the first one's affair)
+    L[2 * lane] = (lane > 0 ? before : 0.0) + a0;
     L[2 * lane + 1] = run;
 }
 
