@@ -314,7 +314,8 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             const int r = k + off;
             float v = 0.f;
 #pragma unroll
-            for (int m = 0; m < SUB; m++) v = fmaf(sm.T[r * SUB + m][r * SUB + ty], sm.P[k][m][tx], v);
+            for (int m = 0; m < SUB; m++)
+                if (m <= ty) v = fmaf(sm.T[r * SUB + m][r * SUB + ty], sm.P[k][m][tx], v);       // (a later row need not be finite)
             sm.T[k * SUB + tx][r * SUB + ty] = -v;
         }
     }
@@ -348,8 +349,9 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             for (int cc = 0; cc < 4; cc++) acc[r][cc] = 0.f;
         for (int J = 0; J <= ty >> 2; J++) {
             f32x2 part[4][2] = {{0ull, 0ull}, {0ull, 0ull}, {0ull, 0ull}, {0ull, 0ull}};
-#pragma unroll
-            for (int jj = 0; jj < SUB; jj++) {
+            const int before = J < ty >> 2 ? SUB : 4 * (ty & 3);      // tokens ahead of all four rows, then their own, of which a row
+#pragma unroll 4                                                      // takes those up to itself (a later one need not be finite)
+            for (int jj = 0; jj < before; jj++) {
                 const ulonglong2 v = ldp(&sm.R[16 * J + jj][4 * tx]);
                 const float4 t4 = ld4(&sm.T[16 * J + jj][4 * ty]);
                 const f32x2 t0 = pack2(t4.x, t4.x), t1 = pack2(t4.y, t4.y), t2 = pack2(t4.z, t4.z), t3 = pack2(t4.w, t4.w);
@@ -357,6 +359,19 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
                 fma2(part[1][0], t1, v.x); fma2(part[1][1], t1, v.y);
                 fma2(part[2][0], t2, v.x); fma2(part[2][1], t2, v.y);
                 fma2(part[3][0], t3, v.x); fma2(part[3][1], t3, v.y);
+            }
+            if (J == ty >> 2) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const ulonglong2 v = ldp(&sm.R[4 * ty + q][4 * tx]);
+                    const float4 t4 = ld4(&sm.T[4 * ty + q][4 * ty]);
+                    const float t[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+                    for (int r = q; r < 4; r++) {
+                        const f32x2 tr = pack2(t[r], t[r]);
+                        fma2(part[r][0], tr, v.x); fma2(part[r][1], tr, v.y);
+                    }
+                }
             }
 #pragma unroll
             for (int r = 0; r < 4; r++) {
@@ -535,6 +550,17 @@ delta_scan_kernel(float* __restrict__ scratch, float* __restrict__ state, size_t
 // 32, a lane has 8 x 4 sums in two groups of four rows.
 constexpr int OUT_THREADS = 128, OK = 32;
 
+// One number of it over the tokens up to its own only; sums in delta_out_kernel's order.
+__device__ __noinline__ float out_number(const float* X, const float* Z, int row, int d, int dv) {
+    float acc = 0.f;
+    for (int k0 = 0; k0 <= d + row; k0 += OK) {
+        float part = 0.f;
+        for (int k = k0; k < k0 + OK && k <= d + row; k++) part = fmaf(X[(size_t)k * PC + row], Z[(size_t)k * dv], part);
+        acc += part;
+    }
+    return acc;
+}
+
 __global__ void __launch_bounds__(OUT_THREADS)
 delta_out_kernel(const float* __restrict__ scratch, float* __restrict__ out, GfbBatch b, int first_chunk, int H, int d, int dv) {
     __shared__ __align__(16) float X[2][OK][PC], Z[2][OK][64];
@@ -586,6 +612,22 @@ delta_out_kernel(const float* __restrict__ scratch, float* __restrict__ out, Gfb
         for (int i = 0; i < 8; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) acc[i][j] += part[i][j];
+    }
+    // The zeros of B meet later tokens' u above: one that is not finite makes NaN of them.  Such a block (and one whose own numbers are not
+    // finite) works its numbers out once more, each from the tokens up to its own.
+    bool odd = false;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) odd |= r0 + (i & 3) + 16 * (i >> 2) < c.n && !(fabsf(acc[i][j]) <= 3.4028235e38f);
+    if (__syncthreads_or(odd)) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int row = r0 + (i & 3) + 16 * (i >> 2);
+                if (row < c.n) acc[i][j] = out_number(m + z.qb(), m + z.su() + v0 + c0 + j, row, d, dv);
+            }
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {

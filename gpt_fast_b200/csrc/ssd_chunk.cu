@@ -264,6 +264,25 @@ struct OutSmem {
     double L[PC];
 };
 
+// One output number ahead of the skip, over the tokens up to its own only; sums in ssd_out_kernel's order.
+__device__ __noinline__ float out_number(const float* CT, const float* S0, const float* scores, const float* x, int ldx, const double* L, const float* dt,
+                                         int row, int N, int P) {
+    float acc = 0.f;
+    for (int k0 = 0; k0 < N; k0 += OK) {
+        float part = 0.f;
+        for (int k = k0; k < k0 + OK; k++) part = fmaf(CT[(size_t)k * PC + row], S0[(size_t)k * P], part);
+        acc += part;
+    }
+    acc = __fmul_rn(acc, exp2f((float)L[row]));             // (not an FMA with the first sum below)
+    for (int j0 = 0; j0 <= row; j0 += OK) {
+        float part = 0.f;
+        for (int j = j0; j < j0 + OK && j <= row; j++)
+            part = fmaf(scores[(size_t)j * PC + row] * (exp2f((float)(L[row] - L[j])) * dt[j]), x[(size_t)j * ldx], part);
+        acc += part;
+    }
+    return acc;
+}
+
 template <typename TD>
 __global__ void __launch_bounds__(OUT_THREADS)
 ssd_out_kernel(const float* __restrict__ x, int ldx, const TD* __restrict__ dt_raw, int ld_dt, int dt_off, const void* __restrict__ dt_bias,
@@ -344,6 +363,22 @@ ssd_out_kernel(const float* __restrict__ x, int ldx, const TD* __restrict__ dt_r
         for (int i = 0; i < 8; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) acc[i][j] += part[i][j];
+    }
+    // The zeros ahead of the diagonal meet later tokens' x above: one that is not finite makes NaN of them.  Such a block (and one whose own
+    // numbers are not finite) works its numbers out once more, each from the tokens up to its own.
+    bool odd = false;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) odd |= r0 + (i & 3) + 16 * (i >> 2) < c.n && !(fabsf(acc[i][j]) <= 3.4028235e38f);
+    if (__syncthreads_or(odd)) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int row = r0 + (i & 3) + 16 * (i >> 2);
+                if (row < c.n) acc[i][j] = out_number(CT, S0 + c0 + j, scores, xg + (size_t)c.t0 * ldx + c0 + j, ldx, sm.L, sm.dt, row, N, z.P);
+            }
     }
     const float dskip = skip != nullptr ? ldw(skip, w_dt, h) : 0.f;
 #pragma unroll

@@ -1,4 +1,5 @@
-"""Numbers that are not finite in the chunked recurrences: a decay that is infinite forgets and nothing else, as token by token."""
+"""Numbers that are not finite in the chunked recurrences: a decay that is infinite forgets and nothing else, and a token that is spoiled
+spoils itself and what comes behind it, as in the token-by-token kernels."""
 import pytest
 import torch
 
@@ -8,7 +9,7 @@ from test_kernels_gpu import DEV
 
 pytestmark = pytest.mark.gpu
 LENS, H, D = [100, 70], 2, 128
-INF = float("inf")
+INF, NAN = float("inf"), float("nan")
 
 
 def both(which, x, dim=D, **kw):
@@ -50,3 +51,26 @@ def test_state_space_forgets():
     x["a_log"][1] = 60.0
     close(*both(ssd, x, 64))
 
+
+J = H * D
+SPOILED = [(delta, "qkv", 2 + 5, D), (delta, "qkv", 2 + J + 5, D), (delta, "qkv", 2 + 2 * J + 5, D), (delta, "beta", 1, D), (delta, "a", 2 + 5, D),
+           (ssd, "x", 5, 64), (ssd, "x", H * 64 + 4 + 7, 64), (ssd, "x", H * 64 + 4 + D + 7, 64), (ssd, "dt", 1, 64)]
+
+
+@pytest.mark.parametrize("value", [NAN, INF])
+@pytest.mark.parametrize("t", [5, 37, 63, 64, 90, 100])
+@pytest.mark.parametrize("which,name,column,dim", SPOILED, ids=["q", "k", "v", "beta", "a", "x", "B", "C", "dt"])
+def test_a_spoiled_token_spoils_nothing_ahead_of_it(which, name, column, dim, t, value):
+    x = which.inputs(LENS, H, H, D, D, False, 0.0) if which is delta else which.inputs(LENS, H, dim, D, 1, 0.0)
+    clean = both(which, x, dim)[1][0]
+    x[name] = x[name].clone()
+    x[name][t, column] = value
+    (by_token, token_state), (in_chunks, chunk_state) = both(which, x, dim)
+    first, last = (0, LENS[0]) if t < LENS[0] else (LENS[0], sum(LENS))
+    ahead = torch.ones(sum(LENS), dtype=torch.bool, device=DEV)
+    ahead[t:last] = False                                # the other sequence's tokens too
+    assert torch.equal(in_chunks[ahead], clean[ahead])
+    if not (value == INF and name in ("beta", "a")):     # (an infinite gate or decay input is a number: one, or a decay that forgets)
+        assert bool(torch.isnan(in_chunks[t, 0]).any() or torch.isinf(in_chunks[t, 0]).any())
+    assert torch.equal(torch.isfinite(in_chunks), torch.isfinite(by_token))
+    assert torch.equal(torch.isfinite(chunk_state), torch.isfinite(token_state))
