@@ -1073,7 +1073,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 // tensor memory as the A operand (128 columns), only the rest (80 KB) in shared memory.
 //   tensor memory: O 0..255, two score buffers of 64 columns (P overwrites the first 32 of its own) 256..383, Q's half 384..511
 //
-// Measured (16 heads, R = 512, one prompt): 4,096 tokens 449 us, 650 TFLOP/s of scores and weighted sums, where the
+// Measured (16 heads, R = 512, one prompt): 4,096 tokens 492 us, 590 TFLOP/s of scores and weighted sums, where the
 // mma.sync kernel (gfb_latent_attention, which decode steps and other sizes keep) took 1,723 us, 169 TFLOP/s.
 constexpr int LK = 64;                          // keys per iteration: one page
 constexpr int PIECE_BYTES = LK * 128;           // [64 keys][64 dims]
@@ -1281,9 +1281,11 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     for (int i = 2; i < 16; i += 2) mx4[c] = max3(mx4[c], x[i], x[i + 1]);
                 }
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-                // the reference maximum follows lazily, in steps of 2^8 (as in the kernels above)
-                float m_new = m_run;
-                if (mx > m_run && (m_run == -INFINITY || (mx - m_run) * scale_log2e > 8.f)) m_new = mx;
+                // The reference is the true maximum and the sum that of the rounded weights: with a reference that lags by up to 2^8 (as in the
+                // kernels above, where keys and values are not the same rows) the largest weight is rounded too, and rows with few large ones were
+                // up to 20 % further from 64 bits than the mma.sync kernel's (1,024 tokens, queries of twice unit size: 0.00209 for 0.00174; so
+                // 0.00173).  It costs a tenth of the time.
+                const float m_new = fmaxf(m_run, mx);
                 const float corr = (m_run == -INFINITY || m_new == m_run) ? 1.f : fast_exp2((m_run - m_new) * scale_log2e);
                 const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * scale_log2e;
                 float rsum[2] = {0.f, 0.f};
@@ -1296,8 +1298,9 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         float a0, a1;
                         fma2(v[c][i], v[c][i + 1], scale_log2e, mneg, a0, a1);
                         const float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
-                        add2(rsum[c], odd, p0, p1);
-                        pk[i >> 1] = pack2(p0, p1);
+                        const uint32_t both = pack2(p0, p1);
+                        add2(rsum[c], odd, __uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u));
+                        pk[i >> 1] = both;
                     }
                     rsum[c] += odd;
                     tmem_st16(lane_base + LCOL_S + s * LK + c * 16, pk);

@@ -1,11 +1,13 @@
 """Prompts against a shared latent on tcgen05: every rank the kernel takes, heads that fill a tile of 128 (token, head) rows or straddle it,
 one to many pages, windows and sinks, sequences that go on behind cached tokens, against 64-bit softmax attention."""
 import dataclasses
+from ctypes import c_float, c_int
 
 import pytest
 import torch
 
 from gpt_fast_b200 import ops
+from gpt_fast_b200.ops.cuda import _ptr, _stream
 from gpt_fast_b200.ops.types import PagedKV
 from test_kernels_gpu import DEV, REF, make_batch, rnd
 
@@ -64,3 +66,26 @@ def test_one_warp_that_rescales_every_page():
     want = torch.empty(n, H * R, dtype=torch.float64)
     REF.attention(q.cpu(), PagedKV(kv.k_pool.cpu(), kv.v_pool.cpu(), table.cpu(), 64), cpu, want, H, 1, R + 64, 0.25, v_head_dim=R, values_in_keys=True)
     assert float((runs[0].double().cpu() - want).norm() / want.norm()) < 5e-3
+
+
+@pytest.mark.parametrize("size", [0.5, 1.0, 2.0, 4.0])
+def test_no_further_from_64_bits_than_the_kernel_of_decode_steps(size):
+    """Rows with many weights of one size, and rows with few large ones."""
+    dtype, H, R, n, scale = torch.bfloat16, 8, 512, 600, 0.0722
+    batch, table, n_pages = make_batch([n], [0], 1, 64, 16, seed=6)
+    kv = PagedKV(rnd(n_pages, 1, 64, R + 64, dtype=dtype, seed=1), torch.zeros(n_pages, 1, 64, 0, dtype=dtype, device=DEV), table, 64)
+    q = rnd(n, H, R + 64, dtype=dtype, scale=size, seed=2)
+    rows = kv.k_pool[table[0, :-(-n // 64)].long(), 0].reshape(-1, R + 64)[:n].double()
+    s = torch.einsum("thd,kd->htk", q.double(), rows) * scale
+    s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device=DEV).triu(1), -torch.inf)
+    want = torch.einsum("htk,kr->thr", s.softmax(-1), rows[:, :R]).reshape(n, H * R)
+    tc, other = (torch.empty(n, H * R, dtype=dtype, device=DEV) for _ in range(2))
+    ops.attention(q, kv, batch, tc, H, 1, R + 64, scale, v_head_dim=R, values_in_keys=True)
+    k = ops.kernels()
+    k._call("latent", "gfb_latent_attention", _ptr(q), _ptr(other), _ptr(kv.k_pool), _ptr(table), c_int(table.shape[1]), c_int(64), c_int(n_pages),
+            *k._batch_args(batch), c_int(n), c_int(H), c_int(R + 64), c_int(R), c_float(scale), c_int(0), _ptr(None), c_int(1), _ptr(None),
+            _ptr(batch.status), _stream())
+    ops.check_status(batch.status)
+    err = lambda got: float((got.double() - want).norm() / want.norm())  # noqa: E731
+    # the norm of 2.5e6 roundings of 2^-9: half a percent is far more than two draws of them differ
+    assert err(tc) <= 1.005 * err(other)
