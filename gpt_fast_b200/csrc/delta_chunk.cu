@@ -148,7 +148,8 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
     // Thread (ty, tx) owns tokens ty + 16 r (one per sub-chunk) against tokens tx + 16 c: B in [0], A in [1]
     // (far: sub-chunks (1,0), (2,1), (2,0), (3,2), (3,1), (3,0)),
     // and every sum as that of its even and that of its odd channels
-    f32x2 far[2][6] = {{0ull, 0ull, 0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull, 0ull, 0ull}}, near[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, diag = 0ull;
+    f32x2 far[2][6] = {{0ull, 0ull, 0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull, 0ull, 0ull}}, diag = 0ull;
+    double own_sub[2][2] = {{0.0, 0.0}, {0.0, 0.0}};      // of the two pairs within a sub-chunk: pieces of 16 terms, added in 64 bits
     // Pairs within a sub-chunk: row u has u earlier tokens and row 15 - u has 15 - u, so that the two together fill 15 of 16 lanes, and the last
     // lane takes the later row's own pair.  128 threads are a sub-chunk, which leaves two sub-chunks to a thread where a square has four; the
     // first eight tokens' own pairs, whose decay is one, are taken by eight threads each.
@@ -219,6 +220,7 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             out[1] = make_float4(gi[4], gi[5], gi[6], gi[7]);
         }
         __syncthreads();
+        f32x2 near[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll 1
         for (int x = 0; x < DT; x += 4) {
             {
@@ -251,6 +253,14 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
                 fma2(near[1][r], c2.x, ex); fma2(near[1][r], c2.y, ey);
             }
         }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            float even, odd;
+            unpack2(near[0][r], even, odd);
+            own_sub[0][r] += (double)even + (double)odd;
+            unpack2(near[1][r], even, odd);
+            own_sub[1][r] += (double)even + (double)odd;
+        }
         {
             const ulonglong2 q2 = ldp(&sm.q[di][(tid & 7) * 4]), k2 = ldp(&sm.k[di][(tid & 7) * 4]);
             fma2(diag, q2.x, k2.x); fma2(diag, q2.y, k2.y);
@@ -275,8 +285,8 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         const int i = fi + 32 * r, j = fj + 32 * r;
-        sm.R[j][i] = half_sum(near[0][r]);
-        if (j < i) sm.N[i][j] = sm.beta[i] * half_sum(near[1][r]);
+        sm.R[j][i] = (float)own_sub[0][r];
+        if (j < i) sm.N[i][j] = sm.beta[i] * (float)own_sub[1][r];
     }
     float own = half_sum(diag);
 #pragma unroll

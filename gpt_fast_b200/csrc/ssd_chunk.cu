@@ -20,7 +20,8 @@
 // 64 heads of 128 x 64: 1,135 us).  Here 2.4 GFMA and the S_0s' way through L2: about 220 us (alone and with cold caches ssd_scores_kernel 10,
 // ssd_add_kernel 77, ssd_state_kernel 78, ssd_out_kernel 121).  With the state in a block's registers, walking over a sequence's chunks as it
 // added them up, the longest sequence's 24 chunks took 6.5 us each on less than a block per SM: 274 us.  Against 64-bit sums (700 tokens of
-// 4 heads, outputs): 1.8e-7 where the decays are close to one (token by token 6.2e-7), 1.3e-7 where they are fast (0.9e-7 to 1.1e-7).
+// 4 heads, outputs): 1.7e-7 where the decays are close to one (token by token 6.2e-7), 0.7e-7 to 0.9e-7 where they are fast (0.9e-7 to
+// 1.1e-7), 0.8e-7 to 1.1e-7 with steps of 0.001 to 0.1 and A of 1 to 16 (1.1e-7 to 1.4e-7).
 #include "common.cuh"
 
 GFB_DEFINE_LAST_ERROR()
@@ -146,21 +147,24 @@ ssd_scores_kernel(const float* __restrict__ x, int ldx, int b_off, int c_off, co
     copy_wait<0>();
     __syncthreads();
     const int i = tid & 15, jg = tid >> 4;
-    float4 acc[4];                                   // four sums per score, of every fourth term
+    // The scores are sums of N terms that every later step multiplies, so they are made in 64 bits and rounded once: with 32-bit sums of 32
+    // terms the outputs were a fifth to two fifths further from 64 bits than token by token where decays are fast.
+    double acc[4][2];
 #pragma unroll
-    for (int r = 0; r < 4; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+    for (int r = 0; r < 4; r++) acc[r][0] = acc[r][1] = 0.0;
+#pragma unroll 2
     for (int k = 0; k < N; k += 4) {
         const float4 cv = ld4(&Cs[i][k]);
+        const double c0 = cv.x, c1 = cv.y, c2 = cv.z, c3 = cv.w;
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const float4 bv = ld4(&Bs[jg + 16 * r][k]);
-            acc[r].x = fmaf(cv.x, bv.x, acc[r].x); acc[r].y = fmaf(cv.y, bv.y, acc[r].y);
-            acc[r].z = fmaf(cv.z, bv.z, acc[r].z); acc[r].w = fmaf(cv.w, bv.w, acc[r].w);
+            acc[r][0] = fma(c0, (double)bv.x, acc[r][0]); acc[r][1] = fma(c1, (double)bv.y, acc[r][1]);
+            acc[r][0] = fma(c2, (double)bv.z, acc[r][0]); acc[r][1] = fma(c3, (double)bv.w, acc[r][1]);
         }
     }
 #pragma unroll
-    for (int r = 0; r < 4; r++) mine[z.scores(g) + (size_t)(jg + 16 * r) * PC + i0 + i] = (acc[r].x + acc[r].y) + (acc[r].z + acc[r].w);
+    for (int r = 0; r < 4; r++) mine[z.scores(g) + (size_t)(jg + 16 * r) * PC + i0 + i] = (float)(acc[r][0] + acc[r][1]);
     for (int k = jg; k < N; k += 16) mine[z.c_t(g) + (size_t)k * PC + i0 + i] = Cs[i][k];
 }
 
