@@ -23,11 +23,12 @@
 // do, which keeps their rounding where it was.  T is made from the inverses of its four 16 x 16 diagonal blocks.
 //
 // What bounds it: the token-by-token kernel took 0.48 us per token whatever the hardware's width (a chain of dependent instructions;
-// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 302 us, of which delta_chunk_kernel 145 (shared
-// memory and the latency of its staging loads, issue slots 31 %; single FMAs instead of pairs 168, pairs of a sub-chunk as a square 158),
-// delta_scan_kernel 120 (shared memory, 76 %), delta_out_kernel 42.  Against 64-bit
-// sums (700 tokens of 4 heads, outputs): 2.3e-7 where the decays are close to one (token by token 3.6e-7), 1.6e-7 to 1.8e-7 where they are
-// fast (1.5e-7).
+// 2,048 tokens of 16 heads of 128 x 128: 980 us).  Here the chain is one step per 64 tokens: 313 us, of which delta_chunk_kernel 150 (shared
+// memory and the latency of its staging loads; with single FMAs instead of pairs 23 more, with the pairs of a sub-chunk as a square 13),
+// delta_scan_kernel 120 (shared memory, 76 %), delta_out_kernel 43.  Against 64-bit sums (700 tokens of 4 heads, outputs): 2.0e-7 where
+// the decays are close to one (token by token 3.4e-7), 1.4e-7 to 1.6e-7 where they are fast (1.5e-7 to 1.7e-7), 1.8e-7 with steps of 0.001
+// to 0.1 and A of 1 to 16 (2.2e-7 to 3.7e-7).  Keys that are alike make T far from the identity: at a correlation of 0.9 and beta near one
+// 1.8e-7 to 4.1e-7 (1.6e-7 to 3.8e-7), of 0.99 up to 7.0e-7 (3.9e-7).
 #include "common.cuh"
 
 GFB_DEFINE_LAST_ERROR()
@@ -103,6 +104,7 @@ struct ChunkSmem {
         struct { float N[PC][AP], T[PC][AP], R[PC][AP]; };     // diag(beta) A, its inverse, right-hand sides
     };
     float P[3][SUB][SUB + 1];
+    double sums[16][THREADS];     // of A and B so far, a thread's own: six far pairs of B, of A, two near ones of B, of A
     double tot[8][DT];            // decay sums of half sub-chunks
     float M[4][DT];               // decay of a whole sub-chunk, and of all behind it
     float qn[PC], kn[PC], beta[PC];
@@ -146,10 +148,11 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
     __syncthreads();
     const float rate = expf(ldw(a_log, w_dt, h)) * LOG2E;
     // Thread (ty, tx) owns tokens ty + 16 r (one per sub-chunk) against tokens tx + 16 c: B in [0], A in [1]
-    // (far: sub-chunks (1,0), (2,1), (2,0), (3,2), (3,1), (3,0)),
-    // and every sum as that of its even and that of its odd channels
-    f32x2 far[2][6] = {{0ull, 0ull, 0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull, 0ull, 0ull}}, diag = 0ull;
-    double own_sub[2][2] = {{0.0, 0.0}, {0.0, 0.0}};      // of the two pairs within a sub-chunk: pieces of 16 terms, added in 64 bits
+    // (far: sub-chunks (1,0), (2,1), (2,0), (3,2), (3,1), (3,0)).
+    // The sums that make T and B are what the outputs' error hangs on, most of all where keys are alike and T is far from the identity: a pass
+    // sums 16 even and 16 odd channels in 32 bits, and the passes add up in 64 (strongly alike keys, beta near one: chains of 64 terms
+    // left the outputs 1.0e-6 from 64 bits, token by token 3.9e-7).
+    f32x2 diag = 0ull;
     // Pairs within a sub-chunk: row u has u earlier tokens and row 15 - u has 15 - u, so that the two together fill 15 of 16 lanes, and the last
     // lane takes the later row's own pair.  128 threads are a sub-chunk, which leaves two sub-chunks to a thread where a square has four; the
     // first eight tokens' own pairs, whose decay is one, are taken by eight threads each.
@@ -220,7 +223,7 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             out[1] = make_float4(gi[4], gi[5], gi[6], gi[7]);
         }
         __syncthreads();
-        f32x2 near[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+        f32x2 far[2][6] = {{0ull, 0ull, 0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull, 0ull, 0ull}}, near[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll 1
         for (int x = 0; x < DT; x += 4) {
             {
@@ -254,12 +257,11 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             }
         }
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
+        for (int f = 0; f < 16; f++) {
             float even, odd;
-            unpack2(near[0][r], even, odd);
-            own_sub[0][r] += (double)even + (double)odd;
-            unpack2(near[1][r], even, odd);
-            own_sub[1][r] += (double)even + (double)odd;
+            unpack2(f < 12 ? far[f / 6][f % 6] : near[(f - 12) / 2][f % 2], even, odd);
+            const double both = (double)even + (double)odd;
+            sm.sums[f][tid] = d0 == 0 ? both : sm.sums[f][tid] + both;
         }
         {
             const ulonglong2 q2 = ldp(&sm.q[di][(tid & 7) * 4]), k2 = ldp(&sm.k[di][(tid & 7) * 4]);
@@ -278,15 +280,15 @@ delta_chunk_kernel(const float* __restrict__ qkv, int ldq, int q_off, int k_off,
             const int f = cc < r ? (r == 1 ? 0 : r == 2 ? 2 - cc : 5 - cc) : 0;
             sm.T[j][i] = 0.f;
             if (cc == r && tx <= ty) continue;       // below
-            sm.R[j][i] = cc < r ? half_sum(far[0][f]) : 0.f;
-            if (cc < r) sm.N[i][j] = be * half_sum(far[1][f]);
+            sm.R[j][i] = cc < r ? (float)sm.sums[f][tid] : 0.f;
+            if (cc < r) sm.N[i][j] = be * (float)sm.sums[6 + f][tid];
         }
     }
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         const int i = fi + 32 * r, j = fj + 32 * r;
-        sm.R[j][i] = (float)own_sub[0][r];
-        if (j < i) sm.N[i][j] = sm.beta[i] * (float)own_sub[1][r];
+        sm.R[j][i] = (float)sm.sums[12 + r][tid];
+        if (j < i) sm.N[i][j] = sm.beta[i] * (float)sm.sums[14 + r][tid];
     }
     float own = half_sum(diag);
 #pragma unroll

@@ -48,3 +48,18 @@ def test_state_space(rate):
     x = ssd.inputs(LENS, H, 64, D, 1, rate or 0.0)
     by_token, in_chunks = errors(ssd, model_decays(x, H) if rate is None else x, 64)
     assert in_chunks <= 1.1 * by_token
+
+
+# Keys that are alike make the chunk's triangular system far from the identity, and the rounding of its 32-bit entries counts with it: the
+# entries' sums are made in 64 bits from pieces of 16 terms (chains of 64 terms left the outputs 2.7 times as far as token by token)
+@pytest.mark.parametrize("alike,most", [(0.5, 1.15), (0.9, 1.6), (0.99, 2.1)])
+@pytest.mark.parametrize("rate", [-6.0, -3.0])
+@pytest.mark.parametrize("head_decay", [False, True])
+def test_delta_rule_with_keys_that_are_alike(alike, most, rate, head_decay):
+    x = delta.inputs(LENS, H, H, D, D, head_decay, rate)
+    k = x["qkv"][:, 2 + H * D:2 + 2 * H * D]
+    one = torch.randn(1, H * D, generator=torch.Generator().manual_seed(7)).to(DEV)
+    k.copy_(alike ** 0.5 * one + (1 - alike) ** 0.5 * k)
+    x["beta"] += 4.0
+    by_token, in_chunks = errors(delta, x, D, head_decay=head_decay)
+    assert in_chunks <= most * by_token
