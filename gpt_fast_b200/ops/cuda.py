@@ -84,13 +84,14 @@ def router_in_one_launch(n_tokens: int, n_rows: int, dim: int, wide: bool) -> bo
     works on CUDA cores, 16 rows per pass of a block, where the product of two launches is on the tensor cores for bfloat16.  us in one |
     in two, captured: bfloat16, rows of 1,024: 16 of them 65 tokens 12.2 | 14.0, 3,072 16.9 | 18.5, 4,096 22.9 | 19.9; 17 of them 65 tokens
     16.6 | 14.2; rows of 2,048: 16 of them 512 tokens 18.0 | 15.5, 1,024 (from 513 on the product has other tiles) 19.2 | 22.1, 2,048
-    19.9 | 23.4, 4,096 32.4 | 26.0; 64 of them 256 tokens 40 | 16.  32-bit: 16 rows of 2,048 24 | 41, 64 of 1,024 37 | 41, 64 of 2,048 52 | 42, 16
+    19.9 | 23.4, 4,096 32.4 | 26.0; 64 of them 256 tokens 40 | 16.  Up to 512 tokens a step of such layers waits for its launches, so 16 rows
+    of 2,048 are one there too (16 layers of 16 experts, 256 tokens: 3.43 ms | 3.66).  32-bit: 16 rows of 2,048 24 | 41, 64 of 1,024 37 | 41, 64 of 2,048 52 | 42, 16
     of 4,096 256 tokens 41 | 42, 4,096 tokens 129 | 120."""
     if n_tokens <= 64:
         return True
     if wide:
         return -(-n_rows // 16) * dim <= 4096 and (dim < 4096 or n_tokens <= 1024)
-    return n_rows <= 16 and (n_tokens <= 3072 if dim <= 1024 else 512 < n_tokens <= 2048)
+    return n_rows <= 16 and n_tokens <= (3072 if dim <= 1024 else 2048) and (dim <= 2048 or n_tokens > 512)
 
 
 def plan_with_rows(pairs: int, n_experts: int, dim: int) -> bool:

@@ -13,7 +13,7 @@ def test_three_where_two_would_need_a_second_round(T, top, E, N, want):
 
 
 @pytest.mark.parametrize("T,rows,D,wide,want", [(64, 128, 4096, False, True), (65, 16, 1024, False, True), (65, 17, 1024, False, False), (3072, 16, 1024, False, True),
-                                                (4096, 16, 1024, False, False), (256, 16, 2048, False, False), (1024, 16, 2048, False, True),
+                                                (4096, 16, 1024, False, False), (256, 16, 2048, False, True), (1024, 16, 2048, False, True), (512, 16, 4096, False, False),
                                                 (2048, 8, 4096, False, True), (4096, 8, 4096, False, False), (256, 64, 2048, False, False),
                                                 (256, 32, 2048, True, True), (256, 64, 1024, True, True), (256, 64, 2048, True, False), (2048, 16, 4096, True, False)])
 def test_the_router_in_one_launch_where_that_is_faster(T, rows, D, wide, want):
