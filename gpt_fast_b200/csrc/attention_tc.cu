@@ -1281,10 +1281,9 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     for (int i = 2; i < 16; i += 2) mx4[c] = max3(mx4[c], x[i], x[i + 1]);
                 }
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-                // The reference is the true maximum and the sum that of the rounded weights: with a reference that lags by up to 2^8 (as in the
-                // kernels above, where keys and values are not the same rows) the largest weight is rounded too, and rows with few large ones were
-                // up to 20 % further from 64 bits than the mma.sync kernel's (1,024 tokens, queries of twice unit size: 0.00209 for 0.00174; so
-                // 0.00173).  It costs a tenth of the time.
+                // The reference is the true maximum, so that a row's largest weight is one, and the sum is that of the rounded weights.  With a
+                // reference that lags by up to 2^8, as in the kernels above, rows with few large weights were up to 20 % further from 64 bits than
+                // the mma.sync kernel's (1,024 tokens, queries of twice unit size: 0.00209 for 0.00174; so 0.00173).  It costs a tenth of the time.
                 const float m_new = fmaxf(m_run, mx);
                 const float corr = (m_run == -INFINITY || m_new == m_run) ? 1.f : fast_exp2((m_run - m_new) * scale_log2e);
                 const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * scale_log2e;

@@ -1,6 +1,6 @@
 // Mixture of experts: a router that picks `top` of E small gated feed-forwards per token, and the experts.
 //
-// gfb_moe_router        few tokens: router logits and choice in one launch (a block per token)
+// gfb_moe_router        router logits and choice in one launch: a block per token, or per eight tokens of a prompt
 // gfb_moe_route         from 32-bit router logits: s = sigmoid(z); the `top` experts with the largest s + correction
 //                       (lowest index on ties); weights s / (sum of the chosen s + 1e-20) * scale.  Or (mode ROUTE_SOFTMAX_TOP)
 //                       the `top` largest logits themselves, weighted by the softmax over just those, times scale.  Or (mode

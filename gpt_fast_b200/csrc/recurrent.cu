@@ -19,7 +19,9 @@
 // The two recurrences share one layout: a block owns one (sequence, head) and a slice of the state's columns and
 // walks through the sequence's tokens of this step; a lane keeps RPT rows of one column of S in registers.  Sums
 // over the rows are added per lane in ascending order and then over the lanes of the column in a fixed butterfly, so
-// a token's result is the same bits however the sequence was cut into steps or batched.  Everything is 32-bit.
+// a token's result in these kernels is the same bits however the sequence was cut into steps (RPT changes once, at 512
+// (sequence, head) pairs).  Longer prompts take the forms in chunks (delta_chunk.cu, ssd_chunk.cu), chosen by the step's
+// work: they agree with these to rounding, not to the bit.  Everything is 32-bit.
 #include "common.cuh"
 
 GFB_DEFINE_LAST_ERROR()
