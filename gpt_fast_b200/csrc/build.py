@@ -26,6 +26,7 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fP
 LIBRARIES = {
     "core": (["core.cu"], [], []),
     "gemm_simt": (["gemm_simt.cu"], [], []),
+    "gemm_split": (["gemm_split.cu"], [], []),
     "attention_generic": (["attention_generic.cu"], [], []),
     "sampling": (["sampling.cu"], [], []),
     "gemm_tc": (["gemm_tc.cu"], [], []),

@@ -1,9 +1,9 @@
 // C[M,N] = A[M,K] * W[N,K]^T on CUDA cores, any M, N, K, both precisions.
 //
-// This is the product kernel of the true 32-bit path (FFMA only, no tensor
-// cores, so no reduced-precision matrix mode) and the fallback of the bfloat16
-// path for shapes the tensor-core kernel refuses (rows that are no multiple of
-// 16 bytes).  It stands where gpt-fast calls nn.Linear (model.py:195, :215,
+// This is the 32-bit product for short sums and for rows that are no multiple of
+// 16 bytes (gemm_split.cu has the others), and the fallback of the bfloat16
+// path for shapes the tensor-core kernel refuses (such rows too).
+// It stands where gpt-fast calls nn.Linear (model.py:195, :215,
 // :227, :145).  Each output element is a sum over slices of SLICE numbers of k:
 // a slice is one thread's sum in ascending order, and the slices are added in
 // ascending order, whatever M, the tile's size and its position are: a row's

@@ -920,6 +920,11 @@ class CudaKernels:
         self._call("elementwise", "gfb_activation", _ptr(x), _ptr(out), c_int(_dt(x)), c_long(x.numel()), c_int(_EPI[kind]), _stream())
 
     # -- matrix products -----------------------------------------------------------
+    # From this K on a 32-bit product is done in bfloat16 pieces, up to three launches for one or two on CUDA cores; whatever M is, since a row's bits
+    # do not depend on the batch.  us in pieces | on CUDA cores, captured, 4,096 columns: K = 128: 1 row 6.2 | 4.7, 64 7.7 | 10.7, 2,048 26.7 | 49.7;
+    # K = 256: 1 row 9.0 | 8.1, 64 10.5 | 19.4; K = 512: 1 row 7.9 | 15.0, 64 9.4 | 36.7, 2,048 109 | 181
+    SPLIT_LEAST_K = 384
+
     def linear(self, a, w, out, mode="store", defer=False):
         M, K = a.shape
         N = w.shape[0]
@@ -940,6 +945,13 @@ class CudaKernels:
             return self._linear_tc(a, w, out, mode, defer=defer and mode in ("store", "add"))
         if a.dtype == torch.float32 and out.dtype != torch.float32:
             _fail("a float32 product is stored as float32")
+        if a.dtype == torch.float32 and K >= self.SPLIT_LEAST_K and K % 4 == 0 and w.data_ptr() % 16 == 0:
+            # three bfloat16 pieces per number on the tensor cores, nearer to 64 bits than sums on CUDA cores
+            fn = self._f("gemm_split", "gfb_gemm_split_scratch_bytes")
+            fn.restype = c_long
+            scratch = torch.empty(fn(c_int(M), c_int(N), c_int(K)), dtype=torch.uint8, device=a.device)
+            return self._call("gemm_split", "gfb_gemm_split", _ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_int(_EPI[mode]),
+                              _ptr(scratch), _ptr(self.status), _stream())
         fn = self._f("gemm_simt", "gfb_gemm_simt_scratch_floats")
         fn.restype = c_long
         need = fn(c_int(M), c_int(N), c_int(K))

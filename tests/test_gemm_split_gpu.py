@@ -1,0 +1,97 @@
+"""The 32-bit product in bfloat16 pieces at the edges of its tiles, stages and portions of K, against 64-bit sums: no further from them than
+the product on CUDA cores, the same bits in every batch, and what is not finite as 32-bit sums have it."""
+from ctypes import c_int, c_long, c_void_p
+
+import pytest
+import torch
+
+from gpt_fast_b200 import ops
+from gpt_fast_b200.csrc import build
+from test_kernels_gpu import DEV, rnd
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["store", "add", "swiglu", "gelu", "gelu_tanh", "silu", "relu2"])
+@pytest.mark.parametrize("M,N,K", [(1, 2, 384), (16, 128, 416), (17, 130, 388), (33, 66, 2052), (64, 6, 412), (65, 258, 1000), (129, 4, 500), (256, 126, 448),
+                                   (257, 3072, 512), (520, 20000, 384), (40, 64, 380), (40, 64, 4)])
+def test_edges(mode, M, N, K):
+    a, w = rnd(M, K, seed=1), rnd(N, K, scale=K ** -0.5, seed=2)
+    got = rnd(M, N // 2 if mode == "swiglu" else N, seed=3)
+    z = a.double() @ w.double().t()
+    f = torch.nn.functional
+    want = {"store": lambda: z, "add": lambda: got.double() + z, "swiglu": lambda: f.silu(z[:, 0::2]) * z[:, 1::2], "gelu": lambda: f.gelu(z),
+            "gelu_tanh": lambda: f.gelu(z, approximate="tanh"), "silu": lambda: f.silu(z), "relu2": lambda: f.relu(z) ** 2}[mode]()
+    ops.linear(a, w, got, mode)
+    # sums of unit scale, each of at most 64 accumulators of which every one loses at most 3 units of 2^-23 of its size, and squared or
+    # multiplied with one another
+    torch.testing.assert_close(got.double(), want, rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("spread", [0.0, 1.0, 4.0])
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 512), (40, 5120, 3072), (240, 3072, 8192), (300, 20000, 1024)])
+def test_nearer_to_64_bits_than_on_cuda_cores(M, N, K, spread):
+    """Numbers of one scale, and numbers whose scales spread over e^(+-3) and e^(+-12).  In the last a sum is little more than its largest
+    product, which is rounded once on CUDA cores (2.8e-8) and cut off once on tensor cores (5.5e-8): one unit of 2^-24 at most."""
+    a, w = rnd(M, K, seed=4), rnd(N, K, seed=5)
+    if spread:
+        a, w = a * torch.exp(spread * rnd(M, K, seed=6)), w * torch.exp(spread * rnd(N, K, seed=7))
+    want = a.double() @ w.double().t()
+    ours, cores = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.linear(a, w, ours)
+    lib = build.library("gemm_simt")
+    lib.gfb_gemm_simt_scratch_floats.restype = c_long
+    room = torch.empty(max(1, lib.gfb_gemm_simt_scratch_floats(M, N, K)), device=DEV)
+    ptr = lambda t: c_void_p(t.data_ptr())  # noqa: E731
+    assert lib.gfb_gemm_simt(ptr(a), ptr(w), ptr(cores), 0, 0, c_int(M), c_int(N), c_int(K), 0, ptr(room), c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    error = [((x.double() - want).norm() / want.norm()).item() for x in (ours, cores)]
+    assert error[0] <= (error[1] if spread < 4.0 else max(error[1], 2.0 ** -24)), error
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(96, 2100), (20000, 1000)])          # portions of K in blocks of their own; one block per tile
+def test_a_row_has_the_same_bits_in_every_batch(N, K):
+    a, w = rnd(600, K, seed=8), rnd(N, K, seed=9)
+    whole = torch.empty(600, N, device=DEV)
+    ops.linear(a, w, whole)
+    for lo, hi in ((0, 1), (0, 16), (3, 36), (250, 450), (100, 400), (599, 600)):
+        part = torch.empty(hi - lo, N, device=DEV)
+        ops.linear(a[lo:hi].contiguous(), w, part)
+        assert torch.equal(part, whole[lo:hi]), (lo, hi)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(96, 2100), (20000, 388)])
+def test_not_finite_and_extreme_numbers(N, K):
+    """An infinity against a bfloat16 number and against its own sign, NaNs, numbers that truncation keeps finite, sums that overflow."""
+    a, w = rnd(40, K, seed=10), rnd(N, K, seed=11)
+    a[3, 5] = float("inf")
+    w[:, 5] = 1.0
+    a[4, 7], a[4, 8] = float("inf"), float("inf")
+    a[5, 9] = float("nan")
+    a[6, 10] = torch.tensor(0x7F800001, dtype=torch.int32).view(torch.float32)       # a NaN whose upper half is an infinity's
+    w[50, 11] = float("-inf")
+    a[7] = 0.0
+    a[7, 12] = torch.finfo(torch.float32).max
+    a[8] = 2e38
+    a[9] = 1e-30
+    want = (a.double() @ w.double().t()).float()
+    got = torch.empty(40, N, device=DEV)
+    ops.linear(a, w, got)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[3], torch.full_like(got[3], float("inf")).where(torch.arange(N, device=DEV) != 50, want[3]))
+    fine = want.isfinite() & got.isfinite()
+    scale = a.abs().nan_to_num(0.0, 0.0, 0.0).double() @ w.abs().nan_to_num(0.0, 0.0, 0.0).double().t()
+    assert bool(((got.double() - want.double()).abs() <= 1e-6 * scale + 1e-37)[fine].all())
+
+
+def test_scratch_is_bounded():
+    lib = build.library("gemm_split")
+    lib.gfb_gemm_split_scratch_bytes.restype = c_long
+    for N in (1, 70, 3072, 4096, 28672, 151936, 3000000):
+        for K in (4, 512, 3072, 14336, 500000):
+            one = lib.gfb_gemm_split_scratch_bytes(c_int(256), c_int(N), c_int(K))
+            for M in (1, 17, 198, 600, 8192, 70000):
+                got = lib.gfb_gemm_split_scratch_bytes(c_int(M), c_int(N), c_int(K))
+                assert 6 * min(M, 256) * K <= got <= max((256 << 20) + 256, one), (M, N, K)
