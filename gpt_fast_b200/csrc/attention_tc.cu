@@ -25,6 +25,7 @@
 #include "common.cuh"
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 GFB_DEFINE_LAST_ERROR()
 
@@ -142,6 +143,7 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t saddr, uint32_t half_b
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int b_mn_major) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+__host__ __device__ constexpr uint32_t idesc_f16(int M, int N, int b_mn_major) { return idesc_bf16(M, N, b_mn_major) & ~((1u << 7) | (1u << 10)); }
 __device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -257,6 +259,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+__device__ __forceinline__ uint32_t pack2_half(float a, float b) {
+    __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
@@ -1479,6 +1485,458 @@ headwise_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
 }
 
+// ---- prompts with their keys and values expanded -------------------------------------------------------
+// A prompt whose keys are mostly its own new tokens is better off with every head's keys and values written out once: a (query, key, head)
+// then takes 2 (192 + 128) operations where attention on the latent takes 2 (576 + 512), and the expansion, 2 * 512 * 256 per key and head,
+// is what the queries' way into the latent space and the outputs' way back cost per token.  latent_expand_kernel makes them,
+// latent_heads_kernel attends.
+//
+// Keys are rounded to bfloat16, as queries are on the other way.  A rounded value where that way rounds the sum of values would cost precision in rows
+// that see few keys (1,200 tokens: 0.00274 from 64 bits for 0.00265), so values and weights are float16, each column of values times the power of two
+// that takes its largest possible number (v_scale, from the weights; a normed latent is bounded) to 2^14 .. 2^15: a number keeps 11 bits down to 2^-29
+// of that.  4,096 tokens of 16 heads, the whole layer: 0.0042 from 64 bits, attention on the latent 0.0046.
+//
+// Measured there (R = 512): expansion 25 us, attention 129 (700 and 670 TFLOP/s), where the queries' and outputs' products and attention on the latent take
+// 34 + 64 and 491.
+//
+// keys, values [H][n_seqs * cap][128]: key j of sequence i in row i * cap + j, cap a multiple of 128.  A block takes 128 keys of one head, two
+// pages of the cache: both products over the latent share the page's tile (A); B is Wuk_h [128][R] as it lies, and Wuv_h [R][128], an
+// MN-major operand in two pieces of 64 columns.  Two stages of 64 k (48 KB each), so that two blocks share an SM and one's epilogue runs under
+// the other's loads, which bound it: 32 KB of weights per 64 k from L2.  Rows past the sequence's end, or of pages ahead of the
+// window, are zeros, so that no weight of zero meets a NaN.
+constexpr int LE_STAGES = 2, LE_STAGE_BYTES = 3 * HALF_BYTES;
+constexpr uint32_t LE_SMEM = 1024 + LE_STAGES * LE_STAGE_BYTES + 128;
+static_assert(4 * 32 * HW_PITCH * 4 <= LE_STAGES * LE_STAGE_BYTES, "the epilogue's rows take the ring's place");
+
+struct LeBars {
+    unsigned long long full[LE_STAGES], empty[LE_STAGES], done;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+__global__ void __launch_bounds__(192)
+latent_expand_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_uk, const __grid_constant__ CUtensorMap map_uv,
+                     __nv_bfloat16* __restrict__ keys, __half* __restrict__ values, const float* __restrict__ v_scale, const int* __restrict__ page_table,
+                     int max_pages, int n_pages_pool, GfbBatch b, int H, int R, int cap, int window, int* status) {
+    extern __shared__ uint8_t smem_raw[];
+    if (threadIdx.x == 0) { prefetch_map(&map_c); prefetch_map(&map_uk); prefetch_map(&map_uv); }
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
+    LeBars* bars = reinterpret_cast<LeBars*>(aligned + LE_STAGES * LE_STAGE_BYTES);
+    volatile int* abort_flag = &bars->abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tiles = cap / KEYS, tile = blockIdx.x / H, h = blockIdx.x - tile * H, seq = tile / tiles, key0 = (tile - seq * tiles) * KEYS;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < LE_STAGES; s++) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
+        mbar_init(smem_u32(&bars->done), 1);
+        bars->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(256u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    const int slot = b.slots[seq], start = b.lengths[slot], new_tokens = b.cu_seqlens[seq + 1] - b.cu_seqlens[seq], len = start + new_tokens;
+    const int lo = window > 0 ? max(0, start - window + 1) : 0;      // the first key that any new token sees
+    const bool idle = new_tokens <= 0 || key0 >= len || key0 + KEYS <= lo;
+    if (idle) {
+    } else if (warp == 0) {
+        if (lane == 0) {
+            int page[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {                            // (a page that no token sees: another one, its rows become zeros)
+                const int pi = min(max(key0 / PAGE + i, lo / PAGE), (len - 1) / PAGE);
+                page[i] = pi < max_pages ? page_table[(size_t)slot * max_pages + pi] : -1;
+                if (page[i] < 0 || page[i] >= n_pages_pool) { gfb_report(status, GFB_ERR_PAGE_TABLE, slot, pi); page[i] = 0; }
+            }
+            for (int kb = 0; kb < R / 64; kb++) {
+                const int s = kb % LE_STAGES;
+                if (!mbar_wait(smem_u32(&bars->empty[s]), ((uint32_t)(kb / LE_STAGES) & 1u) ^ 1u, abort_flag, status, 41)) break;
+                const uint32_t full = smem_u32(&bars->full[s]), at = base + s * LE_STAGE_BYTES;
+                mbar_expect_tx(full, LE_STAGE_BYTES);
+                tma_load_2d(at, &map_c, kb * 64, page[0] * PAGE, full);
+                tma_load_2d(at + PIECE_BYTES, &map_c, kb * 64, page[1] * PAGE, full);
+                tma_load_2d(at + HALF_BYTES, &map_uk, kb * 64, h * D, full);
+                tma_load_2d(at + 2 * HALF_BYTES, &map_uv, 0, h * R + kb * 64, full);
+                tma_load_2d(at + 2 * HALF_BYTES + PIECE_BYTES, &map_uv, 64, h * R + kb * 64, full);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc_k = idesc_bf16(ROWS, D, 0), idesc_v = idesc_bf16(ROWS, D, 1);
+            bool ok = true;
+            for (int kb = 0; kb < R / 64 && ok; kb++) {
+                const int s = kb % LE_STAGES;
+                ok = mbar_wait(smem_u32(&bars->full[s]), (uint32_t)(kb / LE_STAGES) & 1u, abort_flag, status, 42);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t at = base + s * LE_STAGE_BYTES;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    umma_ss(tmem, desc_kmajor(at) + 2 * k, desc_kmajor(at + HALF_BYTES) + 2 * k, idesc_k, (kb | k) != 0);
+                    umma_ss(tmem + D, desc_kmajor(at) + 2 * k, desc_mnmajor(at + 2 * HALF_BYTES + k * 2048, PIECE_BYTES), idesc_v, (kb | k) != 0);
+                }
+                umma_commit(smem_u32(&bars->empty[s]));
+            }
+            if (ok) umma_commit(smem_u32(&bars->done));
+        }
+    } else {
+        const int q = warp & 3;
+        float* mine = reinterpret_cast<float*>(aligned) + q * 32 * HW_PITCH;
+        if (mbar_wait(smem_u32(&bars->done), 0, abort_flag, status, 43)) {      // every copy has landed and been read
+            tc_fence_after();
+            const size_t row0 = ((size_t)h * b.n_seqs + seq) * cap + key0 + q * 32;
+#pragma unroll 1
+            for (int half = 0; half < 2; half++) {
+#pragma unroll 1
+                for (int c = 0; c < D; c += 32) {
+                    float v[32];
+                    tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + half * D + c, v);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(mine + lane * HW_PITCH + c + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                }
+                __syncwarp();
+                uint16_t* out = (half ? reinterpret_cast<uint16_t*>(values) : reinterpret_cast<uint16_t*>(keys)) + row0 * D + lane * 4;
+                const float4 sc = half ? *reinterpret_cast<const float4*>(v_scale + h * D + lane * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll 4
+                for (int r = 0; r < 32; r++) {
+                    const float4 v = *reinterpret_cast<const float4*>(mine + r * HW_PITCH + lane * 4);
+                    const int key = key0 + q * 32 + r;
+                    const bool there = key < len && key >= (lo & ~(PAGE - 1));
+                    const uint2 both = half ? make_uint2(pack2_half(v.x * sc.x, v.y * sc.y), pack2_half(v.z * sc.z, v.w * sc.w))
+                                            : make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+                    *reinterpret_cast<uint2*>(out + (size_t)r * D) = there ? both : make_uint2(0u, 0u);
+                }
+                __syncwarp();
+            }
+        }
+    }
+    if (*abort_flag) {
+        unsigned long long w0 = global_ns();
+        while (global_ns() - w0 < 50000ull) __nanosleep(1000);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+    }
+}
+
+// Attention of one head over its expanded keys [128 | the 64 rotated numbers all heads share, in the cache's rows] and values [128], the output
+// times a sigmoid gate.  As attn_prefill_tc2_kernel: two tiles of 128 tokens per block, each with four softmax warps, share every 128 keys, and
+// the tensor pipe alternates between them.  Q of both tiles (96 KB) leaves a ring of eight slots of 16 KB for three pieces of K, [128 keys][64
+// dims], and two of V, [64 keys][128 dims], per 128 keys, in the order in which they are freed: V_j, K_(j+1), V_(j+1), ...; a
+// piece takes the slot of the eighth piece before it.
+// The reference of the exponentials lags a row's maximum by up to 2^8, as there: float16 weights lose nothing by it that bfloat16 ones would.
+//   tensor memory: S of tile x in columns 128 x .. 128 x + 127 (P overwrites the first half), O of tile x in 256 + 128 x ..
+constexpr int LH_Q_BYTES = 3 * HALF_BYTES, LH_SLOTS = 8;
+struct LhBars {
+    unsigned long long q_full;
+    unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];   // of even and odd key blocks
+    unsigned long long s_full[2], p_ready[2], pv_done[2];              // per tile
+    uint32_t tmem_base;
+    int abort_flag;
+};
+constexpr uint32_t LH_SMEM = 1024 + 2 * LH_Q_BYTES + LH_SLOTS * HALF_BYTES + sizeof(LhBars);
+static_assert(LH_SMEM <= 227 * 1024, "shared memory");
+
+__global__ void __launch_bounds__(320, 1)
+latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qr, const __grid_constant__ CUtensorMap map_k,
+                    const __grid_constant__ CUtensorMap map_kr, const __grid_constant__ CUtensorMap map_v, int q_off, __nv_bfloat16* __restrict__ out,
+                    const float* __restrict__ v_unscale, const __nv_bfloat16* __restrict__ gate, int ld_gate, int gate_off, int gate_per_head, const int* __restrict__ page_table,
+                    int max_pages, int n_pages_pool, GfbBatch b, int H, int R, int cap, float scale_log2e, int window, const float* __restrict__ sink,
+                    int n_x, int* status) {
+    extern __shared__ uint8_t smem_raw[];
+    if (threadIdx.x == 0) { prefetch_map(&map_q); prefetch_map(&map_qr); prefetch_map(&map_k); prefetch_map(&map_kr); prefetch_map(&map_v); }
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t qs = base, ring = base + 2 * LH_Q_BYTES;
+    LhBars* bars = reinterpret_cast<LhBars*>(aligned + 2 * LH_Q_BYTES + LH_SLOTS * HALF_BYTES);
+    volatile int* abort_flag = &bars->abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&bars->q_full), 1);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(smem_u32(&bars->k_full[s]), 1);
+            mbar_init(smem_u32(&bars->k_empty[s]), 1);
+            mbar_init(smem_u32(&bars->v_full[s]), 1);
+            mbar_init(smem_u32(&bars->v_empty[s]), 1);
+            mbar_init(smem_u32(&bars->s_full[s]), 1);
+            mbar_init(smem_u32(&bars->p_ready[s]), 4);
+            mbar_init(smem_u32(&bars->pv_done[s]), 1);
+        }
+        bars->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+
+    // the item: two tiles of tokens (the latest of the last sequence first: they see the most keys) of one head
+    const int xi = (int)blockIdx.x / H, head = (int)blockIdx.x - xi * H;
+    int seq = -1, tq0 = 0;
+    {
+        int left = n_x - 1 - xi;
+        for (int i = 0; i < b.n_seqs; i++) {
+            const int nt = (b.cu_seqlens[i + 1] - b.cu_seqlens[i] + 2 * ROWS - 1) / (2 * ROWS);
+            if (left < nt) { seq = i; tq0 = left * 2 * ROWS; break; }
+            left -= nt;
+        }
+    }
+    if (seq >= 0) {
+        const int t_first = b.cu_seqlens[seq], qlen = b.cu_seqlens[seq + 1] - t_first, slot = b.slots[seq], len0 = b.lengths[slot];
+        if (threadIdx.x == 0 && len0 + qlen > cap) gfb_report(status, GFB_ERR_CACHE_RANGE, t_first + qlen - 1, len0 + qlen - 1);   // more than the host's bound
+        // per tile: tokens [tq0 + 128 x, +nq), positions from pos0, key blocks [lo_blk, hi_blk)
+        int nq[2], pos0[2], lo_blk[2], hi_blk[2];
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            nq[x] = min(ROWS, qlen - (tq0 + x * ROWS));
+            pos0[x] = len0 + tq0 + x * ROWS;
+            lo_blk[x] = nq[x] > 0 ? first_key(pos0[x], window, 0) / KEYS : 0;
+            hi_blk[x] = nq[x] > 0 ? (pos0[x] + nq[x] - 1) / KEYS + 1 : 0;
+        }
+        const int blk0 = lo_blk[0], n_iter = max(hi_blk[0], hi_blk[1]) - blk0;      // (the second tile's tokens are later ones)
+        auto active = [&](int x, int j) { return blk0 + j >= lo_blk[x] && blk0 + j < hi_blk[x]; };
+
+        if (warp == 0) {
+            if (lane == 0) {
+                mbar_expect_tx(smem_u32(&bars->q_full), 2 * LH_Q_BYTES);
+#pragma unroll
+                for (int x = 0; x < 2; x++) {                                // rows beyond the batch are filled with zeros
+                    const int t = t_first + tq0 + x * ROWS;
+                    tma_load_2d(qs + x * LH_Q_BYTES, &map_q, q_off + head * 192, t, smem_u32(&bars->q_full));
+                    tma_load_2d(qs + x * LH_Q_BYTES + HALF_BYTES, &map_q, q_off + head * 192 + 64, t, smem_u32(&bars->q_full));
+                    tma_load_2d(qs + x * LH_Q_BYTES + 2 * HALF_BYTES, &map_qr, head * 64, t, smem_u32(&bars->q_full));
+                }
+                const int* pt = page_table + (size_t)slot * max_pages;
+                const int row0 = (head * b.n_seqs + seq) * cap, lo_page = first_key(len0, window, 0) / PAGE, last_page = (len0 + qlen - 1) / PAGE;
+                auto slot_at = [&](int piece) { return ring + (uint32_t)(piece % LH_SLOTS) * HALF_BYTES; };
+                // pieces 5 j .. 5 j + 2 are K of block j, 5 j + 3 and 5 j + 4 its V
+                auto load_k = [&](int j) -> bool {
+                    const uint32_t full = smem_u32(&bars->k_full[j & 1]), ph = ((uint32_t)(j >> 1) & 1u) ^ 1u;
+                    const int row = row0 + (blk0 + j) * KEYS;
+                    if (!mbar_wait(smem_u32(&bars->k_empty[j & 1]), ph, abort_flag, status, 44)) return false;       // K of block j - 2
+                    mbar_expect_tx(full, 3 * HALF_BYTES);
+                    tma_load_2d(slot_at(5 * j), &map_k, 0, row, full);
+                    if (!mbar_wait(smem_u32(&bars->v_empty[j & 1]), ph, abort_flag, status, 45)) return false;       // V of block j - 2
+                    tma_load_2d(slot_at(5 * j + 1), &map_k, 64, row, full);
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {                        // (no such page, or one ahead of the window: any other, masked later)
+                        const int pi = min(max((blk0 + j) * 2 + i, lo_page), last_page);
+                        int page = pi < max_pages ? pt[pi] : -1;
+                        if (page < 0 || page >= n_pages_pool) { gfb_report(status, GFB_ERR_PAGE_TABLE, slot, pi); page = 0; }
+                        tma_load_2d(slot_at(5 * j + 2) + i * PIECE_BYTES, &map_kr, R, page * PAGE, full);
+                    }
+                    return true;
+                };
+                bool ok = load_k(0);
+                for (int j = 0; j < n_iter && ok; j++) {
+                    const uint32_t full = smem_u32(&bars->v_full[j & 1]);
+                    const int row = row0 + (blk0 + j) * KEYS;
+                    if (j > 0) ok = mbar_wait(smem_u32(&bars->k_empty[(j - 1) & 1]), (uint32_t)((j - 1) >> 1) & 1u, abort_flag, status, 46);   // K of block j - 1
+                    if (!ok) break;
+                    mbar_expect_tx(full, 2 * HALF_BYTES);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        tma_load_2d(slot_at(5 * j + 3 + (i >> 1)) + (i & 1) * PIECE_BYTES, &map_v, (i & 1) * 64, row + (i >> 1) * 64, full);
+                    if (j + 1 < n_iter) ok = load_k(j + 1);
+                }
+            }
+        } else if (warp == 1) {
+            if (lane == 0) {
+                constexpr uint32_t idesc_s = idesc_bf16(ROWS, KEYS, 0), idesc_o = idesc_f16(ROWS, D, 1);
+                uint32_t n_pv[2] = {0, 0};                                   // P V products issued per tile
+                bool ok = mbar_wait(smem_u32(&bars->q_full), 0, abort_flag, status, 47);
+                auto slot_at = [&](int piece) { return ring + (uint32_t)(piece % LH_SLOTS) * HALF_BYTES; };
+                auto issue_s = [&](int x, int j) {                           // K of block j is known to be loaded
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        const uint64_t da = desc_kmajor(qs + x * LH_Q_BYTES + c * HALF_BYTES), db = desc_kmajor(slot_at(5 * j + c));
+#pragma unroll
+                        for (int k = 0; k < 4; k++) umma_ss(tmem + 128 * x, da + 2 * k, db + 2 * k, idesc_s, (c | k) != 0);
+                    }
+                    umma_commit(smem_u32(&bars->s_full[x]));
+                };
+                auto k_ready = [&](int j) { return mbar_wait(smem_u32(&bars->k_full[j & 1]), (uint32_t)(j >> 1) & 1u, abort_flag, status, 48); };
+                ok = ok && k_ready(0);
+                if (ok) {
+                    tc_fence_after();
+                    if (active(0, 0)) issue_s(0, 0);
+                    if (active(1, 0)) issue_s(1, 0);
+                    umma_commit(smem_u32(&bars->k_empty[0]));
+                }
+                for (int j = 0; j < n_iter && ok; j++) {
+                    bool k_next = false;                                     // whether K of block j + 1 has been waited for
+                    ok = mbar_wait(smem_u32(&bars->v_full[j & 1]), (uint32_t)(j >> 1) & 1u, abort_flag, status, 49);
+#pragma unroll
+                    for (int x = 0; x < 2 && ok; x++) {
+                        if (active(x, j)) {
+                            ok = mbar_wait(smem_u32(&bars->p_ready[x]), n_pv[x] & 1u, abort_flag, status, 50);
+                            if (!ok) break;
+                            tc_fence_after();
+#pragma unroll
+                            for (int kk = 0; kk < 8; kk++)                   // 16 keys per MMA: 8 columns of P, 2 KB of either half of the dims
+                                umma_ts(tmem + 256 + 128 * x, tmem + 128 * x + kk * 8,
+                                        desc_mnmajor(slot_at(5 * j + 3 + (kk >> 2)) + (kk & 3) * 2048, PIECE_BYTES), idesc_o, (n_pv[x] | (uint32_t)kk) != 0);
+                            umma_commit(smem_u32(&bars->pv_done[x]));
+                            n_pv[x]++;
+                        }
+                        if (j + 1 < n_iter && active(x, j + 1)) {            // the tile's next scores, behind its P V
+                            if (!k_next) { ok = k_ready(j + 1); k_next = true; if (!ok) break; tc_fence_after(); }
+                            issue_s(x, j + 1);
+                        }
+                    }
+                    if (!ok) break;
+                    umma_commit(smem_u32(&bars->v_empty[j & 1]));
+                    if (j + 1 < n_iter) {
+                        if (!k_next) { ok = k_ready(j + 1); if (!ok) break; }
+                        umma_commit(smem_u32(&bars->k_empty[(j + 1) & 1]));
+                    }
+                }
+            }
+        } else {
+            const int x = (warp - 2) >> 2;                                   // warps 2..5: tile 0, warps 6..9: tile 1
+            const int q = warp & 3, r = q * 32 + lane;
+            const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
+            const uint32_t col_s = 128 * x, col_o = 256 + 128 * x;
+            const bool row_ok = r < nq[x];
+            const int row_pos = pos0[x] + r, row_lo = first_key(row_pos, window, 0), last_lo = first_key(pos0[x] + max(nq[x], 1) - 1, window, 0);
+            float m_run = -INFINITY, l_run = 0.f;
+            uint32_t n_done = 0;                                             // blocks of this tile finished
+            bool ok = true;
+            for (int j = 0; j < n_iter && ok; j++) {
+                if (!active(x, j)) continue;
+                const int key0 = (blk0 + j) * KEYS;
+                ok = mbar_wait(smem_u32(&bars->s_full[x]), n_done & 1u, abort_flag, status, 51);
+                if (!ok) break;
+                tc_fence_after();
+                float v[4][32];
+                tmem_ld_row128(lane_base + col_s, v);
+                if (key0 + KEYS - 1 > pos0[x] || key0 < last_lo || nq[x] < ROWS) {
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+#pragma unroll
+                        for (int i = 0; i < 32; i++) {
+                            const int kj = key0 + c * 32 + i;
+                            if (!(row_ok && kj <= row_pos && kj >= row_lo)) v[c][i] = -INFINITY;
+                        }
+                }
+                float mx4[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    mx4[c] = fmaxf(v[c][0], v[c][1]);
+#pragma unroll
+                    for (int i = 2; i < 32; i += 2) mx4[c] = max3(mx4[c], v[c][i], v[c][i + 1]);
+                }
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                float m_new = m_run;
+                if (mx > m_run && (m_run == -INFINITY || (mx - m_run) * scale_log2e > 8.f)) m_new = mx;
+                const float corr = (m_run == -INFINITY || m_new == m_run) ? 1.f : fast_exp2((m_run - m_new) * scale_log2e);
+                const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * scale_log2e;
+                float rsum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    uint32_t pk[16];
+                    float odd = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float a0, a1;
+                        fma2(v[c][i], v[c][i + 1], scale_log2e, mneg, a0, a1);
+                        const float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
+                        add2(rsum[c], odd, p0, p1);
+                        pk[i >> 1] = pack2_half(p0, p1);
+                    }
+                    rsum[c] += odd;
+                    tmem_st16(lane_base + col_s + c * 16, pk);               // (all of this row's scores are in registers by now)
+                }
+                // O follows a new reference, rarely (S of this block was issued behind the tile's previous P V, so that the wait only orders the accesses)
+                if (n_done > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
+                    ok = mbar_wait(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 52);
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < 4; c++) {
+                        float o[32];
+                        tmem_ld32(lane_base + col_o + c * 32, o);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) o[i] *= corr;
+                        tmem_st32(lane_base + col_o + c * 32, o);
+                    }
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&bars->p_ready[x]));
+                l_run = l_run * corr + (rsum[0] + rsum[1]) + (rsum[2] + rsum[3]);
+                m_run = m_new;
+                n_done++;
+            }
+            if (ok && n_done > 0) ok = mbar_wait(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 53);
+            if (ok && n_done > 0) {
+                tc_fence_after();
+                if (sink != nullptr && m_run != -INFINITY) l_run += fast_exp2(sink[head] * 1.4426950408889634f - m_run * scale_log2e);
+                const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+                const size_t t = (size_t)(t_first + tq0 + x * ROWS + (row_ok ? r : 0));
+                __nv_bfloat16* dst = out + (t * H + head) * D;
+                const __nv_bfloat16* gt = gate + t * ld_gate + gate_off;
+                const float per_head = gate_per_head ? 1.0f / (1.0f + expf(-__bfloat162float(gt[head]))) : 1.f;
+#pragma unroll 1
+                for (int c = 0; c < 4; c++) {
+                    float o[32];
+                    tmem_ld32(lane_base + col_o + c * 32, o);
+                    if (row_ok) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 8) {
+                            const float4 u0 = *reinterpret_cast<const float4*>(v_unscale + head * D + c * 32 + i);
+                            const float4 u1 = *reinterpret_cast<const float4*>(v_unscale + head * D + c * 32 + i + 4);
+                            const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+                            float y[8];
+#pragma unroll
+                            for (int e = 0; e < 8; e++) y[e] = o[i + e] * inv * u[e] * per_head;
+                            if (!gate_per_head) {
+                                const uint4 g8 = *reinterpret_cast<const uint4*>(gt + head * D + c * 32 + i);
+                                const uint32_t g4[4] = {g8.x, g8.y, g8.z, g8.w};
+#pragma unroll
+                                for (int e = 0; e < 4; e++) {
+                                    y[2 * e] *= 1.0f / (1.0f + expf(-__uint_as_float(g4[e] << 16)));
+                                    y[2 * e + 1] *= 1.0f / (1.0f + expf(-__uint_as_float(g4[e] & 0xffff0000u)));
+                                }
+                            }
+                            *reinterpret_cast<uint4*>(dst + c * 32 + i) = make_uint4(pack2(y[0], y[1]), pack2(y[2], y[3]), pack2(y[4], y[5]), pack2(y[6], y[7]));
+                        }
+                    }
+                }
+            }
+        }
+    }
+    if (*abort_flag) {
+        unsigned long long w0 = global_ns();
+        while (global_ns() - w0 < 50000ull) __nanosleep(1000);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1801,4 +2259,50 @@ GFB_API int gfb_headwise_linear_tc(const void* in, int ld_in, int in_off, int in
     e = gfb_launch(headwise_tc_kernel, dim3((n_tokens + ROWS - 1) / ROWS, H, N / 128), dim3(192), HW_SMEM, stream, ma, mw, in_off, in_stride,
                    (__nv_bfloat16*)out, ld_out, out_off, out_stride, (const __nv_bfloat16*)gate, ld_gate, gate_off, gate_cols, n_tokens, K, N, status);
     return gfb_check(e, "gfb_headwise_linear_tc");
+}
+
+// Prompts with every head's keys and values expanded (head and value size 128, 64 rotated numbers, rank R a multiple of 64).  proj bfloat16 [T, ld]:
+// at q_off H heads of 192 query numbers of which the first 128 are read, at gate_off H gates (gate_per_head) or H * 128; q_rot [T, H, 64]: the
+// rotated query parts; wuk [H, 128, R], wuv [H, R, 128]; v_scale float32 [2][H * 128]: powers of two and
+// their reciprocals, by which the values stay within float16; keys, values [H, n_seqs * cap, 128]: scratch, cap a multiple of 128 that no sequence's length
+// exceeds; out [T, H * 128].  The cache holds the new tokens' rows already.  Everything 16-byte aligned, ld, q_off and gate_off multiples of 8.
+GFB_API int gfb_latent_expanded(const void* proj, int ld, int q_off, int gate_off, int gate_per_head, const void* q_rot, const void* wuk, const void* wuv,
+                                const float* v_scale, void* keys, void* values, void* out, void* k_pool, const int* page_table, int max_pages, int page_size, int n_pages,
+                                const int* cu_seqlens, const int* tok_seq, const int* slots, const int* lengths, int n_seqs, int n_tokens, int H, int R,
+                                int cap, float scale, int window, const float* sink, int* status, cudaStream_t stream) {
+    if (n_tokens <= 0 || H <= 0) return 0;
+    if (page_size != PAGE || R < 64 || R % 64 || cap < KEYS || cap % KEYS || !(scale > 0.f) || ld % 8 || q_off % 8 || gate_off % 8)
+        return gfb_fail("gfb_latent_expanded: rank %d, pages of %d, rows of %d, scale %f", R, page_size, ld, scale);
+    if (((uintptr_t)proj | (uintptr_t)q_rot | (uintptr_t)wuk | (uintptr_t)wuv | (uintptr_t)v_scale | (uintptr_t)keys | (uintptr_t)values | (uintptr_t)out | (uintptr_t)k_pool) & 15)
+        return gfb_fail("gfb_latent_expanded: operands must be 16-byte aligned");
+    const long long rows = (long long)n_seqs * cap, n_x = ((long long)n_tokens + 2 * ROWS - 1) / (2 * ROWS) + n_seqs;   // an upper bound of the tiles
+    if ((long long)n_pages * PAGE > 2147483647LL || rows * H > 2147483647LL || (long long)H * R > 2147483647LL || n_x * H > 2147483647LL)
+        return gfb_fail("gfb_latent_expanded: %d pages, %lld rows of %d heads do not fit the 32-bit row coordinate of a tensor map", n_pages, rows, H);
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return gfb_fail("gfb_latent_expanded: the driver does not export cuTensorMapEncodeTiled");
+    CUtensorMap maps[7];
+    const struct { const void* p; long long cols, rows; int box; } what[7] = {
+        {k_pool, R + 64, (long long)n_pages * PAGE, PAGE}, {wuk, R, (long long)H * D, D}, {wuv, D, (long long)H * R, 64}, {proj, ld, n_tokens, ROWS},
+        {q_rot, (long long)H * 64, n_tokens, ROWS}, {keys, D, rows * H, KEYS}, {values, D, rows * H, 64}};
+    for (int i = 0; i < 7; i++) {
+        cuuint64_t dims[2] = {(cuuint64_t)what[i].cols, (cuuint64_t)what[i].rows};
+        cuuint64_t strides[1] = {dims[0] * 2};
+        cuuint32_t box[2] = {64, (cuuint32_t)what[i].box};
+        cuuint32_t es[2] = {1, 1};
+        CUresult r = enc(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(what[i].p), dims, strides, box, es,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return gfb_fail("gfb_latent_expanded: tensor map %d refused (%d)", i, (int)r);
+    }
+    GfbBatch b{cu_seqlens, tok_seq, slots, lengths, n_seqs, n_tokens};
+    cudaError_t e = cudaFuncSetAttribute(latent_expand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LE_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(latent_heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LH_SMEM);
+    if (e != cudaSuccess) return gfb_fail("gfb_latent_expanded: %u and %u bytes of shared memory refused: %s", LE_SMEM, LH_SMEM, cudaGetErrorString(e));
+    e = gfb_launch(latent_expand_kernel, dim3((unsigned)(rows / KEYS * H)), dim3(192), LE_SMEM, stream, maps[0], maps[1], maps[2], (__nv_bfloat16*)keys,
+                   (__half*)values, v_scale, page_table, max_pages, n_pages, b, H, R, cap, window, status);
+    if (gfb_check(e, "gfb_latent_expanded (keys and values)")) return 1;
+    e = gfb_launch(latent_heads_kernel, dim3((unsigned)(n_x * H)), dim3(320), LH_SMEM, stream, maps[3], maps[4], maps[5], maps[0], maps[6], q_off,
+                   (__nv_bfloat16*)out, v_scale + (size_t)H * D, (const __nv_bfloat16*)proj, ld, gate_off, gate_per_head, page_table, max_pages, n_pages, b, H, R, cap,
+                   scale * 1.4426950408889634f, window, sink, (int)n_x, status);
+    return gfb_check(e, "gfb_latent_expanded");
 }

@@ -30,7 +30,7 @@ __device__ __forceinline__ void pair_index(int i, int rot, int pairing, int& a, 
 }
 
 template <typename T>
-__global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int q_off, int kv_off, T* __restrict__ q_out,
+__global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int q_off, int kv_off, T* __restrict__ q_out, int q_pitch, int q_at,
                                       GfbPagedKV kv, GfbBatch b, const float* __restrict__ table, int table_len,
                                       const void* __restrict__ norm_w, int w_dt, float eps, int H, int d, int rot, int rank,
                                       int pairing, int append, int* status) {
@@ -48,7 +48,6 @@ __global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int q_o
     const int half = rot / 2;
 
     // every head's rotated query part
-    const int qrow = rank + rot;
     for (int i = threadIdx.x; i < H * half; i += blockDim.x) {
         const int h = i / half, p = i - h * half;
         int ia, ib;
@@ -56,7 +55,7 @@ __global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int q_o
         const T* q = row + q_off + (size_t)h * (d + rot) + d;
         const float u = gfb_to_f32(q[ia]), v = gfb_to_f32(q[ib]);
         const float c = cs[2 * p], sn = cs[2 * p + 1];
-        T* o = q_out + ((size_t)t * H + h) * qrow + rank;
+        T* o = q_out + ((size_t)t * H + h) * q_pitch + q_at;
         o[ia] = gfb_from_f32<T>(u * c - v * sn);
         o[ib] = gfb_from_f32<T>(v * c + u * sn);
     }
@@ -75,7 +74,7 @@ __global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int q_o
     ss = gfb_block_sum(ss, scratch);
     if (page < 0) return;
     const float r = 1.0f / sqrtf(ss / (float)rank + eps);
-    T* krow = (T*)kv.k_pool + ((size_t)page * kv.page_size + (pos % kv.page_size)) * qrow;
+    T* krow = (T*)kv.k_pool + ((size_t)page * kv.page_size + (pos % kv.page_size)) * (rank + rot);
     for (int i = threadIdx.x; i < rank; i += blockDim.x)
         krow[i] = gfb_from_f32<T>(gfb_to_f32(dkv[i]) * r * ld_any(norm_w, w_dt, i));
     for (int p = threadIdx.x; p < half; p += blockDim.x) {
@@ -89,9 +88,9 @@ __global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int q_o
 }
 
 // src [T, ld]: at q_off H heads of (d + rot) numbers (d unrotated, then rot rotated), at kv_off rank + rot numbers.
-// q_out [T, H, rank + rot]: only the last rot numbers of every head are written here.  The cache entry has one
+// q_out [T, H, q_pitch]: only rot numbers of every head, from q_at on, are written here.  The cache entry has one
 // key head of rank + rot numbers per token (its value pool is not used).  table float32 [table_len, rot/2, 2].
-GFB_API int gfb_latent_prepare(const void* src, int dt, int ld, int q_off, int kv_off, void* q_out, void* k_pool,
+GFB_API int gfb_latent_prepare(const void* src, int dt, int ld, int q_off, int kv_off, void* q_out, int q_pitch, int q_at, void* k_pool,
                                const int* page_table, int max_pages, int page_size, int n_pages, const int* cu_seqlens,
                                const int* tok_seq, const int* slots, const int* lengths, int n_seqs, int n_tokens,
                                const float* table, int table_len, const void* norm_w, int w_dt, float eps, int H, int d,
@@ -103,10 +102,10 @@ GFB_API int gfb_latent_prepare(const void* src, int dt, int ld, int q_off, int k
     cudaError_t e;
     if (dt == GFB_BF16)
         e = gfb_launch(latent_prepare_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(128), 0, stream, (const __nv_bfloat16*)src, ld, q_off,
-                       kv_off, (__nv_bfloat16*)q_out, kv, b, table, table_len, norm_w, w_dt, eps, H, d, rot, rank, pairing, append, status);
+                       kv_off, (__nv_bfloat16*)q_out, q_pitch, q_at, kv, b, table, table_len, norm_w, w_dt, eps, H, d, rot, rank, pairing, append, status);
     else if (dt == GFB_F32)
         e = gfb_launch(latent_prepare_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, (const float*)src, ld, q_off, kv_off,
-                       (float*)q_out, kv, b, table, table_len, norm_w, w_dt, eps, H, d, rot, rank, pairing, append, status);
+                       (float*)q_out, q_pitch, q_at, kv, b, table, table_len, norm_w, w_dt, eps, H, d, rot, rank, pairing, append, status);
     else
         return gfb_fail("gfb_latent_prepare: unknown type %d", dt);
     return gfb_check(e, "gfb_latent_prepare");

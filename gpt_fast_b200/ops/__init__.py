@@ -176,6 +176,26 @@ def latent_prepare(src, q_off: int, kv_off: int, q_out, kv: PagedKV, batch: Batc
                                     table, pairing, append)
 
 
+def value_scales(wuv, norm_weight):
+    """[2, n_head * v_head_dim]: the power of two that takes the largest number a value column can hold, given that a latent is a normed vector times
+    norm_weight, to between 2^14 and 2^15, and its reciprocal.  wuv [n_head, rank, v_head_dim]."""
+    bound = wuv.shape[1] ** 0.5 * (wuv.float().abs() * norm_weight.float().abs().view(1, -1, 1)).sum(1).flatten()
+    power = torch.where(bound.isfinite() & (bound > 0), 14 - bound.clamp(2.0 ** -100, 2.0 ** 100).log2().floor(), 0.0)
+    return torch.stack([torch.exp2(power), torch.exp2(-power)])
+
+
+def latent_expanded(proj, q_off: int, kv_off: int, gate_off: int, gate_per_head: bool, out, kv: PagedKV, batch: BatchMeta, n_head: int, head_dim: int,
+                    rot_dim: int, v_head_dim: int, rank: int, norm_weight, eps: float, table, pairing: str, append: bool, wuk, wuv, v_scale, scale: float,
+                    window: Optional[int] = None, sink=None) -> bool:
+    """A step's latent attention in one call: `latent_prepare`, then causal attention of every head over keys and values expanded
+    from the cached latents (wuk [n_head, head_dim, rank], wuv [n_head, rank, v_head_dim]; v_scale from `value_scales`) and, as 32-bit numbers, times the sigmoid of the gates at
+    column gate_off of proj, written to out [T, n_head * v_head_dim].  The kernels decide where that is the faster form; elsewhere, and
+    where a set of kernels has none, nothing is done and False returned."""
+    fused = getattr(kernels(), "latent_expanded", None)
+    return fused is not None and fused(proj, q_off, kv_off, gate_off, gate_per_head, out, kv, batch, n_head, head_dim, rot_dim, v_head_dim, rank,
+                                       norm_weight, eps, table, pairing, append, wuk, wuv, v_scale, scale, window, sink)
+
+
 def headwise_linear(a, w, out, n_head: int, k: int, n: int, a_off: int = 0, a_stride: Optional[int] = None, out_off: int = 0,
                     out_stride: Optional[int] = None, gate=None, gate_off: int = 0, gate_per_head: bool = False):
     """A product with a weight per head: out[t, h, :] = a[t, h, :] W_h.  a [T, Wa]: head h's k inputs start at column

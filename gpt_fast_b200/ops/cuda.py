@@ -139,6 +139,12 @@ def ssd_in_chunks(n_tokens: int, n_seqs: int, longest: int, n_head: int, head_di
     return max(longest, busy) + 2.3 * w * n_seqs >= line * (1 + each * chunks)
 
 
+def expand_latents(n_tokens: int, n_seqs: int, longest: int, cap: int) -> bool:
+    """Whether a prompt's latents are expanded to keys and values per head: where its keys, at most `cap` for every sequence, are mostly its own
+    new tokens.  A cached key costs 262,144 operations per head to expand and saves 1,536 for every query that sees it."""
+    return longest > 1 and n_seqs * cap <= 3 * n_tokens + 128 * n_seqs
+
+
 class CudaKernels:
     """The operations of `ops`, bound to the sm_100a libraries.  A library is
     compiled and loaded when its first function is needed."""
@@ -433,13 +439,14 @@ class CudaKernels:
                    _stream())
 
     def latent_prepare(self, src, q_off, kv_off, q_out, kv, batch, n_head, head_dim, rot_dim, rank, norm_weight, eps, table,
-                       pairing="interleaved", append=True):
+                       pairing="interleaved", append=True, rotated_only=False):
         T = batch.n_tokens
+        q_at = 0 if rotated_only else rank              # (rotated_only: q_out holds the rotated parts and nothing else)
         W = src.shape[1]
         _need(src, q_out.dtype, (T, W), "projection")
         if max(q_off + n_head * (head_dim + rot_dim), kv_off + rank + rot_dim) > W:
             _fail(f"queries at {q_off} and the down projection at {kv_off} do not fit rows of {W}")
-        _need(q_out, shape=(T, n_head, rank + rot_dim), name="q_out")
+        _need(q_out, shape=(T, n_head, q_at + rot_dim), name="q_out")
         _need(norm_weight, shape=(rank,), name="latent norm weight")
         _need(table, torch.float32, name="rotary table")
         if table.shape[1] * 2 != rot_dim:
@@ -449,10 +456,39 @@ class CudaKernels:
             if tuple(kv.k_pool.shape[1:]) != (1, kv.page_size, rank + rot_dim):
                 _fail(f"cache pages are {tuple(kv.k_pool.shape[1:])}, the layer needs {(1, kv.page_size, rank + rot_dim)}")
         self._call("latent", "gfb_latent_prepare", _ptr(src), c_int(_dt(src)), c_int(W), c_int(q_off), c_int(kv_off), _ptr(q_out),
-                   _ptr(kv.k_pool), _ptr(kv.page_table), c_int(kv.page_table.shape[1]), c_int(kv.page_size), c_int(kv.k_pool.shape[0]),
-                   *self._batch_args(batch), _ptr(table), c_int(table.shape[0]), _ptr(norm_weight), c_int(_dt(norm_weight)),
+                   c_int(q_at + rot_dim), c_int(q_at), _ptr(kv.k_pool), _ptr(kv.page_table), c_int(kv.page_table.shape[1]), c_int(kv.page_size),
+                   c_int(kv.k_pool.shape[0]), *self._batch_args(batch), _ptr(table), c_int(table.shape[0]), _ptr(norm_weight), c_int(_dt(norm_weight)),
                    c_float(eps), c_int(n_head), c_int(head_dim), c_int(rot_dim), c_int(rank), c_int(_PAIRING[pairing]),
                    c_int(1 if append else 0), _ptr(batch.status), _stream())
+
+    def latent_expanded(self, proj, q_off, kv_off, gate_off, gate_per_head, out, kv, batch, n_head, head_dim, rot_dim, v_head_dim, rank, norm_weight,
+                        eps, table, pairing, append, wuk, wuv, v_scale, scale, window=None, sink=None) -> bool:
+        """All of a prompt's latent attention between the input and the output product, with keys and values written out per head.  Returns False, having
+        done nothing, where attention on the latent itself is to run."""
+        T, W = proj.shape
+        H, R = n_head, rank
+        cap = -(-max(int(batch.max_kv_len), 1) // 128) * 128
+        if not (proj.dtype == torch.bfloat16 and expand_latents(T, batch.n_seqs, batch.max_q_len, cap)
+                and head_dim == 128 and v_head_dim == 128 and rot_dim == 64 and R % 64 == 0 and kv.page_size == 64 and scale > 0
+                and (W | q_off | gate_off) % 8 == 0 and (proj.data_ptr() | wuk.data_ptr() | wuv.data_ptr() | out.data_ptr() | kv.k_pool.data_ptr()) % 16 == 0
+                and H * max(R, batch.n_seqs * cap) < 2 ** 31):
+            return False
+        _need(wuk, proj.dtype, (H, 128, R), "key expansion")
+        _need(wuv, proj.dtype, (H, R, 128), "value expansion")
+        _need(v_scale, torch.float32, (2, H * 128), "scales of the values")
+        _need(out, proj.dtype, (T, H * 128), "attention output")
+        if gate_off + (H if gate_per_head else H * 128) > W:
+            _fail(f"gates at {gate_off} do not fit rows of {W}")
+        if sink is not None:
+            _need(sink, torch.float32, (H,), "sink")
+        q_rot = torch.empty(T, H, rot_dim, dtype=proj.dtype, device=proj.device)
+        self.latent_prepare(proj, q_off, kv_off, q_rot, kv, batch, H, head_dim, rot_dim, R, norm_weight, eps, table, pairing, append, rotated_only=True)
+        keys, values = torch.empty(2, H, batch.n_seqs * cap, 128, dtype=proj.dtype, device=proj.device)
+        self._call("attention_tc", "gfb_latent_expanded", _ptr(proj), c_int(W), c_int(q_off), c_int(gate_off), c_int(1 if gate_per_head else 0), _ptr(q_rot),
+                   _ptr(wuk), _ptr(wuv), _ptr(v_scale), _ptr(keys), _ptr(values), _ptr(out), _ptr(kv.k_pool), _ptr(kv.page_table), c_int(kv.page_table.shape[1]),
+                   c_int(kv.page_size), c_int(kv.k_pool.shape[0]), *self._batch_args(batch), c_int(H), c_int(R), c_int(cap), c_float(scale),
+                   c_int(window or 0), _ptr(sink), _ptr(batch.status), _stream())
+        return True
 
     # up to this many tokens the smaller tiles of the mma.sync form (16 heads, 128 -> 512, us with it | on tcgen05: 16 tokens 22.1 | 22.9,
     # 48 23.4 | 23.4, 64 26.8 | 22.8, 256 29.2 | 18.9)

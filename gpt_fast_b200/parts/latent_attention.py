@@ -13,7 +13,8 @@ exponential joins the softmax denominator without a value).
 Only (c, rot(k_r)) is cached: one row of rank + rot_dim numbers per token.  Since k_h and v_h are linear in c, the
 mixer attends on the latent itself: the query of head h becomes [Wuk,h^T q_u,h | rot(q_r,h)] (rank + rot_dim numbers),
 all heads read the same cached rows as keys and their first rank numbers as values, and Wuv,h expands the attended
-latent afterwards.  Nothing is ever expanded per cached token, in prompts or in decoding."""
+latent afterwards: nothing is expanded per cached token.  Where most keys are a prompt's own new tokens, expanding those takes fewer
+operations, and the kernels do that instead (`ops.latent_expanded`); what is cached is the same."""
 from typing import Optional
 
 import torch
@@ -36,7 +37,7 @@ class LatentAttention:
         self.scale, self.eps, self.dtype, self.position, self.window = float(scale), float(eps), dtype, position, window
         self.head_gate, self.has_sink = bool(head_gate), bool(sink)
         self.gates = n_head if head_gate else n_head * v_head_dim
-        self.w_in = self.wuk = self.wuv = self.wo = self.latent_norm = self.sink = None
+        self.w_in = self.wuk = self.wuv = self.v_scale = self.wo = self.latent_norm = self.sink = None
 
     def param_specs(self):
         H, d, r, dv, R, D = self.n_head, self.head_dim, self.rot_dim, self.v_head_dim, self.rank, self.dim
@@ -53,6 +54,7 @@ class LatentAttention:
         self.wuk = tensors["wuk"].view(self.n_head, self.head_dim, self.rank)         # [H][k = head_dim][n = rank]
         self.wuv = tensors["wuv"].view(self.n_head, self.v_head_dim, self.rank).transpose(1, 2).contiguous()   # [H][k = rank][n = v_head_dim]
         self.wo, self.latent_norm = tensors["wo"], tensors["latent_norm"]
+        self.v_scale = ops.value_scales(self.wuv, self.latent_norm)
         if self.has_sink:
             self._sink_stored = tensors["sink"]
             self.sink = tensors["sink"].float().contiguous()
@@ -76,12 +78,16 @@ class LatentAttention:
         q_off, kv_off, g_off = 0, H * (d + r), H * (d + r) + R + r
         proj = torch.empty(T, self.w_in.shape[0], dtype=self.dtype, device=h.device)
         ops.linear(h, self.w_in, proj)
+        y = torch.empty(T, H * dv, dtype=self.dtype, device=h.device)
+        if ops.latent_expanded(proj, q_off, kv_off, g_off, self.head_gate, y, view.kv, batch, H, d, r, dv, R, self.latent_norm, self.eps,
+                               self.position.table, self.position.pairing, append, self.wuk, self.wuv, self.v_scale, self.scale, self.window, self.sink):
+            as_residual(residual).add_linear(y, self.wo)
+            return
         q = torch.empty(T, H, R + r, dtype=self.dtype, device=h.device)
         ops.latent_prepare(proj, q_off, kv_off, q, view.kv, batch, H, d, r, R, self.latent_norm, self.eps,
                            self.position.table, self.position.pairing, append)
         ops.headwise_linear(proj, self.wuk, q.view(T, H * (R + r)), H, d, R, a_off=q_off, a_stride=d + r, out_stride=R + r)
         o = torch.empty(T, H * R, dtype=self.dtype, device=h.device)
         ops.attention(q, view.kv, batch, o, H, 1, R + r, self.scale, self.window, sink=self.sink, v_head_dim=R, values_in_keys=True)
-        y = torch.empty(T, H * dv, dtype=self.dtype, device=h.device)
         ops.headwise_linear(o, self.wuv, y, H, R, dv, gate=proj, gate_off=g_off, gate_per_head=self.head_gate)
         as_residual(residual).add_linear(y, self.wo)
