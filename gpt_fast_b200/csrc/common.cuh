@@ -75,6 +75,30 @@ static int gfb_pdl_state = -1;
 __device__ __forceinline__ void gfb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void gfb_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ---- blocks of a cluster -------------------------------------------------------------
+// Every thread of every block comes here; what they wrote before is visible behind it.
+__device__ __forceinline__ void gfb_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// four (two) neighbouring 32-bit numbers out of block `rank`'s shared memory, at the address that `mine` has in this block's
+__device__ __forceinline__ uint32_t gfb_cluster_addr(const void* mine, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float4 gfb_cluster_load4(const void* mine, uint32_t rank) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(gfb_cluster_addr(mine, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 gfb_cluster_load2(const void* mine, uint32_t rank) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(gfb_cluster_addr(mine, rank)) : "memory");
+    return v;
+}
+
 static inline bool gfb_pdl_enabled() {
     if (gfb_pdl_state < 0) {
         const char* e = getenv("GFB_NO_PDL");
@@ -99,10 +123,10 @@ static inline cudaError_t gfb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// The same with a thread-block cluster of `cluster_x` blocks along x (grid.x must be a multiple of it).
+// The same with thread-block clusters (the grid must be a multiple of them).
 template <typename... KArgs, typename... Args>
-static inline cudaError_t gfb_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                             unsigned cluster_x, Args... args) {
+static inline cudaError_t gfb_launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                              dim3 cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -110,14 +134,21 @@ static inline cudaError_t gfb_launch_cluster(void (*kernel)(KArgs...), dim3 grid
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster_x;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = cluster.x;
+    attr[0].val.clusterDim.y = cluster.y;
+    attr[0].val.clusterDim.z = cluster.z;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = gfb_pdl_enabled() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// ... of `cluster_x` blocks along x.
+template <typename... KArgs, typename... Args>
+static inline cudaError_t gfb_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                             unsigned cluster_x, Args... args) {
+    return gfb_launch_clusters(kernel, grid, block, smem, stream, dim3(cluster_x, 1, 1), args...);
 }
 
 static inline int gfb_check(cudaError_t e, const char* what) {
