@@ -179,8 +179,8 @@ def latent_prepare(src, q_off: int, kv_off: int, q_out, kv: PagedKV, batch: Batc
 def value_scales(wuv, norm_weight):
     """[2, n_head * v_head_dim]: the power of two that takes the largest number a value column can hold, given that a latent is a normed vector times
     norm_weight, to between 2^14 and 2^15, and its reciprocal.  wuv [n_head, rank, v_head_dim]."""
-    bound = wuv.shape[1] ** 0.5 * (wuv.float().abs() * norm_weight.float().abs().view(1, -1, 1)).sum(1).flatten()
-    power = torch.where(bound.isfinite() & (bound > 0), 14 - bound.clamp(2.0 ** -100, 2.0 ** 100).log2().floor(), 0.0)
+    bound = torch.matmul(norm_weight.abs().float(), wuv.abs().float()).flatten() * wuv.shape[1] ** 0.5
+    power = 14 - bound.nan_to_num(1.0, 1.0).clamp(2.0 ** -100, 2.0 ** 100).log2().floor()
     return torch.stack([torch.exp2(power), torch.exp2(-power)])
 
 
