@@ -133,7 +133,7 @@ def test_scales_of_values():
     fine = (bound > 2.0 ** -100) & (bound < 2.0 ** 100)                    # (not the columns of zeros and of an infinity)
     assert bool((s * back == 1.0).all()) and bool((s.log2() == s.log2().round()).all())
     assert bool(((bound * s)[fine] < 2.0 ** 15).all()) and bool(((bound * s)[fine] >= 2.0 ** 14 * 0.999).all())
-assert bool(s.isfinite().all()) and float(s.min()) > 0.0
+    assert bool(s.isfinite().all()) and float(s.min()) > 0.0
 
 
 @pytest.mark.gpu
