@@ -139,6 +139,14 @@ def ssd_in_chunks(n_tokens: int, n_seqs: int, longest: int, n_head: int, head_di
     return max(longest, busy) + 2.3 * w * n_seqs >= line * (1 + each * chunks)
 
 
+def rows_share_keys(rows: int, longest: int, max_kv_len: int, line: int) -> bool:
+    """Whether the rows (token, head) of a step's 32-bit attention share the keys and values of sixteen rows per block; the bits are the same.  A block
+    then has sixteen rows' work in a row, so it takes rows enough, fewer where keys are many.  us shared | a block per row: 64 tokens of
+    24 heads over 8 18.9 | 19.1, of 16 over 16 14.9 | 12.5; 16 tokens behind 2,000, 16 heads 160 | 178, four times 16 behind 500 62 | 92; 2 tokens
+    behind 1,000 98 | 101, alone 11.3 | 6.7; 512 tokens of 24 heads 148 | 572."""
+    return longest > 1 and (rows >= line or (rows * 6 >= line and max_kv_len > 512))
+
+
 def expand_latents(n_tokens: int, n_seqs: int, longest: int, cap: int) -> bool:
     """Whether a prompt's latents are expanded to keys and values per head: where its keys, at most `cap` for every sequence, are mostly its own
     new tokens.  A cached key costs 262,144 operations per head to expand and saves 1,536 for every query that sees it."""
@@ -1129,11 +1137,15 @@ class CudaKernels:
             return self._attention_bf16(q, kv, batch, out, n_head, n_kv, head_dim, scale, window, chunk=chunk, sink=sink,
                                         bias=bias, slopes=slopes, softcap=softcap, keep_first=keep_first)
         self._call("attention_generic", "gfb_attention_generic", _ptr(q), _ptr(out), c_int(_dt(q)),
-                   *self._kv_args(kv), *self._batch_args(batch), c_int(n_head), c_int(n_kv), c_int(head_dim), c_int(dv),
-                   c_float(scale), c_int(window or 0), c_int(chunk or 0), _ptr(sink), c_int(1 if values_in_keys else 0),
+                   *self._kv_args(kv), *self._batch_args(batch),
+                   c_int(1 if rows_share_keys(T * n_head, batch.max_q_len, batch.max_kv_len, self.SHARING_ROWS) else 0), c_int(n_head), c_int(n_kv),
+                   c_int(head_dim), c_int(dv), c_float(scale), c_int(window or 0), c_int(chunk or 0), _ptr(sink), c_int(1 if values_in_keys else 0),
                    _ptr(bias), c_int(bias.shape[0] if bias is not None else 0), _ptr(slopes), c_float(softcap or 0.0),
                    c_int(int(keep_first)), c_int(maps), c_float(diff[0] if diff else 0.0), c_float(diff[1] if diff else 0.0),
                    c_float(diff[2] if diff else 1.0), _ptr(batch.status), _stream())
+
+    # rows (token, head) from which a 32-bit prompt's rows share keys and values (`rows_share_keys`)
+    SHARING_ROWS = 1536
 
     def decode_slices(self, max_kv_len, page_size, blocks) -> int:
         return decode_slices(max_kv_len, page_size, blocks, self.sm_count)
