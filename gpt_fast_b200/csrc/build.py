@@ -10,6 +10,7 @@ the call fails with the reason.
 import ctypes
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -146,13 +147,38 @@ def build(name: str, verbose=True) -> str:
     return path
 
 
+_PROTOTYPE = re.compile(r"GFB_API\s+(int|long|void|const char\*)\s+(gfb_\w+)\(([^)]*)\)")
+_C_TYPES = {"int": ctypes.c_int, "float": ctypes.c_float, "long": ctypes.c_long, "long long": ctypes.c_longlong,
+            "unsigned long long": ctypes.c_ulonglong, "cudaStream_t": ctypes.c_void_p}
+
+
+def prototypes(name: str) -> dict:
+    """The C functions that library `name` exports, by its sources: {function: (type of the result, types of the arguments)}."""
+    found = {}
+    for source in LIBRARIES[name][0]:
+        with open(os.path.join(HERE, source)) as f:
+            text = f.read()
+        for result, function, arguments in _PROTOTYPE.findall(text):
+            types = []
+            for a in arguments.split(","):
+                a = " ".join(a.replace("const ", "").split())
+                if a:
+                    types.append(ctypes.c_void_p if "*" in a else _C_TYPES[a.rsplit(" ", 1)[0]])
+            found[function] = ({"int": ctypes.c_int, "long": ctypes.c_long, "void": None}.get(result, ctypes.c_char_p), types)
+    return found
+
+
 def library(name: str) -> ctypes.CDLL:
-    """The loaded library `name` (built first if needed)."""
+    """The loaded library `name` (built first if needed), its functions declared, so that numbers and addresses are passed as they are."""
     with _lock:
         lib = _loaded.get(name)
         if lib is None:
             lib = ctypes.CDLL(build(name))
+            for function, (result, arguments) in prototypes(name).items():
+                fn = getattr(lib, function)
+                fn.restype, fn.argtypes = result, arguments
             lib.gfb_last_error.restype = ctypes.c_char_p
+            lib.gfb_set_overlap.argtypes = [ctypes.c_int]
             _loaded[name] = lib
         return lib
 

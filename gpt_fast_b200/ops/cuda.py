@@ -1,7 +1,6 @@
 """ctypes bindings of the kernel libraries: host-side checks, kernel choice,
 launch on the current stream."""
 import ctypes
-from ctypes import c_float, c_int, c_long, c_longlong, c_ulonglong, c_void_p
 from typing import Optional
 
 import torch
@@ -28,7 +27,7 @@ def _dt(t: torch.Tensor) -> int:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return c_void_p(0 if t is None else t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _need(t: torch.Tensor, dtype=None, shape=None, name="tensor"):
@@ -38,19 +37,20 @@ def _need(t: torch.Tensor, dtype=None, shape=None, name="tensor"):
         _fail(f"{name} must be contiguous")
     if dtype is not None and t.dtype != dtype:
         _fail(f"{name} must be {dtype}, got {t.dtype}")
-    if shape is not None and tuple(t.shape) != tuple(shape):
+    if shape is not None and t.shape != shape:
         _fail(f"{name} must have shape {tuple(shape)}, got {tuple(t.shape)}")
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream():
     """The current stream of the current device as a handle for the kernels.  Asked for at every launch (a capture
     runs on a stream of its own); the short way through torch's C module costs a tenth of `current_stream()`."""
     if _raw_stream is not None:
-        return c_void_p(_raw_stream(torch.cuda.current_device()))
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def decode_slices(max_kv_len: int, page_size: int, blocks: int, sm_count: int) -> int:
@@ -165,6 +165,7 @@ class CudaKernels:
         self._status = None
         self.trace = None                  # a list: (label, start event, stop event) of every launch is appended
         self._label = None                 # what the next launch is called in the trace (default: the entry point)
+        self._plans = {}                   # of the tensor-core products, by sizes and epilogue
         self._bias_cache = {}              # distance biases in the tensor-core prefill kernel's layout, by table
         self._overlap = True               # kernels may start while their predecessor drains (programmatic dependent launch)
 
@@ -176,7 +177,6 @@ class CudaKernels:
             if not self._overlap:
                 handle.gfb_set_overlap(0)
             fn = getattr(handle, name)
-            fn.restype = c_int
             self._fn[key] = fn
             fn._lib = handle
         return fn
@@ -212,8 +212,8 @@ class CudaKernels:
         _need(tokens, torch.int32, name="tokens")
         _need(table, name="embedding table")
         _need(out, torch.float32, (T, D), "embedding output")
-        self._call("core", "gfb_embed", _ptr(tokens), _ptr(table), c_int(_dt(table)), _ptr(out),
-                   c_int(T), c_int(D), c_int(V), c_float(scale), _ptr(status), _stream())
+        self._call("core", "gfb_embed", _ptr(tokens), _ptr(table), _dt(table), _ptr(out),
+                   T, D, V, scale, _ptr(status), _stream())
 
     def embed_normed(self, tokens, table, weight, eps, out, status, scale=1.0):
         T = tokens.shape[0]
@@ -222,8 +222,8 @@ class CudaKernels:
         _need(table, name="embedding table")
         _need(weight, shape=(D,), name="embedding norm weight")
         _need(out, torch.float32, (T, D), "embedding output")
-        self._call("embedding", "gfb_embed_normed", _ptr(tokens), _ptr(table), c_int(_dt(table)), _ptr(weight), c_int(_dt(weight)), _ptr(out),
-                   c_int(T), c_int(D), c_int(V), c_float(scale), c_float(eps), _ptr(status), _stream())
+        self._call("embedding", "gfb_embed_normed", _ptr(tokens), _ptr(table), _dt(table), _ptr(weight), _dt(weight), _ptr(out),
+                   T, D, V, scale, eps, _ptr(status), _stream())
 
     MAX_STREAMS = 16
 
@@ -248,7 +248,7 @@ class CudaKernels:
             if y is not None:
                 S = y.shape[0] if y.dim() == 3 else 0
                 _need(y, torch.float32, (S, T, D) if S else (T, D), "output of a sublayer")
-            b_args += [_ptr(y), c_int(S)]
+            b_args += [_ptr(y), S]
         R = T
         if rows is not None:
             if out is None or x_out is not None:
@@ -261,9 +261,9 @@ class CudaKernels:
             _need(out, shape=(R, D), name="norm output")
         if weight is not None:
             _need(weight, shape=(D,), name="norm weight")
-        self._call("streams", "gfb_streams", _ptr(x), c_long(0 if shared else T * D), _ptr(x_out), c_long(T * D), c_int(n), _ptr(mix), _ptr(leave),
-                   *b_args, c_long(T * D), _ptr(enter), _ptr(weight), c_int(_dt(weight) if weight is not None else 0), c_float(eps), _ptr(out),
-                   c_int(_dt(out) if out is not None else 0), _ptr(rows), c_int(R), c_int(D), _stream())
+        self._call("streams", "gfb_streams", _ptr(x), 0 if shared else T * D, _ptr(x_out), T * D, n, _ptr(mix), _ptr(leave),
+                   *b_args, T * D, _ptr(enter), _ptr(weight), _dt(weight) if weight is not None else 0, eps, _ptr(out),
+                   _dt(out) if out is not None else 0, _ptr(rows), R, D, _stream())
 
     def embed_hashed(self, tokens, table, extra, out, batch, prev, buckets, mul_prev, mul_cur, scale=1.0):
         T = tokens.shape[0]
@@ -273,9 +273,9 @@ class CudaKernels:
         _need(extra, table.dtype, (buckets + 1, D), "hashed embedding table")
         _need(out, torch.float32, (T, D), "embedding output")
         _need(prev, torch.int32, name="previous tokens")
-        self._call("embedding", "gfb_embed_hashed", _ptr(tokens), _ptr(table), _ptr(extra), c_int(_dt(table)), _ptr(out),
-                   *self._batch_args(batch), _ptr(prev), c_int(D), c_int(V), c_int(buckets), c_longlong(mul_prev), c_longlong(mul_cur),
-                   c_float(scale), _ptr(batch.status), _stream())
+        self._call("embedding", "gfb_embed_hashed", _ptr(tokens), _ptr(table), _ptr(extra), _dt(table), _ptr(out),
+                   *self._batch_args(batch), _ptr(prev), D, V, buckets, mul_prev, mul_cur,
+                   scale, _ptr(batch.status), _stream())
 
     def embed_positions(self, tokens, table, positions, out, batch, scale=1.0):
         T = tokens.shape[0]
@@ -284,13 +284,13 @@ class CudaKernels:
         _need(table, name="embedding table")
         _need(positions, table.dtype, (positions.shape[0], D), "position table")
         _need(out, torch.float32, (T, D), "embedding output")
-        self._call("embedding", "gfb_embed_positions", _ptr(tokens), _ptr(table), _ptr(positions), c_int(_dt(table)), _ptr(out),
-                   *self._batch_args(batch), c_int(D), c_int(V), c_int(positions.shape[0]), c_float(scale), _ptr(batch.status),
+        self._call("embedding", "gfb_embed_positions", _ptr(tokens), _ptr(table), _ptr(positions), _dt(table), _ptr(out),
+                   *self._batch_args(batch), D, V, positions.shape[0], scale, _ptr(batch.status),
                    _stream())
 
     def softcap(self, x, cap):
         _need(x, torch.float32, name="logits")
-        self._call("core", "gfb_softcap", _ptr(x), c_long(x.numel()), c_float(cap), _stream())
+        self._call("core", "gfb_softcap", _ptr(x), x.numel(), cap, _stream())
 
     def rmsnorm(self, x, weight, eps, out, rows=None, pending=None):
         D = x.shape[-1]
@@ -309,26 +309,26 @@ class CudaKernels:
         if pending is not None:
             S = pending.shape[0]
             _need(pending, torch.float32, (S,) + tuple(x.shape), "pending partial sums")
-        self._call("core", "gfb_rmsnorm", _ptr(x), _ptr(pending), c_int(S), c_long(x.numel()), _ptr(weight),
-                   c_int(_dt(weight)), _ptr(out), c_int(_dt(out)), _ptr(rows), c_int(R), c_int(D), c_float(eps), _stream())
+        self._call("core", "gfb_rmsnorm", _ptr(x), _ptr(pending), S, x.numel(), _ptr(weight),
+                   _dt(weight), _ptr(out), _dt(out), _ptr(rows), R, D, eps, _stream())
 
     def add_partials(self, x, pending):
         _need(x, torch.float32, name="sum")
         _need(pending, torch.float32, (pending.shape[0],) + tuple(x.shape), "pending partial sums")
-        self._call("core", "gfb_add_partials", _ptr(x), _ptr(pending), c_int(pending.shape[0]), c_long(x.numel()), _stream())
+        self._call("core", "gfb_add_partials", _ptr(x), _ptr(pending), pending.shape[0], x.numel(), _stream())
 
     def rope_table(self, inv_freq, table, amplitude=1.0):
         P, half, two = table.shape
         _need(inv_freq, torch.float32, (half,), "inv_freq")
         _need(table, torch.float32, name="rotary table")
-        self._call("core", "gfb_rope_table", _ptr(inv_freq), _ptr(table), c_int(P), c_int(half), c_float(amplitude), _stream())
+        self._call("core", "gfb_rope_table", _ptr(inv_freq), _ptr(table), P, half, amplitude, _stream())
 
     def _batch_args(self, b: BatchMeta):
-        return (_ptr(b.cu_seqlens), _ptr(b.tok_seq), _ptr(b.slots), _ptr(b.lengths), c_int(b.n_seqs), c_int(b.n_tokens))
+        return (_ptr(b.cu_seqlens), _ptr(b.tok_seq), _ptr(b.slots), _ptr(b.lengths), b.n_seqs, b.n_tokens)
 
     def _kv_args(self, kv: PagedKV):
-        return (_ptr(kv.k_pool), _ptr(kv.v_pool), _ptr(kv.page_table), c_int(kv.page_table.shape[1]),
-                c_int(kv.page_size), c_int(kv.k_pool.shape[0]))
+        return (_ptr(kv.k_pool), _ptr(kv.v_pool), _ptr(kv.page_table), kv.page_table.shape[1],
+                kv.page_size, kv.k_pool.shape[0])
 
     def rope_append(self, qkv, q_out, kv, batch, table, n_head, n_kv, head_dim, pairing, append, partials=None):
         T = batch.n_tokens
@@ -346,18 +346,18 @@ class CudaKernels:
             _need(kv.k_pool, qkv.dtype, name="key pool")
             if tuple(kv.k_pool.shape[1:]) != (n_kv, kv.page_size, head_dim):
                 _fail(f"key pool pages are {tuple(kv.k_pool.shape[1:])}, the layer needs {(n_kv, kv.page_size, head_dim)}")
-        self._call("core", "gfb_rope_append", _ptr(src), c_int(n_part), _ptr(q_out), c_int(_dt(q_out)), *self._kv_args(kv),
-                   *self._batch_args(batch), _ptr(table), c_int(table.shape[0]), c_int(n_head), c_int(n_kv),
-                   c_int(head_dim), c_int(_PAIRING[pairing]), c_int(1 if append else 0), _ptr(batch.status), _stream())
+        self._call("core", "gfb_rope_append", _ptr(src), n_part, _ptr(q_out), _dt(q_out), *self._kv_args(kv),
+                   *self._batch_args(batch), _ptr(table), table.shape[0], n_head, n_kv,
+                   head_dim, _PAIRING[pairing], 1 if append else 0, _ptr(batch.status), _stream())
 
     def advance_lengths(self, batch):
         self._call("core", "gfb_advance_lengths", _ptr(batch.lengths), _ptr(batch.slots), _ptr(batch.cu_seqlens),
-                   c_int(batch.n_seqs), _stream())
+                   batch.n_seqs, _stream())
 
     def add_into(self, out, y):
         _need(out, torch.float32, name="sum")
         _need(y, shape=out.shape, name="addend")
-        self._call("core", "gfb_add_into", _ptr(out), _ptr(y), c_int(_dt(y)), c_long(out.numel()), _stream())
+        self._call("core", "gfb_add_into", _ptr(out), _ptr(y), _dt(y), out.numel(), _stream())
 
     # -- layer norm, q/k/v preparation, retention, activations ---------------------------
     def layernorm(self, x, weight, bias, eps, out, rows=None, branch=None, rms=False):
@@ -392,10 +392,10 @@ class CudaKernels:
                 _need(y, torch.float32, (T, D), "branch")
         elif out is None:
             return
-        self._call("layernorm", "gfb_layernorm", _ptr(x), _ptr(y), c_int(S), c_long(T * D), _ptr(pw), _ptr(pb),
-                   c_int(_dt(pw) if pw is not None else 0), c_float(peps), c_float(mult), _ptr(weight if out is not None else None),
-                   _ptr(bias if out is not None and weight is not None else None), c_int(_dt(weight) if out is not None and weight is not None else 0), c_float(eps),
-                   _ptr(out), c_int(_dt(out) if out is not None else 0), _ptr(rows), c_int(R), c_int(D), c_int(1 if rms else 0),
+        self._call("layernorm", "gfb_layernorm", _ptr(x), _ptr(y), S, T * D, _ptr(pw), _ptr(pb),
+                   _dt(pw) if pw is not None else 0, peps, mult, _ptr(weight if out is not None else None),
+                   _ptr(bias if out is not None and weight is not None else None), _dt(weight) if out is not None and weight is not None else 0, eps,
+                   _ptr(out), _dt(out) if out is not None else 0, _ptr(rows), R, D, 1 if rms else 0,
                    _stream())
 
     def layernorm_multi(self, x, branches=(), outs=(), rows=None, rms=False):
@@ -417,7 +417,7 @@ class CudaKernels:
                 if scale is not None:
                     _need(scale, shape=(D,), name="branch factor")
                     scale_dt = _dt(scale)
-            b_args += [_ptr(y), c_int(S), _ptr(scale)]
+            b_args += [_ptr(y), S, _ptr(scale)]
         scales = [s for _, s in branches if s is not None]
         if len(scales) == 2 and scales[0].dtype != scales[1].dtype:
             _fail("the branch factors must have one type")
@@ -432,7 +432,7 @@ class CudaKernels:
                     _fail("the row itself can only be the one output")
                 _need(out, shape=(R, D), name="norm output")
                 out_dt = _dt(out)
-            o_args += [_ptr(w), c_float(eps), _ptr(out)]
+            o_args += [_ptr(w), eps, _ptr(out)]
         if len(outs) == 2 and (outs[0][0].dtype != outs[1][0].dtype or outs[0][2].dtype != outs[1][2].dtype
                                or outs[0][2].shape != outs[1][2].shape):
             _fail("the two outputs must agree in shape and types")
@@ -442,8 +442,8 @@ class CudaKernels:
             _fail(f"norm output has {R} rows, input {T}")
         if not branches and not outs:
             return
-        self._call("layernorm", "gfb_layernorm_multi", _ptr(x), *b_args[:3], *b_args[3:], c_int(scale_dt), c_long(T * D),
-                   *o_args[:3], *o_args[3:], c_int(w_dt), c_int(out_dt), _ptr(rows), c_int(R), c_int(D), c_int(1 if rms else 0),
+        self._call("layernorm", "gfb_layernorm_multi", _ptr(x), *b_args[:3], *b_args[3:], scale_dt, T * D,
+                   *o_args[:3], *o_args[3:], w_dt, out_dt, _ptr(rows), R, D, 1 if rms else 0,
                    _stream())
 
     def latent_prepare(self, src, q_off, kv_off, q_out, kv, batch, n_head, head_dim, rot_dim, rank, norm_weight, eps, table,
@@ -463,11 +463,11 @@ class CudaKernels:
             _need(kv.k_pool, q_out.dtype, name="key pool")
             if tuple(kv.k_pool.shape[1:]) != (1, kv.page_size, rank + rot_dim):
                 _fail(f"cache pages are {tuple(kv.k_pool.shape[1:])}, the layer needs {(1, kv.page_size, rank + rot_dim)}")
-        self._call("latent", "gfb_latent_prepare", _ptr(src), c_int(_dt(src)), c_int(W), c_int(q_off), c_int(kv_off), _ptr(q_out),
-                   c_int(q_at + rot_dim), c_int(q_at), _ptr(kv.k_pool), _ptr(kv.page_table), c_int(kv.page_table.shape[1]), c_int(kv.page_size),
-                   c_int(kv.k_pool.shape[0]), *self._batch_args(batch), _ptr(table), c_int(table.shape[0]), _ptr(norm_weight), c_int(_dt(norm_weight)),
-                   c_float(eps), c_int(n_head), c_int(head_dim), c_int(rot_dim), c_int(rank), c_int(_PAIRING[pairing]),
-                   c_int(1 if append else 0), _ptr(batch.status), _stream())
+        self._call("latent", "gfb_latent_prepare", _ptr(src), _dt(src), W, q_off, kv_off, _ptr(q_out),
+                   q_at + rot_dim, q_at, _ptr(kv.k_pool), _ptr(kv.page_table), kv.page_table.shape[1], kv.page_size,
+                   kv.k_pool.shape[0], *self._batch_args(batch), _ptr(table), table.shape[0], _ptr(norm_weight), _dt(norm_weight),
+                   eps, n_head, head_dim, rot_dim, rank, _PAIRING[pairing],
+                   1 if append else 0, _ptr(batch.status), _stream())
 
     def latent_expanded(self, proj, q_off, kv_off, gate_off, gate_per_head, out, kv, batch, n_head, head_dim, rot_dim, v_head_dim, rank, norm_weight,
                         eps, table, pairing, append, wuk, wuv, v_scale, scale, window=None, sink=None) -> bool:
@@ -492,10 +492,10 @@ class CudaKernels:
         q_rot = torch.empty(T, H, rot_dim, dtype=proj.dtype, device=proj.device)
         self.latent_prepare(proj, q_off, kv_off, q_rot, kv, batch, H, head_dim, rot_dim, R, norm_weight, eps, table, pairing, append, rotated_only=True)
         keys, values = torch.empty(2, H, batch.n_seqs * cap, 128, dtype=proj.dtype, device=proj.device)
-        self._call("attention_tc", "gfb_latent_expanded", _ptr(proj), c_int(W), c_int(q_off), c_int(gate_off), c_int(1 if gate_per_head else 0), _ptr(q_rot),
-                   _ptr(wuk), _ptr(wuv), _ptr(v_scale), _ptr(keys), _ptr(values), _ptr(out), _ptr(kv.k_pool), _ptr(kv.page_table), c_int(kv.page_table.shape[1]),
-                   c_int(kv.page_size), c_int(kv.k_pool.shape[0]), *self._batch_args(batch), c_int(H), c_int(R), c_int(cap), c_float(scale),
-                   c_int(window or 0), _ptr(sink), _ptr(batch.status), _stream())
+        self._call("attention_tc", "gfb_latent_expanded", _ptr(proj), W, q_off, gate_off, 1 if gate_per_head else 0, _ptr(q_rot),
+                   _ptr(wuk), _ptr(wuv), _ptr(v_scale), _ptr(keys), _ptr(values), _ptr(out), _ptr(kv.k_pool), _ptr(kv.page_table), kv.page_table.shape[1],
+                   kv.page_size, kv.k_pool.shape[0], *self._batch_args(batch), H, R, cap, scale,
+                   window or 0, _ptr(sink), _ptr(batch.status), _stream())
         return True
 
     # up to this many tokens the smaller tiles of the mma.sync form (16 heads, 128 -> 512, us with it | on tcgen05: 16 tokens 22.1 | 22.9,
@@ -521,13 +521,13 @@ class CudaKernels:
         if (a.dtype == torch.bfloat16 and T > self.HEADWISE_FEW_TOKENS and k % 64 == 0 and n % 128 == 0
                 and (a.shape[1] | a_off | a_stride) % 8 == 0 and (out.shape[1] | out_off | out_stride) % 4 == 0
                 and (a.data_ptr() | w.data_ptr()) % 16 == 0 and out.data_ptr() % 8 == 0):
-            self._call("attention_tc", "gfb_headwise_linear_tc", _ptr(a), c_int(a.shape[1]), c_int(a_off), c_int(a_stride), _ptr(w), _ptr(out),
-                       c_int(out.shape[1]), c_int(out_off), c_int(out_stride), _ptr(gate), c_int(gate.shape[1] if gate is not None else 0),
-                       c_int(gate_off), c_int(1 if gate_per_head else n), c_int(T), c_int(n_head), c_int(k), c_int(n), _ptr(self.status), _stream())
+            self._call("attention_tc", "gfb_headwise_linear_tc", _ptr(a), a.shape[1], a_off, a_stride, _ptr(w), _ptr(out),
+                       out.shape[1], out_off, out_stride, _ptr(gate), gate.shape[1] if gate is not None else 0,
+                       gate_off, 1 if gate_per_head else n, T, n_head, k, n, _ptr(self.status), _stream())
             return
-        self._call("latent", "gfb_headwise_linear", _ptr(a), c_int(_dt(a)), c_int(a.shape[1]), c_int(a_off), c_int(a_stride), _ptr(w), _ptr(out), c_int(out.shape[1]), c_int(out_off), c_int(out_stride), _ptr(gate),
-                   c_int(gate.shape[1] if gate is not None else 0), c_int(gate_off), c_int(1 if gate_per_head else n), c_int(T), c_int(n_head),
-                   c_int(k), c_int(n),
+        self._call("latent", "gfb_headwise_linear", _ptr(a), _dt(a), a.shape[1], a_off, a_stride, _ptr(w), _ptr(out), out.shape[1], out_off, out_stride, _ptr(gate),
+                   gate.shape[1] if gate is not None else 0, gate_off, 1 if gate_per_head else n, T, n_head,
+                   k, n,
                    _stream())
 
     @staticmethod
@@ -535,7 +535,7 @@ class CudaKernels:
         _need(state, torch.float32, name="per-sequence state")
         if state.dim() != 2 or state_off < 0 or state_off + need > state.shape[1]:
             _fail(f"{need} numbers of state at column {state_off} do not fit rows of {tuple(state.shape)}")
-        return c_void_p(state.data_ptr() + 4 * state_off), c_long(state.shape[1])
+        return state.data_ptr() + 4 * state_off, state.shape[1]
 
     _LOG2E = 1.4426950408889634
 
@@ -554,19 +554,18 @@ class CudaKernels:
         if not tau > 0:
             _fail(f"tau = {tau} must be positive")
         sp, sld = self._state_args(state, state_off, H * d * dv)
-        factor = c_float(self._LOG2E / tau)
-        cols = (c_int(q_off), c_int(k_off), c_int(v_off), c_int(low_off))
-        if (batch.max_q_len == 1 and T == batch.n_seqs and dv % 4 == 0 and dv <= 2048 and state.shape[1] % 4 == 0 and sp.value % 16 == 0
+        factor = self._LOG2E / tau
+        cols = (q_off, k_off, v_off, low_off)
+        if (batch.max_q_len == 1 and T == batch.n_seqs and dv % 4 == 0 and dv <= 2048 and state.shape[1] % 4 == 0 and sp % 16 == 0
                 and (512 // (dv // 4) * dv + 3 * d + rank) * 4 <= 48 * 1024):
-            return self._call("gla", "gfb_gla_decode", _ptr(src), c_int(_dt(src)), c_int(W), *cols, c_int(g_off), c_int(rank), _ptr(a2),
-                              _ptr(bias), c_int(_dt(bias)), factor, sp, sld, _ptr(norm), c_int(_dt(norm)), c_float(eps), _ptr(out),
-                              *self._batch_args(batch), c_int(H), c_int(d), c_int(dv), c_float(q_scale), _stream())
+            return self._call("gla", "gfb_gla_decode", _ptr(src), _dt(src), W, *cols, g_off, rank, _ptr(a2),
+                              _ptr(bias), _dt(bias), factor, sp, sld, _ptr(norm), _dt(norm), eps, _ptr(out),
+                              *self._batch_args(batch), H, d, dv, q_scale, _stream())
         fn = self._f("gla", "gfb_gla_scratch_floats")
-        fn.restype = c_long
-        scratch = torch.empty(fn(c_int(T), c_int(batch.n_seqs), c_int(H), c_int(d), c_int(dv)), dtype=torch.float32, device=src.device)
+        scratch = torch.empty(fn(T, batch.n_seqs, H, d, dv), dtype=torch.float32, device=src.device)
         o = torch.empty(T, H * dv, dtype=torch.float32, device=src.device)
-        self._call("gla", "gfb_gla", _ptr(src), c_int(_dt(src)), c_int(W), *cols, c_int(rank), _ptr(a2), _ptr(bias), c_int(_dt(bias)), factor,
-                   sp, sld, _ptr(o), _ptr(scratch), *self._batch_args(batch), c_int(H), c_int(d), c_int(dv), c_float(q_scale), _stream())
+        self._call("gla", "gfb_gla", _ptr(src), _dt(src), W, *cols, rank, _ptr(a2), _ptr(bias), _dt(bias), factor,
+                   sp, sld, _ptr(o), _ptr(scratch), *self._batch_args(batch), H, d, dv, q_scale, _stream())
         self.gated_norm(o, src, g_off, norm, out, dv, eps, act="silu", gate_first=False)
 
     def token_gate(self, z, tokens, table, off, out, status):
@@ -578,8 +577,8 @@ class CudaKernels:
         _need(out, table.dtype, (T, n), "gated side rows")
         if off < 0 or off + n > W:
             _fail(f"columns {off} .. {off + n - 1} of a side table of {W}")
-        self._call("embedding", "gfb_token_gate", _ptr(tokens), _ptr(table), c_int(_dt(table)), c_int(V), c_int(W), c_int(off), _ptr(z), _ptr(out),
-                   c_int(_dt(out)), c_int(T), c_int(n), _ptr(status), _stream())
+        self._call("embedding", "gfb_token_gate", _ptr(tokens), _ptr(table), _dt(table), V, W, off, _ptr(z), _ptr(out),
+                   _dt(out), T, n, _ptr(status), _stream())
 
     def pass_entry(self, x, x0, step, cat, y):
         T, D = x.shape
@@ -588,8 +587,8 @@ class CudaKernels:
         _need(step, shape=(D,), name="vector of the pass")
         _need(cat, shape=(T, 2 * D), name="input of the entry product")
         _need(y, torch.float32, (T, D), "new stream")
-        self._call("elementwise", "gfb_pass_entry", _ptr(x), _ptr(x0), _ptr(step), c_int(_dt(step)), _ptr(cat), c_int(_dt(cat)), _ptr(y), c_int(T),
-                   c_int(D), _stream())
+        self._call("elementwise", "gfb_pass_entry", _ptr(x), _ptr(x0), _ptr(step), _dt(step), _ptr(cat), _dt(cat), _ptr(y), T,
+                   D, _stream())
 
     def short_conv(self, src, col_off, channels, weight, bias, state, state_off, out, batch, act=True, in_bias=None):
         T = batch.n_tokens
@@ -604,9 +603,9 @@ class CudaKernels:
             _need(in_bias, weight.dtype, (channels,), "bias of the convolution's inputs")
         _need(out, torch.float32, (T, channels), "convolution output")
         sp, sld = self._state_args(state, state_off, (taps - 1) * channels)
-        self._call("recurrent", "gfb_short_conv", _ptr(src), c_int(_dt(src)), c_int(src.shape[1]), c_int(col_off), c_int(channels),
-                   _ptr(weight), _ptr(bias), _ptr(in_bias), c_int(_dt(weight)), c_int(taps), sp, sld, _ptr(out), *self._batch_args(batch),
-                   c_int(int(batch.max_q_len)), c_int(1 if act else 0), _stream())
+        self._call("recurrent", "gfb_short_conv", _ptr(src), _dt(src), src.shape[1], col_off, channels,
+                   _ptr(weight), _ptr(bias), _ptr(in_bias), _dt(weight), taps, sp, sld, _ptr(out), *self._batch_args(batch),
+                   int(batch.max_q_len), 1 if act else 0, _stream())
 
     def rglru(self, u, w_a, w_i, b_a, b_i, lam, decay_scale, y_src, y_off, y_bias, state, state_off, out, batch):
         T = batch.n_tokens
@@ -625,13 +624,11 @@ class CudaKernels:
         _need(out, shape=(T, C), name="recurrence output")
         sp, sld = self._state_args(state, state_off, C)
         fn = self._f("recurrent", "gfb_rglru_scratch_floats")
-        fn.restype = c_long
-        need = fn(c_int(T), c_int(batch.n_seqs), c_int(int(batch.max_q_len)), c_int(C))
-        fn.restype = c_int
+        need = fn(T, batch.n_seqs, int(batch.max_q_len), C)
         scratch = torch.empty(need, dtype=torch.float32, device=u.device)
-        self._call("recurrent", "gfb_rglru", _ptr(u), _ptr(w_a), _ptr(w_i), c_int(_dt(w_a)), _ptr(b_a), _ptr(b_i), _ptr(lam), _ptr(y_bias),
-                   c_int(_dt(b_a)), c_float(decay_scale), _ptr(y_src), c_int(_dt(y_src)), c_int(y_src.shape[1]), c_int(y_off), sp, sld,
-                   _ptr(out), c_int(_dt(out)), _ptr(scratch), *self._batch_args(batch), c_int(int(batch.max_q_len)), c_int(C), c_int(blocks),
+        self._call("recurrent", "gfb_rglru", _ptr(u), _ptr(w_a), _ptr(w_i), _dt(w_a), _ptr(b_a), _ptr(b_i), _ptr(lam), _ptr(y_bias),
+                   _dt(b_a), decay_scale, _ptr(y_src), _dt(y_src), y_src.shape[1], y_off, sp, sld,
+                   _ptr(out), _dt(out), _ptr(scratch), *self._batch_args(batch), int(batch.max_q_len), C, blocks,
                    _stream())
 
     # what a step in chunks costs at least, in tokens of a lone sequence token by token (`ssd_in_chunks`)
@@ -654,20 +651,19 @@ class CudaKernels:
                 and out.data_ptr() % 16 == 0
                 and ssd_in_chunks(T, batch.n_seqs, int(batch.max_q_len), n_head, head_dim, n_state, self.SSD_CHUNK_TOKENS)):
             fn = self._f("ssd_chunk", "gfb_ssd_chunks_scratch_floats")
-            fn.restype = c_long
-            need = fn(c_int(T), c_int(batch.n_seqs), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups))
+            need = fn(T, batch.n_seqs, n_head, head_dim, n_state, n_groups)
             scratch = torch.empty(need, dtype=torch.float32, device=x.device)
-            return self._call("ssd_chunk", "gfb_ssd_chunks", _ptr(x), c_int(x.shape[1]), c_int(b_off), c_int(c_off), _ptr(dt_src), c_int(_dt(dt_src)),
-                              c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
-                              _ptr(out), _ptr(scratch), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state),
-                              c_int(n_groups), _stream())
-        if batch.max_q_len == 1 and T == batch.n_seqs and n_state <= 512 and head_dim % 4 == 0 and state.shape[1] % 4 == 0 and sp.value % 16 == 0:
-            return self._call("recurrent", "gfb_ssd_decode", _ptr(x), c_int(x.shape[1]), c_int(b_off), c_int(c_off), _ptr(dt_src), c_int(_dt(dt_src)),
-                              c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
-                              _ptr(out), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups), _stream())
-        self._call("recurrent", "gfb_ssd_scan", _ptr(x), c_int(x.shape[1]), c_int(b_off), c_int(c_off), _ptr(dt_src), c_int(_dt(dt_src)),
-                   c_int(dt_src.shape[1]), c_int(dt_off), _ptr(dt_bias), _ptr(a_log), _ptr(skip), c_int(_dt(dt_bias)), sp, sld,
-                   _ptr(out), *self._batch_args(batch), c_int(n_head), c_int(head_dim), c_int(n_state), c_int(n_groups), _stream())
+            return self._call("ssd_chunk", "gfb_ssd_chunks", _ptr(x), x.shape[1], b_off, c_off, _ptr(dt_src), _dt(dt_src),
+                              dt_src.shape[1], dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(skip), _dt(dt_bias), sp, sld,
+                              _ptr(out), _ptr(scratch), *self._batch_args(batch), n_head, head_dim, n_state,
+                              n_groups, _stream())
+        if batch.max_q_len == 1 and T == batch.n_seqs and n_state <= 512 and head_dim % 4 == 0 and state.shape[1] % 4 == 0 and sp % 16 == 0:
+            return self._call("recurrent", "gfb_ssd_decode", _ptr(x), x.shape[1], b_off, c_off, _ptr(dt_src), _dt(dt_src),
+                              dt_src.shape[1], dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(skip), _dt(dt_bias), sp, sld,
+                              _ptr(out), *self._batch_args(batch), n_head, head_dim, n_state, n_groups, _stream())
+        self._call("recurrent", "gfb_ssd_scan", _ptr(x), x.shape[1], b_off, c_off, _ptr(dt_src), _dt(dt_src),
+                   dt_src.shape[1], dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(skip), _dt(dt_bias), sp, sld,
+                   _ptr(out), *self._batch_args(batch), n_head, head_dim, n_state, n_groups, _stream())
 
     # the same for the delta rule (`delta_in_chunks`)
     DELTA_CHUNK_TOKENS = 132
@@ -691,25 +687,24 @@ class CudaKernels:
         if (head_dim in (64, 128) and v_head_dim % 64 == 0 and out.data_ptr() % 16 == 0
                 and delta_in_chunks(T, batch.n_seqs, int(batch.max_q_len), n_head, head_dim, v_head_dim, self.DELTA_CHUNK_TOKENS)):
             fn = self._f("delta_chunk", "gfb_delta_chunks_scratch_floats")
-            fn.restype = c_long
-            need = fn(c_int(T), c_int(batch.n_seqs), c_int(n_head), c_int(head_dim), c_int(v_head_dim))
+            need = fn(T, batch.n_seqs, n_head, head_dim, v_head_dim)
             scratch = torch.empty(need, dtype=torch.float32, device=qkv.device)
-            return self._call("delta_chunk", "gfb_delta_chunks", _ptr(qkv), c_int(qkv.shape[1]), c_int(q_off), c_int(k_off), c_int(v_off),
-                              _ptr(beta_src), c_int(_dt(beta_src)), c_int(beta_src.shape[1]), c_int(beta_off), _ptr(a_src),
-                              c_int(a_src.shape[1]), c_int(a_off), _ptr(dt_bias), _ptr(a_log), c_int(_dt(dt_bias)), sp, sld, _ptr(out),
-                              _ptr(scratch), *self._batch_args(batch), c_int(n_head), c_int(n_qk), c_int(head_dim), c_int(v_head_dim),
-                              c_float(q_scale), c_float(unit_eps), c_int(1 if head_decay else 0), _stream())
-        if batch.max_q_len == 1 and T == batch.n_seqs and head_dim <= 256 and v_head_dim % 4 == 0 and state.shape[1] % 4 == 0 and sp.value % 16 == 0:
-            return self._call("recurrent", "gfb_delta_decode", _ptr(qkv), c_int(qkv.shape[1]), c_int(q_off), c_int(k_off), c_int(v_off),
-                              _ptr(beta_src), c_int(_dt(beta_src)), c_int(beta_src.shape[1]), c_int(beta_off), _ptr(a_src),
-                              c_int(a_src.shape[1]), c_int(a_off), _ptr(dt_bias), _ptr(a_log), c_int(_dt(dt_bias)), sp, sld, _ptr(out),
-                              *self._batch_args(batch), c_int(n_head), c_int(n_qk), c_int(head_dim), c_int(v_head_dim), c_float(q_scale),
-                              c_float(unit_eps), c_int(1 if head_decay else 0), _stream())
-        self._call("recurrent", "gfb_delta_rule", _ptr(qkv), c_int(qkv.shape[1]), c_int(q_off), c_int(k_off), c_int(v_off),
-                   _ptr(beta_src), c_int(_dt(beta_src)), c_int(beta_src.shape[1]), c_int(beta_off), _ptr(a_src), c_int(a_src.shape[1]),
-                   c_int(a_off), _ptr(dt_bias), _ptr(a_log), c_int(_dt(dt_bias)), sp, sld, _ptr(out), *self._batch_args(batch),
-                   c_int(n_head), c_int(n_qk), c_int(head_dim), c_int(v_head_dim), c_float(q_scale), c_float(unit_eps),
-                   c_int(1 if head_decay else 0), _stream())
+            return self._call("delta_chunk", "gfb_delta_chunks", _ptr(qkv), qkv.shape[1], q_off, k_off, v_off,
+                              _ptr(beta_src), _dt(beta_src), beta_src.shape[1], beta_off, _ptr(a_src),
+                              a_src.shape[1], a_off, _ptr(dt_bias), _ptr(a_log), _dt(dt_bias), sp, sld, _ptr(out),
+                              _ptr(scratch), *self._batch_args(batch), n_head, n_qk, head_dim, v_head_dim,
+                              q_scale, unit_eps, 1 if head_decay else 0, _stream())
+        if batch.max_q_len == 1 and T == batch.n_seqs and head_dim <= 256 and v_head_dim % 4 == 0 and state.shape[1] % 4 == 0 and sp % 16 == 0:
+            return self._call("recurrent", "gfb_delta_decode", _ptr(qkv), qkv.shape[1], q_off, k_off, v_off,
+                              _ptr(beta_src), _dt(beta_src), beta_src.shape[1], beta_off, _ptr(a_src),
+                              a_src.shape[1], a_off, _ptr(dt_bias), _ptr(a_log), _dt(dt_bias), sp, sld, _ptr(out),
+                              *self._batch_args(batch), n_head, n_qk, head_dim, v_head_dim, q_scale,
+                              unit_eps, 1 if head_decay else 0, _stream())
+        self._call("recurrent", "gfb_delta_rule", _ptr(qkv), qkv.shape[1], q_off, k_off, v_off,
+                   _ptr(beta_src), _dt(beta_src), beta_src.shape[1], beta_off, _ptr(a_src), a_src.shape[1],
+                   a_off, _ptr(dt_bias), _ptr(a_log), _dt(dt_bias), sp, sld, _ptr(out), *self._batch_args(batch),
+                   n_head, n_qk, head_dim, v_head_dim, q_scale, unit_eps,
+                   1 if head_decay else 0, _stream())
 
     def gated_norm(self, y, gate, gate_off, weight, out, group, eps, act="silu", gate_first=False):
         T, C = y.shape
@@ -721,9 +716,9 @@ class CudaKernels:
             _fail(f"groups of {group}, a gate of {tuple(gate.shape)} at {gate_off} or a weight of {tuple(weight.shape)} do not fit {C} columns")
         if act not in ("silu", "sigmoid"):
             _fail(f"unknown gate activation '{act}'")
-        self._call("recurrent", "gfb_gated_norm", _ptr(y), _ptr(gate), c_int(_dt(gate)), c_int(gate.shape[1]), c_int(gate_off),
-                   _ptr(weight), c_int(_dt(weight)), c_int(weight.shape[0]), _ptr(out), c_int(_dt(out)), c_int(T), c_int(C // group),
-                   c_int(group), c_float(eps), c_int(1 if act == "sigmoid" else 0), c_int(1 if gate_first else 0), _stream())
+        self._call("recurrent", "gfb_gated_norm", _ptr(y), _ptr(gate), _dt(gate), gate.shape[1], gate_off,
+                   _ptr(weight), _dt(weight), weight.shape[0], _ptr(out), _dt(out), T, C // group,
+                   group, eps, 1 if act == "sigmoid" else 0, 1 if gate_first else 0, _stream())
 
     def qkv_prepare(self, src, partials, offsets, q_out, kv, batch, n_head, n_kv, head_dim, v_head_dim, table=None, rot_dims=0,
                     pairing="half", q_norm=None, k_norm=None, norm_eps=0.0, k_scale=1.0, append=True, norm_whole=False,
@@ -762,12 +757,12 @@ class CudaKernels:
             if tuple(kv.k_pool.shape[1:]) != (n_kv, kv.page_size, head_dim * maps) or tuple(kv.v_pool.shape[1:]) != (n_kv, kv.page_size, v_head_dim):
                 _fail(f"cache pages are {tuple(kv.k_pool.shape[1:])} / {tuple(kv.v_pool.shape[1:])}, the layer needs "
                       f"{(n_kv, kv.page_size, head_dim * maps)} / {(n_kv, kv.page_size, v_head_dim)}")
-        self._call("qkv_prepare", "gfb_qkv_prepare", _ptr(source), c_int(n_part), c_int(W), c_int(q_off), c_int(k_off), c_int(v_off),
-                   _ptr(bias), c_int(_dt(bias) if bias is not None else 0), _ptr(q_out), c_int(_dt(q_out)), *self._kv_args(kv), *self._batch_args(batch), _ptr(table),
-                   c_int(table.shape[0] if table is not None else 0), c_int(rot_dims if table is not None else 0),
-                   c_int(_PAIRING[pairing]), _ptr(q_norm), _ptr(k_norm), c_int(w_dt), c_float(norm_eps), c_float(k_scale),
-                   c_int(n_head), c_int(n_kv), c_int(head_dim), c_int(v_head_dim), c_int(1 if append else 0),
-                   c_int((1 if norm_whole else 0) | (2 if norm_bare else 0) | (4 if norm_last else 0) | (8 if q_spread else 0)), c_int(maps),
+        self._call("qkv_prepare", "gfb_qkv_prepare", _ptr(source), n_part, W, q_off, k_off, v_off,
+                   _ptr(bias), _dt(bias) if bias is not None else 0, _ptr(q_out), _dt(q_out), *self._kv_args(kv), *self._batch_args(batch), _ptr(table),
+                   table.shape[0] if table is not None else 0, rot_dims if table is not None else 0,
+                   _PAIRING[pairing], _ptr(q_norm), _ptr(k_norm), w_dt, norm_eps, k_scale,
+                   n_head, n_kv, head_dim, v_head_dim, 1 if append else 0,
+                   (1 if norm_whole else 0) | (2 if norm_bare else 0) | (4 if norm_last else 0) | (8 if q_spread else 0), maps,
                    _ptr(batch.status), _stream())
 
     def retention(self, src, offsets, state, out, batch, n_head, head_dim, v_head_dim, decay, table=None, rot_dims=0,
@@ -787,15 +782,13 @@ class CudaKernels:
                 _fail(f"the rotary table serves {table.shape[1] * 2} dimensions, the mixer rotates {rot_dims}")
         # prompts of several chunks run their chunks side by side and need room for one state per chunk
         fn = self._f("retention", "gfb_retention_scratch_floats")
-        fn.restype = c_long
-        need = fn(c_int(T), c_int(batch.n_seqs), c_int(int(batch.max_q_len)), c_int(n_head), c_int(head_dim), c_int(v_head_dim))
-        fn.restype = c_long
+        need = fn(T, batch.n_seqs, int(batch.max_q_len), n_head, head_dim, v_head_dim)
         scratch = torch.empty(need, dtype=torch.float32, device=src.device) if need > 0 else None
-        self._call("retention", "gfb_retention", _ptr(src), c_int(_dt(src)), c_int(W), c_int(q_off), c_int(k_off), c_int(v_off),
-                   _ptr(state), _ptr(out), *self._batch_args(batch), c_int(int(batch.max_q_len)), _ptr(table),
-                   c_int(table.shape[0] if table is not None else 0), c_int(rot_dims if table is not None else 0),
-                   c_int(_PAIRING[pairing]), _ptr(decay), c_float(k_scale), c_int(n_head), c_int(head_dim), c_int(v_head_dim),
-                   _ptr(scratch), c_long(need), _ptr(batch.status), _stream())
+        self._call("retention", "gfb_retention", _ptr(src), _dt(src), W, q_off, k_off, v_off,
+                   _ptr(state), _ptr(out), *self._batch_args(batch), int(batch.max_q_len), _ptr(table),
+                   table.shape[0] if table is not None else 0, rot_dims if table is not None else 0,
+                   _PAIRING[pairing], _ptr(decay), k_scale, n_head, head_dim, v_head_dim,
+                   _ptr(scratch), need, _ptr(batch.status), _stream())
 
     def retention_gate(self, o, src, gate_offset, out, n_head, v_head_dim, eps):
         T, W = src.shape
@@ -804,8 +797,8 @@ class CudaKernels:
         _need(out, src.dtype, (T, n_head * v_head_dim), "gated output")
         if gate_offset + n_head * v_head_dim > W:
             _fail(f"a gate at column {gate_offset} does not fit rows of {W}")
-        self._call("retention", "gfb_retention_gate", _ptr(o), _ptr(src), c_int(_dt(src)), c_int(W), c_int(gate_offset), _ptr(out),
-                   c_int(T), c_int(n_head), c_int(v_head_dim), c_float(eps), _stream())
+        self._call("retention", "gfb_retention_gate", _ptr(o), _ptr(src), _dt(src), W, gate_offset, _ptr(out),
+                   T, n_head, v_head_dim, eps, _stream())
 
     def sigmoid_gate(self, y, gate, gate_off, group):
         T, C = y.shape
@@ -815,8 +808,8 @@ class CudaKernels:
             _fail(f"a gate of {gate.dtype} on a tensor of {y.dtype}")
         if gate.dim() != 2 or gate.shape[0] != T or group < 1 or C % group or gate_off + C // group > gate.shape[1]:
             _fail(f"gates for groups of {group} of {C} columns at column {gate_off} do not fit {tuple(gate.shape)}")
-        self._call("elementwise", "gfb_sigmoid_gate", _ptr(y), _ptr(gate), c_int(_dt(y)), c_int(_dt(gate)), c_int(T), c_int(C), c_int(gate.shape[1]),
-                   c_int(gate_off), c_int(group), _stream())
+        self._call("elementwise", "gfb_sigmoid_gate", _ptr(y), _ptr(gate), _dt(y), _dt(gate), T, C, gate.shape[1],
+                   gate_off, group, _stream())
 
     # -- mixture of experts ------------------------------------------------------------------
     MOE_TILE_ROWS = 64                 # rows of a tile of the sorted form on CUDA cores
@@ -833,8 +826,8 @@ class CudaKernels:
     def _route_args(self, score, groups, shared):
         if score not in self._ROUTE_SCORES:
             _fail(f"unknown router score '{score}'")
-        return (c_int(self._ROUTE_SCORES[score]), c_int(groups[0]), c_int(groups[1]), c_int(groups[2] if len(groups) > 2 else 1),
-                c_int(1 if shared else 0))
+        return (self._ROUTE_SCORES[score], groups[0], groups[1], groups[2] if len(groups) > 2 else 1,
+                1 if shared else 0)
 
     def moe_route(self, logits, correction, top, scale, idx, weights, score="sigmoid", groups=(1, 1), shared=False):
         T, slots = logits.shape[0], top + (1 if shared else 0)
@@ -847,8 +840,8 @@ class CudaKernels:
         _need(correction, name="router correction")
         _need(idx, torch.int32, (T, slots), "chosen experts")
         _need(weights, torch.float32, (T, slots), "expert weights")
-        self._call("moe", "gfb_moe_route", _ptr(logits), c_int(logits.shape[1]), _ptr(correction), c_int(_dt(correction)), c_int(E),
-                   c_int(top), c_float(scale), _ptr(idx), _ptr(weights), c_int(T), *self._route_args(score, groups, shared), _stream())
+        self._call("moe", "gfb_moe_route", _ptr(logits), logits.shape[1], _ptr(correction), _dt(correction), E,
+                   top, scale, _ptr(idx), _ptr(weights), T, *self._route_args(score, groups, shared), _stream())
 
     MOE_ROUTER_FEW_TOKENS = 64         # up to this many tokens a block per token, beyond it one per eight tokens (rows of whole 16-byte pieces)
 
@@ -879,9 +872,9 @@ class CudaKernels:
         _need(correction, name="router correction")
         _need(idx, torch.int32, (T, slots), "chosen experts")
         _need(weights, torch.float32, (T, slots), "expert weights")
-        self._call("moe", "gfb_moe_router", _ptr(h), _ptr(router), c_int(_dt(h)), _ptr(correction), c_int(_dt(correction)), c_int(E),
-                   c_int(top), c_float(scale), _ptr(idx), _ptr(weights), c_int(T), c_int(D), *self._route_args(score, groups, shared),
-                   c_int(n_extra), _ptr(extra), _stream())
+        self._call("moe", "gfb_moe_router", _ptr(h), _ptr(router), _dt(h), _ptr(correction), _dt(correction), E,
+                   top, scale, _ptr(idx), _ptr(weights), T, D, *self._route_args(score, groups, shared),
+                   n_extra, _ptr(extra), _stream())
         return True
 
     def moe_experts(self, h, idx, weights, w13, w2, x, limit, alpha, shift=1.0, act="glu", store=False):
@@ -891,15 +884,15 @@ class CudaKernels:
             _fail(f"unknown activation of the experts '{act}'")
         relu2 = act == "relu2"
         F, top = N1 if relu2 else N1 // 2, idx.shape[1]
-        kind, keep = c_int(1 if relu2 else 0), c_int(1 if store else 0)
+        kind, keep = 1 if relu2 else 0, 1 if store else 0
         _need(h, name="expert input")
         _need(w13, h.dtype, (E, N1, D), "gate/up weights")
         _need(w2, h.dtype, (E, D, F), "down weights")
         _need(idx, torch.int32, (T, top), "chosen experts")
         _need(weights, torch.float32, (T, top), "expert weights")
         _need(x, torch.float32, (T, D), "residual stream")
-        dt = c_int(_dt(h))
-        sizes = (c_int(T), c_int(top), c_int(E), c_int(F), c_int(D))
+        dt = _dt(h)
+        sizes = (T, top, E, F, D)
         if h.dtype == torch.bfloat16 and T > self.MOE_TC_FEW_TOKENS and D % 8 == 0 and F % 8 == 0 and E * max(N1, D) < 2 ** 31:
             # sorted by expert in tiles, both products on the tensor cores: gather the rows, gate/up with the
             # activation in the epilogue, down into 32-bit rows, then the weighted sum into the stream in pair order
@@ -914,31 +907,31 @@ class CudaKernels:
             tile_expert, tiles_used = plan[tiles * rows + pairs:-1], plan[-1:]
             hs = torch.empty(tiles * rows, D, dtype=h.dtype, device=h.device)
             if rows <= 64 and plan_with_rows(pairs, E, D):
-                self._call("moe", "gfb_moe_plan_gather", _ptr(idx), c_int(pairs), c_int(E), c_int(rows), _ptr(h), _ptr(hs), c_int(top), c_int(D),
-                           _ptr(row_pair), _ptr(pair_row), _ptr(tile_expert), c_int(tiles), _ptr(tiles_used), _stream())
+                self._call("moe", "gfb_moe_plan_gather", _ptr(idx), pairs, E, rows, _ptr(h), _ptr(hs), top, D,
+                           _ptr(row_pair), _ptr(pair_row), _ptr(tile_expert), tiles, _ptr(tiles_used), _stream())
             else:
-                self._call("moe", "gfb_moe_plan", _ptr(idx), c_int(pairs), c_int(E), c_int(rows), _ptr(row_pair), _ptr(pair_row),
-                           _ptr(tile_expert), c_int(tiles), _ptr(tiles_used), _stream())
-                self._call("moe", "gfb_moe_gather_rows", _ptr(h), _ptr(row_pair), _ptr(hs), c_int(tiles * rows), c_int(top), c_int(D), _stream())
+                self._call("moe", "gfb_moe_plan", _ptr(idx), pairs, E, rows, _ptr(row_pair), _ptr(pair_row),
+                           _ptr(tile_expert), tiles, _ptr(tiles_used), _stream())
+                self._call("moe", "gfb_moe_gather_rows", _ptr(h), _ptr(row_pair), _ptr(hs), tiles * rows, top, D, _stream())
             mid = torch.empty(tiles * rows, F, dtype=h.dtype, device=h.device)
             self._label = f"moe_{act}_tc {N1}x{D}"
-            self._call("gemm_tc", "gfb_gemm_tc_grouped", _ptr(hs), _ptr(w13), _ptr(mid), c_int(_dt(mid)), c_int(tiles * rows), c_int(rows), c_int(E),
-                       c_int(N1), c_int(D), c_int(_EPI["relu2"] if relu2 else self._EPI_GLU_CLAMP), _ptr(tile_expert), _ptr(tiles_used), c_float(limit), c_float(alpha),
-                       c_float(shift), c_int(expert_blocks_per_sm(T, top, E, N1, self.sm_count)), _ptr(self.status), _stream())
+            self._call("gemm_tc", "gfb_gemm_tc_grouped", _ptr(hs), _ptr(w13), _ptr(mid), _dt(mid), tiles * rows, rows, E,
+                       N1, D, _EPI["relu2"] if relu2 else self._EPI_GLU_CLAMP, _ptr(tile_expert), _ptr(tiles_used), limit, alpha,
+                       shift, expert_blocks_per_sm(T, top, E, N1, self.sm_count), _ptr(self.status), _stream())
             y = torch.empty(tiles * rows, D, dtype=torch.float32, device=h.device)
             self._label = f"moe_down_tc {D}x{F}"
-            self._call("gemm_tc", "gfb_gemm_tc_grouped", _ptr(mid), _ptr(w2), _ptr(y), c_int(_dt(y)), c_int(tiles * rows), c_int(rows), c_int(E),
-                       c_int(D), c_int(F), c_int(_EPI["store"]), _ptr(tile_expert), _ptr(tiles_used), c_float(0.0), c_float(0.0), c_float(0.0),
-                       c_int(expert_blocks_per_sm(T, top, E, D, self.sm_count)), _ptr(self.status), _stream())
-            self._call("moe", "gfb_moe_combine_rows", _ptr(y), _ptr(pair_row), _ptr(weights), _ptr(x), c_int(T), c_int(top), c_int(D), keep,
+            self._call("gemm_tc", "gfb_gemm_tc_grouped", _ptr(mid), _ptr(w2), _ptr(y), _dt(y), tiles * rows, rows, E,
+                       D, F, _EPI["store"], _ptr(tile_expert), _ptr(tiles_used), 0.0, 0.0, 0.0,
+                       expert_blocks_per_sm(T, top, E, D, self.sm_count), _ptr(self.status), _stream())
+            self._call("moe", "gfb_moe_combine_rows", _ptr(y), _ptr(pair_row), _ptr(weights), _ptr(x), T, top, D, keep,
                        _stream())
             return
         if T <= self.MOE_FEW_TOKENS:
             mid = torch.empty(T * top, F, dtype=h.dtype, device=h.device)
-            self._call("moe", "gfb_moe_glu", _ptr(h), _ptr(idx), _ptr(w13), _ptr(mid), dt, kind, *sizes, c_float(limit), c_float(alpha),
-                       c_float(shift), _ptr(None), _ptr(None), c_int(0), _stream())
+            self._call("moe", "gfb_moe_glu", _ptr(h), _ptr(idx), _ptr(w13), _ptr(mid), dt, kind, *sizes, limit, alpha,
+                       shift, _ptr(None), _ptr(None), 0, _stream())
             self._call("moe", "gfb_moe_down", _ptr(mid), _ptr(idx), _ptr(weights), _ptr(w2), _ptr(x), dt, *sizes, _ptr(None), _ptr(None),
-                       c_int(0), _ptr(None), keep, _stream())
+                       0, _ptr(None), keep, _stream())
             return
         # the sorted form: pairs grouped by expert, every expert's rows padded to whole tiles
         rows = self.MOE_TILE_ROWS
@@ -946,14 +939,14 @@ class CudaKernels:
         tiles = (pairs + min(E, pairs) * (rows - 1)) // rows
         plan = torch.empty(tiles * rows + pairs + tiles, dtype=torch.int32, device=h.device)
         row_pair, pair_row, tile_expert = plan[:tiles * rows], plan[tiles * rows:tiles * rows + pairs], plan[tiles * rows + pairs:]
-        self._call("moe", "gfb_moe_plan", _ptr(idx), c_int(pairs), c_int(E), c_int(rows), _ptr(row_pair), _ptr(pair_row),
-                   _ptr(tile_expert), c_int(tiles), _ptr(None), _stream())
+        self._call("moe", "gfb_moe_plan", _ptr(idx), pairs, E, rows, _ptr(row_pair), _ptr(pair_row),
+                   _ptr(tile_expert), tiles, _ptr(None), _stream())
         mid = torch.empty(tiles * rows, F, dtype=h.dtype, device=h.device)
         y = torch.empty(pairs, D, dtype=torch.float32, device=h.device)
-        self._call("moe", "gfb_moe_glu", _ptr(h), _ptr(idx), _ptr(w13), _ptr(mid), dt, kind, *sizes, c_float(limit), c_float(alpha),
-                   c_float(shift), _ptr(row_pair), _ptr(tile_expert), c_int(tiles), _stream())
+        self._call("moe", "gfb_moe_glu", _ptr(h), _ptr(idx), _ptr(w13), _ptr(mid), dt, kind, *sizes, limit, alpha,
+                   shift, _ptr(row_pair), _ptr(tile_expert), tiles, _stream())
         self._call("moe", "gfb_moe_down", _ptr(mid), _ptr(idx), _ptr(weights), _ptr(w2), _ptr(x), dt, *sizes, _ptr(row_pair),
-                   _ptr(tile_expert), c_int(tiles), _ptr(y), keep, _stream())
+                   _ptr(tile_expert), tiles, _ptr(y), keep, _stream())
 
     def activation(self, x, kind, out=None):
         if kind not in _UNARY:
@@ -961,7 +954,7 @@ class CudaKernels:
         out = x if out is None else out
         _need(x, name="activation input")
         _need(out, x.dtype, x.shape, "activation output")
-        self._call("elementwise", "gfb_activation", _ptr(x), _ptr(out), c_int(_dt(x)), c_long(x.numel()), c_int(_EPI[kind]), _stream())
+        self._call("elementwise", "gfb_activation", _ptr(x), _ptr(out), _dt(x), x.numel(), _EPI[kind], _stream())
 
     # -- matrix products -----------------------------------------------------------
     # From this K on a 32-bit product is done in bfloat16 pieces, up to three launches for one or two on CUDA cores; whatever M is, since a row's bits
@@ -992,16 +985,14 @@ class CudaKernels:
         if a.dtype == torch.float32 and K >= self.SPLIT_LEAST_K and K % 4 == 0 and w.data_ptr() % 16 == 0:
             # three bfloat16 pieces per number on the tensor cores, nearer to 64 bits than sums on CUDA cores
             fn = self._f("gemm_split", "gfb_gemm_split_scratch_bytes")
-            fn.restype = c_long
-            scratch = torch.empty(fn(c_int(M), c_int(N), c_int(K)), dtype=torch.uint8, device=a.device)
-            return self._call("gemm_split", "gfb_gemm_split", _ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_int(_EPI[mode]),
+            scratch = torch.empty(fn(M, N, K), dtype=torch.uint8, device=a.device)
+            return self._call("gemm_split", "gfb_gemm_split", _ptr(a), _ptr(w), _ptr(out), M, N, K, _EPI[mode],
                               _ptr(scratch), _ptr(self.status), _stream())
         fn = self._f("gemm_simt", "gfb_gemm_simt_scratch_floats")
-        fn.restype = c_long
-        need = fn(c_int(M), c_int(N), c_int(K))
+        need = fn(M, N, K)
         partial = torch.empty(need, dtype=torch.float32, device=a.device) if need > 0 else None
-        self._call("gemm_simt", "gfb_gemm_simt", _ptr(a), _ptr(w), _ptr(out), c_int(_dt(a)), c_int(_dt(out)),
-                   c_int(M), c_int(N), c_int(K), c_int(_EPI[mode]), _ptr(partial), _stream())
+        self._call("gemm_simt", "gfb_gemm_simt", _ptr(a), _ptr(w), _ptr(out), _dt(a), _dt(out),
+                   M, N, K, _EPI[mode], _ptr(partial), _stream())
 
     def _tc_fits(self, M, N, K, mode) -> bool:
         """The tensor-core kernel takes rows of whole 16-byte units (TMA) and stores in 16-byte vectors."""
@@ -1054,12 +1045,18 @@ class CudaKernels:
     def _linear_tc(self, a, w, out, mode, plan=None, defer=False):
         M, K = a.shape
         N = w.shape[0]
-        swap, bn, splits, stages = plan or self.tc_plan(M, N, K, mode)
+        if plan is None:
+            plan = self._plans.get((M, N, K, mode))
+            if plan is None:
+                if len(self._plans) > 4096:
+                    self._plans.clear()
+                plan = self._plans[(M, N, K, mode)] = self.tc_plan(M, N, K, mode)
+        swap, bn, splits, stages = plan
         ws = torch.empty(splits, M, N, dtype=torch.float32, device=a.device) if splits > 1 else None
-        used = c_int(1)
-        self._call("gemm_tc", "gfb_gemm_tc", _ptr(a), _ptr(w), _ptr(out), c_int(_dt(out)), c_int(M), c_int(N), c_int(K),
-                   c_int(_EPI[mode]), c_int(swap), c_int(bn), c_int(splits), c_int(stages), _ptr(ws),
-                   c_int(0 if defer else 1), ctypes.byref(used), _ptr(self.status), _stream())
+        used = ctypes.c_int(1)
+        self._call("gemm_tc", "gfb_gemm_tc", _ptr(a), _ptr(w), _ptr(out), _dt(out), M, N, K,
+                   _EPI[mode], swap, bn, splits, stages, _ptr(ws),
+                   0 if defer else 1, ctypes.byref(used), _ptr(self.status), _stream())
         if defer and used.value > 1:
             return ws[:used.value]
         return None
@@ -1084,8 +1081,8 @@ class CudaKernels:
             self.attention(q, kv, batch, both, n_head * maps, n_kv, maps * head_dim, scale, window, chunk, sink, dv, values_in_keys,
                            bias, slopes, softcap, keep_first)
             _need(out, q.dtype, (T, n_head * dv), "attention output")
-            return self._call("elementwise", "gfb_diff_combine", _ptr(both), _ptr(out), c_int(_dt(out)), c_int(T), c_int(n_head), c_int(dv),
-                              c_float(diff[0]), c_float(diff[1]), c_float(diff[2]), _stream())
+            return self._call("elementwise", "gfb_diff_combine", _ptr(both), _ptr(out), _dt(out), T, n_head, dv,
+                              diff[0], diff[1], diff[2], _stream())
         if maps not in (1, 2) or (maps == 2) != (diff is not None):
             _fail("two score maps per head come with (lambda, eps, out_scale), one map without")
         if keep_first and not window:
@@ -1111,8 +1108,8 @@ class CudaKernels:
                 # prompts at the sizes the tcgen05 kernel is built for (it takes the maximum of unscaled scores, so scale > 0)
                 self._label = "gfb_latent_attention"
                 return self._call("attention_tc", "gfb_latent_prefill_tc", _ptr(q), _ptr(out), _ptr(kv.k_pool), _ptr(kv.page_table),
-                                  c_int(kv.page_table.shape[1]), c_int(kv.page_size), c_int(kv.k_pool.shape[0]), *self._batch_args(batch),
-                                  c_int(n_head), c_int(head_dim), c_int(dv), c_float(scale), c_int(window or 0), _ptr(sink), _ptr(batch.status),
+                                  kv.page_table.shape[1], kv.page_size, kv.k_pool.shape[0], *self._batch_args(batch),
+                                  n_head, head_dim, dv, scale, window or 0, _ptr(sink), _ptr(batch.status),
                                   _stream())
             # a latent that all heads share: the tensor-core kernel that fetches every cached row once per 64 (token, head)
             # pairs of a sequence (a decode step's heads are the rows of one MMA)
@@ -1126,9 +1123,9 @@ class CudaKernels:
                 if splits > 1:
                     scratch = torch.empty(T * n_head * splits * (dv + 2), dtype=torch.float32, device=q.device)
             return self._call("latent", "gfb_latent_attention", _ptr(q), _ptr(out), _ptr(kv.k_pool), _ptr(kv.page_table),
-                              c_int(kv.page_table.shape[1]), c_int(kv.page_size), c_int(kv.k_pool.shape[0]), *self._batch_args(batch),
-                              c_int(int(batch.max_q_len)), c_int(n_head), c_int(head_dim), c_int(dv), c_float(scale), c_int(window or 0),
-                              _ptr(sink), c_int(splits), _ptr(scratch), _ptr(batch.status), _stream())
+                              kv.page_table.shape[1], kv.page_size, kv.k_pool.shape[0], *self._batch_args(batch),
+                              int(batch.max_q_len), n_head, head_dim, dv, scale, window or 0,
+                              _ptr(sink), splits, _ptr(scratch), _ptr(batch.status), _stream())
         if (not values_in_keys and maps == 1 and dv == head_dim and q.dtype == torch.bfloat16 and kv.page_size == 64 and n_head // n_kv <= 8
                 and (head_dim in (64, 128) or (plain and head_dim % 8 == 0 and head_dim <= 256)) and (not (biased or capped) or scale > 0)
                 and not (keep_first and (biased or sink is not None))):
@@ -1136,13 +1133,13 @@ class CudaKernels:
             # head sizes they are built for
             return self._attention_bf16(q, kv, batch, out, n_head, n_kv, head_dim, scale, window, chunk=chunk, sink=sink,
                                         bias=bias, slopes=slopes, softcap=softcap, keep_first=keep_first)
-        self._call("attention_generic", "gfb_attention_generic", _ptr(q), _ptr(out), c_int(_dt(q)),
+        self._call("attention_generic", "gfb_attention_generic", _ptr(q), _ptr(out), _dt(q),
                    *self._kv_args(kv), *self._batch_args(batch),
-                   c_int(1 if rows_share_keys(T * n_head, batch.max_q_len, batch.max_kv_len, self.SHARING_ROWS) else 0), c_int(n_head), c_int(n_kv),
-                   c_int(head_dim), c_int(dv), c_float(scale), c_int(window or 0), c_int(chunk or 0), _ptr(sink), c_int(1 if values_in_keys else 0),
-                   _ptr(bias), c_int(bias.shape[0] if bias is not None else 0), _ptr(slopes), c_float(softcap or 0.0),
-                   c_int(int(keep_first)), c_int(maps), c_float(diff[0] if diff else 0.0), c_float(diff[1] if diff else 0.0),
-                   c_float(diff[2] if diff else 1.0), _ptr(batch.status), _stream())
+                   1 if rows_share_keys(T * n_head, batch.max_q_len, batch.max_kv_len, self.SHARING_ROWS) else 0, n_head, n_kv,
+                   head_dim, dv, scale, window or 0, chunk or 0, _ptr(sink), 1 if values_in_keys else 0,
+                   _ptr(bias), bias.shape[0] if bias is not None else 0, _ptr(slopes), softcap or 0.0,
+                   int(keep_first), maps, diff[0] if diff else 0.0, diff[1] if diff else 0.0,
+                   diff[2] if diff else 1.0, _ptr(batch.status), _stream())
 
     # rows (token, head) from which a 32-bit prompt's rows share keys and values (`rows_share_keys`)
     SHARING_ROWS = 1536
@@ -1188,20 +1185,20 @@ class CudaKernels:
                 # kept first positions are merged into the rows behind the windowed attention, which leaves each row's log-sum-exp
                 lse = torch.empty(T * n_head, dtype=torch.float32, device=q.device) if keep_first else None
                 self._call("attention_tc", "gfb_attn_prefill_tc_capped", _ptr(q), _ptr(out), *self._kv_args(kv), *self._batch_args(batch),
-                           c_int(n_head), c_int(n_kv), c_int(head_dim), c_float(scale), c_int(window or 0), c_int(chunk or 0),
-                           _ptr(sink), _ptr(arrays), c_int(length), c_int(top), _ptr(per_head), c_float(softcap or 0.0),
-                           c_int(int(keep_first or 0)), _ptr(lse), c_int(tiles), c_int(max_blocks), _ptr(batch.status), _stream())
+                           n_head, n_kv, head_dim, scale, window or 0, chunk or 0,
+                           _ptr(sink), _ptr(arrays), length, top, _ptr(per_head), softcap or 0.0,
+                           int(keep_first or 0), _ptr(lse), tiles, max_blocks, _ptr(batch.status), _stream())
                 return
             if bias is not None or slopes is not None:
                 arrays, length, top, per_head = self._distance_arrays(bias, slopes, scale)
                 self._call("attention_tc", "gfb_attn_prefill_tc_biased", _ptr(q), _ptr(out), *self._kv_args(kv), *self._batch_args(batch),
-                           c_int(n_head), c_int(n_kv), c_int(head_dim), c_float(scale), c_int(window or 0), c_int(chunk or 0),
-                           _ptr(sink), _ptr(arrays), c_int(length), c_int(top), _ptr(per_head), c_int(tiles), c_int(max_blocks),
+                           n_head, n_kv, head_dim, scale, window or 0, chunk or 0,
+                           _ptr(sink), _ptr(arrays), length, top, _ptr(per_head), tiles, max_blocks,
                            _ptr(batch.status), _stream())
                 return
             self._call("attention_tc", "gfb_attn_prefill_tc_masked", _ptr(q), _ptr(out), *self._kv_args(kv), *self._batch_args(batch),
-                       c_int(n_head), c_int(n_kv), c_int(head_dim), c_float(scale), c_int(window or 0), c_int(chunk or 0), _ptr(sink),
-                       c_int(tiles), c_int(max_blocks), _ptr(batch.status), _stream())
+                       n_head, n_kv, head_dim, scale, window or 0, chunk or 0, _ptr(sink),
+                       tiles, max_blocks, _ptr(batch.status), _stream())
             return
         if splits is None:
             splits = 1
@@ -1218,19 +1215,19 @@ class CudaKernels:
             scratch = torch.empty(T * n_head * splits * (head_dim + 2), dtype=torch.float32, device=q.device)
         if capped:
             self._call("attention_bf16", "gfb_attn_decode_capped", _ptr(q), _ptr(out), *self._kv_args(kv), *self._batch_args(batch),
-                       c_int(n_head), c_int(n_kv), c_int(head_dim), c_float(scale), c_int(window or 0), c_int(chunk or 0), _ptr(sink),
-                       _ptr(bias), c_int(bias.shape[0] if bias is not None else 0), _ptr(slopes), c_float(softcap or 0.0),
-                       c_int(int(keep_first or 0)), c_int(splits), _ptr(scratch), _ptr(batch.status), _stream())
+                       n_head, n_kv, head_dim, scale, window or 0, chunk or 0, _ptr(sink),
+                       _ptr(bias), bias.shape[0] if bias is not None else 0, _ptr(slopes), softcap or 0.0,
+                       int(keep_first or 0), splits, _ptr(scratch), _ptr(batch.status), _stream())
             return
         if bias is not None or slopes is not None:
             self._call("attention_bf16", "gfb_attn_decode_biased", _ptr(q), _ptr(out), *self._kv_args(kv), *self._batch_args(batch),
-                       c_int(n_head), c_int(n_kv), c_int(head_dim), c_float(scale), c_int(window or 0), c_int(chunk or 0), _ptr(sink),
-                       _ptr(bias), c_int(bias.shape[0] if bias is not None else 0), _ptr(slopes), c_int(splits), _ptr(scratch),
+                       n_head, n_kv, head_dim, scale, window or 0, chunk or 0, _ptr(sink),
+                       _ptr(bias), bias.shape[0] if bias is not None else 0, _ptr(slopes), splits, _ptr(scratch),
                        _ptr(batch.status), _stream())
             return
         self._call("attention_bf16", "gfb_attn_decode_masked", _ptr(q), _ptr(out), *self._kv_args(kv), *self._batch_args(batch),
-                   c_int(n_head), c_int(n_kv), c_int(head_dim), c_float(scale), c_int(window or 0), c_int(chunk or 0), _ptr(sink),
-                   c_int(splits), _ptr(scratch), _ptr(batch.status), _stream())
+                   n_head, n_kv, head_dim, scale, window or 0, chunk or 0, _ptr(sink),
+                   splits, _ptr(scratch), _ptr(batch.status), _stream())
 
     def rope_append_attention(self, qkv, partials, kv, batch, table, out, n_head, n_kv, head_dim, pairing, append,
                               scale, window=None, lengths_early=None) -> bool:
@@ -1258,10 +1255,10 @@ class CudaKernels:
         scratch = None
         if splits > 1:
             scratch = torch.empty(T * n_head * splits * (head_dim + 2), dtype=torch.float32, device=out.device)
-        self._call("attention_bf16", "gfb_attn_decode_rope", _ptr(src), c_int(n_part), _ptr(out), *self._kv_args(kv),
-                   *self._batch_args(batch), _ptr(table), c_int(table.shape[0]), c_int(n_head), c_int(n_kv), c_int(head_dim),
-                   c_int(_PAIRING[pairing]), c_int(1 if append else 0), c_float(scale), c_int(window or 0), c_int(splits),
-                   _ptr(scratch), _ptr(batch.status), _ptr(lengths_early), c_int(int(batch.max_kv_len)), _stream())
+        self._call("attention_bf16", "gfb_attn_decode_rope", _ptr(src), n_part, _ptr(out), *self._kv_args(kv),
+                   *self._batch_args(batch), _ptr(table), table.shape[0], n_head, n_kv, head_dim,
+                   _PAIRING[pairing], 1 if append else 0, scale, window or 0, splits,
+                   _ptr(scratch), _ptr(batch.status), _ptr(lengths_early), int(batch.max_kv_len), _stream())
         return True
 
     # -- sampling --------------------------------------------------------------------------
@@ -1269,7 +1266,7 @@ class CudaKernels:
         B, V = logits.shape
         _need(logits, torch.float32, name="logits")
         _need(out, torch.int32, (B,), "token output")
-        self._call("sampling", "gfb_argmax", _ptr(logits), _ptr(out), c_int(B), c_int(V), _stream())
+        self._call("sampling", "gfb_argmax", _ptr(logits), _ptr(out), B, V, _stream())
 
     def sample(self, logits, out, temperature, top_k, seed, request_ids=None, token_index=None, index_map=None,
                noise_out=None, seed_dev=None):
@@ -1286,6 +1283,6 @@ class CudaKernels:
             _fail("token index has fewer entries than logits has rows")
         if noise_out is not None:
             _need(noise_out, torch.float32, (B, V), "noise output")
-        self._call("sampling", "gfb_sample", _ptr(logits), _ptr(out), c_int(B), c_int(V), c_float(temperature),
-                   c_int(int(top_k) if top_k else 0), c_ulonglong(seed & (2 ** 64 - 1)), _ptr(seed_dev), _ptr(request_ids),
+        self._call("sampling", "gfb_sample", _ptr(logits), _ptr(out), B, V, temperature,
+                   int(top_k) if top_k else 0, seed & (2 ** 64 - 1), _ptr(seed_dev), _ptr(request_ids),
                    _ptr(token_index), _ptr(index_map), _ptr(noise_out), _stream())
