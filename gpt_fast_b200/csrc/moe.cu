@@ -627,16 +627,26 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __r
 
 // ------------------------------------------------------------------------------------ around the tensor-core tiles ----
 // The tensor cores' tiles read their rows where TMA finds them: side by side in the sorted order.  hs[row] = h[row_pair[row] / top]
-// (zeros for padding rows), 16 bytes per thread and step.
-__global__ void __launch_bounds__(128)
-moe_gather_rows_kernel(const uint4* __restrict__ h, const int* __restrict__ row_pair, uint4* __restrict__ hs, int top, int vec_per_row) {
+// (zeros for padding rows), 16 bytes per thread and step, GATHER_ROWS rows' pieces in flight together.  10,240 rows of
+// 2,048: a row per block 15.3 us, so 11.1.
+constexpr int GATHER_ROWS = 4;
+
+__global__ void __launch_bounds__(256)
+moe_gather_rows_kernel(const uint4* __restrict__ h, const int* __restrict__ row_pair, uint4* __restrict__ hs, int top, int vec_per_row, int rows) {
     gfb_pdl_launch();
     gfb_pdl_wait();
-    const int row = blockIdx.x;
-    const int p = row_pair[row];
-    const uint4* src = p < 0 ? nullptr : h + (size_t)(p / top) * vec_per_row;
-    uint4* dst = hs + (size_t)row * vec_per_row;
-    for (int i = threadIdx.x; i < vec_per_row; i += blockDim.x) dst[i] = src ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+    const int row0 = blockIdx.x * GATHER_ROWS;
+    int p[GATHER_ROWS];
+#pragma unroll
+    for (int k = 0; k < GATHER_ROWS; k++) p[k] = row0 + k < rows ? row_pair[row0 + k] : -1;
+    for (int i = threadIdx.x; i < vec_per_row; i += blockDim.x) {
+        uint4 v[GATHER_ROWS];
+#pragma unroll
+        for (int k = 0; k < GATHER_ROWS; k++) v[k] = p[k] >= 0 ? h[(size_t)(p[k] / top) * vec_per_row + i] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < GATHER_ROWS; k++)
+            if (row0 + k < rows) hs[(size_t)(row0 + k) * vec_per_row + i] = v[k];
+    }
 }
 
 // h [T, D] bfloat16 with D % 8 == 0 -> hs [rows, D] in the plan's sorted order
@@ -644,8 +654,8 @@ GFB_API int gfb_moe_gather_rows(const void* h, const int* row_pair, void* hs, in
     if (rows <= 0) return 0;
     if (D % 8 || ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(hs)) & 15))
         return gfb_fail("gfb_moe_gather_rows: rows of %d bfloat16 numbers are not whole 16-byte pieces", D);
-    cudaError_t e = gfb_launch(moe_gather_rows_kernel, dim3((unsigned)rows), dim3(128), 0, stream, (const uint4*)h, row_pair, (uint4*)hs, top,
-                               D / 8);
+    cudaError_t e = gfb_launch(moe_gather_rows_kernel, dim3((unsigned)((rows + GATHER_ROWS - 1) / GATHER_ROWS)), dim3(256), 0, stream, (const uint4*)h,
+                               row_pair, (uint4*)hs, top, D / 8, rows);
     return gfb_check(e, "gfb_moe_gather_rows");
 }
 

@@ -18,7 +18,7 @@
 //
 // What bounds it: the token-by-token kernel is a chain of dependent instructions per token (sequences of 77, 788 and 1,500 tokens,
 // 64 heads of 128 x 64: 1,135 us).  Here 2.4 GFMA and the S_0s' way through L2: about 230 us (alone and with cold caches ssd_scores_kernel 18,
-// ssd_add_kernel 77, ssd_state_kernel 80, ssd_out_kernel 123).  With the state in a block's registers, walking over a sequence's chunks as it
+// ssd_add_kernel 77, ssd_state_kernel 69, ssd_out_kernel 123).  With the state in a block's registers, walking over a sequence's chunks as it
 // added them up, the longest sequence's 24 chunks took 6.5 us each on less than a block per SM: 274 us.  Against 64-bit sums (700 tokens of
 // 4 heads, outputs): 1.7e-7 where the decays are close to one (token by token 6.2e-7), 0.7e-7 to 0.9e-7 where they are fast (0.9e-7 to
 // 1.1e-7), 0.8e-7 to 1.1e-7 with steps of 0.001 to 0.1 and A of 1 to 16 (1.1e-7 to 1.4e-7).
@@ -226,8 +226,8 @@ ssd_add_kernel(const float* __restrict__ x, int ldx, int b_off, float* __restric
 }
 
 // The walk over a sequence's chunks, four numbers of the state per thread: S_0 of a chunk takes the place of what the chunk adds, S <- decay S + dS.
-// Bound by that traffic; AHEAD chunks' loads are in flight together.
-constexpr int AHEAD = 4;
+// Bound by that traffic; AHEAD chunks' loads are in flight together (sequences of 77, 788 and 1,500 tokens, 64 heads of 128 x 64: four 66 us, eight 55).
+constexpr int AHEAD = 8;
 
 __global__ void __launch_bounds__(THREADS)
 ssd_state_kernel(float* scratch, float* __restrict__ state, size_t state_ld, GfbBatch b, int first_chunk, int n_chunks, Sizes z) {
