@@ -230,6 +230,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
+// one column: a number per lane
+__device__ __forceinline__ void tmem_st1(uint32_t taddr, float v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(__float_as_uint(v)) : "memory");
+}
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
+    uint32_t r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r) :: "memory");
+    return __uint_as_float(r);
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
@@ -1496,7 +1506,7 @@ headwise_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 // that takes its largest possible number (v_scale, from the weights; a normed latent is bounded) to 2^14 .. 2^15: a number keeps 11 bits down to 2^-29
 // of that.  4,096 tokens of 16 heads, the whole layer: 0.0042 from 64 bits, attention on the latent 0.0046.
 //
-// Measured there (R = 512): expansion 25 us, attention 129 (700 and 670 TFLOP/s), where the queries' and outputs' products and attention on the latent take
+// Measured there (R = 512): expansion 25 us, attention 123 (700 and 700 TFLOP/s), where the queries' and outputs' products and attention on the latent take
 // 34 + 64 and 491.
 //
 // keys, values [H][n_seqs * cap][128]: key j of sequence i in row i * cap + j, cap a multiple of 128.  A block takes 128 keys of one head, two
@@ -1630,8 +1640,10 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_con
 }
 
 // Attention of one head over its expanded keys [128 | the 64 rotated numbers all heads share, in the cache's rows] and values [128], the output
-// times a sigmoid gate.  As attn_prefill_tc2_kernel: two tiles of 128 tokens per block, each with four softmax warps, share every 128 keys, and
-// the tensor pipe alternates between them.  Q of both tiles (96 KB) leaves a ring of eight slots of 16 KB for three pieces of K, [128 keys][64
+// times a sigmoid gate.  As attn_prefill_tc2_kernel: two tiles of 128 tokens per block share every 128 keys, and the tensor pipe alternates between
+// them.  What bounds it is a tile's chain of scores, softmax and P V, so each has eight softmax warps: two threads share a row, 64 keys each, and
+// tell each other their maximum (and in the end their sum) through a column of tensor memory that the scores have left (4,096 tokens of
+// 16 heads: a thread per row 129 us, two 123; the products of both tiles behind one another 137).  Q of both tiles (96 KB) leaves a ring of eight slots of 16 KB for three pieces of K, [128 keys][64
 // dims], and two of V, [64 keys][128 dims], per 128 keys, in the order in which they are freed: V_j, K_(j+1), V_(j+1), ...; a
 // piece takes the slot of the eighth piece before it.
 // The reference of the exponentials lags a row's maximum by up to 2^8, as there: float16 weights lose nothing by it that bfloat16 ones would.
@@ -1641,13 +1653,15 @@ struct LhBars {
     unsigned long long q_full;
     unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];   // of even and odd key blocks
     unsigned long long s_full[2], p_ready[2], pv_done[2];              // per tile
+    unsigned long long told[2][4];                                     // per tile and quarter of its rows: both halves of the keys have told
     uint32_t tmem_base;
     int abort_flag;
 };
+constexpr int LH_THREADS = 64 + 2 * 256;
 constexpr uint32_t LH_SMEM = 1024 + 2 * LH_Q_BYTES + LH_SLOTS * HALF_BYTES + sizeof(LhBars);
 static_assert(LH_SMEM <= 227 * 1024, "shared memory");
 
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(LH_THREADS, 1)
 latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qr, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_kr, const __grid_constant__ CUtensorMap map_v, int q_off, __nv_bfloat16* __restrict__ out,
                     const float* __restrict__ v_unscale, const __nv_bfloat16* __restrict__ gate, int ld_gate, int gate_off, int gate_per_head, const int* __restrict__ page_table,
@@ -1670,8 +1684,9 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             mbar_init(smem_u32(&bars->v_full[s]), 1);
             mbar_init(smem_u32(&bars->v_empty[s]), 1);
             mbar_init(smem_u32(&bars->s_full[s]), 1);
-            mbar_init(smem_u32(&bars->p_ready[s]), 4);
+            mbar_init(smem_u32(&bars->p_ready[s]), 8);
             mbar_init(smem_u32(&bars->pv_done[s]), 1);
+            for (int k = 0; k < 4; k++) mbar_init(smem_u32(&bars->told[s][k]), 2);
         }
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1731,17 +1746,21 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 auto load_k = [&](int j) -> bool {
                     const uint32_t full = smem_u32(&bars->k_full[j & 1]), ph = ((uint32_t)(j >> 1) & 1u) ^ 1u;
                     const int row = row0 + (blk0 + j) * KEYS;
+                    int page[2];                                         // (asked for ahead of the waits)
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {                        // (no such page, or one ahead of the window: any other, masked later)
+                        const int pi = min(max((blk0 + j) * 2 + i, lo_page), last_page);
+                        page[i] = pi < max_pages ? pt[pi] : -1;
+                    }
                     if (!mbar_wait(smem_u32(&bars->k_empty[j & 1]), ph, abort_flag, status, 44)) return false;       // K of block j - 2
                     mbar_expect_tx(full, 3 * HALF_BYTES);
                     tma_load_2d(slot_at(5 * j), &map_k, 0, row, full);
                     if (!mbar_wait(smem_u32(&bars->v_empty[j & 1]), ph, abort_flag, status, 45)) return false;       // V of block j - 2
                     tma_load_2d(slot_at(5 * j + 1), &map_k, 64, row, full);
 #pragma unroll
-                    for (int i = 0; i < 2; i++) {                        // (no such page, or one ahead of the window: any other, masked later)
-                        const int pi = min(max((blk0 + j) * 2 + i, lo_page), last_page);
-                        int page = pi < max_pages ? pt[pi] : -1;
-                        if (page < 0 || page >= n_pages_pool) { gfb_report(status, GFB_ERR_PAGE_TABLE, slot, pi); page = 0; }
-                        tma_load_2d(slot_at(5 * j + 2) + i * PIECE_BYTES, &map_kr, R, page * PAGE, full);
+                    for (int i = 0; i < 2; i++) {
+                        if (page[i] < 0 || page[i] >= n_pages_pool) { gfb_report(status, GFB_ERR_PAGE_TABLE, slot, (blk0 + j) * 2 + i); page[i] = 0; }
+                        tma_load_2d(slot_at(5 * j + 2) + i * PIECE_BYTES, &map_kr, R, page[i] * PAGE, full);
                     }
                     return true;
                 };
@@ -1811,10 +1830,27 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 }
             }
         } else {
-            const int x = (warp - 2) >> 2;                                   // warps 2..5: tile 0, warps 6..9: tile 1
+            const int x = (warp - 2) >> 3, half = (warp - 2) >> 2 & 1;       // warps 2..9: tile 0, 10..17: tile 1; the first four of them keys 0..63
             const int q = warp & 3, r = q * 32 + lane;
             const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
-            const uint32_t col_s = 128 * x, col_o = 256 + 128 * x;
+            const uint32_t col_s = 128 * x, col_o = 256 + 128 * x + 64 * half;       // (each half also rescales and writes half of O)
+            const uint32_t told = smem_u32(&bars->told[x][q]);
+            // the last column of either half of the scores: its own half's thread writes it behind its loads, the other reads it ahead of
+            // what comes next there (P of the second half in columns 32 .. 63, the next scores)
+            const uint32_t col_mine = lane_base + col_s + 63 + 64 * half, col_other = lane_base + col_s + 63 + 64 * (half ^ 1);
+            uint32_t n_told = 0;
+            auto exchange = [&](float mine, float& other) -> bool {
+                tmem_st1(col_mine, mine);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(told);
+                if (!mbar_wait(told, n_told & 1u, abort_flag, status, 54)) return false;
+                n_told++;
+                tc_fence_after();
+                other = tmem_ld1(col_other);
+                return true;
+            };
             const bool row_ok = r < nq[x];
             const int row_pos = pos0[x] + r, row_lo = first_key(row_pos, window, 0), last_lo = first_key(pos0[x] + max(nq[x], 1) - 1, window, 0);
             float m_run = -INFINITY, l_run = 0.f;
@@ -1822,15 +1858,23 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             bool ok = true;
             for (int j = 0; j < n_iter && ok; j++) {
                 if (!active(x, j)) continue;
-                const int key0 = (blk0 + j) * KEYS;
+                const int key0 = (blk0 + j) * KEYS + 64 * half;
                 ok = mbar_wait(smem_u32(&bars->s_full[x]), n_done & 1u, abort_flag, status, 51);
                 if (!ok) break;
                 tc_fence_after();
-                float v[4][32];
-                tmem_ld_row128(lane_base + col_s, v);
-                if (key0 + KEYS - 1 > pos0[x] || key0 < last_lo || nq[x] < ROWS) {
+                uint32_t raw[2][32];
+                tmem_ld32_issue(lane_base + col_s + 64 * half, raw[0]);
+                tmem_ld32_issue(lane_base + col_s + 64 * half + 32, raw[1]);
+                tmem_ld_wait32(raw[0]);
+                tmem_ld_wait32(raw[1]);
+                float v[2][32];
 #pragma unroll
-                    for (int c = 0; c < 4; c++)
+                for (int c = 0; c < 2; c++)
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[c][i] = __uint_as_float(raw[c][i]);
+                if (key0 + 63 > pos0[x] || key0 < last_lo || nq[x] < ROWS) {
+#pragma unroll
+                    for (int c = 0; c < 2; c++)
 #pragma unroll
                         for (int i = 0; i < 32; i++) {
                             const int kj = key0 + c * 32 + i;
@@ -1840,18 +1884,22 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 float mx4[4];
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    mx4[c] = fmaxf(v[c][0], v[c][1]);
+                    const float* y = &v[c >> 1][(c & 1) * 16];
+                    mx4[c] = fmaxf(y[0], y[1]);
 #pragma unroll
-                    for (int i = 2; i < 32; i += 2) mx4[c] = max3(mx4[c], v[c][i], v[c][i + 1]);
+                    for (int i = 2; i < 16; i += 2) mx4[c] = max3(mx4[c], y[i], y[i + 1]);
                 }
-                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])), theirs;
+                ok = exchange(mx, theirs);
+                if (!ok) break;
+                mx = fmaxf(mx, theirs);
                 float m_new = m_run;
                 if (mx > m_run && (m_run == -INFINITY || (mx - m_run) * scale_log2e > 8.f)) m_new = mx;
                 const float corr = (m_run == -INFINITY || m_new == m_run) ? 1.f : fast_exp2((m_run - m_new) * scale_log2e);
                 const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * scale_log2e;
-                float rsum[4] = {0.f, 0.f, 0.f, 0.f};
+                float rsum[2] = {0.f, 0.f};
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
+                for (int c = 0; c < 2; c++) {
                     uint32_t pk[16];
                     float odd = 0.f;
 #pragma unroll
@@ -1863,7 +1911,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         pk[i >> 1] = pack2_half(p0, p1);
                     }
                     rsum[c] += odd;
-                    tmem_st16(lane_base + col_s + c * 16, pk);               // (all of this row's scores are in registers by now)
+                    tmem_st16(lane_base + col_s + 32 * half + c * 16, pk);   // (both halves of this row's scores are in registers by now)
                 }
                 // O follows a new reference, rarely (S of this block was issued behind the tile's previous P V, so that the wait only orders the accesses)
                 if (n_done > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
@@ -1871,7 +1919,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll 1
-                    for (int c = 0; c < 4; c++) {
+                    for (int c = 0; c < 2; c++) {
                         float o[32];
                         tmem_ld32(lane_base + col_o + c * 32, o);
 #pragma unroll
@@ -1883,34 +1931,40 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bars->p_ready[x]));
-                l_run = l_run * corr + (rsum[0] + rsum[1]) + (rsum[2] + rsum[3]);
+                l_run = l_run * corr + (rsum[0] + rsum[1]);
                 m_run = m_new;
                 n_done++;
             }
             if (ok && n_done > 0) ok = mbar_wait(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 53);
             if (ok && n_done > 0) {
                 tc_fence_after();
+                float theirs;
+                ok = exchange(l_run, theirs);                                // (the last P has been read)
+                l_run = half ? theirs + l_run : l_run + theirs;
+            }
+            if (ok && n_done > 0) {
                 if (sink != nullptr && m_run != -INFINITY) l_run += fast_exp2(sink[head] * 1.4426950408889634f - m_run * scale_log2e);
                 const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
                 const size_t t = (size_t)(t_first + tq0 + x * ROWS + (row_ok ? r : 0));
-                __nv_bfloat16* dst = out + (t * H + head) * D;
+                const int dim0 = 64 * half;
+                __nv_bfloat16* dst = out + (t * H + head) * D + dim0;
                 const __nv_bfloat16* gt = gate + t * ld_gate + gate_off;
                 const float per_head = gate_per_head ? 1.0f / (1.0f + expf(-__bfloat162float(gt[head]))) : 1.f;
 #pragma unroll 1
-                for (int c = 0; c < 4; c++) {
+                for (int c = 0; c < 2; c++) {
                     float o[32];
                     tmem_ld32(lane_base + col_o + c * 32, o);
                     if (row_ok) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
-                            const float4 u0 = *reinterpret_cast<const float4*>(v_unscale + head * D + c * 32 + i);
-                            const float4 u1 = *reinterpret_cast<const float4*>(v_unscale + head * D + c * 32 + i + 4);
+                            const float* un = v_unscale + head * D + dim0 + c * 32 + i;
+                            const float4 u0 = *reinterpret_cast<const float4*>(un), u1 = *reinterpret_cast<const float4*>(un + 4);
                             const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
                             float y[8];
 #pragma unroll
                             for (int e = 0; e < 8; e++) y[e] = o[i + e] * inv * u[e] * per_head;
                             if (!gate_per_head) {
-                                const uint4 g8 = *reinterpret_cast<const uint4*>(gt + head * D + c * 32 + i);
+                                const uint4 g8 = *reinterpret_cast<const uint4*>(gt + head * D + dim0 + c * 32 + i);
                                 const uint32_t g4[4] = {g8.x, g8.y, g8.z, g8.w};
 #pragma unroll
                                 for (int e = 0; e < 4; e++) {
@@ -2301,7 +2355,7 @@ GFB_API int gfb_latent_expanded(const void* proj, int ld, int q_off, int gate_of
     e = gfb_launch(latent_expand_kernel, dim3((unsigned)(rows / KEYS * H)), dim3(192), LE_SMEM, stream, maps[0], maps[1], maps[2], (__nv_bfloat16*)keys,
                    (__half*)values, v_scale, page_table, max_pages, n_pages, b, H, R, cap, window, status);
     if (gfb_check(e, "gfb_latent_expanded (keys and values)")) return 1;
-    e = gfb_launch(latent_heads_kernel, dim3((unsigned)(n_x * H)), dim3(320), LH_SMEM, stream, maps[3], maps[4], maps[5], maps[0], maps[6], q_off,
+    e = gfb_launch(latent_heads_kernel, dim3((unsigned)(n_x * H)), dim3(LH_THREADS), LH_SMEM, stream, maps[3], maps[4], maps[5], maps[0], maps[6], q_off,
                    (__nv_bfloat16*)out, v_scale + (size_t)H * D, (const __nv_bfloat16*)proj, ld, gate_off, gate_per_head, page_table, max_pages, n_pages, b, H, R, cap,
                    scale * 1.4426950408889634f, window, sink, (int)n_x, status);
     return gfb_check(e, "gfb_latent_expanded");

@@ -87,6 +87,85 @@ __global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int q_o
     }
 }
 
+// The same for bfloat16 in rows of whole 16-byte pieces and neighbouring pairs: eight numbers per access.  It only moves data (4,096 tokens of 16
+// heads: 26 MB), but two bytes at a time its accesses took 20.7 us; 13.3 so.
+constexpr int PREPARE_THREADS = 128;
+
+// four neighbouring pairs turned by their angles; cs: (cos, sin) of each
+__device__ __forceinline__ uint4 turn_four(uint4 v, const float* __restrict__ cs) {
+    const float4 a = *reinterpret_cast<const float4*>(cs), b = *reinterpret_cast<const float4*>(cs + 4);
+    const float c[4] = {a.x, a.z, b.x, b.z}, s[4] = {a.y, a.w, b.y, b.w};
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float x = __uint_as_float(w[i] << 16), y = __uint_as_float(w[i] & 0xffff0000u);
+        const __nv_bfloat162 o = __floats2bfloat162_rn(x * c[i] - y * s[i], y * c[i] + x * s[i]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&o);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__global__ void __launch_bounds__(PREPARE_THREADS)
+latent_prepare_wide_kernel(const __nv_bfloat16* __restrict__ src, int ld, int q_off, int kv_off, __nv_bfloat16* __restrict__ q_out, int q_pitch, int q_at,
+                           GfbPagedKV kv, GfbBatch b, const float* __restrict__ table, int table_len, const void* __restrict__ norm_w, int w_dt, float eps,
+                           int H, int d, int rot, int rank, int append, int* status) {
+    __shared__ float scratch[32];
+    gfb_pdl_launch();
+    gfb_pdl_wait();
+    const int t = blockIdx.x, tid = threadIdx.x;
+    const int s = b.tok_seq[t];
+    const int slot = b.slots[s];
+    const int pos = b.lengths[slot] + (t - b.cu_seqlens[s]);
+    const __nv_bfloat16* row = src + (size_t)t * ld;
+    const bool pos_ok = pos >= 0 && pos < table_len;
+    if (!pos_ok && tid == 0) gfb_report(status, GFB_ERR_CACHE_RANGE, t, pos);
+    const float* cs = table + (size_t)(pos_ok ? pos : 0) * rot;          // [rot/2][2]
+    const int units = rot / 8;
+    for (int i = tid; i < H * units; i += PREPARE_THREADS) {
+        const int h = i / units, u = (i - h * units) * 8;
+        const uint4 v = *reinterpret_cast<const uint4*>(row + q_off + (size_t)h * (d + rot) + d + u);
+        *reinterpret_cast<uint4*>(q_out + ((size_t)t * H + h) * q_pitch + q_at + u) = turn_four(v, cs + u);
+    }
+    if (!append) return;
+    const int pi = pos / kv.page_size;
+    int page = (pos_ok && pi < kv.max_pages) ? kv.page_table[(size_t)slot * kv.max_pages + pi] : -1;
+    if (page < 0 || page >= kv.n_pages) {
+        if (tid == 0 && pos_ok) gfb_report(status, GFB_ERR_PAGE_TABLE, slot, pi);
+        page = -1;
+    }
+    const __nv_bfloat16* dkv = row + kv_off;
+    float ss = 0.f;
+    for (int i = tid * 8; i < rank; i += PREPARE_THREADS * 8) {
+        const uint4 v = *reinterpret_cast<const uint4*>(dkv + i);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float x = __uint_as_float(w[k] << 16), y = __uint_as_float(w[k] & 0xffff0000u);
+            ss += x * x;
+            ss += y * y;
+        }
+    }
+    ss = gfb_block_sum(ss, scratch);
+    if (page < 0) return;
+    const float r = 1.0f / sqrtf(ss / (float)rank + eps);
+    __nv_bfloat16* krow = (__nv_bfloat16*)kv.k_pool + ((size_t)page * kv.page_size + (pos % kv.page_size)) * (rank + rot);
+    for (int i = tid * 8; i < rank + rot; i += PREPARE_THREADS * 8) {
+        const uint4 v = *reinterpret_cast<const uint4*>(dkv + i);
+        if (i >= rank) {
+            *reinterpret_cast<uint4*>(krow + i) = turn_four(v, cs + (i - rank));
+            continue;
+        }
+        uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const __nv_bfloat162 o = __floats2bfloat162_rn(__uint_as_float(w[k] << 16) * r * ld_any(norm_w, w_dt, i + 2 * k),
+                                                           __uint_as_float(w[k] & 0xffff0000u) * r * ld_any(norm_w, w_dt, i + 2 * k + 1));
+            w[k] = *reinterpret_cast<const uint32_t*>(&o);
+        }
+        *reinterpret_cast<uint4*>(krow + i) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 // src [T, ld]: at q_off H heads of (d + rot) numbers (d unrotated, then rot rotated), at kv_off rank + rot numbers.
 // q_out [T, H, q_pitch]: only rot numbers of every head, from q_at on, are written here.  The cache entry has one
 // key head of rank + rot numbers per token (its value pool is not used).  table float32 [table_len, rot/2, 2].
@@ -100,7 +179,11 @@ GFB_API int gfb_latent_prepare(const void* src, int dt, int ld, int q_off, int k
     GfbPagedKV kv{k_pool, nullptr, page_table, max_pages, page_size, n_pages};
     GfbBatch b{cu_seqlens, tok_seq, slots, lengths, n_seqs, n_tokens};
     cudaError_t e;
-    if (dt == GFB_BF16)
+    if (dt == GFB_BF16 && pairing == 0 && (rot | rank | d | ld | q_off | kv_off | q_pitch | q_at) % 8 == 0 &&
+        (((uintptr_t)src | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)table) & 15) == 0)
+        e = gfb_launch(latent_prepare_wide_kernel, dim3(n_tokens), dim3(PREPARE_THREADS), 0, stream, (const __nv_bfloat16*)src, ld, q_off, kv_off,
+                       (__nv_bfloat16*)q_out, q_pitch, q_at, kv, b, table, table_len, norm_w, w_dt, eps, H, d, rot, rank, append, status);
+    else if (dt == GFB_BF16)
         e = gfb_launch(latent_prepare_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(128), 0, stream, (const __nv_bfloat16*)src, ld, q_off,
                        kv_off, (__nv_bfloat16*)q_out, q_pitch, q_at, kv, b, table, table_len, norm_w, w_dt, eps, H, d, rot, rank, pairing, append, status);
     else if (dt == GFB_F32)
