@@ -370,6 +370,11 @@ __device__ __forceinline__ void load_pairs(const RopeSource& r, const size_t* e0
 
 constexpr int MERGE_SLICES = 8;              // the largest portable cluster
 
+// What a slice adds to a row's sum of weights and to its outputs, rounded as written in both forms of the merge, whatever the compiler makes
+// of the code around it.
+__device__ __forceinline__ float plus_slice_sum(float l, float slice, float weight) { return __fadd_rn(l, __fmul_rn(slice, weight)); }
+__device__ __forceinline__ float plus_slice(float o, float slice, float weight) { return __fmaf_rn(slice, weight, o); }
+
 template <int D, int SRC, int DECODE_NBUF>
 __global__ void __launch_bounds__(THREADS)
 attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -800,9 +805,9 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             for (int k = 0; k < MERGE_SLICES; k++)
                 if (k < splits && part[k].x != -INFINITY) {
                     const float e = exp2f(part[k].x - m);
-                    l += part[k].y * e;
-                    o0 += row[k].x * e;
-                    o1 += row[k].y * e;
+                    l = plus_slice_sum(l, part[k].y, e);
+                    o0 = plus_slice(o0, row[k].x, e);
+                    o1 = plus_slice(o1, row[k].y, e);
                 }
             const float inv = l > 0.f ? 1.f / l : 0.f;
             *reinterpret_cast<__nv_bfloat162*>(out + ((size_t)t * H + head) * D + dim) = __floats2bfloat162_rn(o0 * inv, o1 * inv);
@@ -844,13 +849,14 @@ __global__ void attn_combine_kernel(const float* __restrict__ scratch_o, const f
     const float sk = sink != nullptr ? sink[head] * 1.4426950408889634f : -INFINITY;
     m = fmaxf(m, sk);
     float l = sink != nullptr ? exp2f(sk - m) : 0.f;
-    for (int z = 0; z < splits; z++) l += (ml[2 * z] == -INFINITY) ? 0.f : ml[2 * z + 1] * exp2f(ml[2 * z] - m);
+    for (int z = 0; z < splits; z++)
+        if (ml[2 * z] != -INFINITY) l = plus_slice_sum(l, ml[2 * z + 1], exp2f(ml[2 * z] - m));
     float inv = l > 0.f ? 1.f / l : 0.f;
     for (int dim = threadIdx.x; dim < d; dim += blockDim.x) {
         float o = 0.f;
         for (int z = 0; z < splits; z++) {
             if (ml[2 * z] == -INFINITY) continue;
-            o += scratch_o[(((size_t)t * H + head) * splits + z) * d + dim] * exp2f(ml[2 * z] - m);
+            o = plus_slice(o, scratch_o[(((size_t)t * H + head) * splits + z) * d + dim], exp2f(ml[2 * z] - m));
         }
         out[((size_t)t * H + head) * d + dim] = __float2bfloat16_rn(o * inv);
     }
@@ -954,10 +960,11 @@ cudaError_t launch_decode_mma(int d, int src, dim3 grid, cudaStream_t stream, co
 
 }  // namespace
 
-// whether the tensor-core kernel's slices merge within a cluster
-static int merged(int splits) { return splits > 1 && splits <= MERGE_SLICES; }
+// Whether the tensor-core kernel's slices merge within a cluster: up to MERGE_SLICES of them, where the caller has no scratch for a merge behind.
+static int merged(int splits, const float* scratch) { return scratch == nullptr && splits > 1 && splits <= MERGE_SLICES; }
 
-// Bytes of scratch the decode kernel needs for `splits` > 1: [T, H, splits, d + 2] floats.
+// Bytes of scratch in which the decode kernel leaves `splits` > 1 slices for a merge behind it: [T, H, splits, d + 2] floats.  Without
+// scratch up to 8 slices of head_dim 64 or 128 merge within a cluster of blocks, to the same bits.
 GFB_API long gfb_attn_decode_scratch_bytes(int T, int H, int d, int splits) {
     return splits > 1 ? (long)T * H * splits * (d + 2) * 4 : 0;
 }
@@ -1033,7 +1040,8 @@ GFB_API int gfb_attn_decode_capped(const void* q, void* out, void* k_pool, void*
     if (d % 8 || d > THREADS * MAX_DPT) return gfb_fail("gfb_attn_decode: head_dim %d must be a multiple of 8, at most %d", d, THREADS * MAX_DPT);
     if (G <= 0 || H % G || H / G > MAX_REP) return gfb_fail("gfb_attn_decode: %d heads over %d groups (at most %d per group)", H, G, MAX_REP);
     if (splits < 1 || G > 65535 || splits > 65535) return gfb_fail("gfb_attn_decode: bad split count %d", splits);
-    if (splits > 1 && scratch == nullptr) return gfb_fail("gfb_attn_decode: %d slices need scratch memory", splits);
+    const bool mma = d == 128 || d == 64;
+    if (splits > 1 && scratch == nullptr && !(mma && merged(splits, scratch))) return gfb_fail("gfb_attn_decode: %d slices need scratch memory", splits);
     const int rep = H / G;
     size_t smem = (size_t)4 * PAGE * d * 2 + (size_t)rep * d * 4 + (size_t)rep * PAGE * 4;
     static size_t configured = 0;
@@ -1048,7 +1056,7 @@ GFB_API int gfb_attn_decode_capped(const void* q, void* out, void* k_pool, void*
     float* sml = scratch ? scratch + (size_t)n_tokens * H * splits * d : nullptr;
     dim3 grid(n_tokens, G, splits);
     cudaError_t e;
-    if (d == 128 || d == 64) {
+    if (mma) {
         RopeSource rs{};
         rs.chunk = chunk;
         rs.sink = sink;
@@ -1057,7 +1065,7 @@ GFB_API int gfb_attn_decode_capped(const void* q, void* out, void* k_pool, void*
         rs.slopes = slopes;
         rs.keep_first = keep_first;
         rs.softcap = softcap;
-        rs.merge = merged(splits);
+        rs.merge = merged(splits, scratch);
         e = launch_decode_mma(d, SRC_Q, grid, stream, q, out, so, sml, kv, b, H, G, scale, window, splits, status, rs, 0);
         if (e == cudaErrorInvalidValue && gfb_error_text[0]) return 1;
     } else {
@@ -1065,7 +1073,7 @@ GFB_API int gfb_attn_decode_capped(const void* q, void* out, void* k_pool, void*
                        (__nv_bfloat16*)out, so, sml, kv, b, H, G, d, scale * 1.4426950408889634f, window, splits, status);
     }
     if (gfb_check(e, "gfb_attn_decode")) return 1;
-    if (splits > 1 && !((d == 128 || d == 64) && merged(splits))) {
+    if (splits > 1 && scratch != nullptr) {
         dim3 cgrid(n_tokens, H);
         e = gfb_launch(attn_combine_kernel, cgrid, dim3(128), 0, stream, (const float*)so, (const float*)sml,
                        (__nv_bfloat16*)out, H, d, splits, sink);
@@ -1093,7 +1101,7 @@ GFB_API int gfb_attn_decode_rope(const void* src, int n_part, void* out, void* k
     if (d != 64 && d != 128) return gfb_fail("gfb_attn_decode_rope: head_dim %d (64 or 128)", d);
     if (G <= 0 || H % G || H / G > MAX_REP) return gfb_fail("gfb_attn_decode_rope: %d heads over %d groups (at most %d per group)", H, G, MAX_REP);
     if (splits < 1 || G > 65535 || splits > 65535) return gfb_fail("gfb_attn_decode_rope: bad split count %d", splits);
-    if (splits > 1 && scratch == nullptr) return gfb_fail("gfb_attn_decode_rope: %d slices need scratch memory", splits);
+    if (splits > 1 && scratch == nullptr && !merged(splits, scratch)) return gfb_fail("gfb_attn_decode_rope: %d slices need scratch memory", splits);
     if (pairing != 0 && pairing != 1) return gfb_fail("gfb_attn_decode_rope: unknown pairing %d", pairing);
     if ((uintptr_t)src % 8) return gfb_fail("gfb_attn_decode_rope: the q/k/v product must start on an 8-byte boundary");
     GfbPagedKV kv{k_pool, v_pool, page_table, max_pages, page_size, n_pages};
@@ -1102,7 +1110,7 @@ GFB_API int gfb_attn_decode_rope(const void* src, int n_part, void* out, void* k
     float* sml = scratch ? scratch + (size_t)n_tokens * H * splits * d : nullptr;
     RopeSource rs{src, n_part, (size_t)n_tokens * (H + 2 * G) * d, table, table_len, pairing, append, lengths_early,
                   n_tokens == n_seqs ? 1 : 0, 0, nullptr};
-    rs.merge = merged(splits);
+    rs.merge = merged(splits, scratch);
     const int pages = max_kv_len > 0 ? (max_kv_len + PAGE - 1) / PAGE : 0;
     cudaError_t e = launch_decode_mma(d, n_part > 0 ? SRC_PARTIALS : SRC_QKV, dim3(n_tokens, G, splits), stream, nullptr, out, so, sml,
                                       kv, b, H, G, scale, window, splits, status, rs, (pages + splits - 1) / splits);

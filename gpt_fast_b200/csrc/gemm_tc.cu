@@ -1375,7 +1375,8 @@ int dispatch_epi(int epi, int out_dt, const CUtensorMap& mx, const CUtensorMap& 
 // (bn 128 or 256); swap = 1: 128 weight rows x bn tokens (bn 16, 32, 64 or 128, M <= bn * tiles).
 // splits > 1 (swap only) writes partials to `workspace` ([splits, M, N] f32); with reduce != 0 they are
 // summed and the epilogue applied by a second kernel, with reduce == 0 the caller's next kernel consumes
-// them.  *splits_used receives the number of slices that were written.
+// them.  With reduce != 0 and no workspace up to 8 slices merge within a cluster of blocks, to the same bits.
+// *splits_used receives the number of slices.
 GFB_API int gfb_gemm_tc(const void* A, const void* W, void* out, int out_dt, int M, int N, int K, int epi, int swap,
                         int bn, int splits, int stages, float* workspace, int reduce, int* splits_used, int* status,
                         cudaStream_t stream) {
@@ -1397,7 +1398,8 @@ GFB_API int gfb_gemm_tc(const void* A, const void* W, void* out, int out_dt, int
     splits = (total_kb + kbps - 1) / kbps;                 // no empty split
     if (splits_used) *splits_used = splits;
     if (splits > 1 && !swap) return gfb_fail("gfb_gemm_tc: a split over K needs the swapped orientation");
-    if (splits > 1 && workspace == nullptr) return gfb_fail("gfb_gemm_tc: a split over K needs a workspace");
+    const bool merge = splits > 1 && reduce && workspace == nullptr && splits <= MERGE_SPLITS;
+    if (splits > 1 && workspace == nullptr && !merge) return gfb_fail("gfb_gemm_tc: a split over K needs a workspace");
 
     const int ldo = epi == EPI_SWIGLU ? N / 2 : N;
     const int R = swap ? N : M, Cc = swap ? M : N;
@@ -1448,7 +1450,7 @@ GFB_API int gfb_gemm_tc(const void* A, const void* W, void* out, int out_dt, int
         if (out_dt == GFB_F32) return launch_persistent<EPI_STORE, float>(mx, my2, out, M, N, K, ldo, st, sm_count, status, stream);
         return launch_persistent<EPI_STORE, bf16>(mx, my2, out, M, N, K, ldo, st, sm_count, status, stream);
     }
-    if (swap && splits > 1 && reduce && splits <= MERGE_SPLITS) {
+    if (merge) {
 #define MERGED(B) return dispatch_merged<B>(epi, out_dt, mx, my, out, R, Cc, K, ldo, splits, kbps, stages, status, stream)
         if (bn == 16) MERGED(16);
         if (bn == 32) MERGED(32);

@@ -139,6 +139,15 @@ def ssd_in_chunks(n_tokens: int, n_seqs: int, longest: int, n_head: int, head_di
     return max(longest, busy) + 2.3 * w * n_seqs >= line * (1 + each * chunks)
 
 
+MERGED_SLICES = 8                      # slices of a sum that merge within a cluster of blocks, without scratch
+
+
+def split_parts(K: int, splits: int) -> int:
+    """The parts that a product split over K has: portions of whole stages of 64 numbers, none of them empty."""
+    stages = -(-K // 64)
+    return -(-stages // -(-stages // min(splits, stages)))
+
+
 def rows_share_keys(rows: int, longest: int, max_kv_len: int, line: int) -> bool:
     """Whether the rows (token, head) of a step's 32-bit attention share the keys and values of sixteen rows per block; the bits are the same.  A block
     then has sixteen rows' work in a row, so it takes rows enough, fewer where keys are many.  us shared | a block per row: 64 tokens of
@@ -1042,7 +1051,8 @@ class CudaKernels:
             self._status = torch.zeros(4, dtype=torch.int32, device="cuda")
         return self._status
 
-    def _linear_tc(self, a, w, out, mode, plan=None, defer=False):
+    def _linear_tc(self, a, w, out, mode, plan=None, defer=False, merge=True):
+        """merge=False: the parts of a split over K always go through memory (the same bits)."""
         M, K = a.shape
         N = w.shape[0]
         if plan is None:
@@ -1052,7 +1062,9 @@ class CudaKernels:
                     self._plans.clear()
                 plan = self._plans[(M, N, K, mode)] = self.tc_plan(M, N, K, mode)
         swap, bn, splits, stages = plan
-        ws = torch.empty(splits, M, N, dtype=torch.float32, device=a.device) if splits > 1 else None
+        parts = split_parts(K, splits)
+        merge = merge and not defer and parts <= MERGED_SLICES
+        ws = torch.empty(parts, M, N, dtype=torch.float32, device=a.device) if parts > 1 and not merge else None
         used = ctypes.c_int(1)
         self._call("gemm_tc", "gfb_gemm_tc", _ptr(a), _ptr(w), _ptr(out), _dt(out), M, N, K,
                    _EPI[mode], swap, bn, splits, stages, _ptr(ws),
@@ -1174,7 +1186,8 @@ class CudaKernels:
         return arrays, length, top, per_head
 
     def _attention_bf16(self, q, kv, batch, out, n_head, n_kv, head_dim, scale, window, splits=None, prefill=None, tiles=0,
-                        max_blocks=0, chunk=None, sink=None, bias=None, slopes=None, softcap=None, keep_first=0):
+                        max_blocks=0, chunk=None, sink=None, bias=None, slopes=None, softcap=None, keep_first=0, merge=True):
+        """merge=False: the slices of a decode step always go through memory (the same bits)."""
         T = batch.n_tokens
         capped = bool(softcap) or bool(keep_first)
         if prefill is None:
@@ -1211,7 +1224,7 @@ class CudaKernels:
             if keep_first:
                 splits += 1                                 # the kept first positions are a slice of their own, the grid's last
         scratch = None
-        if splits > 1:
+        if splits > 1 and not (merge and splits <= MERGED_SLICES and head_dim in (64, 128)):
             scratch = torch.empty(T * n_head * splits * (head_dim + 2), dtype=torch.float32, device=q.device)
         if capped:
             self._call("attention_bf16", "gfb_attn_decode_capped", _ptr(q), _ptr(out), *self._kv_args(kv), *self._batch_args(batch),
@@ -1230,11 +1243,11 @@ class CudaKernels:
                    splits, _ptr(scratch), _ptr(batch.status), _stream())
 
     def rope_append_attention(self, qkv, partials, kv, batch, table, out, n_head, n_kv, head_dim, pairing, append,
-                              scale, window=None, lengths_early=None) -> bool:
+                              scale, window=None, lengths_early=None, merge=True) -> bool:
         """Rotary encoding, cache append and attention of a decode step in one launch, where the kernel for
         it fits (bfloat16, one token per sequence, head_dim 64 or 128, pages of 64, at most 8 query heads per
         key/value head).  Returns False, having done nothing, where it does not.  lengths_early (tests only):
-        what the kernel's read of the lengths ahead of its dependency wait is to see."""
+        what the kernel's read of the lengths ahead of its dependency wait is to see; merge as in _attention_bf16."""
         T = batch.n_tokens
         if not (out.dtype == torch.bfloat16 and batch.max_q_len == 1 and head_dim in (64, 128) and kv.page_size == 64
                 and n_head // n_kv <= 8):
@@ -1253,7 +1266,7 @@ class CudaKernels:
             _fail(f"key pool pages are {tuple(kv.k_pool.shape[1:])}, the layer needs {(n_kv, kv.page_size, head_dim)}")
         splits = self.decode_slices(batch.max_kv_len, kv.page_size, T * n_kv)
         scratch = None
-        if splits > 1:
+        if splits > 1 and not (merge and splits <= MERGED_SLICES):
             scratch = torch.empty(T * n_head * splits * (head_dim + 2), dtype=torch.float32, device=out.device)
         self._call("attention_bf16", "gfb_attn_decode_rope", _ptr(src), n_part, _ptr(out), *self._kv_args(kv),
                    *self._batch_args(batch), _ptr(table), table.shape[0], n_head, n_kv, head_dim,
