@@ -109,6 +109,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         __nanosleep(64);
     }
 }
+// The same for a whole warp: one answer for all its lanes.  Where a wait runs out lanes can differ (one sees the abort flag, another its barrier), and
+// a warp that parted there would never meet again at the aligned instructions behind it.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int which) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, which));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -556,7 +561,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 // the table of this item's heads: wait until no warp reads the previous item's, write a share, wait for all shares
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bars->tbl_free));
-                ok = mbar_wait(smem_u32(&bars->tbl_free), it & 1u, abort_flag, status, 15);
+                ok = mbar_wait_warp(smem_u32(&bars->tbl_free), it & 1u, abort_flag, status, 15);
                 if (!ok) break;
                 for (int k = (warp - 2) * 32 + lane; k < rep * db.s_len; k += 256) {
                     const int hl = k / db.s_len, kk = k - hl * db.s_len;
@@ -565,14 +570,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bars->tbl_full));
-                ok = mbar_wait(smem_u32(&bars->tbl_full), it & 1u, abort_flag, status, 16);
+                ok = mbar_wait_warp(smem_u32(&bars->tbl_full), it & 1u, abort_flag, status, 16);
                 if (!ok) break;
             }
             float m_run = -INFINITY, l_run = 0.f;                        // l_run: this warp's half of the row's sum
             for (int j = 0; j < t.n_iter && ok; j++, jj++) {
                 const uint32_t sb = jj & 1u;
                 const int key0 = (t.blk0 + j) * KEYS + half * 64;        // this warp's first key
-                ok = mbar_wait(smem_u32(&bars->s_full[sb]), (jj >> 1) & 1u, abort_flag, status, 8);
+                ok = mbar_wait_warp(smem_u32(&bars->s_full[sb]), (jj >> 1) & 1u, abort_flag, status, 8);
                 if (!ok) break;
                 tc_fence_after();
                 // a block needs no mask when the tile's first row sees its last key and its last row (whose window or chunk
@@ -639,7 +644,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 bars->mx_half[sb][half][r] = mx;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bars->xch[q]));
-                ok = mbar_wait(smem_u32(&bars->xch[q]), jj & 1u, abort_flag, status, 13);
+                ok = mbar_wait_warp(smem_u32(&bars->xch[q]), jj & 1u, abort_flag, status, 13);
                 if (!ok) break;
                 mx = fmaxf(mx, bars->mx_half[sb][half ^ 1][r]);
                 // The running maximum only has to keep the exponentials in range, so it follows the true maximum
@@ -674,7 +679,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 // were issued behind the P V of block jj - 2, and the phase after it (block jj + 1) cannot have begun,
                 // since that P V is issued behind this block's, which waits for this warp's arrival below.
                 if (j > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
-                    ok = mbar_wait(smem_u32(&bars->pv_done[(jj - 1u) & 1u]), ((jj - 1u) >> 1) & 1u, abort_flag, status, 9);
+                    ok = mbar_wait_warp(smem_u32(&bars->pv_done[(jj - 1u) & 1u]), ((jj - 1u) >> 1) & 1u, abort_flag, status, 9);
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll 1
@@ -696,14 +701,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // All P V of the item have landed: a barrier of its own with one phase per item.  (A parity wait on pv_done
             // is only valid while that barrier can be neither a phase behind nor a phase ahead of the awaited one; at the
             // end of an item, with the waits of the earlier blocks left out, it could be either.)
-            if (ok) ok = mbar_wait(smem_u32(&bars->o_full), it & 1u, abort_flag, status, 10);
+            if (ok) ok = mbar_wait_warp(smem_u32(&bars->o_full), it & 1u, abort_flag, status, 10);
             if (!ok) break;
             tc_fence_after();
             // the row's sum: both halves are under the same reference
             bars->l_half[it & 1u][half][r] = l_run;
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars->fin[q]));
-            ok = mbar_wait(smem_u32(&bars->fin[q]), it & 1u, abort_flag, status, 14);
+            ok = mbar_wait_warp(smem_u32(&bars->fin[q]), it & 1u, abort_flag, status, 14);
             if (!ok) break;
             l_run += bars->l_half[it & 1u][half ^ 1][r];
             it++;
@@ -970,7 +975,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         for (int j = 0; j < n_iter && ok; j++) {
             if (!active(x, j)) continue;
             const int key0 = (blk0 + j) * KEYS;
-            ok = mbar_wait(smem_u32(&bars->s_full[x]), n_done & 1u, abort_flag, status, 8);
+            ok = mbar_wait_warp(smem_u32(&bars->s_full[x]), n_done & 1u, abort_flag, status, 8);
             if (!ok) break;
             tc_fence_after();
             const bool need_mask = key0 + KEYS - 1 > pos0[x] || key0 < last_lo || nq[x] < TQ;
@@ -1020,7 +1025,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             // O follows the reference maximum, rarely (S of this block was issued behind the tile's previous P V, so
             // that phase is over and the wait only orders the accesses)
             if (n_done > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
-                ok = mbar_wait(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 9);
+                ok = mbar_wait_warp(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 9);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll 1
@@ -1040,7 +1045,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             m_run = m_new;
             n_done++;
         }
-        if (ok && n_done > 0) ok = mbar_wait(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 10);
+        if (ok && n_done > 0) ok = mbar_wait_warp(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 10);
         if (ok && n_done > 0) {
             tc_fence_after();
             const int head = g * rep + (r - tq * rep);
@@ -1265,7 +1270,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             bool ok = true;
             for (int j = 0; j < n_iter; j++) {
                 const int s = j & 1, key0 = (blk0 + j) * LK;
-                ok = mbar_wait(smem_u32(&bars->s_full[s]), (uint32_t)(j >> 1) & 1u, abort_flag, status, 28);
+                ok = mbar_wait_warp(smem_u32(&bars->s_full[s]), (uint32_t)(j >> 1) & 1u, abort_flag, status, 28);
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t raw[2][32];
@@ -1323,7 +1328,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 // O follows a new reference, behind the previous P V: the scores of this page were issued behind the P V of page j - 2,
                 // and that of page j + 1 waits for this warp, so the barrier's phase is the awaited one or the one before it
                 if (j > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
-                    ok = mbar_wait(smem_u32(&bars->pv_done[(j - 1) & 1]), (uint32_t)((j - 1) >> 1) & 1u, abort_flag, status, 29);
+                    ok = mbar_wait_warp(smem_u32(&bars->pv_done[(j - 1) & 1]), (uint32_t)((j - 1) >> 1) & 1u, abort_flag, status, 29);
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll 1
@@ -1342,7 +1347,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 l_run = l_run * corr + (rsum[0] + rsum[1]);
                 m_run = m_new;
             }
-            if (ok) ok = mbar_wait(smem_u32(&bars->o_full), 0, abort_flag, status, 30);
+            if (ok) ok = mbar_wait_warp(smem_u32(&bars->o_full), 0, abort_flag, status, 30);
             if (ok) {
                 tc_fence_after();
                 if (sink != nullptr && m_run != -INFINITY) l_run += fast_exp2(sink[(m0 + r) % H] * 1.4426950408889634f - m_run * scale_log2e);
@@ -1457,7 +1462,7 @@ headwise_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     } else {
         const int q = warp & 3;
         float* mine = reinterpret_cast<float*>(aligned) + q * 32 * HW_PITCH;
-        if (mbar_wait(smem_u32(&bars->done), 0, abort_flag, status, 33)) {      // every copy has landed and been read
+        if (mbar_wait_warp(smem_u32(&bars->done), 0, abort_flag, status, 33)) {      // every copy has landed and been read
             tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < 128; c += 32) {
@@ -1599,7 +1604,7 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_con
     } else {
         const int q = warp & 3;
         float* mine = reinterpret_cast<float*>(aligned) + q * 32 * HW_PITCH;
-        if (mbar_wait(smem_u32(&bars->done), 0, abort_flag, status, 43)) {      // every copy has landed and been read
+        if (mbar_wait_warp(smem_u32(&bars->done), 0, abort_flag, status, 43)) {      // every copy has landed and been read
             tc_fence_after();
             const size_t row0 = ((size_t)h * b.n_seqs + seq) * cap + key0 + q * 32;
 #pragma unroll 1
@@ -1859,7 +1864,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int j = 0; j < n_iter && ok; j++) {
                 if (!active(x, j)) continue;
                 const int key0 = (blk0 + j) * KEYS + 64 * half;
-                ok = mbar_wait(smem_u32(&bars->s_full[x]), n_done & 1u, abort_flag, status, 51);
+                ok = mbar_wait_warp(smem_u32(&bars->s_full[x]), n_done & 1u, abort_flag, status, 51);
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t raw[2][32];
@@ -1915,7 +1920,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 }
                 // O follows a new reference, rarely (S of this block was issued behind the tile's previous P V, so that the wait only orders the accesses)
                 if (n_done > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
-                    ok = mbar_wait(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 52);
+                    ok = mbar_wait_warp(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 52);
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll 1
@@ -1935,7 +1940,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 m_run = m_new;
                 n_done++;
             }
-            if (ok && n_done > 0) ok = mbar_wait(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 53);
+            if (ok && n_done > 0) ok = mbar_wait_warp(smem_u32(&bars->pv_done[x]), (n_done - 1u) & 1u, abort_flag, status, 53);
             if (ok && n_done > 0) {
                 tc_fence_after();
                 float theirs;

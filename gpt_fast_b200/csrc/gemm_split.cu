@@ -96,6 +96,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         __nanosleep(64);
     }
 }
+// The same for a whole warp: one answer for all its lanes.  Where a wait runs out lanes can differ (one sees the abort flag, another its barrier), and
+// a warp that parted there would never meet again at the aligned instructions behind it.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int which) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, which));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -353,7 +358,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         for (int i = 0; i < n_stages + NP - 1 && ok; i++) {
             if (i < n_stages) {                  // (the planes are free: stage i - NP has been added up below)
                 const int s = i % NW, b = i % NP;
-                ok = mbar_wait(smem_u32(&bars->w_full[s]), (uint32_t)(i / NW & 1), abort_flag, status, 6);
+                ok = mbar_wait_warp(smem_u32(&bars->w_full[s]), (uint32_t)(i / NW & 1), abort_flag, status, 6);
                 if (!ok) break;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
@@ -379,7 +384,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
             if (const int d = i - (NP - 1); d >= 0) {
                 const int b = d % NP;
-                ok = mbar_wait(smem_u32(&bars->done[b]), (uint32_t)(d / NP & 1), abort_flag, status, 7);
+                ok = mbar_wait_warp(smem_u32(&bars->done[b]), (uint32_t)(d / NP & 1), abort_flag, status, 7);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 32 * CH + g0 * 16);

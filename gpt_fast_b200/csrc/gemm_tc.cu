@@ -114,6 +114,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         __nanosleep(64);
     }
 }
+// The same for a whole warp: one answer for all its lanes.  Where a wait runs out lanes can differ (one sees the abort flag, another its barrier), and
+// a warp that parted there would never meet again at the aligned instructions behind it.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int which) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, which));
+}
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
@@ -522,7 +527,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     } else {
         const int q = warp & 3;                             // tensor-memory lanes 32q .. 32q+31 belong to this warp
         const int r = row0 + q * 32 + lane;
-        bool ok = mbar_wait(smem_u32(&bars->accum), 0, abort_flag, status, 3);
+        bool ok = mbar_wait_warp(smem_u32(&bars->accum), 0, abort_flag, status, 3);
         tc_fence_after();
         {
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
@@ -908,7 +913,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             const int ab = ti & 1;
             const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
             const int row0 = (tile % row_tiles) * BM, col0 = (tile / row_tiles) * PBN;
-            if (!mbar_wait(smem_u32(&bars->acc_full[ab]), (uint32_t)(ti >> 1) & 1u, abort_flag, status, 3)) break;
+            if (!mbar_wait_warp(smem_u32(&bars->acc_full[ab]), (uint32_t)(ti >> 1) & 1u, abort_flag, status, 3)) break;
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * PBN);
             const int rows = min(32, R - (row0 + q * 32));
@@ -1110,7 +1115,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             const int ab = ti & 1;
             const int tile = pair + ti * n_pairs;
             const int row0 = (tile % row_tiles) * 256 + (int)rank * 128, col0 = (tile / row_tiles) * 256;
-            if (!mbar_wait(smem_u32(&bars->acc_full[ab]), (uint32_t)(ti >> 1) & 1u, abort_flag, status, 3)) break;
+            if (!mbar_wait_warp(smem_u32(&bars->acc_full[ab]), (uint32_t)(ti >> 1) & 1u, abort_flag, status, 3)) break;
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * 256);
             const int rows = min(32, R - (row0 + q * 32));

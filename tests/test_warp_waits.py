@@ -26,7 +26,7 @@ def waits(text):
             start = i + 1
         if i in calls and blocks:                        # (at file level: the helpers' own heads)
             around = blocks + [text[start:i]]
-            if not any(re.search(r"bool mbar_wait", b) for b in around):
+            if not any(re.search(r"bool (?:mbar_wait|$)", b) for b in around):
                 one = any(re.search(r"\blane == 0\b|\bthreadIdx\.x == 0\b|\btid == 0\b", b) for b in around)
                 found.append((text.count("\n", 0, i) + 1, calls[i], one))
     return found
