@@ -1,6 +1,6 @@
 // C[M,N] = A[M,K] * W[N,K]^T of 32-bit numbers on the tensor cores, each number as the sum of three bfloat16.
 //
-// a = a1 + a2 + a3 without a remainder (8 bits each; a1 truncated, so that the largest numbers stay finite), likewise w, and
+// a = a1 + a2 + a3 without a remainder from 2^-110 on (8 bits each; a1 truncated, so that the largest numbers stay finite), likewise w, and
 //     a w = a1 w1 + (a1 w2 + a2 w1) + (a1 w3 + a2 w2 + a3 w1) + terms below 2^-22 of it and of either sign:
 // six bfloat16 products with exact 16-bit results.  What is left to lose is the order and the rounding of the sum, which the tensor cores cut
 // off instead of rounding.  So an accumulator in tensor memory holds 32 numbers of k at most, its small terms first, and a thread
@@ -20,8 +20,8 @@
 // rows of a tile are the rows of the MMA, up to 256 tokens its columns.  The activations come in three planes that `split_rows_kernel`
 // wrote, since every block reads them; a weight is read, and split, once per 256 tokens.
 //
-// A sum that is not finite (an infinite or NaN operand: its pieces cannot hold it; an overflow on the way) is worked out once more
-// from the 32-bit numbers, by a warp, before the epilogue.  Every wait is bounded by time, as in the bfloat16 product.
+// A sum that is not finite (an infinite or NaN operand: its pieces cannot hold it; an overflow on the way), or so small that the operands' pieces
+// may have missed bits that count, is worked out once more from the 32-bit numbers, by a warp, before the epilogue.  Every wait is bounded by time, as in the bfloat16 product.
 //
 // Epilogues as in gemm_simt.cu, which keeps the products this kernel does not take (rows that are no multiple of 16 bytes, bfloat16).
 #include "common.cuh"
@@ -186,11 +186,18 @@ __device__ __noinline__ float whole_dot(const float* __restrict__ A, const float
     return (float)s;
 }
 
-// Four neighbouring sums of row m, from column n on: those that are not finite are worked out once more (a whole warp comes here).
-__device__ __forceinline__ void mend(float (&v)[4], const float* __restrict__ A, const float* __restrict__ W, int m, int n, int N, int K) {
+// Where pieces miss a number.  bfloat16 ends at 2^-133 (and as normal numbers at 2^-126), so a number below 2^-110 loses its last bits, at most
+// 2^-126 of it however the tensor cores take subnormal pieces.  A row of A without a number of 2^-96 has all its sums worked out from the 32-bit
+// numbers.  In any other row its own numbers lose less than 2^-30 of the largest, and the weights' losses, K 2^-126 times that
+// largest at most, are below 2^-26 of every sum from K 2^-100 times the largest (and 2^-100 K) on; smaller sums are worked out as well.
+constexpr float SMALL_ROW = 0x1p-96f, SMALL_SUM = 0x1p-100f;
+
+// Four neighbouring sums of row m, from column n on: those that are not finite, or smaller than the row's `least`, are worked out once more (a whole
+// warp comes here).  A row of zeros has a `least` of zero.
+__device__ __forceinline__ void mend(float (&v)[4], const float* __restrict__ A, const float* __restrict__ W, float least, int m, int n, int N, int K) {
     uint32_t bad = 0;
 #pragma unroll
-    for (int u = 0; u < 4; u++) bad |= (n + u < N && !isfinite(v[u])) ? 1u << u : 0u;
+    for (int u = 0; u < 4; u++) bad |= (n + u < N && (!isfinite(v[u]) || fabsf(v[u]) < least)) ? 1u << u : 0u;
     uint32_t lanes = __ballot_sync(0xffffffffu, bad != 0);
     while (lanes) {
         const int l = __ffs(lanes) - 1;
@@ -229,30 +236,44 @@ __device__ __forceinline__ void finish4(float* __restrict__ C, int m, int n, int
         if (n + u < N) c[u] = EPI == EPI_ADD ? c[u] + v[u] : unary<EPI>(v[u]);
 }
 
-// planes[p][m][k]: piece p of A[m][k], zeros from K to Kp.  A thread takes eight numbers.
-__global__ void __launch_bounds__(256)
-split_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ planes, int M, int K, int Kp, int wide) {
+// planes[p][m][k]: piece p of A[m][k], zeros from K to Kp.  A block takes a row, eight numbers per thread and step, and says below which size
+// the row's sums are not to be had from pieces (see `mend`).
+constexpr int ROW_THREADS = 1024;            // at most
+
+__global__ void __launch_bounds__(ROW_THREADS)
+split_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ planes, float* __restrict__ least, int M, int K, int Kp, int wide) {
+    __shared__ uint32_t warps[ROW_THREADS / 32];
     gfb_pdl_launch();
     gfb_pdl_wait();
-    const int units = Kp >> 3;
-    const size_t e = (size_t)blockIdx.x * 256 + threadIdx.x;
-    if (e >= (size_t)M * units) return;
-    const int m = (int)(e / units), k = (int)(e - (size_t)m * units) * 8;
-    const float* a = A + (size_t)m * K + k;
-    float v[8];
-    if (wide && k + 8 <= K) {
-        const float4 lo = *reinterpret_cast<const float4*>(a), hi = *reinterpret_cast<const float4*>(a + 4);
-        v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-    } else {
+    const int m = blockIdx.x;
+    uint32_t largest = 0;                                            // by its bits: infinities and NaNs are the largest
+    for (int k = threadIdx.x * 8; k < Kp; k += blockDim.x * 8) {
+        const float* a = A + (size_t)m * K + k;
+        float v[8];
+        if (wide && k + 8 <= K) {
+            const float4 lo = *reinterpret_cast<const float4*>(a), hi = *reinterpret_cast<const float4*>(a + 4);
+            v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = k + i < K ? a[i] : 0.f;
+            for (int i = 0; i < 8; i++) v[i] = k + i < K ? a[i] : 0.f;
+        }
+        uint32_t p[3][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            split2(v[2 * i], v[2 * i + 1], p[0][i], p[1][i], p[2][i]);
+            largest = max(largest, max(__float_as_uint(v[2 * i]) & 0x7fffffffu, __float_as_uint(v[2 * i + 1]) & 0x7fffffffu));
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            *reinterpret_cast<uint4*>(planes + (size_t)q * M * Kp + (size_t)m * Kp + k) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
     }
-    uint32_t p[3][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) split2(v[2 * i], v[2 * i + 1], p[0][i], p[1][i], p[2][i]);
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-        *reinterpret_cast<uint4*>(planes + (size_t)q * M * Kp + (size_t)m * Kp + k) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = largest;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    largest = __reduce_max_sync(0xffffffffu, threadIdx.x < blockDim.x / 32 ? warps[threadIdx.x] : 0u);
+    const float top = __uint_as_float(largest);
+    if (threadIdx.x == 0) least[m] = largest == 0 ? 0.f : top < SMALL_ROW ? INFINITY : (float)K * SMALL_SUM * fmaxf(top, 1.f);
 }
 
 // A tile of 128 weight rows (blockIdx.y) by bn tokens (blockIdx.x; bn a multiple of 16, at most 32 * CH) over one portion of K (blockIdx.z).
@@ -260,7 +281,8 @@ split_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ plane
 template <int CH, int EPI, bool PARTIAL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ A,
-                  const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int stages_per_split, int* status) {
+                  const float* __restrict__ W, const float* __restrict__ least, float* __restrict__ C, int M, int N, int K, int bn, int stages_per_split,
+                  int* status) {
     constexpr int NW = Ring<CH>::W, NX = Ring<CH>::X, NP = Ring<CH>::P, LAG = NW - NX;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -349,6 +371,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int q = warp & 3, half = (warp - 2) >> 2, w8 = warp - 2;
         const int groups = bn >> 4, low = (groups + 1) >> 1;
         const int g0 = half ? low : 0, mine = half ? groups - low : low;           // this warp's groups of 16 columns
+        const int n_tok = min(bn, M - m0);
+        const float lowest = !PARTIAL && w8 + SPLITTERS * lane < n_tok ? least[m0 + w8 + SPLITTERS * lane] : 0.f;     // of the warp's tokens below, one per lane
         float sum[CH][16];
 #pragma unroll
         for (int c = 0; c < CH; c++)
@@ -410,7 +434,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                     for (int j = 0; j < 16; j++) tile[((g0 + c) * 16 + j) * BM + q * 32 + lane] = sum[c][j];
             asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
-            const int n_tok = min(bn, M - m0), n = n0 + 4 * lane;
+            const int n = n0 + 4 * lane;
 #pragma unroll 2
             for (int j = w8; j < n_tok; j += SPLITTERS) {
                 const float4 t = *reinterpret_cast<const float4*>(tile + j * BM + 4 * lane);
@@ -418,7 +442,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 if (PARTIAL) {
                     finish4<EPI_STORE>(C + (size_t)blockIdx.z * M * N, m0 + j, n, N, v);
                 } else {
-                    mend(v, A, W, m0 + j, n, N, K);
+                    mend(v, A, W, __shfl_sync(0xffffffffu, lowest, j / SPLITTERS), m0 + j, n, N, K);
                     finish4<EPI>(C, m0 + j, n, N, v);
                 }
             }
@@ -440,8 +464,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 // the portions of every sum, in ascending order, and the epilogue; a thread per four columns
 template <int EPI>
 __global__ void __launch_bounds__(256)
-split_sum_kernel(const float* __restrict__ partial, const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
-                 int K, int splits) {
+split_sum_kernel(const float* __restrict__ partial, const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ least,
+                 float* __restrict__ C, int M, int N, int K, int splits) {
     gfb_pdl_launch();
     gfb_pdl_wait();
     const int units = (N + 3) / 4;
@@ -466,7 +490,7 @@ split_sum_kernel(const float* __restrict__ partial, const float* __restrict__ A,
             for (int u = 0; u < 4; u++) v[u] = s == 0 ? t[u] : v[u] + t[u];
         }
     }
-    mend(v, A, W, m, n, N, K);
+    mend(v, A, W, least[m], m, n, N, K);
     finish4<EPI>(C, m, n, N, v);
 }
 
@@ -525,14 +549,16 @@ int splits_of(int N, int K) {
     return ((K + BK - 1) / BK + per - 1) / per;
 }
 
+long aligned(long bytes) { return (bytes + 255) / 256 * 256; }
+
 // The rows of A that one launch takes: its planes and partial sums stay below 256 MB (or are one tile's).
 constexpr long SCRATCH_BYTES = 256L << 20;
 long row_bytes(int N, int K) {
     const int splits = splits_of(N, K);
-    return 6L * ((K + 7) / 8 * 8) + (splits > 1 ? 4L * splits * N : 0);
+    return 4 + 6L * ((K + 7) / 8 * 8) + (splits > 1 ? 4L * splits * N : 0);
 }
 int portion(int M, int N, int K) {
-    long most = SCRATCH_BYTES / row_bytes(N, K) / 256 * 256;
+    long most = (SCRATCH_BYTES - 512) / row_bytes(N, K) / 256 * 256;
     if (most < 256) most = 256;
     return M < most ? M : (int)most;
 }
@@ -542,7 +568,7 @@ template <int CH> size_t smem_bytes() {
 }
 
 template <int CH, int EPI, bool PARTIAL>
-int launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, float* C, int M, int N, int K, int bn, int* status, cudaStream_t stream) {
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, const float* least, float* C, int M, int N, int K, int bn, int* status, cudaStream_t stream) {
     static_assert(Ring<CH>::W * W_STAGE + Ring<CH>::P * 3 * W_PLANE + Ring<CH>::X * 3 * 32 * CH * X_ROW >= 32 * CH * BM * 4, "the tile of sums fits the rings");
     static_assert(Ring<CH>::X <= Ring<CH>::W && Ring<CH>::W <= MAX_RING, "rings");
     auto kern = gemm_split_kernel<CH, EPI, PARTIAL>;
@@ -555,33 +581,34 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const f
     }
     const dim3 grid((M + bn - 1) / bn, (N + BM - 1) / BM, PARTIAL ? splits_of(N, K) : 1);
     const int per = PARTIAL ? stages_per_split(N, K) : (K + BK - 1) / BK;
-    return gfb_check(gfb_launch(kern, grid, dim3(THREADS), smem, stream, mw, mx, A, W, C, M, N, K, bn, per, status), "gfb_gemm_split");
+    return gfb_check(gfb_launch(kern, grid, dim3(THREADS), smem, stream, mw, mx, A, W, least, C, M, N, K, bn, per, status), "gfb_gemm_split");
 }
 
 template <int EPI, bool PARTIAL>
-int launch_by_width(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, float* C, int M, int N, int K, int bn, int* status,
+int launch_by_width(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, const float* least, float* C, int M, int N, int K, int bn, int* status,
                     cudaStream_t stream) {
-    if (bn <= 32) return launch<1, EPI, PARTIAL>(mw, mx, A, W, C, M, N, K, bn, status, stream);
-    if (bn <= 64) return launch<2, EPI, PARTIAL>(mw, mx, A, W, C, M, N, K, bn, status, stream);
-    if (bn <= 128) return launch<4, EPI, PARTIAL>(mw, mx, A, W, C, M, N, K, bn, status, stream);
-    return launch<8, EPI, PARTIAL>(mw, mx, A, W, C, M, N, K, bn, status, stream);
+    if (bn <= 32) return launch<1, EPI, PARTIAL>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
+    if (bn <= 64) return launch<2, EPI, PARTIAL>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
+    if (bn <= 128) return launch<4, EPI, PARTIAL>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
+    return launch<8, EPI, PARTIAL>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
 }
 
 template <int EPI>
 int run(const float* A, const float* W, float* C, int M, int N, int K, uint8_t* scratch, int* status, cudaStream_t stream) {
     const int Kp = (K + 7) / 8 * 8, splits = splits_of(N, K);
     __nv_bfloat16* planes = reinterpret_cast<__nv_bfloat16*>(scratch);
-    float* partial = reinterpret_cast<float*>(scratch + ((size_t)6 * M * Kp + 255) / 256 * 256);
-    const size_t units = (size_t)M * (Kp / 8);
-    if (gfb_check(gfb_launch(split_rows_kernel, dim3((unsigned)((units + 255) / 256)), dim3(256), 0, stream, A, planes, M, K, Kp,
-                             (int)(((uintptr_t)A & 15) == 0)), "gfb_gemm_split (rows)")) return 1;
+    float* least = reinterpret_cast<float*>(scratch + aligned(6L * M * Kp));
+    float* partial = reinterpret_cast<float*>(scratch + aligned(6L * M * Kp) + aligned(4L * M));
+    const int steps = (Kp / 8 + ROW_THREADS - 1) / ROW_THREADS, row_threads = ((Kp / 8 + steps - 1) / steps + 31) / 32 * 32;
+    if (gfb_check(gfb_launch(split_rows_kernel, dim3((unsigned)M), dim3((unsigned)row_threads), 0, stream, A, planes, least, M, K, Kp, (int)(((uintptr_t)A & 15) == 0)),
+                  "gfb_gemm_split (rows)")) return 1;
     const int tiles = (M + 255) / 256, bn = ((M + tiles - 1) / tiles + 15) / 16 * 16;
     CUtensorMap mw, mx;
     if (make_maps(&mw, &mx, W, planes, M, N, K, Kp, bn)) return 1;
-    if (splits == 1) return launch_by_width<EPI, false>(mw, mx, A, W, C, M, N, K, bn, status, stream);
-    if (launch_by_width<EPI_STORE, true>(mw, mx, A, W, partial, M, N, K, bn, status, stream)) return 1;
+    if (splits == 1) return launch_by_width<EPI, false>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
+    if (launch_by_width<EPI_STORE, true>(mw, mx, A, W, least, partial, M, N, K, bn, status, stream)) return 1;
     const size_t sums = (size_t)M * ((N + 3) / 4);
-    return gfb_check(gfb_launch(split_sum_kernel<EPI>, dim3((unsigned)((sums + 255) / 256)), dim3(256), 0, stream, (const float*)partial, A, W, C, M, N, K,
+    return gfb_check(gfb_launch(split_sum_kernel<EPI>, dim3((unsigned)((sums + 255) / 256)), dim3(256), 0, stream, (const float*)partial, A, W, (const float*)least, C, M, N, K,
                                 splits), "gfb_gemm_split (sum)");
 }
 
@@ -600,7 +627,7 @@ int portions(const float* A, const float* W, float* C, int M, int N, int K, uint
 GFB_API long gfb_gemm_split_scratch_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     const long rows = portion(M, N, K);
-    return (6L * rows * ((K + 7) / 8 * 8) + 255) / 256 * 256 + (splits_of(N, K) > 1 ? 4L * splits_of(N, K) * rows * N : 0);
+    return aligned(6L * rows * ((K + 7) / 8 * 8)) + aligned(4L * rows) + (splits_of(N, K) > 1 ? 4L * splits_of(N, K) * rows * N : 0);
 }
 
 // A, W, C 32-bit; W 16-byte aligned with rows of whole 16-byte units; scratch: gfb_gemm_split_scratch_bytes, 256-byte aligned.

@@ -86,6 +86,29 @@ def test_not_finite_and_extreme_numbers(N, K):
     assert bool(((got.double() - want.double()).abs() <= 1e-6 * scale + 1e-37)[fine].all())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(96, 2100), (20000, 388)])          # portions of K in blocks of their own; one block per tile
+@pytest.mark.parametrize("rows,weights", [(1.0, 1e-24), (1.0, 1e-27), (1.0, 1e-33), (1.0, 1e-36), (1e12, 1e-36), (1e-24, 1.0), (1e-28, 1.0), (1e-30, 1.0),
+                                          (1e-34, 1.0), (1e-36, 1.0), (1e-15, 1e-15), (1e-20, 1e-16), (1e30, 1e-36), (1e-36, 1e30)])
+def test_small_numbers_keep_their_bits(N, K, rows, weights):
+    """Numbers whose third and second pieces bfloat16 does not reach, on either side: each row is as near to 64 bits, by its own size, as sums
+    on CUDA cores.  A row of zeros, a zero weight and a lone small number among ordinary ones stay what they are."""
+    a, w = rnd(24, K, seed=12) * rows, rnd(N, K, seed=13) * weights
+    a[5] = 0.0
+    w[7] = 0.0
+    a[6, 1:] = 0.0
+    want = a.double() @ w.double().t()
+    got, cores = torch.empty(24, N, device=DEV), torch.empty(24, N, device=DEV)
+    ops.linear(a, w, got)
+    lib = build.library("gemm_simt")
+    room = torch.empty(max(1, lib.gfb_gemm_simt_scratch_floats(24, N, K)), device=DEV)
+    assert lib.gfb_gemm_simt(a.data_ptr(), w.data_ptr(), cores.data_ptr(), 0, 0, 24, N, K, 0, room.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    ours, theirs = ((x.double() - want).norm(dim=1) / want.norm(dim=1) for x in (got, cores))
+    some = torch.arange(24, device=DEV) != 5
+    assert float(ours[some].max()) <= max(2.0 ** -24, float(theirs[some].max())), (ours, theirs)
+    assert not got[5].any() and not got[:, 7].any()
+
+
 def test_scratch_is_bounded():
     lib = build.library("gemm_split")
     lib.gfb_gemm_split_scratch_bytes.restype = c_long
