@@ -21,7 +21,10 @@
 // wrote, since every block reads them; a weight is read, and split, once per 256 tokens.
 //
 // A sum that is not finite (an infinite or NaN operand: its pieces cannot hold it; an overflow on the way), or so small that the operands' pieces
-// may have missed bits that count, is worked out once more from the 32-bit numbers, by a warp, before the epilogue.  Every wait is bounded by time, as in the bfloat16 product.
+// may have missed bits that count, is worked out once more from the 32-bit numbers, by a warp, before the epilogue: eight columns that read a row of A
+// once, given up where all are NaN.  That is for the odd row.  Where every sum needs it, 198 rows of 3,072 numbers times 16,384 columns
+// take 1.4 ms with NaNs throughout and 10.2 ms with an infinity in every row (column by column 23.1), 16 rows of 1,024 times 4,096 0.1 and 0.2 ms.
+// Every wait is bounded by time, as in the bfloat16 product.
 //
 // Epilogues as in gemm_simt.cu, which keeps the products this kernel does not take (rows that are no multiple of 16 bytes, bfloat16).
 #include "common.cuh"
@@ -175,42 +178,72 @@ __device__ __forceinline__ float unary(float z) {
     return z;
 }
 
-// Row m of A times row n of W by a whole warp, in 64 bits, so that only infinities and NaNs of the operands, or a sum beyond 32 bits, come
-// out as such.
-__device__ __noinline__ float whole_dot(const float* __restrict__ A, const float* __restrict__ W, int m, int n, int K) {
-    const float *a = A + (size_t)m * K, *w = W + (size_t)n * K;
-    double s = 0.0;
-    for (int k = threadIdx.x & 31; k < K; k += 32) s = fma((double)a[k], (double)w[k], s);
+// Row m of A times rows n .. n + COLS - 1 of W (the last of them at most N - 1) by a whole warp, in 64 bits, so that only infinities and NaNs of the
+// operands, or a sum beyond 32 bits, come out as such.  Column n + u's sum goes to lane u.  The order of a sum is that of its k alone.
+constexpr int COLS = 8, LOOK = 512;
+__device__ __noinline__ float whole_dots(const float* __restrict__ A, const float* __restrict__ W, int m, int n, int N, int K) {
+    const int lane = threadIdx.x & 31;
+    const float* a = A + (size_t)m * K;
+    double s[COLS];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return (float)s;
+    for (int u = 0; u < COLS; u++) s[u] = 0.0;
+    for (int k0 = 0; k0 < K; k0 += LOOK) {
+        const int end = min(K, k0 + LOOK);
+#pragma unroll 4
+        for (int k = k0 + lane; k < end; k += 32) {
+            const double x = a[k];
+#pragma unroll
+            for (int u = 0; u < COLS; u++) s[u] = fma(x, (double)W[(size_t)min(n + u, N - 1) * K + k], s[u]);
+        }
+        bool over = true;                        // NaNs stay what they are
+#pragma unroll
+        for (int u = 0; u < COLS; u++) over = over && __any_sync(0xffffffffu, isnan(s[u]));
+        if (over) break;
+    }
+    float mine = 0.f;
+#pragma unroll
+    for (int u = 0; u < COLS; u++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+        if (lane == u) mine = (float)s[u];
+    }
+    return mine;
 }
 
 // Where pieces miss a number.  bfloat16 ends at 2^-133 (and as normal numbers at 2^-126), so a number below 2^-110 loses its last bits, at most
 // 2^-126 of it however the tensor cores take subnormal pieces.  A row of A without a number of 2^-96 has all its sums worked out from the 32-bit
-// numbers.  In any other row its own numbers lose less than 2^-30 of the largest, and the weights' losses, K 2^-126 times that
+// numbers (`least` infinite), a row of zeros none (zero).  In any other row its own numbers lose less than 2^-30 of the largest, and the weights' losses, K 2^-126 times that
 // largest at most, are below 2^-26 of every sum from K 2^-100 times the largest (and 2^-100 K) on; smaller sums are worked out as well.
 constexpr float SMALL_ROW = 0x1p-96f, SMALL_SUM = 0x1p-100f;
 
-// Four neighbouring sums of row m, from column n on: those that are not finite, or smaller than the row's `least`, are worked out once more (a whole
-// warp comes here).  A row of zeros has a `least` of zero.
-__device__ __forceinline__ void mend(float (&v)[4], const float* __restrict__ A, const float* __restrict__ W, float least, int m, int n, int N, int K) {
+// Whether a sum of a row may have to be worked out once more: not finite, or smaller than the row's `least` (as bits: not in [least, infinity)).
+__device__ __forceinline__ bool doubtful(float v, uint32_t least) { return (__float_as_uint(v) & 0x7fffffffu) - least >= 0x7f800000u - least; }
+
+// Four neighbouring sums of row m, from column n on: the doubtful ones are worked out once more (a whole warp comes here).  A sum of zero is
+// left in any row but a small one: its weights are zeros, or none of them is a number of bfloat16 (2^-133).
+__device__ __noinline__ float4 mended(float4 sums, const float* __restrict__ A, const float* __restrict__ W, uint32_t least, int m, int n, int N, int K) {
+    float v[4] = {sums.x, sums.y, sums.z, sums.w};
+    const int lane = threadIdx.x & 31;
     uint32_t bad = 0;
 #pragma unroll
-    for (int u = 0; u < 4; u++) bad |= (n + u < N && (!isfinite(v[u]) || fabsf(v[u]) < least)) ? 1u << u : 0u;
-    uint32_t lanes = __ballot_sync(0xffffffffu, bad != 0);
-    while (lanes) {
-        const int l = __ffs(lanes) - 1;
-        lanes &= lanes - 1;
-        const uint32_t which = __shfl_sync(0xffffffffu, bad, l);
-        const int mm = __shfl_sync(0xffffffffu, m, l), nn = __shfl_sync(0xffffffffu, n, l);
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (which >> u & 1) {
-                const float s = whole_dot(A, W, mm, nn + u, K);
-                if ((int)(threadIdx.x & 31) == l) v[u] = s;
-            }
+    for (int u = 0; u < 4; u++) {
+        if (n + u < N && doubtful(v[u], least) && (v[u] != 0.f || least == 0x7f800000u)) bad |= 1u << u;
     }
+    uint32_t lanes = __ballot_sync(0xffffffffu, bad != 0);
+    while (lanes) {                              // two lanes' columns at a time, where they are neighbours in a row
+        const int l = __ffs(lanes) - 1;
+        const int mm = __shfl_sync(0xffffffffu, m, l), nn = __shfl_sync(0xffffffffu, n, l);
+        const bool pair = l < 31 && __shfl_sync(0xffffffffu, m, (l + 1) & 31) == mm && __shfl_sync(0xffffffffu, n, (l + 1) & 31) == nn + 4;
+        const float s = whole_dots(A, W, mm, nn, N, K);
+        const int from = lane == l ? 0 : 4;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float x = __shfl_sync(0xffffffffu, s, from + u);
+            if ((lane == l || (pair && lane == l + 1)) && (bad >> u & 1)) v[u] = x;
+        }
+        lanes &= ~((pair ? 3u : 1u) << l);
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
 }
 
 // four neighbouring sums through the epilogue; n is a multiple of four
@@ -236,12 +269,12 @@ __device__ __forceinline__ void finish4(float* __restrict__ C, int m, int n, int
         if (n + u < N) c[u] = EPI == EPI_ADD ? c[u] + v[u] : unary<EPI>(v[u]);
 }
 
-// planes[p][m][k]: piece p of A[m][k], zeros from K to Kp.  A block takes a row, eight numbers per thread and step, and says below which size
-// the row's sums are not to be had from pieces (see `mend`).
+// planes[p][m][k]: piece p of A[m][k], zeros from K to Kp.  A block takes a row, eight numbers per thread and step, and says from which size
+// on (by its bits) the row's sums are to be had from pieces (see below).
 constexpr int ROW_THREADS = 1024;            // at most
 
 __global__ void __launch_bounds__(ROW_THREADS)
-split_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ planes, float* __restrict__ least, int M, int K, int Kp, int wide) {
+split_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ planes, uint32_t* __restrict__ least, int M, int K, int Kp, int wide) {
     __shared__ uint32_t warps[ROW_THREADS / 32];
     gfb_pdl_launch();
     gfb_pdl_wait();
@@ -273,7 +306,7 @@ split_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ plane
     if (threadIdx.x >= 32) return;
     largest = __reduce_max_sync(0xffffffffu, threadIdx.x < blockDim.x / 32 ? warps[threadIdx.x] : 0u);
     const float top = __uint_as_float(largest);
-    if (threadIdx.x == 0) least[m] = largest == 0 ? 0.f : top < SMALL_ROW ? INFINITY : (float)K * SMALL_SUM * fmaxf(top, 1.f);
+    if (threadIdx.x == 0) least[m] = largest == 0 ? 0u : __float_as_uint(top < SMALL_ROW ? INFINITY : (float)K * SMALL_SUM * fmaxf(top, 1.f));
 }
 
 // A tile of 128 weight rows (blockIdx.y) by bn tokens (blockIdx.x; bn a multiple of 16, at most 32 * CH) over one portion of K (blockIdx.z).
@@ -281,7 +314,7 @@ split_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ plane
 template <int CH, int EPI, bool PARTIAL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ A,
-                  const float* __restrict__ W, const float* __restrict__ least, float* __restrict__ C, int M, int N, int K, int bn, int stages_per_split,
+                  const float* __restrict__ W, const uint32_t* __restrict__ least, float* __restrict__ C, int M, int N, int K, int bn, int stages_per_split,
                   int* status) {
     constexpr int NW = Ring<CH>::W, NX = Ring<CH>::X, NP = Ring<CH>::P, LAG = NW - NX;
     extern __shared__ uint8_t smem_raw[];
@@ -372,7 +405,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int groups = bn >> 4, low = (groups + 1) >> 1;
         const int g0 = half ? low : 0, mine = half ? groups - low : low;           // this warp's groups of 16 columns
         const int n_tok = min(bn, M - m0);
-        const float lowest = !PARTIAL && w8 + SPLITTERS * lane < n_tok ? least[m0 + w8 + SPLITTERS * lane] : 0.f;     // of the warp's tokens below, one per lane
+        const uint32_t lowest = !PARTIAL && w8 + SPLITTERS * lane < n_tok ? least[m0 + w8 + SPLITTERS * lane] : 0u;     // of the warp's tokens below, one per lane
         float sum[CH][16];
 #pragma unroll
         for (int c = 0; c < CH; c++)
@@ -437,14 +470,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const int n = n0 + 4 * lane;
 #pragma unroll 2
             for (int j = w8; j < n_tok; j += SPLITTERS) {
-                const float4 t = *reinterpret_cast<const float4*>(tile + j * BM + 4 * lane);
-                float v[4] = {t.x, t.y, t.z, t.w};
-                if (PARTIAL) {
-                    finish4<EPI_STORE>(C + (size_t)blockIdx.z * M * N, m0 + j, n, N, v);
-                } else {
-                    mend(v, A, W, __shfl_sync(0xffffffffu, lowest, j / SPLITTERS), m0 + j, n, N, K);
-                    finish4<EPI>(C, m0 + j, n, N, v);
+                float4 t = *reinterpret_cast<const float4*>(tile + j * BM + 4 * lane);
+                if (!PARTIAL) {
+                    const uint32_t low = __shfl_sync(0xffffffffu, lowest, j / SPLITTERS);
+                    if (__any_sync(0xffffffffu, doubtful(t.x, low) || doubtful(t.y, low) || doubtful(t.z, low) || doubtful(t.w, low)))
+                        t = mended(t, A, W, low, m0 + j, n, N, K);
                 }
+                const float v[4] = {t.x, t.y, t.z, t.w};
+                if (PARTIAL) finish4<EPI_STORE>(C + (size_t)blockIdx.z * M * N, m0 + j, n, N, v);
+                else finish4<EPI>(C, m0 + j, n, N, v);
             }
         }
     }
@@ -463,8 +497,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
 // the portions of every sum, in ascending order, and the epilogue; a thread per four columns
 template <int EPI>
-__global__ void __launch_bounds__(256)
-split_sum_kernel(const float* __restrict__ partial, const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ least,
+__global__ void __launch_bounds__(256, 5)        // (the rare call may spill; the sums want many blocks under way)
+split_sum_kernel(const float* __restrict__ partial, const float* __restrict__ A, const float* __restrict__ W, const uint32_t* __restrict__ least,
                  float* __restrict__ C, int M, int N, int K, int splits) {
     gfb_pdl_launch();
     gfb_pdl_wait();
@@ -490,7 +524,11 @@ split_sum_kernel(const float* __restrict__ partial, const float* __restrict__ A,
             for (int u = 0; u < 4; u++) v[u] = s == 0 ? t[u] : v[u] + t[u];
         }
     }
-    mend(v, A, W, least[m], m, n, N, K);
+    const uint32_t low = least[m];
+    if (__any_sync(0xffffffffu, in && (doubtful(v[0], low) || doubtful(v[1], low) || doubtful(v[2], low) || doubtful(v[3], low)))) {
+        const float4 t = mended(make_float4(v[0], v[1], v[2], v[3]), A, W, low, m, n, N, K);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    }
     finish4<EPI>(C, m, n, N, v);
 }
 
@@ -568,7 +606,7 @@ template <int CH> size_t smem_bytes() {
 }
 
 template <int CH, int EPI, bool PARTIAL>
-int launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, const float* least, float* C, int M, int N, int K, int bn, int* status, cudaStream_t stream) {
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, const uint32_t* least, float* C, int M, int N, int K, int bn, int* status, cudaStream_t stream) {
     static_assert(Ring<CH>::W * W_STAGE + Ring<CH>::P * 3 * W_PLANE + Ring<CH>::X * 3 * 32 * CH * X_ROW >= 32 * CH * BM * 4, "the tile of sums fits the rings");
     static_assert(Ring<CH>::X <= Ring<CH>::W && Ring<CH>::W <= MAX_RING, "rings");
     auto kern = gemm_split_kernel<CH, EPI, PARTIAL>;
@@ -585,7 +623,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const f
 }
 
 template <int EPI, bool PARTIAL>
-int launch_by_width(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, const float* least, float* C, int M, int N, int K, int bn, int* status,
+int launch_by_width(const CUtensorMap& mw, const CUtensorMap& mx, const float* A, const float* W, const uint32_t* least, float* C, int M, int N, int K, int bn, int* status,
                     cudaStream_t stream) {
     if (bn <= 32) return launch<1, EPI, PARTIAL>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
     if (bn <= 64) return launch<2, EPI, PARTIAL>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
@@ -597,7 +635,7 @@ template <int EPI>
 int run(const float* A, const float* W, float* C, int M, int N, int K, uint8_t* scratch, int* status, cudaStream_t stream) {
     const int Kp = (K + 7) / 8 * 8, splits = splits_of(N, K);
     __nv_bfloat16* planes = reinterpret_cast<__nv_bfloat16*>(scratch);
-    float* least = reinterpret_cast<float*>(scratch + aligned(6L * M * Kp));
+    uint32_t* least = reinterpret_cast<uint32_t*>(scratch + aligned(6L * M * Kp));
     float* partial = reinterpret_cast<float*>(scratch + aligned(6L * M * Kp) + aligned(4L * M));
     const int steps = (Kp / 8 + ROW_THREADS - 1) / ROW_THREADS, row_threads = ((Kp / 8 + steps - 1) / steps + 31) / 32 * 32;
     if (gfb_check(gfb_launch(split_rows_kernel, dim3((unsigned)M), dim3((unsigned)row_threads), 0, stream, A, planes, least, M, K, Kp, (int)(((uintptr_t)A & 15) == 0)),
@@ -608,7 +646,7 @@ int run(const float* A, const float* W, float* C, int M, int N, int K, uint8_t* 
     if (splits == 1) return launch_by_width<EPI, false>(mw, mx, A, W, least, C, M, N, K, bn, status, stream);
     if (launch_by_width<EPI_STORE, true>(mw, mx, A, W, least, partial, M, N, K, bn, status, stream)) return 1;
     const size_t sums = (size_t)M * ((N + 3) / 4);
-    return gfb_check(gfb_launch(split_sum_kernel<EPI>, dim3((unsigned)((sums + 255) / 256)), dim3(256), 0, stream, (const float*)partial, A, W, (const float*)least, C, M, N, K,
+    return gfb_check(gfb_launch(split_sum_kernel<EPI>, dim3((unsigned)((sums + 255) / 256)), dim3(256), 0, stream, (const float*)partial, A, W, (const uint32_t*)least, C, M, N, K,
                                 splits), "gfb_gemm_split (sum)");
 }
 

@@ -87,6 +87,24 @@ def test_not_finite_and_extreme_numbers(N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(98, 2100), (18946, 388), (131, 1000)])      # (the last columns are no group of eight)
+def test_sums_that_all_need_the_32_bit_numbers(N, K):
+    """Every sum of a tile, and every other one, worked out from the 32-bit numbers: infinities at the end of every row, NaNs from the start, small rows
+    beside ordinary ones."""
+    a, w = rnd(37, K, seed=14), rnd(N, K, seed=15)
+    a[:20, K - 1] = float("inf")
+    a[20:25] = float("nan")
+    a[25:36] *= 1e-33
+    w[::2, K - 1] = 0.0                                               # infinity times zero
+    want = (a.double() @ w.double().t()).float()
+    got = torch.empty(37, N, device=DEV)
+    ops.linear(a, w, got)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[:20].nan_to_num(), want[:20].nan_to_num())
+    torch.testing.assert_close(got[25:36], want[25:36], rtol=2.0 ** -22, atol=0.0)       # (rounded once each, but for sums in another order of 64 bits)
+    torch.testing.assert_close(got[36], want[36], rtol=0.0, atol=1e-5 * K ** 0.5)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("N,K", [(96, 2100), (20000, 388)])          # portions of K in blocks of their own; one block per tile
 @pytest.mark.parametrize("rows,weights", [(1.0, 1e-24), (1.0, 1e-27), (1.0, 1e-33), (1.0, 1e-36), (1e12, 1e-36), (1e-24, 1.0), (1e-28, 1.0), (1e-30, 1.0),
                                           (1e-34, 1.0), (1e-36, 1.0), (1e-15, 1e-15), (1e-20, 1e-16), (1e30, 1e-36), (1e-36, 1e30)])
