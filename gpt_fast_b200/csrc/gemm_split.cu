@@ -574,7 +574,11 @@ int stages_per_split(int N, int K) {
     const int all = (K + BK - 1) / BK;
     int best = all;
     double best_cost = 0;
-    for (int s = 1; s <= 16 && s <= all; s++) {
+    // Few tiles of long rows take more portions.  us for one row | on CUDA cores: 8,192 numbers times 256 columns 13.1 | 15.4 (16 portions: 16.7), 14,336 times
+    // 256 15.3 | 22.6 (24.8), times 2 14.8 | 13.9 (24.7), 28,672 times 2 20.9 | 14.8 (43.9), times 512 27.8 | 39.1 (44.4).
+    const long few = K / (256 * (tiles > 2 ? tiles / 2 : 1));
+    const int most = few > 64 ? 64 : few < 16 ? 16 : (int)few;
+    for (int s = 1; s <= most && s <= all; s++) {
         const int per = (all + s - 1) / s, real = (all + per - 1) / per;
         if (real != s) continue;
         const double cost = (double)((tiles * s + 147) / 148) * (per + 6) + (s > 1 ? 4 + s * (N / 3000.0) : 0);

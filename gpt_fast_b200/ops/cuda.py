@@ -968,7 +968,8 @@ class CudaKernels:
     # -- matrix products -----------------------------------------------------------
     # From this K on a 32-bit product is done in bfloat16 pieces, up to three launches for one or two on CUDA cores; whatever M is, since a row's bits
     # do not depend on the batch.  us in pieces | on CUDA cores, captured, 4,096 columns: K = 128: 1 row 6.2 | 4.7, 64 7.7 | 10.7, 2,048 26.7 | 49.7;
-    # K = 256: 1 row 9.0 | 8.1, 64 10.5 | 19.4; K = 512: 1 row 7.9 | 15.0, 64 9.4 | 36.7, 2,048 109 | 181
+    # K = 256: 1 row 9.0 | 8.1, 64 10.5 | 19.4; K = 512: 1 row 7.9 | 15.0, 64 9.4 | 36.7, 2,048 112 | 181.  K = 384, 2 columns: 1 row 5.4 | 10.6, 2,048
+    # 12.4 | 27.2, 128 columns 5.7 | 11.4 and 14.5 | 27.7; from 2 to 2,048 columns and up to 14,336 numbers pieces are behind by 1.4 us at most
     SPLIT_LEAST_K = 384
 
     def linear(self, a, w, out, mode="store", defer=False):

@@ -87,6 +87,21 @@ def test_not_finite_and_extreme_numbers(N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(2, 28672), (256, 14340), (300, 14336), (130, 8196)])
+def test_few_columns_of_long_rows_take_more_portions(N, K):
+    """More than 16 portions of K, the last of them shorter: as near to 64 bits as elsewhere, and the same bits in every batch."""
+    a, w = rnd(70, K, seed=16), rnd(N, K, seed=17)
+    want = a.double() @ w.double().t()
+    whole, one = torch.empty(70, N, device=DEV), torch.empty(1, N, device=DEV)
+    ops.linear(a, w, whole)
+    assert float((whole.double() - want).norm() / want.norm()) < 2.5e-7
+    ops.linear(a[69:].contiguous(), w, one)
+    assert torch.equal(one[0], whole[69])
+    lib = build.library("gemm_split")
+    assert lib.gfb_gemm_split_scratch_bytes(70, N, K) > 6 * 70 * K + 16 * 4 * 70 * N
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("N,K", [(98, 2100), (18946, 388), (131, 1000)])      # (the last columns are no group of eight)
 def test_sums_that_all_need_the_32_bit_numbers(N, K):
     """Every sum of a tile, and every other one, worked out from the 32-bit numbers: infinities at the end of every row, NaNs from the start, small rows
