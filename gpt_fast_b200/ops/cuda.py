@@ -148,12 +148,17 @@ def split_parts(K: int, splits: int) -> int:
     return -(-stages // -(-stages // min(splits, stages)))
 
 
-def rows_share_keys(rows: int, longest: int, max_kv_len: int, line: int) -> bool:
-    """Whether the rows (token, head) of a step's 32-bit attention share the keys and values of sixteen rows per block; the bits are the same.  A block
-    then has sixteen rows' work in a row, so it takes rows enough, fewer where keys are many.  us shared | a block per row: 64 tokens of
-    24 heads over 8 18.9 | 19.1, of 16 over 16 14.9 | 12.5; 16 tokens behind 2,000, 16 heads 160 | 178, four times 16 behind 500 62 | 92; 2 tokens
-    behind 1,000 98 | 101, alone 11.3 | 6.7; 512 tokens of 24 heads 148 | 572."""
-    return longest > 1 and (rows >= line or (rows * 6 >= line and max_kv_len > 512))
+def rows_share_keys(rows: int, longest: int, max_kv_len: int, line: int, blocks: Optional[int] = None) -> bool:
+    """Whether the rows (token, head) of a step's 32-bit attention share the keys and values of sixteen rows per block; the bits are the same.  `blocks`: of
+    sixteen rows of one sequence and key head at most (default: all full).  A block has sixteen rows' work in a row and stages every key of its sequence, so
+    it takes rows enough, fewer where keys are many, and more where blocks are not full or a block per row has few keys to read: a fit to
+    432 steps of 1 to 64 sequences, 2 to 200 new tokens, 0 to 2,000 cached ones and 4 to 32 heads.  us shared | a block per row, the form taken first: 64
+    sequences of 4 tokens with 8 heads of their own keys 30.9 | 13.5 and 16 of 8 tokens of 24 heads over 8 18.0 | 15.7 (a block per row), behind 100 tokens
+    46.4 | 51.0 and 26.0 | 67.8 (shared); 512 tokens of 24 heads 148 | 572; 64 tokens of 16 heads over 16 14.9 | 12.5; 16 tokens behind 2,000, 16 heads 160 | 178."""
+    if longest <= 1 or not (rows >= line or (rows * 6 >= line and max_kv_len > 512)):
+        return False
+    blocks, keys = -(-rows // 16) if blocks is None else blocks, max_kv_len - longest / 2
+    return rows * (4 + keys) >= line * (20 - keys / 64 + blocks * (0.1 + keys / 768))
 
 
 def expand_latents(n_tokens: int, n_seqs: int, longest: int, cap: int) -> bool:
@@ -1146,9 +1151,10 @@ class CudaKernels:
             # head sizes they are built for
             return self._attention_bf16(q, kv, batch, out, n_head, n_kv, head_dim, scale, window, chunk=chunk, sink=sink,
                                         bias=bias, slopes=slopes, softcap=softcap, keep_first=keep_first)
+        blocks = n_kv * max(batch.n_seqs, -(-T * (n_head // n_kv) // 16))
         self._call("attention_generic", "gfb_attention_generic", _ptr(q), _ptr(out), _dt(q),
                    *self._kv_args(kv), *self._batch_args(batch),
-                   1 if rows_share_keys(T * n_head, batch.max_q_len, batch.max_kv_len, self.SHARING_ROWS) else 0, n_head, n_kv,
+                   1 if rows_share_keys(T * n_head, batch.max_q_len, batch.max_kv_len, self.SHARING_ROWS, blocks) else 0, n_head, n_kv,
                    head_dim, dv, scale, window or 0, chunk or 0, _ptr(sink), 1 if values_in_keys else 0,
                    _ptr(bias), bias.shape[0] if bias is not None else 0, _ptr(slopes), softcap or 0.0,
                    int(keep_first), maps, diff[0] if diff else 0.0, diff[1] if diff else 0.0,

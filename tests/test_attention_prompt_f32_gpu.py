@@ -60,3 +60,10 @@ def test_values_in_keys_and_what_a_row_does_not_see(sharing):
 def test_the_rule():
     assert rows_share_keys(198 * 24, 137, 137, 1536) and rows_share_keys(256, 16, 2016, 1536)
     assert not rows_share_keys(198 * 24, 1, 137, 1536) and not rows_share_keys(1024, 64, 64, 1536) and not rows_share_keys(80, 2, 800, 1536)
+
+
+def test_the_rule_counts_blocks_that_are_not_full():
+    few_live = [(64 * 4 * 8, 4, 4, 1536, 8 * 64), (64 * 2 * 32, 2, 2, 1536, 32 * 64), (16 * 8 * 24, 8, 8, 1536, 8 * 24)]       # a block per row is the faster form
+    full = [(64 * 8 * 24, 8, 108, 1536, 8 * 96), (16 * 32 * 32, 32, 32, 1536, 8 * 128), (64 * 4 * 32, 4, 604, 1536, 8 * 64), (200 * 16, 200, 200, 1536, 200)]
+    assert not any(rows_share_keys(*c) for c in few_live) and all(rows_share_keys(*c) for c in full)
+    assert rows_share_keys(198 * 24, 137, 137, 1536, 8 * 38) and rows_share_keys(8, 2, 2, 1, 4)
