@@ -161,10 +161,15 @@ def rows_share_keys(rows: int, longest: int, max_kv_len: int, line: int, blocks:
     return rows * (4 + keys) >= line * (20 - keys / 64 + blocks * (0.1 + keys / 768))
 
 
-def expand_latents(n_tokens: int, n_seqs: int, longest: int, cap: int) -> bool:
-    """Whether a prompt's latents are expanded to keys and values per head: where its keys, at most `cap` for every sequence, are mostly its own
-    new tokens.  A cached key costs 262,144 operations per head to expand and saves 1,536 for every query that sees it."""
-    return longest > 1 and n_seqs * cap <= 3 * n_tokens + 128 * n_seqs
+def expand_latents(n_tokens: int, n_seqs: int, longest: int, cap: int, n_head: int = 16) -> bool:
+    """Whether a prompt's latents are expanded to keys and values per head: where its keys, at most `cap` (whole blocks of 128) for every sequence, are
+    at most three times its new tokens, but for one block each (which bounds the scratch by what attention on the latent takes), and
+    expanding them costs less than it saves.  A block of 128 keys costs what 23 new tokens save, a sequence, whose last tiles are not full, what 37 do,
+    and two launches less are worth 1,000 tokens of 16 heads.  us expanded | on the latent, 16 heads, one launch behind the other, the form taken first:
+    one prompt of 4,096 tokens 277 | 724, of 100 81 | 98, 16 of 64 tokens 99 | 112, 64 of 64 291 | 299 (expanded); 64 sequences of 2 tokens behind
+    126 cached ones 199 | 99, of 35 tokens 243 | 180, of 64 behind 126 351 | 330, 16 of 35 behind 126 108 | 104 (on the latent)."""
+    return (longest > 1 and n_seqs * cap <= 3 * n_tokens + 128 * n_seqs
+            and n_head * (23 * n_seqs * (cap // 128) + 37 * n_seqs - n_tokens) <= 16000)
 
 
 class CudaKernels:
@@ -490,7 +495,7 @@ class CudaKernels:
         T, W = proj.shape
         H, R = n_head, rank
         cap = -(-max(int(batch.max_kv_len), 1) // 128) * 128
-        if not (proj.dtype == torch.bfloat16 and expand_latents(T, batch.n_seqs, batch.max_q_len, cap)
+        if not (proj.dtype == torch.bfloat16 and expand_latents(T, batch.n_seqs, batch.max_q_len, cap, H)
                 and head_dim == 128 and v_head_dim == 128 and rot_dim == 64 and R % 64 == 0 and kv.page_size == 64 and scale > 0
                 and (W | q_off | gate_off) % 8 == 0 and (proj.data_ptr() | wuk.data_ptr() | wuv.data_ptr() | out.data_ptr() | kv.k_pool.data_ptr()) % 16 == 0
                 and H * max(R, batch.n_seqs * cap) < 2 ** 31):

@@ -168,3 +168,9 @@ def test_the_rule():
     assert expand_latents(4096, 1, 4096, 4096) and expand_latents(20, 1, 20, 128) and expand_latents(2056, 16, 256, 256)
     assert not expand_latents(16, 16, 1, 128)                            # a decode step
     assert not expand_latents(100, 1, 100, 2176) and expand_latents(300, 1, 300, 1024)
+
+
+def test_the_rule_refuses_many_short_continuations():
+    slower = [(128, 64, 2, 128, 16), (512, 64, 8, 128, 16), (2240, 64, 35, 128, 16), (4096, 64, 64, 256, 16), (32, 16, 2, 128, 128)]
+    faster = [(4096, 64, 64, 128, 16), (1024, 16, 64, 256, 16), (32, 16, 2, 128, 16), (3200, 16, 200, 512, 16), (4096, 1, 4096, 4096, 128), (100, 1, 100, 128, 128)]
+    assert not any(expand_latents(*c) for c in slower) and all(expand_latents(*c) for c in faster)
