@@ -1651,9 +1651,13 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_con
 // 16 heads: a thread per row 129 us, two 123; the products of both tiles behind one another 137).  Q of both tiles (96 KB) leaves a ring of eight slots of 16 KB for three pieces of K, [128 keys][64
 // dims], and two of V, [64 keys][128 dims], per 128 keys, in the order in which they are freed: V_j, K_(j+1), V_(j+1), ...; a
 // piece takes the slot of the eighth piece before it.
-// The reference of the exponentials lags a row's maximum by up to 2^8, as there: float16 weights lose nothing by it that bfloat16 ones would.
+// float16 has more bits than bfloat16 and far fewer exponents, so weights are lifted to the top of its range: the reference of the exponentials lags a
+// row's maximum by up to 2^LH_LAG and stands for 2^LH_LIFT, so that the largest weight of a row lies between 2^LH_LIFT and 2^15, one 2^29 below
+// it keeps ten bits and one 2^35 below it is not lost; and the sum takes the weights as they are rounded for P V.  (Sums of unrounded weights up to 2^8
+// lost a flat tail 2^25.5 below a row's peak, and kept it in the denominator: 2.8e-3 of a row at 131,072 keys.)
 //   tensor memory: S of tile x in columns 128 x .. 128 x + 127 (P overwrites the first half), O of tile x in 256 + 128 x ..
 constexpr int LH_Q_BYTES = 3 * HALF_BYTES, LH_SLOTS = 8;
+constexpr float LH_LAG = 3.f, LH_LIFT = 15.f - LH_LAG;
 struct LhBars {
     unsigned long long q_full;
     unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];   // of even and odd key blocks
@@ -1899,9 +1903,9 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (!ok) break;
                 mx = fmaxf(mx, theirs);
                 float m_new = m_run;
-                if (mx > m_run && (m_run == -INFINITY || (mx - m_run) * scale_log2e > 8.f)) m_new = mx;
+                if (mx > m_run && (m_run == -INFINITY || (mx - m_run) * scale_log2e > LH_LAG)) m_new = mx;
                 const float corr = (m_run == -INFINITY || m_new == m_run) ? 1.f : fast_exp2((m_run - m_new) * scale_log2e);
-                const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * scale_log2e;
+                const float mneg = (m_new == -INFINITY) ? 0.f : LH_LIFT - m_new * scale_log2e;
                 float rsum[2] = {0.f, 0.f};
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
@@ -1911,9 +1915,10 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     for (int i = 0; i < 32; i += 2) {
                         float a0, a1;
                         fma2(v[c][i], v[c][i + 1], scale_log2e, mneg, a0, a1);
-                        const float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
-                        add2(rsum[c], odd, p0, p1);
-                        pk[i >> 1] = pack2_half(p0, p1);
+                        const __half2 p = __floats2half2_rn(fast_exp2(a0), fast_exp2(a1));
+                        const float2 rounded = __half22float2(p);        // what P V takes is what the sum takes
+                        add2(rsum[c], odd, rounded.x, rounded.y);
+                        pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&p);
                     }
                     rsum[c] += odd;
                     tmem_st16(lane_base + col_s + 32 * half + c * 16, pk);   // (both halves of this row's scores are in registers by now)
@@ -1948,7 +1953,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 l_run = half ? theirs + l_run : l_run + theirs;
             }
             if (ok && n_done > 0) {
-                if (sink != nullptr && m_run != -INFINITY) l_run += fast_exp2(sink[head] * 1.4426950408889634f - m_run * scale_log2e);
+                if (sink != nullptr && m_run != -INFINITY) l_run += fast_exp2(sink[head] * 1.4426950408889634f + (LH_LIFT - m_run * scale_log2e));
                 const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
                 const size_t t = (size_t)(t_first + tq0 + x * ROWS + (row_ok ? r : 0));
                 const int dim0 = 64 * half;

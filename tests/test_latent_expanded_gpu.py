@@ -123,6 +123,33 @@ def test_value_columns_of_every_scale():
     assert float(err.max()) < 6e-3, err
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("depth", [8.0, 14.5, 20.0, 25.5, 30.0, 34.0])
+@pytest.mark.parametrize("peak", [0, 400, 699])
+def test_a_flat_tail_far_below_a_peak(depth, peak):
+    """One key whose weight is 2^depth times every other one's, ahead of the others, among them and behind them.  Half of the value columns hold nothing
+    of the peak: what they get is the tail's share, as far below the row as that is, and no worse than on the latent."""
+    c = case(2, 128, [700], [0], None, False, True)
+    R, kv_off = 128, c["kv_off"]
+    c["position"].table[..., 0], c["position"].table[..., 1] = 1.0, 0.0                    # no rotation: a score is set by one number of the key
+    c["norm"] = torch.ones(R, device=DEV)
+    c["proj"][:, :c["g_off"]] = 0.0
+    q = c["proj"][:, :kv_off].view(700, 2, 192)
+    q[:, :, 128] = 64.0
+    others = torch.arange(700, device=DEV) != peak
+    c["proj"][others, kv_off:kv_off + 64] = rnd(1, 64, dtype=BF, seed=9)                   # the tail's latent, the same for all: its errors add up
+    c["proj"][peak, kv_off + 64:kv_off + 128] = rnd(64, dtype=BF, seed=10)
+    c["proj"][others, kv_off + R] = -depth / (1.4426950408889634 * 64.0 * c["scale"])
+    c["wuv"][:, 64:, :64] = 0.0
+    c["wuv"][:, :64, 64:] = 0.0
+    y = [f(c).double().view(700, 2, 128)[1:] for f in (expanded, on_the_latent)]
+    ref = want(c).view(700, 2, 128)[1:]
+    sees = torch.arange(1, 700, device=DEV) >= peak
+    for cols, rows in ((slice(0, 64), slice(None)), (slice(64, 128), sees)):
+        err = [float(((v - ref)[rows][..., cols]).norm() / ref[rows][..., cols].norm()) for v in y]
+        assert err[0] <= max(1.05 * err[1], 2.0 ** -8), (depth, peak, err)                 # (2^-9 is the output's rounding, at most)
+
+
 def test_scales_of_values():
     w = torch.randn(3, 64, 16) * torch.logspace(-30, 30, 16)
     w[0, :, 3] = 0.0
