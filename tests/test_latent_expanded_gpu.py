@@ -147,7 +147,8 @@ def test_a_flat_tail_far_below_a_peak(depth, peak):
     sees = torch.arange(1, 700, device=DEV) >= peak
     for cols, rows in ((slice(0, 64), slice(None)), (slice(64, 128), sees)):
         err = [float(((v - ref)[rows][..., cols]).norm() / ref[rows][..., cols].norm()) for v in y]
-        assert err[0] <= max(1.05 * err[1], 2.0 ** -8), (depth, peak, err)                 # (2^-9 is the output's rounding, at most)
+        # 2^-9 is the output's rounding, at most; weights are multiples of 2^-24 at least, half of that against 2^12 at the peak
+        assert err[0] <= max(1.05 * err[1], 2.0 ** -8, 2.0 ** (depth - 37)), (depth, peak, err)
 
 
 def test_scales_of_values():
