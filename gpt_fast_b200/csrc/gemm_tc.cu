@@ -21,9 +21,14 @@
 // Roles in a block of 192 threads: warp 0 = TMA producer (one lane), warp 1 =
 // tensor-memory allocation + MMA issue (one lane), warps 2..5 = epilogue (one
 // quarter of the 128 accumulator lanes each).  Stages of the shared-memory ring
-// are handed over through mbarriers.  Every wait is bounded by wall-clock time:
-// when one runs out the block records GFB_ERR_WAIT_TIMEOUT in `status`, lets
-// copies in flight land, frees its tensor memory and returns.
+// are handed over through mbarriers.  Every wait on one is bounded by wall-clock time:
+// when it runs out the block records GFB_ERR_WAIT_TIMEOUT in `status`, lets
+// copies in flight land, frees its tensor memory and returns.  The waits for the
+// preceding kernel, for tensor memory and for the other blocks of a cluster have
+// no limit; they end because a block tells the next kernel to start only when it
+// holds shared and tensor memory, because its kernel's blocks on one SM never need
+// more than the 512 columns, and because every block of a cluster passes the same
+// cluster barriers on every path.
 #include "common.cuh"
 
 #include <cuda.h>

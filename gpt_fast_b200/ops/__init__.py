@@ -190,7 +190,8 @@ def latent_expanded(proj, q_off: int, kv_off: int, gate_off: int, gate_per_head:
     """A step's latent attention in one call: `latent_prepare`, then causal attention of every head over keys and values expanded
     from the cached latents (wuk [n_head, head_dim, rank], wuv [n_head, rank, v_head_dim]; v_scale from `value_scales`) and, as 32-bit numbers, times the sigmoid of the gates at
     column gate_off of proj, written to out [T, n_head * v_head_dim].  The kernels decide where that is the faster form; elsewhere, and
-    where a set of kernels has none, nothing is done and False returned."""
+    where a set of kernels has none, nothing is done and False returned.  The cached rows have to be what a norm with norm_weight makes (no number of a
+    latent beyond sqrt(rank) times its weight), as `latent_prepare` writes them: v_scale fits the values of such rows into float16, larger ones overflow."""
     fused = getattr(kernels(), "latent_expanded", None)
     return fused is not None and fused(proj, q_off, kv_off, gate_off, gate_per_head, out, kv, batch, n_head, head_dim, rot_dim, v_head_dim, rank,
                                        norm_weight, eps, table, pairing, append, wuk, wuv, v_scale, scale, window, sink)
