@@ -8,9 +8,9 @@
 // rounds 32 times.  Against 64 bits, numbers of unit scale: 0.9e-7 (K = 512) to 2.1e-7 (14,336), on CUDA cores 4.1e-7; sums that are
 // little more than their largest product 5.5e-8, there 2.8e-8, since the one sum that counts is cut off here and rounded there.
 //
-// us here | on CUDA cores, K = 3,072: 198 rows times 16,384 columns 110 | 525, times 5,120 50 | 179; one row times 16,384 77 | 103, times 128,256
-// 478 | 700; 2,048 rows times 5,120 339 | 1,417; 198 rows of 8,192 numbers times 3,072 62 | 288.  Shared memory bounds it at 256 tokens (1,740 of some
-// 2,000 cycles per stage: 12 multiplications read 10 KB each beside the copies and the planes), the way from weight to sum at few.
+// us here | on CUDA cores, captured, K = 3,072: 198 rows times 16,384 columns 107 | 525, times 5,120 42 | 179; one row times 16,384 84 | 103, times
+// 128,256 481 | 700; 2,048 rows times 5,120 360 | 1,417; 198 rows of 8,192 numbers times 3,072 57 | 288.  At 198 rows the tensor pipe is busy for 69 % of
+// the time (12 multiplications of 128 x 208 x 16 read 10 KB each per stage, beside the copies and the planes); at few rows the way from weight to sum bounds it.
 //
 // An element's order of summation depends on N and K alone: accumulators of 32 k in ascending order, in `splits_of(N, K)`
 // portions of K whose sums are added in ascending order by a kernel of their own.  A row's bits do not depend on the other rows.
