@@ -1149,6 +1149,8 @@ GFB_API int gfb_attn_decode_noalloc(const void* q, void* out, void* k_pool, void
             return gfb_fail("gfb_attn_decode_noalloc: %d tokens x %d heads x %d slices x (%d + 2) = %lld floats of scratch "
                             "exceed the built-in %d; use fewer slices or gfb_attn_decode with your own scratch",
                             n_tokens, H, splits, d, need, GFB_NOALLOC_SCRATCH_FLOATS);
+    }
+    if (splits > 1 && !((d == 128 || d == 64) && merged(splits, nullptr))) {      // (slices that merge within a cluster leave nothing in memory)
         int dev = -1;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return gfb_fail("gfb_attn_decode_noalloc: cudaGetDevice: %s", cudaGetErrorString(e));

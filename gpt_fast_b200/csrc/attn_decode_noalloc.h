@@ -21,7 +21,9 @@
  *    whose context loads this library keeps that much memory until the
  *    process exits.  A call needs n_tokens * H * splits * (d + 2) floats;
  *    a larger request is refused with an error (gfb_last_error() says so),
- *    nothing is launched.  With splits == 1 no scratch is used at all.
+ *    nothing is launched.  With splits == 1, and with up to 8 slices of
+ *    head_dim 64 or 128 (which merge within a cluster of blocks, to the same
+ *    bits), the array is not used at all; the limit is the same.
  *  - The first call on a device looks up the array's device address
  *    (cudaGetSymbolAddress, once per device, with that device current) and
  *    remembers it.  Make that first call outside any stream capture.
